@@ -445,7 +445,7 @@ rbc3d_status rbc3d_create(const rbc3d_params* prm, rbc3d_ctx** out) {
       ctx->t_mask32.upload(mk32.data(), mk32.size(), ctx->st) || ctx->dcnt.alloc(16) || ctx->xvint.alloc(3) ||
       ctx->dBcoef.upload(ctx->Bcoef, RBC3D_MAX_CELLTYPES, ctx->st))
     return bail(RBC3D_ERR_CUDA);
-  if (self_ff_tables(ctx, c1, c2, dl)) return bail(RBC3D_ERR_CUDA);
+  if (self_ff_tables(ctx, c1, c2, dl) || self_ring_tables(ctx, c1, c2, dl)) return bail(RBC3D_ERR_CUDA);
   Tables& T = ctx->T;
   T.sl_c1 = ctx->t_sl1.p; T.sl_c2 = ctx->t_sl2.p; T.dl_c1 = ctx->t_dl.p; T.mask = ctx->t_mask.p;
   T.sl32 = ctx->t_sl32.p; T.dl32 = ctx->t_dl32.p; T.mask32 = ctx->t_mask32.p;
@@ -569,9 +569,9 @@ rbc3d_status rbc3d_set_cell_grid(rbc3d_ctx* ctx, const double* th, const double*
     if (s) return s;
   }
   {
-    // FP64 Spline_Interp weights per (latitude, patch point) for k_self: with
-    // phi(j) = j 2 pi / nlon, phiG = atan2(...) + phi0 moves the stencil by
-    // whole columns, so only the column offset depends on the target's longitude
+    // Spline_Interp weights per (latitude, patch point): with phi(j) = j 2 pi /
+    // nlon, phiG = atan2(...) + phi0 moves the stencil by whole columns, so
+    // only the column offset depends on the target's longitude
     const int m = 2 * nlat;
     const double hx = RBC3D_TWO_PI / m, hy = RBC3D_TWO_PI / nlon, ihx = 1. / hx, ihy = 1. / hy;
     std::vector<SelfW64> W((size_t)nlat * NQ);
@@ -597,9 +597,9 @@ rbc3d_status rbc3d_set_cell_grid(rbc3d_ctx* ctx, const double* th, const double*
       }
       W[i] = e;
     }
-    CUDA_TRY(ctx->self_w64.upload(reinterpret_cast<const char*>(W.data()), W.size() * sizeof(SelfW64), ctx->st));
     rbc3d_status s = self_ff_grid(ctx, W, pw);
     if (s) return s;
+    if ((s = self_ring_grid(ctx, ring_classes(ctx, thG, phiA, pw)))) return s;
   }
   CUDA_TRY(ctx->thG.upload(thG.data(), thG.size(), ctx->st));
   CUDA_TRY(ctx->phiA.upload(phiA.data(), phiA.size(), ctx->st));

@@ -100,6 +100,15 @@ struct SelfW64 {
   int i1, j1b;
   double w[16];  // the 16 Spline_Interp weight products in spline_w16's order
 };
+// A class of patch points of one target latitude (selfring.cu): the points at
+// azimuth +-a of one radius, which share their colatitude.  Spline row i1 and
+// the theta weights of (u' - u, u_th, u'_th) (u' the next row; u itself has
+// weight 1); per side the column interval j relative to the target's (-1: no
+// such point) and the phi weights; the quadrature weight.
+struct RingClass {
+  int i1, j[2];
+  double x[3], y[2][3], w;
+};
 struct SplW {
   int n11, n12, n21, n22;  // node ids (i1,j1) (i1,j2) (i2,j1) (i2,j2)
   double cx[4], cy[4];

@@ -27,7 +27,6 @@ struct CorrArgs {
   SplGrid G;  // Spline_Create constants of the (2 nlat, nlon) spline grid
   double rc2;
   unsigned long long* queue;  // k_near's item counter
-  const SelfW64* W64;         // k_self: tabulated patch weights (uniform longitudes), or null
   const int* list;            // k_near: items to process (indices), or null for all
   long long list_start;       // k_near over a list: its first entry (the staged pass takes those before)
   int stage_cap;              // the staged pass: entries it takes from the list's head
@@ -73,7 +72,8 @@ __device__ __forceinline__ const double* set_ptr(const CorrArgs& a, int cell, in
   return a.spl + ((size_t)cell * SPL_NSET + set) * (size_t)a.m * a.nlon * SPL_NODE;
 }
 
-// RBC_SingInt: one warp per cell target
+// RBC_SingInt on any longitude grid: one warp per cell target (uniform grids
+// of up to RING_MAX_NLON columns: selfring.cu)
 __global__ void __launch_bounds__(256) k_self(CorrArgs a) {
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
@@ -98,21 +98,11 @@ __global__ void __launch_bounds__(256) k_self(CorrArgs a) {
   for (int q = lane; q < NQ; q += 32) {
     const int irad = q % a.nrad;
     double w16[16];
-    if (a.W64) {
-      // weight products tabulated per (latitude, patch point); longitudes shift the stencil
-      const SelfW64& e = a.W64[(size_t)ilat0 * NQ + q];
-      const int j1 = imod(e.j1b + ilon0, a.nlon), j2 = (j1 + 1 == a.nlon) ? 0 : j1 + 1;
-      const int i2 = (e.i1 + 1 == a.m) ? 0 : e.i1 + 1;
-      W.n11 = e.i1 + a.m * j1; W.n12 = e.i1 + a.m * j2; W.n21 = i2 + a.m * j1; W.n22 = i2 + a.m * j2;
-#pragma unroll
-      for (int k = 0; k < 16; ++k) w16[k] = e.w[k];
-    } else {
-      const double th_j = a.thG[(size_t)ilat0 * NQ + q];
-      const double p = a.phiA[(size_t)ilat0 * NQ + q] + phi0;  // PolarPatch_Build: atan2(...) + phi0
-      const double phi_j = p - floor(p * RBC3D_I_2PI) * RBC3D_TWO_PI;
-      spline_weights_g(th_j, phi_j, a.G, W);
-      spline_w16(W, w16);
-    }
+    const double th_j = a.thG[(size_t)ilat0 * NQ + q];
+    const double pa = a.phiA[(size_t)ilat0 * NQ + q] + phi0;  // PolarPatch_Build: atan2(...) + phi0
+    const double phi_j = pa - floor(pa * RBC3D_I_2PI) * RBC3D_TWO_PI;
+    spline_weights_g(th_j, phi_j, a.G, W);
+    spline_w16(W, w16);
     double xj[3], xx[3];
     spline_eval16(sx, W, w16, 3, xj);
     for (int k = 0; k < 3; ++k) xx[k] = xj[k] - xi[k];
@@ -1050,7 +1040,6 @@ void fill_args(rbc3d_ctx* ctx, int tlist, double c1, double c2, CorrArgs& a, con
   a.nt = t.n; a.tx = t.x.p; a.tA = t.Acoef.p; a.tmeta = t.meta.p; a.v = t.v.p;
   a.ncell = ctx->ncell; a.nlat = ctx->nlat; a.nlon = ctx->nlon; a.m = ctx->m;
   a.G = spl_grid(ctx->m, ctx->nlon);
-  a.W64 = ctx->phi_uniform ? reinterpret_cast<const SelfW64*>(ctx->self_w64.p) : nullptr;
   a.rc2 = ctx->prm.rc * ctx->prm.rc;
   a.th = ctx->th.p; a.phi = ctx->phi.p; a.w = ctx->w.p;
   a.x = ctx->x.p; a.a3 = ctx->a3.p; a.detJ = ctx->detJ.p; a.f = ctx->f.p; a.g = ctx->g.p;
@@ -1073,6 +1062,7 @@ rbc3d_status run_self_corr(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   CorrArgs a;
   fill_args(ctx, tlist, c1, (c2 != 0 && ctx->has_g) ? c2 : 0.0, a, Bc);
   if (c1 != 0 && !ctx->has_f) a.c1 = 0;
+  if (ctx->phi_uniform && ctx->nlon <= RING_MAX_NLON) return run_self_ring(ctx, tlist, a.c1, a.c2);
   long long threads = (long long)t.n * 32;
   { k_self<<<(int)((threads + 255) / 256), 256, 0, ctx->st>>>(a); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());

@@ -207,7 +207,9 @@ struct rbc3d_ctx {
   int s_ntiles = 0;
   DBuf<unsigned long long> near_queue;  // work counter of the near-singular kernel
   DBuf<double> dBcoef;                  // Bcoef per cell type on the device
-  DBuf<char> self_w64;                  // FP64 patch weights per (latitude, patch point)
+  DBuf<char> ring_cls;                  // patch-point classes per latitude (RingClass)
+  DBuf<double> ring_tab, ring_rec;      // FP64 patch: Ewald tables with steps, node values in column order
+  int ring_sets = 0;                    // ring_rec's current sets (bit 0 x, 1 f, 2 g, 3 a3)
   DBuf<double> mtab64;                  // same-cell mask per (latitude, latitude, longitude gap)
   DBuf<float> mtab32;                   // 1 - mask, FP32
   DBuf<int> near_l1, near_l2;           // near-singular candidates after the screen / the FP32 replay
@@ -342,6 +344,15 @@ rbc3d_status wall_spec_predict_dev(rbc3d_ctx* ctx, const double* b_dev, double* 
 rbc3d_status wall_spec_add_dev(rbc3d_ctx* ctx, const double* b_dev, const double* x_dev);
 rbc3d_status wall_spec_apply_dev(rbc3d_ctx* ctx, const double* v_dev, double* out_dev);
 void wall_spec_release(rbc3d_ctx* ctx);
+
+// selfring.cu: the FP64 patch by latitude rings (uniform longitudes, nlon <= RING_MAX_NLON)
+constexpr int RING_MAX_NLON = 256;
+std::vector<RingClass> ring_classes(const rbc3d_ctx* ctx, const std::vector<double>& thG,
+                                    const std::vector<double>& phiA, const std::vector<double>& pw);
+rbc3d_status self_ring_grid(rbc3d_ctx* ctx, const std::vector<RingClass>& C);
+rbc3d_status self_ring_tables(rbc3d_ctx* ctx, const std::vector<double>& c1, const std::vector<double>& c2,
+                              const std::vector<double>& dl);
+rbc3d_status run_self_ring(rbc3d_ctx* ctx, int tlist, double c1, double c2);
 
 // selfmix.cu
 rbc3d_status self_mixed_grid(rbc3d_ctx* ctx, const std::vector<double>& thG, const std::vector<double>& phiA,

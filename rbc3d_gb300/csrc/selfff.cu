@@ -482,9 +482,9 @@ rbc3d_status self_ff_grid(rbc3d_ctx* ctx, const std::vector<SelfW64>& W, const s
 
 // Node records are rebuilt on first use after the positions or densities change.
 void self_ff_invalidate(rbc3d_ctx* ctx, bool geom, bool f, bool g) {
-  if (geom) ctx->ff_sets &= ~(1 | 8);
-  if (f) ctx->ff_sets &= ~2;
-  if (g) ctx->ff_sets &= ~4;
+  const int gone = (geom ? 1 | 8 : 0) | (f ? 2 : 0) | (g ? 4 : 0);
+  ctx->ff_sets &= ~gone;
+  ctx->ring_sets &= ~gone;
 }
 
 // The float-float node records of the sets in `need` (bit 0 x, 1 f, 2 g,

@@ -1,0 +1,36 @@
+"""The own-cell patch by latitude rings against the oracle's RBC_SingInt: the
+grids of RBC_Create and the benchmark's, cell counts that leave a block's last
+places empty, single and double layer alone and together."""
+import math
+
+import numpy as np
+import pytest
+
+from rbc3d_gb300 import geometry as G
+from rbc3d_gb300.abi import FP64, TERM_CORR, TLIST_RBC, Context
+
+pytestmark = pytest.mark.gpu
+C = 1 / (4 * math.pi)
+
+
+@pytest.mark.parametrize("nlat,nlon,ncell", [(12, 24, 1), (14, 28, 11), (24, 48, 6), (25, 50, 4), (36, 72, 4)])
+def test_ring_patch_matches_oracle(gpu, oracle, nlat, nlon, ncell):
+    L = 9.1 if ncell == 1 else 14.0
+    rng = np.random.default_rng(nlat)
+    cells = G.make_cells(rng, ncell, [L] * 3, 3.2, nlat=nlat, nlon=nlon, with_g=True)
+    cells.celltype[:] = np.arange(ncell) % 2
+    prm = dict(Lb=[L] * 3, alpha=G.alpha_for_cutoff(3.0, 1e-6), rc=3.0, eps=1e-6, Nb=[16] * 3, P=4, nlat=nlat,
+               nlon=nlon, ncelltypes=2, viscRat=[5.0, 0.2])
+    ctx = []
+    for lib in (oracle, gpu):
+        c = Context(lib, prm)
+        c.set_cells(cells)
+        c.set_cell_density(f=cells.f, g=cells.g, spl_F=cells.spl_F, spl_G=cells.spl_G)
+        ctx.append(c)
+    # rounding: the separation of the first radial ring (about 0.01) is a
+    # difference of positions up to 14, 2e-16 x 14 / 0.01 = 3e-13; the sums differ in order only
+    for c1, c2 in ((C, C), (C, 0.0), (0.0, C)):
+        ref, out = (c.matvec(TLIST_RBC, c1, c2, TERM_CORR, FP64) for c in ctx)
+        assert np.linalg.norm(out - ref) <= 1e-11 * np.linalg.norm(ref), (c1, c2)
+    for c in ctx:
+        c.close()
