@@ -569,37 +569,11 @@ rbc3d_status rbc3d_set_cell_grid(rbc3d_ctx* ctx, const double* th, const double*
     if (s) return s;
   }
   {
-    // Spline_Interp weights per (latitude, patch point): with phi(j) = j 2 pi /
-    // nlon, phiG = atan2(...) + phi0 moves the stencil by whole columns, so
-    // only the column offset depends on the target's longitude
-    const int m = 2 * nlat;
-    const double hx = RBC3D_TWO_PI / m, hy = RBC3D_TWO_PI / nlon, ihx = 1. / hx, ihy = 1. / hy;
-    std::vector<SelfW64> W((size_t)nlat * NQ);
-    for (size_t i = 0; i < W.size(); ++i) {
-      const double x = thG[i] * ihx, y = phiA[i] * ihy;
-      const int i1 = (int)std::floor(x), j1 = (int)std::floor(y);
-      const double s = x - i1, t = y - j1;
-      SelfW64 e;
-      e.i1 = ((i1 % m) + m) % m;
-      e.j1b = j1;
-      double cx[4], cy[4];
-      cx[0] = 1 + s * s * (-3. + 2. * s); cx[1] = s * s * (3. - 2. * s);
-      cx[2] = hx * s * (1. + s * (-2. + s)); cx[3] = hx * s * s * (-1. + s);
-      cy[0] = 1 + t * t * (-3. + 2. * t); cy[1] = t * t * (3. - 2. * t);
-      cy[2] = hy * t * (1. + t * (-2. + t)); cy[3] = hy * t * t * (-1. + t);
-      // node (i1,j1): u u1 u2 u12, then (i1,j2), (i2,j1), (i2,j2), as spline_w16
-      const int ax[4] = {0, 0, 1, 1}, ay[4] = {0, 1, 0, 1};
-      for (int k = 0; k < 4; ++k) {
-        e.w[4 * k + 0] = cx[ax[k]] * cy[ay[k]];
-        e.w[4 * k + 1] = cx[ax[k] + 2] * cy[ay[k]];
-        e.w[4 * k + 2] = cx[ax[k]] * cy[ay[k] + 2];
-        e.w[4 * k + 3] = cx[ax[k] + 2] * cy[ay[k] + 2];
-      }
-      W[i] = e;
-    }
-    rbc3d_status s = self_ff_grid(ctx, W, pw);
-    if (s) return s;
-    if ((s = self_ring_grid(ctx, ring_classes(ctx, thG, phiA, pw)))) return s;
+    // the patch points' classes: with phi(j) = j 2 pi / nlon, phiG = atan2(...) +
+    // phi0 moves the stencil by whole columns
+    const std::vector<RingClass> R = ring_classes(ctx, thG, phiA, pw);
+    rbc3d_status s;
+    if ((s = self_ff_grid(ctx, R)) || (s = self_ring_grid(ctx, R))) return s;
   }
   CUDA_TRY(ctx->thG.upload(thG.data(), thG.size(), ctx->st));
   CUDA_TRY(ctx->phiA.upload(phiA.data(), phiA.size(), ctx->st));

@@ -94,12 +94,6 @@ __device__ __forceinline__ double dist_on_sphere(double th0, double phi0, double
 // ---------------------------------------------------------------------------
 // Bicubic Hermite interpolation on the doubled-sphere grid (Spline_Interp,
 // ModSpline.F90:150-191).  Node layout: spl[node*SPL_NODE + kind*3 + var].
-// Spline_Interp weights of one patch point for a target latitude: row i1,
-// column offset j1b (before adding the target's longitude index), cx, cy.
-struct SelfW64 {
-  int i1, j1b;
-  double w[16];  // the 16 Spline_Interp weight products in spline_w16's order
-};
 // A class of patch points of one target latitude (selfring.cu): the points at
 // azimuth +-a of one radius, which share their colatitude.  Spline row i1 and
 // the theta weights of (u' - u, u_th, u'_th) (u' the next row; u itself has

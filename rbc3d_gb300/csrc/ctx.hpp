@@ -240,15 +240,13 @@ struct rbc3d_ctx {
   int mix_sets = 0;  // current FP32M node-record parts: bit 0 geometry, 1 f, 2 g
   bool phi_uniform = false;
 
-  // FP32D self patch: float-float node records [cell][slot x quad][node tile][hi, lo],
-  // the patch weights of k_self as hi/lo planes, pw and the Ewald tables as
-  // hi/lo; ff_sets: which record sets (bit 0 x, 1 f, 2 g, 3 a3) are current
-  DBuf<int2> ff_widx;
-  DBuf<float4> ff_rec, ff_w, ff_tab;
-  DBuf<float2> ff_pw;
+  // FP32D self patch: float-float node records [cell][row][slot][quad][column][hi, lo],
+  // the ring classes and the Ewald tables as hi/lo; ff_sets: which record sets
+  // (bit 0 x, 1 f, 2 g, 3 a3) are current
+  DBuf<float4> ff_rec, ff_tab;
+  DBuf<char> ff_cls;
   DBuf<unsigned> ff_bnd;  // [set][cell][slot]: max |value| (float bits) for the sums' offsets
   int ff_sets = 0;
-  DBuf<short> ff_perm;    // [latitude][k]: lane order of the patch points
 
   // membrane mechanics (membrane.cu): transform tables of the degree < nlat
   // expansion and the reference cells' a_rcp and b, [type][4][nv]
@@ -349,6 +347,8 @@ void wall_spec_release(rbc3d_ctx* ctx);
 constexpr int RING_MAX_NLON = 256;
 std::vector<RingClass> ring_classes(const rbc3d_ctx* ctx, const std::vector<double>& thG,
                                     const std::vector<double>& phiA, const std::vector<double>& pw);
+int ring_cells(int ncell, int nlon);                  // cells of one block
+int ring_parts(int classes, int blocks, int nsm);     // blocks that share a ring's classes
 rbc3d_status self_ring_grid(rbc3d_ctx* ctx, const std::vector<RingClass>& C);
 rbc3d_status self_ring_tables(rbc3d_ctx* ctx, const std::vector<double>& c1, const std::vector<double>& c2,
                               const std::vector<double>& dl);
@@ -362,7 +362,7 @@ rbc3d_status self_mixed_density(rbc3d_ctx* ctx, bool f, bool g);
 rbc3d_status run_self_mixed(rbc3d_ctx* ctx, int tlist, double c1, double c2);
 rbc3d_status self_ff_tables(rbc3d_ctx* ctx, const std::vector<double>& c1, const std::vector<double>& c2,
                             const std::vector<double>& dl);
-rbc3d_status self_ff_grid(rbc3d_ctx* ctx, const std::vector<SelfW64>& W, const std::vector<double>& pw);
+rbc3d_status self_ff_grid(rbc3d_ctx* ctx, const std::vector<RingClass>& R);
 void self_ff_invalidate(rbc3d_ctx* ctx, bool geom, bool f, bool g);
 rbc3d_status run_self_ff(rbc3d_ctx* ctx, int tlist, double c1, double c2);
 inline bool valid_prec(int p) {

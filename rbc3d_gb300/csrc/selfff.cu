@@ -28,20 +28,22 @@
 // (rel-L2, 256-cell workload); the interpolation sums carry errors of a few
 // 1e-12 of sum |w v| (x) or of the cell's maxima (f, g, a3).
 //
-// Data layout.  Per node and slot d (u, u_th, u_ph, u_thph) the 12 values x
+// By latitude rings, as selfring.cu does it in FP64: the points of a ring's
+// targets share their colatitudes and pair up about the meridian, so per point
+// pair (class) and column j the theta part U_j, D_j (4 terms each) is computed
+// once for the ring, and a point takes the 4 terms of the phi part from the
+// columns j and j + 1.  About 500 packed instructions of interpolation a point
+// against 900 with 16 terms, and 0.4 KB of loads against 1.7 KB.  256 cells,
+// SL+DL: 6.5 -> 4.8 ms against one warp per target, the FP32D matvec 10.66 -> 8.89.
+//
+// Data layout.  Per row i and slot d (u, u_th, u_ph, u_thph) the 12 values x
 // (relative to the cell centre), f and g density sets and a3 (three
-// components each) are stored as three quads; a quad's hi and lo parts form
-// one 32-byte entry, read with one 256-bit load, in its own plane
-// [cell][d*3 + quad][node tile]: the lanes of a warp interpolate at
-// neighbouring patch points, and with 2 x 2 node tiles per 128-byte line
-// their stencil nodes share lines (a record per node put each lane's load
-// in its own line and kept the L1 data pipe 95% busy; separate hi and lo
-// planes of 16-byte entries took two loads and two lines per quad).
-// Consecutive values share one bicubic weight, so they run in pairs as
-// packed FP32x2 operations.  Patch weights per (target latitude,
-// patch point) are the 16 Spline_Interp products as hi/lo planes (coalesced
-// across the lanes, which walk consecutive patch points); target positions
-// are the FP32M hi/lo records relative to the same cell centre.
+// components each) are stored as three quads in column order; a quad's hi and
+// lo parts form one 32-byte entry, read with one 256-bit load, so that a warp
+// reads 32 consecutive entries: [cell][row][slot][quad][column].
+// Consecutive values share one weight, so they run in pairs as packed FP32x2
+// operations; the weights are stored doubled, as the pairs' operands.  Target
+// positions are the FP32M hi/lo records relative to the same cell centre.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -50,30 +52,18 @@
 
 namespace {
 
-inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
+constexpr int FF_ROW = 12;   // 32-byte entries of a node: 4 slots x 3 quads
+constexpr int FF_CHUNK = 2;  // classes between two barriers: the rows' entries are loaded once for both
 
-constexpr int FF_PLANES = 24;  // float4 per node: 4 slots x 3 quads x (hi, lo)
-
-// Position of spline node (i, j) in a plane: tiles of 2^ti (latitude rows) x
-// 2^tj (longitude columns), one 128-byte line of 32-byte entries per plane.
-// With 16-byte entries (8 per line) 2 x 4 tiles measured best for the
-// 25 x 50 grid (k_self_ff at 256 cells: 6.81 ms; 4 x 2 7.02, 8 x 1 7.07,
-// 1 x 8 7.65); 32-byte entries in 2 x 2 tiles: 6.68 ms in the matvec.
-struct NodeMap {
-  int ti, tj, nti;  // log2 tile sizes, tiles along i
-  long long per;    // padded nodes per plane
-  __device__ __forceinline__ int pos(int i, int j) const {
-    return (((j >> tj) * nti + (i >> ti)) << (ti + tj)) + (i & ((1 << ti) - 1)) + ((j & ((1 << tj) - 1)) << ti);
-  }
+// A class of patch points (RingClass) in hi/lo parts, each weight as the
+// operands (h, h, l, l): the theta weights of (u, u', u_th, u'_th), per side
+// the phi weights of (U_j, U_j+1, D_j, D_j+1).
+struct FFClass {
+  int i1, j[2], pad;
+  float4 x[4], y[2][4];
+  float2 w, pad2;
 };
-inline NodeMap node_map(int m, int n) {
-  NodeMap M;
-  M.ti = 1; M.tj = 1;
-  M.nti = (m + (1 << M.ti) - 1) >> M.ti;
-  const int ntj = (n + (1 << M.tj) - 1) >> M.tj;
-  M.per = (long long)M.nti * ntj << (M.ti + M.tj);
-  return M;
-}
+static_assert(sizeof(FFClass) % 16 == 0, "vector loads of the weights");
 
 // ---------------------------------------------------------------------------
 // float-float arithmetic
@@ -156,26 +146,25 @@ struct Dot2 {
     c = __ffma2_rn(wl, vh, c);
     c = __fadd2_rn(c, sub2(err, ne));
   }
-  __device__ __forceinline__ ff x() const { return two_sum(s.x, c.x); }
-  __device__ __forceinline__ ff y() const { return two_sum(s.y, c.y); }
+  // FAST with the weight's stored operands (h, h, l, l)
+  template <bool FAST>
+  __device__ __forceinline__ void add(float4 w, float2 vh, float2 vl) {
+    add<FAST>(make_float2(w.x, w.y), make_float2(-w.x, -w.y), make_float2(w.z, w.w), vh, vl);
+  }
 };
 
 struct FFArgs {
-  int nt, ncell, nlat, nlon, m, NQ, nrad;
+  int nt, ncell, nlat, nlon, m, NC, G, parts;
   const double* tA;
   double* v;
-  const float4* rec;    // [cell][slot x quad][node tile][hi, lo]
-  const int2* widx;     // (i1, j1b) per (latitude, patch point)
-  const float4* w;      // 8 planes of nlat*NQ: hi of slot d of nodes 0..3 (d = 0..3), then lo
-  const float2* pw;     // patch weights, hi/lo
+  const float4* rec;    // [cell][row][slot][quad][column][hi, lo]
+  const FFClass* cls;   // [latitude][NC]
   const float4* thi;    // target positions relative to the cell centre, hi
   const float4* tlo;    // and lo
   const float4* tab;    // [3][EWALD_NTAB]: {T_i hi, T_i lo, (T_i+1 - T_i) hi, lo}
   const uint4* bnd;     // [set x f g a3][cell]: max |u|, |u_th|, |u_ph|, |u_thph| (float bits)
-  NodeMap map;
-  float hq1, hq2, hq12; // derivative weight-sum bounds: h_th / 4, h_ph / 4, h_th h_ph / 16
+  float hq1, hq2;       // derivative weight-sum bounds: h_th / 4, h_ph / 4
   const int* celltype;
-  const short* perm;    // [latitude][k]: the patch point lane k of the warp's pass takes
   ff c1;                // c1
   ff c2B[RBC3D_MAX_CELLTYPES];  // c2 Bcoef per cell type
   ff rc2, r_eps, ntab_over_rc;
@@ -193,107 +182,72 @@ __device__ __forceinline__ ff dot3(const ff* a, const ff* b) {
   return ff_add(ff_add(ff_mul(a[0], b[0]), ff_mul(a[1], b[1])), ff_mul(a[2], b[2]));
 }
 
-// One target of the own-cell patch: warp index w (cell, latitude ring,
-// longitude), its grid point p, position, DL factor, record base and the
-// starting offsets of its cell's sums (x: the derivative terms'; f, g, a3:
-// all 16 terms').
-struct Tgt {
-  int p, cell, ilat0, ilon0;
-  ff xi[3];
-  ff c2m;
-  const float4* base;
-  float2 offs[6];
+// The pairs of values: (x.x x.y) (x.z f.x) (f.y f.z) (g.x g.y) (g.z a.x) (a.y a.z),
+// value 3 set + component in the order x, f, g, a3.
+constexpr int FF_PAIRS = 6, FF_XPAIRS = 2;  // the first two hold x: value terms by TwoSum
+// Offsets of one cell's sums: of U and D (theta part) and of the point (phi
+// part), the x pairs' for their derivative terms only; and c2 Bcoef.
+struct FFCell {
+  float2 u[FF_PAIRS], d[FF_PAIRS], p[FF_PAIRS];
+  float2 c2m, pad;
 };
 
-template <bool DL>
-__device__ __forceinline__ Tgt target(const FFArgs& a, int w) {
-  Tgt T;
-  const int nv = a.nlat * a.nlon;
-  T.cell = w / nv;
-  const int rr = w - T.cell * nv;
-  T.ilon0 = rr % a.nlon;
-  T.ilat0 = rr / a.nlon;
-  T.p = T.cell * nv + T.ilon0 * a.nlat + T.ilat0;
-  const float4 th4 = a.thi[T.p], tl4 = a.tlo[T.p];
-  T.xi[0] = {th4.x, tl4.x}; T.xi[1] = {th4.y, tl4.y}; T.xi[2] = {th4.z, tl4.z};
-  T.c2m = DL ? a.c2B[a.celltype[T.cell]] : ff{0.f, 0.f};
-  T.base = a.rec + (size_t)T.cell * FF_PLANES * a.map.per;
-  float off[4], offd[2];
-#pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    const uint4 b = __ldg(a.bnd + (size_t)s * a.ncell + T.cell);
-    const float Bd = a.hq1 * __uint_as_float(b.y) + a.hq2 * __uint_as_float(b.z) + a.hq12 * __uint_as_float(b.w);
-    int e;
-    frexpf(2.f * 1.01f * (__uint_as_float(b.x) + Bd), &e);  // 2 B < 2^e
-    off[s] = ldexpf(1.f, e);
-    if (s < 2) {  // x, and f where it shares a pair with x
-      frexpf(2.f * 1.01f * Bd, &e);
-      offd[s] = ldexpf(1.f, e);
-    }
-  }
-  T.offs[0] = make_float2(offd[0], offd[0]); T.offs[1] = make_float2(offd[0], offd[1]);
-  T.offs[2] = make_float2(off[1], off[1]); T.offs[3] = make_float2(off[2], off[2]);
-  T.offs[4] = make_float2(off[2], off[3]); T.offs[5] = make_float2(off[3], off[3]);
-  return T;
+// smallest power of two at least twice b (with a margin for b's rounding)
+__device__ __forceinline__ float sum_offset(float b) {
+  int e;
+  frexpf(2.f * 1.01f * b, &e);
+  return ldexpf(1.f, e);
 }
 
-// Patch point q of target T added to acc (RBC_SingInt's loop body).
-template <bool SL, bool DL>
-__device__ __forceinline__ void patch_point(const FFArgs& a, const Tgt& T, int q, ffacc* acc) {
-  constexpr int NP = DL ? 6 : 3;  // value pairs per slot: (x.x x.y) (x.z f.x) (f.y f.z) | (g.x g.y) (g.z a.x) (a.y a.z)
-  constexpr int NX = 2;           // the pairs that hold x: value terms by TwoSum
-  const size_t per = (size_t)a.map.per;
-  const size_t plane = (size_t)a.nlat * a.NQ;
-  const size_t wi = (size_t)T.ilat0 * a.NQ + q;
-  const int2 ix = __ldg(a.widx + wi);
-  const int j1 = imod(ix.y + T.ilon0, a.nlon), j2 = (j1 + 1 == a.nlon) ? 0 : j1 + 1;
-  const int i1 = ix.x, i2 = (i1 + 1 == a.m) ? 0 : i1 + 1;
-  const int nodes[4] = {a.map.pos(i1, j1), a.map.pos(i1, j2), a.map.pos(i2, j1), a.map.pos(i2, j2)};
-  Dot2 d2[NP];
-#pragma unroll
-  for (int k = 0; k < NP; ++k) { d2[k].s = T.offs[k]; d2[k].c = make_float2(0.f, 0.f); }
-  // slots u_th, u_ph, u_thph first (FastTwoSum from off), then u (the x
-  // pairs: off subtracted, TwoSum; the others: FastTwoSum, off subtracted after)
-#pragma unroll
-  for (int dd = 0; dd < 4; ++dd) {
-    const int d = (dd + 1) & 3;
-    if (d == 0) {
-#pragma unroll
-      for (int k = 0; k < NX; ++k) d2[k].s = sub2(d2[k].s, T.offs[k]);  // exact: off/2 <= s <= 3 off/2
-    }
-    const float4 wh4 = __ldg(a.w + d * plane + wi), wl4 = __ldg(a.w + (4 + d) * plane + wi);
-    const float whs[4] = {wh4.x, wh4.y, wh4.z, wh4.w}, wls[4] = {wl4.x, wl4.y, wl4.z, wl4.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 wh = make_float2(whs[k], whs[k]), nwh = make_float2(-whs[k], -whs[k]);
-      const float2 wl = make_float2(wls[k], wls[k]);
-      const float4* r = T.base + 2 * ((size_t)(3 * d) * per + nodes[k]);
-      float2 vh[DL ? 6 : 4], vl[DL ? 6 : 4];
-#pragma unroll
-      for (int i = 0; i < (DL ? 3 : 2); ++i) {  // SL: quads (x.x x.y x.z f.x) (f.y f.z . .)
-        float4 h, l;
-        ld8(r + 2 * (size_t)i * per, h, l);
-        vh[2 * i] = make_float2(h.x, h.y); vh[2 * i + 1] = make_float2(h.z, h.w);
-        vl[2 * i] = make_float2(l.x, l.y); vl[2 * i + 1] = make_float2(l.z, l.w);
-      }
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        if (d == 0 && i < NX) d2[i].add<false>(wh, nwh, wl, vh[i], vl[i]);
-        else d2[i].add<true>(wh, nwh, wl, vh[i], vl[i]);
-      }
-    }
+__device__ __forceinline__ void cell_offsets(const FFArgs& a, int cell, FFCell& C) {
+  float ou[4], od[4], op[4];
+  for (int s = 0; s < 4; ++s) {
+    const uint4 b = __ldg(a.bnd + (size_t)s * a.ncell + cell);
+    const float u = __uint_as_float(b.x), ut = __uint_as_float(b.y), up = __uint_as_float(b.z), utp = __uint_as_float(b.w);
+    const float D = up + a.hq1 * utp, U = u + a.hq1 * ut;  // bounds of |D_j|, |U_j|
+    const bool x = s == 0;
+    ou[s] = sum_offset(x ? a.hq1 * ut : U);
+    od[s] = sum_offset(D);
+    op[s] = sum_offset(x ? a.hq2 * D : U + a.hq2 * D);
   }
-#pragma unroll
-  for (int k = NX; k < NP; ++k) d2[k].s = sub2(d2[k].s, T.offs[k]);
-  // interpolated x (relative to the cell centre), f, g, a3
+  // f shares its first pair with x: the derivative terms' offset there too
+  const uint4 b = __ldg(a.bnd + (size_t)a.ncell + cell);
+  const float fD = __uint_as_float(b.z) + a.hq1 * __uint_as_float(b.w);
+  const float fu = sum_offset(a.hq1 * __uint_as_float(b.y)), fp = sum_offset(a.hq2 * fD);
+  C.u[0] = make_float2(ou[0], ou[0]); C.u[1] = make_float2(ou[0], fu); C.u[2] = make_float2(ou[1], ou[1]);
+  C.u[3] = make_float2(ou[2], ou[2]); C.u[4] = make_float2(ou[2], ou[3]); C.u[5] = make_float2(ou[3], ou[3]);
+  C.d[0] = make_float2(od[0], od[0]); C.d[1] = make_float2(od[0], od[1]); C.d[2] = make_float2(od[1], od[1]);
+  C.d[3] = make_float2(od[2], od[2]); C.d[4] = make_float2(od[2], od[3]); C.d[5] = make_float2(od[3], od[3]);
+  C.p[0] = make_float2(op[0], op[0]); C.p[1] = make_float2(op[0], fp); C.p[2] = make_float2(op[1], op[1]);
+  C.p[3] = make_float2(op[2], op[2]); C.p[4] = make_float2(op[2], op[3]); C.p[5] = make_float2(op[3], op[3]);
+  const ff c2 = a.c2B[a.celltype[cell]];
+  C.c2m = make_float2(c2.h, c2.l);
+}
+
+__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
+
+// RBC_SingInt's loop body at interpolated values v (s and c of the 6 pairs)
+// for a target at xi: c1 and c2 terms added to the sums acc (stride st).
+template <bool SL, bool DL>
+__device__ __forceinline__ void patch_point(const FFArgs& a, const Dot2* d2, const ff* xi, ff c2m, ff wq, float2* acc,
+                                            int st) {
   ff xx[3], F[3], G[3], A[3];
-  xx[0] = ff_sub(d2[0].x(), T.xi[0]);
-  xx[1] = ff_sub(d2[0].y(), T.xi[1]);
-  xx[2] = ff_sub(d2[1].x(), T.xi[2]);
-  F[0] = d2[1].y(); F[1] = d2[2].x(); F[2] = d2[2].y();
+  xx[0] = ff_sub(fast_two_sum(d2[0].s.x, d2[0].c.x), xi[0]);
+  xx[1] = ff_sub(fast_two_sum(d2[0].s.y, d2[0].c.y), xi[1]);
+  xx[2] = ff_sub(fast_two_sum(d2[1].s.x, d2[1].c.x), xi[2]);
+  if (SL) {
+    F[0] = fast_two_sum(d2[1].s.y, d2[1].c.y);
+    F[1] = fast_two_sum(d2[2].s.x, d2[2].c.x);
+    F[2] = fast_two_sum(d2[2].s.y, d2[2].c.y);
+  }
   if (DL) {
-    G[0] = d2[3].x(); G[1] = d2[3].y(); G[2] = d2[4].x();
-    A[0] = d2[4].y(); A[1] = d2[5].x(); A[2] = d2[5].y();
+    G[0] = fast_two_sum(d2[3].s.x, d2[3].c.x);
+    G[1] = fast_two_sum(d2[3].s.y, d2[3].c.y);
+    G[2] = fast_two_sum(d2[4].s.x, d2[4].c.x);
+    A[0] = fast_two_sum(d2[4].s.y, d2[4].c.y);
+    A[1] = fast_two_sum(d2[5].s.x, d2[5].c.x);
+    A[2] = fast_two_sum(d2[5].s.y, d2[5].c.y);
   }
   const ff r2 = ff_add(ff_add(ff_mul(xx[0], xx[0]), ff_mul(xx[1], xx[1])), ff_mul(xx[2], xx[2]));
   if (ff_ge(r2, a.rc2)) return;  // rr >= rc (ModRbcSingInt.F90:65)
@@ -317,8 +271,6 @@ __device__ __forceinline__ void patch_point(const FFArgs& a, const Tgt& T, int q
   if (it < 0 || it >= EWALD_NTAB) return;
   const ff f1 = two_sum(__fsub_rn(sp.h, fi), sp.l);
   const ff ir2 = ff_mul(ir, ir);
-  const int irad = q % a.nrad;
-  const ff wq = ld_ff(__ldg(a.pw + irad));
   ff cx = {0.f, 0.f}, cf = {0.f, 0.f};  // dv += cx xx + cf f
   if (SL) {
     const ff cs1 = tab_lerp(a.tab, 0, it, f1), cs2 = tab_lerp(a.tab, 1, it, f1);
@@ -333,38 +285,158 @@ __device__ __forceinline__ void patch_point(const FFArgs& a, const Tgt& T, int q
     // c2 Bcoef wq EA xx (xx . g)(xx . a3), EA = cd / r^5
     const ff cd = tab_lerp(a.tab, 2, it, f1);
     const ff EA = ff_mul(cd, ff_mul(ir2, ff_mul(ir2, ir)));
-    const ff t = ff_mul(ff_mul(ff_mul(T.c2m, wq), EA), ff_mul(dot3(xx, G), dot3(xx, A)));
+    const ff t = ff_mul(ff_mul(ff_mul(c2m, wq), EA), ff_mul(dot3(xx, G), dot3(xx, A)));
     cx = SL ? ff_add(cx, t) : t;
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    acc[k].add(ff_mul(cx, xx[k]));
-    if (SL) acc[k].add(ff_mul(cf, F[k]));
+    const float2 z = acc[k * st];
+    ffacc s = {z.x, z.y};
+    s.add(ff_mul(cx, xx[k]));
+    if (SL) s.add(ff_mul(cf, F[k]));
+    acc[k * st] = make_float2(s.s, s.c);
   }
 }
 
-// One warp per target; the 8 warps of a block take 8 consecutive targets of
-// a latitude ring, so that they share weight entries and most stencil nodes
-// in L1.  The lanes of one pass take patch points in the order of their
-// stencil cells' 2 x 2 node tiles (a per-latitude permutation), so that they
-// read fewer distinct lines (6.71 -> 6.60 ms at 256 cells against the
-// radial-ray order; raster order of the stencil cells: 7.25 ms).  (Packing the 8-point tails of 4 targets into one full pass saved
-// 15% of the instructions but not time: the kernel is bound by the L1 data
-// pipe, 7.08 against 6.81 ms at 256 cells.)
+// One block: a ring of G cells, thread = column (cols = G nlon; more than 256
+// columns: several a thread).  Per chunk of FF_CHUNK classes the theta parts
+// go to shared memory, then every column evaluates the points in the interval
+// [j, j + 1]: of the targets j - j[0] and j - j[1] (mod nlon), whose sums lie
+// in shared memory, a side each, so no two threads meet between two barriers.
 template <bool SL, bool DL>
 __global__ void __launch_bounds__(256, 2) k_self_ff(FFArgs a) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= a.ncell * a.nlat * a.nlon) return;
-  const Tgt T = target<DL>(a, w);
-  ffacc acc[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-  const short* pr = a.perm + (size_t)T.ilat0 * a.NQ;
-  for (int k = lane; k < a.NQ; k += 32) patch_point<SL, DL>(a, T, pr[k], acc);
-  double dv[3];
-  for (int k = 0; k < 3; ++k) dv[k] = warp_sum((double)acc[k].s + (double)acc[k].c);
-  if (lane == 0) {
-    const double iA = 1.0 / a.tA[T.p];
-    for (int k = 0; k < 3; ++k) a.v[T.p + (size_t)k * a.nt] += dv[k] * iA;
+  constexpr int NP = DL ? (SL ? 6 : 5) : 3;  // pairs kept; without SL the pair (f.y f.z) is left out
+  extern __shared__ __align__(16) unsigned char smem_ff[];
+  const int nlon = a.nlon, cols = a.G * nlon;
+  float4* ex = reinterpret_cast<float4*>(smem_ff);            // [FF_CHUNK][NP][U, D][cols]: (s, s, c, c)
+  FFCell* sC = reinterpret_cast<FFCell*>(ex + (size_t)FF_CHUNK * NP * 2 * cols);  // [G]
+  float2* acc = reinterpret_cast<float2*>(sC + a.G);          // [2 sides][3][cols]
+  float2* sT = acc + 6 * cols;                                // [3][cols] target positions
+  int b = blockIdx.x;
+  const int part = b % a.parts; b /= a.parts;
+  const int ring = b % a.nlat, cell0 = (b / a.nlat) * a.G;
+  const int ncl = min(a.G, a.ncell - cell0), ncol = ncl * nlon;
+  const int nv = a.nlat * nlon;
+  for (int t = threadIdx.x; t < ncl; t += blockDim.x) cell_offsets(a, cell0 + t, sC[t]);
+  for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
+    const int lc = t / nlon, j = t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
+    const float4 h = a.thi[p], l = a.tlo[p];
+    sT[t] = make_float2(h.x, l.x); sT[cols + t] = make_float2(h.y, l.y); sT[2 * cols + t] = make_float2(h.z, l.z);
+    for (int k = 0; k < 6; ++k) acc[k * cols + t] = make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+  const int k0 = (int)((long long)a.NC * part / a.parts), k1 = (int)((long long)a.NC * (part + 1) / a.parts);
+  const FFClass* cls = a.cls + (size_t)ring * a.NC;
+  for (int kb = k0; kb < k1; kb += FF_CHUNK) {
+    for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
+      const int lc = t / nlon, j = t - lc * nlon;
+      const FFCell& C = sC[lc];
+      const float4* rc = a.rec + 2 * ((size_t)(cell0 + lc) * a.m * FF_ROW * nlon + j);
+#pragma unroll
+      for (int q = 0; q < (DL ? 3 : 2); ++q) {
+        float4 rh[8], rl[8];  // row i1: slots 0..3, row i1 + 1: slots 0..3
+        int have = -1;
+#pragma unroll
+        for (int kk = 0; kk < FF_CHUNK; ++kk) {
+          if (kb + kk >= k1) break;
+          const FFClass& c = cls[kb + kk];
+          if (c.i1 != have) {
+            have = c.i1;
+            const int i2 = have + 1 == a.m ? 0 : have + 1;
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+              ld8(rc + 2 * (size_t)((have * FF_ROW + 3 * d + q) * nlon), rh[d], rl[d]);
+              ld8(rc + 2 * (size_t)((i2 * FF_ROW + 3 * d + q) * nlon), rh[4 + d], rl[4 + d]);
+            }
+          }
+          const float4 w0 = __ldg(c.x), w1 = __ldg(c.x + 1), w2 = __ldg(c.x + 2), w3 = __ldg(c.x + 3);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int P = 2 * q + e;
+            if ((!DL && P >= 3) || (!SL && P == 2)) continue;
+            const int S = (!SL && P > 2) ? P - 1 : P;
+            auto vh = [&](int i) { return e ? hi2(rh[i]) : lo2(rh[i]); };
+            auto vl = [&](int i) { return e ? hi2(rl[i]) : lo2(rl[i]); };
+            Dot2 U, D;
+            const float2 ou = C.u[P], od = C.d[P];
+            U.s = ou; U.c = make_float2(0.f, 0.f);
+            U.add<true>(w2, vh(1), vl(1));
+            U.add<true>(w3, vh(5), vl(5));
+            if (P < FF_XPAIRS) {  // off/2 <= s <= 3 off/2: the subtraction is exact
+              U.s = sub2(U.s, ou);
+              U.add<false>(w0, vh(0), vl(0));
+              U.add<false>(w1, vh(4), vl(4));
+            } else {
+              U.add<true>(w0, vh(0), vl(0));
+              U.add<true>(w1, vh(4), vl(4));
+              U.s = sub2(U.s, ou);
+            }
+            D.s = od; D.c = make_float2(0.f, 0.f);
+            D.add<true>(w2, vh(3), vl(3));
+            D.add<true>(w3, vh(7), vl(7));
+            D.add<true>(w0, vh(2), vl(2));
+            D.add<true>(w1, vh(6), vl(6));
+            D.s = sub2(D.s, od);
+            float4* o = ex + (size_t)((kk * NP + S) * 2) * cols + t;
+            o[0] = make_float4(U.s.x, U.s.y, U.c.x, U.c.y);
+            o[cols] = make_float4(D.s.x, D.s.y, D.c.x, D.c.y);
+          }
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int kk = 0; kk < FF_CHUNK && kb + kk < k1; ++kk) {
+      const FFClass& c = cls[kb + kk];
+      for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
+        const int lc = t / nlon, j = t - lc * nlon, base = t - j;
+        const int tn = j + 1 == nlon ? base : t + 1;
+        const FFCell& C = sC[lc];
+#pragma unroll 1
+        for (int side = 0; side < 2; ++side) {
+          const int js = c.j[side];
+          if (js < 0) break;  // the points on the meridian have no mirror image
+          const int q = base + (j >= js ? j - js : j - js + nlon);  // the target's column
+          const float4* y = c.y[side];
+          const float4 w0 = __ldg(y), w1 = __ldg(y + 1), w2 = __ldg(y + 2), w3 = __ldg(y + 3);
+          Dot2 d2[FF_PAIRS];
+#pragma unroll
+          for (int P = 0; P < FF_PAIRS; ++P) {
+            if ((!DL && P >= 3) || (!SL && P == 2)) continue;
+            const int S = (!SL && P > 2) ? P - 1 : P;
+            const float4* o = ex + (size_t)((kk * NP + S) * 2) * cols;
+            const float4 D0 = o[cols + t], D1 = o[cols + tn], U0 = o[t], U1 = o[tn];
+            const float2 off = C.p[P];
+            Dot2& d = d2[P];
+            d.s = off; d.c = make_float2(0.f, 0.f);
+            d.add<true>(w2, lo2(D0), hi2(D0));
+            d.add<true>(w3, lo2(D1), hi2(D1));
+            if (P < FF_XPAIRS) {
+              d.s = sub2(d.s, off);
+              d.add<false>(w0, lo2(U0), hi2(U0));
+              d.add<false>(w1, lo2(U1), hi2(U1));
+            } else {
+              d.add<true>(w0, lo2(U0), hi2(U0));
+              d.add<true>(w1, lo2(U1), hi2(U1));
+              d.s = sub2(d.s, off);
+            }
+          }
+          const ff xi[3] = {ld_ff(sT[q]), ld_ff(sT[cols + q]), ld_ff(sT[2 * cols + q])};
+          patch_point<SL, DL>(a, d2, xi, ld_ff(C.c2m), ld_ff(__ldg(&c.w)), acc + 3 * side * cols + q, cols);
+        }
+      }
+      __syncthreads();  // the next class's sums may meet these
+    }
+  }
+  for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
+    const int lc = t / nlon, j = t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
+    const double iA = 1.0 / a.tA[p];
+    for (int k = 0; k < 3; ++k) {
+      const float2 z0 = acc[k * cols + t], z1 = acc[(3 + k) * cols + t];
+      const double dv = (((double)z0.x + (double)z1.x) + ((double)z0.y + (double)z1.y)) * iA;
+      if (a.parts == 1) a.v[p + (size_t)k * a.nt] += dv;
+      else atomicAdd(a.v + p + (size_t)k * a.nt, dv);
+    }
   }
 }
 
@@ -375,38 +447,58 @@ __device__ __forceinline__ void split(double v, float* h, float* l) {
   *l = (float)(v - (double)hv);
 }
 
-// node records of the spline sets named in `sets` (bit 0 x, 1 f, 2 g, 3 a3):
+// Node records of the spline sets named in `sets` (bit 0 x, 1 f, 2 g, 3 a3):
 // value 3 s + c of slot d goes to component (3 s + c) % 4 of quad (3 s + c) / 4.
-// bnd[s][cell] collects max |value| per slot (float bits, rounded up; a warp
-// spanning two cells gives both the larger maximum).
-__global__ void k_ff_rec(int ncell, int m, long long per, NodeMap map, const double* __restrict__ spl,
-                         const double* __restrict__ xc, float4* __restrict__ out, unsigned* __restrict__ bnd, int sets) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = idx < (long long)ncell * per;
-  const int cell = valid ? (int)(idx / per) : ncell - 1;
-  const long long node = idx - (long long)cell * per;  // i + m j
-  const int lane = threadIdx.x & 31;
-  const int prev = __shfl_up_sync(0xffffffffu, cell, 1);
-  const bool lead = lane == 0 || prev != cell;
-  const int ni = valid ? (int)(node % m) : 0, nj = valid ? (int)(node / m) : 0;
-  float* o = reinterpret_cast<float*>(out + (size_t)cell * FF_PLANES * map.per) + 8 * (size_t)map.pos(ni, nj);
-  const size_t pstride = 8 * (size_t)map.per;  // floats between planes of 32-byte entries
+// bnd[s][cell] collects max |value| per slot (float bits, rounded up).  A block
+// takes 4 rows x 16 columns of one cell through shared memory (the tables are
+// in row order, the records in column order).
+__global__ void __launch_bounds__(128) k_ff_rec(int ncell, int m, int n, const double* __restrict__ spl,
+                                                const double* __restrict__ xc, float* __restrict__ out,
+                                                unsigned* __restrict__ bnd, int sets) {
+  __shared__ double s[4][16][4][SPL_NODE];  // set, column, row, value
+  __shared__ unsigned smax[16];
+  const int nti = (m + 3) / 4, ntj = (n + 15) / 16;
+  const int jt = blockIdx.x % ntj, it = (blockIdx.x / ntj) % nti, cell = blockIdx.x / (ntj * nti);
   const int src[4] = {SPL_X, SPL_F, SPL_G, SPL_A3};
-  for (int s = 0; s < 4; ++s) {
-    if (!(sets & (1 << s))) continue;
-    const double* sp = spl + (((size_t)cell * SPL_NSET + src[s]) * per + node) * SPL_NODE;
-    for (int d = 0; d < 4; ++d) {
-      unsigned mx = 0;
-      if (valid)
-        for (int c = 0; c < 3; ++c) {
-          double v = sp[3 * d + c];
-          if (s == 0 && d == 0) v -= xc[3 * cell + c];
-          const int q = (3 * s + c) >> 2, e = (3 * s + c) & 3;
-          split(v, o + (3 * d + q) * pstride + e, o + (3 * d + q) * pstride + 4 + e);
-          mx = max(mx, __float_as_uint(__double2float_ru(fabs(v))));
-        }
-      mx = __reduce_max_sync(0xffffffffu, mx);
-      if (valid && lead) atomicMax(bnd + ((size_t)s * ncell + cell) * 4 + d, mx);
+  if (threadIdx.x < 16) smax[threadIdx.x] = 0;
+  __syncthreads();
+  for (int k = 0; k < 4; ++k) {
+    if (!(sets & (1 << k))) continue;
+    const double* in = spl + ((size_t)cell * SPL_NSET + src[k]) * (size_t)m * n * SPL_NODE;
+    for (int e = threadIdx.x; e < 16 * 4 * SPL_NODE; e += blockDim.x) {
+      const int q = e % SPL_NODE, r = (e / SPL_NODE) % 4, c = e / (4 * SPL_NODE);
+      const int j = 16 * jt + c, i = 4 * it + r;
+      double v = 0.;
+      if (j < n && i < m) v = in[((size_t)j * m + i) * SPL_NODE + q];
+      if (k == 0 && q < 3 && j < n && i < m) v -= xc[3 * cell + q];
+      s[k][c][r][q] = v;
+      const unsigned mx = __float_as_uint(__double2float_ru(fabs(v)));
+      atomicMax(&smax[4 * k + q / 3], mx);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 16 && (sets & (1 << (threadIdx.x / 4))))
+    atomicMax(bnd + ((size_t)(threadIdx.x / 4) * ncell + cell) * 4 + threadIdx.x % 4, smax[threadIdx.x]);
+  for (int e = threadIdx.x; e < 4 * FF_ROW * 16; e += blockDim.x) {
+    const int c = e % 16, dq = (e / 16) % FF_ROW, r = e / (16 * FF_ROW);
+    const int j = 16 * jt + c, i = 4 * it + r;
+    if (j >= n || i >= m) continue;
+    float* o = out + 8 * ((((size_t)cell * m + i) * FF_ROW + dq) * n + j);
+    float h[4], l[4];
+    int have = 0;
+    for (int k = 0; k < 4; ++k) {
+      const int val = 4 * (dq % 3) + k, set = val / 3;
+      h[k] = l[k] = 0.f;
+      if (!(sets & (1 << set))) continue;
+      split(s[set][c][r][3 * (dq / 3) + val % 3], h + k, l + k);
+      have |= 1 << k;
+    }
+    if (have == 15) {
+      *reinterpret_cast<float4*>(o) = make_float4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<float4*>(o + 4) = make_float4(l[0], l[1], l[2], l[3]);
+    } else {
+      for (int k = 0; k < 4; ++k)
+        if (have & (1 << k)) { o[k] = h[k]; o[4 + k] = l[k]; }
     }
   }
 }
@@ -435,47 +527,26 @@ rbc3d_status self_ff_tables(rbc3d_ctx* ctx, const std::vector<double>& c1, const
   return RBC3D_OK;
 }
 
-// Patch weights per (latitude, patch point) as hi/lo planes, from the FP64
-// table of k_self, and the patch weights pw as hi/lo.
-rbc3d_status self_ff_grid(rbc3d_ctx* ctx, const std::vector<SelfW64>& W, const std::vector<double>& pw) {
-  const size_t n = W.size();
-  std::vector<int2> idx(n);
-  std::vector<float4> w(8 * n);
-  for (size_t i = 0; i < n; ++i) {
-    idx[i] = make_int2(W[i].i1, W[i].j1b);
-    for (int d = 0; d < 4; ++d) {
-      ff e[4];
-      for (int k = 0; k < 4; ++k) e[k] = hsplit(W[i].w[4 * k + d]);
-      w[(size_t)d * n + i] = make_float4(e[0].h, e[1].h, e[2].h, e[3].h);
-      w[(size_t)(4 + d) * n + i] = make_float4(e[0].l, e[1].l, e[2].l, e[3].l);
+// The ring classes in hi/lo parts (the value weights complete: 1 - x[0] for u).
+rbc3d_status self_ff_grid(rbc3d_ctx* ctx, const std::vector<RingClass>& R) {
+  auto op = [](double v) {
+    const ff e = hsplit(v);
+    return make_float4(e.h, e.h, e.l, e.l);
+  };
+  std::vector<FFClass> C(R.size());
+  for (size_t i = 0; i < R.size(); ++i) {
+    const RingClass& r = R[i];
+    FFClass& c = C[i];
+    c.i1 = r.i1; c.j[0] = r.j[0]; c.j[1] = r.j[1]; c.pad = 0;
+    c.x[0] = op(1. - r.x[0]); c.x[1] = op(r.x[0]); c.x[2] = op(r.x[1]); c.x[3] = op(r.x[2]);
+    for (int s = 0; s < 2; ++s) {
+      c.y[s][0] = op(1. - r.y[s][0]); c.y[s][1] = op(r.y[s][0]); c.y[s][2] = op(r.y[s][1]); c.y[s][3] = op(r.y[s][2]);
     }
+    const ff w = hsplit(r.w);
+    c.w = make_float2(w.h, w.l);
+    c.pad2 = make_float2(0.f, 0.f);
   }
-  std::vector<float2> p(pw.size());
-  for (size_t i = 0; i < pw.size(); ++i) {
-    const ff e = hsplit(pw[i]);
-    p[i] = make_float2(e.h, e.l);
-  }
-  // lane order of the patch points per latitude: by the 2 x 2 tile of their
-  // stencil cell (i1, j1b), then by the cell inside the tile
-  {
-    const int nlat = ctx->nlat, NQ = (int)(n / nlat);
-    std::vector<short> perm(n);
-    std::vector<int> q(NQ);
-    for (int l = 0; l < nlat; ++l) {
-      for (int k = 0; k < NQ; ++k) q[k] = k;
-      auto key = [&](int k) {
-        const int2 t = idx[(size_t)l * NQ + k];
-        const int i = t.x, j = t.y + 4096;  // j1b may be negative
-        return ((long long)(i >> 1) * 100000 + (j >> 1)) * 4 + (i & 1) * 2 + (j & 1);
-      };
-      std::stable_sort(q.begin(), q.end(), [&](int a2, int b2) { return key(a2) < key(b2); });
-      for (int k = 0; k < NQ; ++k) perm[(size_t)l * NQ + k] = (short)q[k];
-    }
-    CUDA_TRY(ctx->ff_perm.upload(perm.data(), perm.size(), ctx->st));
-  }
-  CUDA_TRY(ctx->ff_widx.upload(idx.data(), idx.size(), ctx->st));
-  CUDA_TRY(ctx->ff_w.upload(w.data(), w.size(), ctx->st));
-  CUDA_TRY(ctx->ff_pw.upload(p.data(), p.size(), ctx->st));
+  CUDA_TRY(ctx->ff_cls.upload(reinterpret_cast<const char*>(C.data()), C.size() * sizeof(FFClass), ctx->st));
   CUDA_TRY(cudaStreamSynchronize(ctx->st));
   return RBC3D_OK;
 }
@@ -490,10 +561,9 @@ void self_ff_invalidate(rbc3d_ctx* ctx, bool geom, bool f, bool g) {
 // The float-float node records of the sets in `need` (bit 0 x, 1 f, 2 g,
 // 3 a3) that are out of date, on the current stream.
 rbc3d_status self_ff_records(rbc3d_ctx* ctx, int need) {
-  const long long per = (long long)ctx->m * ctx->nlon;
-  const NodeMap map = node_map(ctx->m, ctx->nlon);
-  if (!ctx->ff_rec.p || ctx->ff_rec.n < (size_t)ctx->ncell * map.per * FF_PLANES) {
-    CUDA_TRY(ctx->ff_rec.alloc((size_t)ctx->ncell * map.per * FF_PLANES));
+  const size_t per = 2 * (size_t)ctx->m * ctx->nlon * FF_ROW;  // float4 a cell
+  if (!ctx->ff_rec.p || ctx->ff_rec.n < ctx->ncell * per) {
+    CUDA_TRY(ctx->ff_rec.alloc(ctx->ncell * per));
     ctx->ff_sets = 0;
   }
   CUDA_TRY(ctx->ff_bnd.alloc(16 * (size_t)ctx->ncell));
@@ -502,9 +572,9 @@ rbc3d_status self_ff_records(rbc3d_ctx* ctx, int need) {
     for (int k = 0; k < 4; ++k)
       if (build & (1 << k))
         CUDA_TRY(cudaMemsetAsync(ctx->ff_bnd.p + 4 * (size_t)k * ctx->ncell, 0, 16 * (size_t)ctx->ncell, ctx->st));
-    { k_ff_rec<<<nblk(ctx->ncell * per, 256), 256, 0, ctx->st>>>(ctx->ncell, ctx->m, per, map, ctx->spl.p,
-                                                                  ctx->mix_xc.p, ctx->ff_rec.p, ctx->ff_bnd.p, build);
-      ++ctx->launches; }
+    const long long nb = (long long)ctx->ncell * ((ctx->m + 3) / 4) * ((ctx->nlon + 15) / 16);
+    { k_ff_rec<<<(int)nb, 128, 0, ctx->st>>>(ctx->ncell, ctx->m, ctx->nlon, ctx->spl.p, ctx->mix_xc.p,
+                                             reinterpret_cast<float*>(ctx->ff_rec.p), ctx->ff_bnd.p, build); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
     ctx->ff_sets |= build;
   }
@@ -517,31 +587,44 @@ rbc3d_status run_self_ff(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   if (!ctx->phi_uniform) return ctx_fail(ctx, RBC3D_ERR_ARG, "FP32D needs phi(j) = j*2*pi/nlon");
   const bool sl = c1 != 0 && ctx->has_f, dl = c2 != 0 && ctx->has_g;
   if (!sl && !dl) return RBC3D_OK;
-  const NodeMap map = node_map(ctx->m, ctx->nlon);
+  const int np = dl ? (sl ? 6 : 5) : 3;
+  auto smem = [&](int G) {
+    const size_t cols = (size_t)G * ctx->nlon;
+    return sizeof(float4) * FF_CHUNK * np * 2 * cols + sizeof(FFCell) * G + sizeof(float2) * 9 * cols;
+  };
+  // a ring wider than shared memory holds (about 500 columns) goes to the FP64 patch
+  if (smem(1) > 227 * 1024) return run_self_corr(ctx, tlist, sl ? c1 : 0., dl ? c2 : 0.);
   // records this call reads: x always, f for SL, g and a3 for DL
   rbc3d_status s = self_ff_records(ctx, 1 | (sl ? 2 : 0) | (dl ? 4 | 8 : 0));
   if (s) return s;
   FFArgs a;
   a.nt = t.n; a.ncell = ctx->ncell; a.nlat = ctx->nlat; a.nlon = ctx->nlon; a.m = ctx->m;
-  a.NQ = ctx->nrad * ctx->nazm; a.nrad = ctx->nrad;
   a.tA = t.Acoef.p; a.v = t.v.p; a.rec = ctx->ff_rec.p;
-  a.widx = ctx->ff_widx.p; a.w = ctx->ff_w.p; a.pw = ctx->ff_pw.p;
+  a.cls = reinterpret_cast<const FFClass*>(ctx->ff_cls.p);
   a.thi = ctx->mix_thi.p; a.tlo = ctx->mix_tlo.p; a.tab = ctx->ff_tab.p; a.celltype = ctx->celltype.p;
-  a.perm = ctx->ff_perm.p;
   a.bnd = reinterpret_cast<const uint4*>(ctx->ff_bnd.p);
-  a.map = map;
-  const double hx = RBC3D_TWO_PI / ctx->m, hy = RBC3D_TWO_PI / ctx->nlon;
-  a.hq1 = (float)(hx / 4); a.hq2 = (float)(hy / 4); a.hq12 = (float)(hx * hy / 16);
+  a.hq1 = (float)(RBC3D_TWO_PI / ctx->m / 4); a.hq2 = (float)(RBC3D_TWO_PI / ctx->nlon / 4);
   const ff z = {0.f, 0.f};
   a.c1 = sl ? hsplit(c1) : z;
   for (int l = 0; l < RBC3D_MAX_CELLTYPES; ++l) a.c2B[l] = dl ? hsplit(c2 * ctx->Bcoef[l]) : z;
   a.rc2 = hsplit(ctx->prm.rc * ctx->prm.rc);
   a.r_eps = hsplit(ctx->T.r_eps);
   a.ntab_over_rc = hsplit(ctx->T.ntab_over_rc);
-  const int grid = (int)((t.n + 7ll) / 8);  // blocks of 8 warps, one target each
-  if (sl && dl) { k_self_ff<true, true><<<grid, 256, 0, ctx->st>>>(a); ++ctx->launches; }
-  else if (sl) { k_self_ff<true, false><<<grid, 256, 0, ctx->st>>>(a); ++ctx->launches; }
-  else { k_self_ff<false, true><<<grid, 256, 0, ctx->st>>>(a); ++ctx->launches; }
-  CUDA_TRY(cudaGetLastError());
-  return RBC3D_OK;
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
+  a.NC = ctx->nrad * (ctx->nazm / 2 + 1);
+  a.G = ring_cells(ctx->ncell, ctx->nlon);
+  const int blocks = (ctx->ncell + a.G - 1) / a.G * ctx->nlat, thr = std::min(256, (a.G * ctx->nlon + 31) / 32 * 32);
+  a.parts = ring_parts(a.NC, blocks, nsm);
+  const size_t bytes = smem(a.G);
+  auto launch = [&](auto kern) -> rbc3d_status {
+    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    kern<<<blocks * a.parts, thr, bytes, ctx->st>>>(a);
+    ++ctx->launches;
+    CUDA_TRY(cudaGetLastError());
+    return RBC3D_OK;
+  };
+  if (sl && dl) return launch(k_self_ff<true, true>);
+  if (sl) return launch(k_self_ff<true, false>);
+  return launch(k_self_ff<false, true>);
 }

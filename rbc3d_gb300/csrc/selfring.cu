@@ -210,6 +210,8 @@ __global__ void __launch_bounds__(256, 1) k_self_ring(RingArgs a) {
   }
 }
 
+}  // namespace
+
 // Cells per block: the most lanes in use (full warps of columns, no empty
 // places in the last block).
 int ring_cells(int ncell, int nlon) {
@@ -223,7 +225,11 @@ int ring_cells(int ncell, int nlon) {
   return best;
 }
 
-}  // namespace
+// Under 12 blocks an SM several share a ring's classes, at least 8 each, and
+// add their sums atomically (a block's set-up costs about half a class).
+int ring_parts(int classes, int blocks, int nsm) {
+  return std::max(1, std::min(classes / 8, (12 * nsm + blocks - 1) / blocks));
+}
 
 // Classes of the patch points per latitude: the points (irad, ia) and (irad,
 // nazm - ia), in the order of their spline rows.
@@ -308,9 +314,7 @@ rbc3d_status run_self_ring(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   a.NC = ctx->nrad * (ctx->nazm / 2 + 1);
   a.G = ring_cells(ctx->ncell, ctx->nlon);
   const int blocks = (ctx->ncell + a.G - 1) / a.G * ctx->nlat, thr = (a.G * ctx->nlon + 31) / 32 * 32;
-  // under 12 blocks an SM several share a ring's classes, at least 8 each, and
-  // add their sums atomically (a block's set-up costs about half a class)
-  a.parts = std::max(1, std::min(a.NC / 8, (12 * nsm + blocks - 1) / blocks));
+  a.parts = ring_parts(a.NC, blocks, nsm);
   a.rec = ctx->ring_rec.p; a.cls = reinterpret_cast<const RingClass*>(ctx->ring_cls.p); a.spl = ctx->spl.p;
   a.th = ctx->th.p; a.phi = ctx->phi.p; a.tA = t.Acoef.p; a.v = t.v.p; a.celltype = ctx->celltype.p; a.Bc = ctx->dBcoef.p;
   a.tab = ctx->ring_tab.p;

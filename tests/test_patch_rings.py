@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from rbc3d_gb300 import geometry as G
-from rbc3d_gb300.abi import FP64, TERM_CORR, TLIST_RBC, Context
+from rbc3d_gb300.abi import FP32D, FP64, TERM_CORR, TERM_LINEAR, TERM_REAL, TLIST_RBC, Context
 
 pytestmark = pytest.mark.gpu
 C = 1 / (4 * math.pi)
@@ -27,10 +27,15 @@ def test_ring_patch_matches_oracle(gpu, oracle, nlat, nlon, ncell):
         c.set_cells(cells)
         c.set_cell_density(f=cells.f, g=cells.g, spl_F=cells.spl_F, spl_G=cells.spl_G)
         ctx.append(c)
-    # rounding: the separation of the first radial ring (about 0.01) is a
-    # difference of positions up to 14, 2e-16 x 14 / 0.01 = 3e-13; the sums differ in order only
+    # FP64: the separation of the first radial ring (about 0.01) is a difference
+    # of positions up to 14, 2e-16 x 14 / 0.01 = 3e-13; the sums differ in order
+    # only.  FP32D: interpolated positions to about 2^-47 of 1.4, 1e-14 / 0.005 =
+    # 2e-12 a point on the finest grid, and the table position to 2^-47 x 8192 steps
     for c1, c2 in ((C, C), (C, 0.0), (0.0, C)):
-        ref, out = (c.matvec(TLIST_RBC, c1, c2, TERM_CORR, FP64) for c in ctx)
+        real = TERM_REAL | TERM_CORR | TERM_LINEAR  # the oracle evaluates the three together
+        ref, out = (c.matvec(TLIST_RBC, c1, c2, real, FP64) for c in ctx)
         assert np.linalg.norm(out - ref) <= 1e-11 * np.linalg.norm(ref), (c1, c2)
+        ref, out = (ctx[1].matvec(TLIST_RBC, c1, c2, TERM_CORR, prec) for prec in (FP64, FP32D))
+        assert np.linalg.norm(out - ref) <= 2e-11 * np.linalg.norm(ref), (c1, c2)
     for c in ctx:
         c.close()
