@@ -7,19 +7,18 @@
 // significant bits):
 //   * the Spline_Interp sums are compensated dot products (Ogita, Rump and
 //     Oishi, "Accurate sum and dot product", SIAM J. Sci. Comput. 26, 2005):
-//     each product w v split exactly by the FMA form of TwoProduct, the high
-//     parts summed error-free, the rounding errors and the lo-part cross
-//     terms summed in FP32.  The sums start from a power of two `off` at
+//     the high parts summed error-free, the rounding errors and the lo-part
+//     cross terms summed in FP32.  The sums start from a power of two `off` at
 //     least twice a bound on their sum of |w v| (the per-cell maxima of the
-//     node values times the weight-sum bounds 1, h/4 and h^2/16), so every
-//     partial sum stays above every product in magnitude and Dekker's
-//     FastTwoSum (3 operations) is exact where Knuth's TwoSum takes 6; off
-//     is subtracted exactly at the end.  The FP32 correction term is rounded
+//     node values times the weight-sum bounds 1 and h/4), so every partial sum
+//     stays above every product in magnitude and one fused multiply-add takes
+//     the place of product and sum with a recoverable error (Dot2); off is
+//     subtracted exactly at the end.  The FP32 correction term is rounded
 //     on the scale of off, so for the position x, whose interpolant is
-//     differenced against the target, the bound covers the 12 derivative
-//     terms only: off is subtracted before the 4 value terms, which are
-//     added with TwoSum (all 16 from the larger offset: the corrections
-//     move from 2.3e-12 to 2.3e-11 of the FP64 patch);
+//     differenced against the target, the bound covers the derivative terms
+//     only: off is subtracted before the value terms, which are added with
+//     Knuth's TwoSum (all from the larger offset: the corrections move from
+//     2.3e-12 to 2.3e-11 of the FP64 patch);
 //   * the Ewald kernel (EwaldCoeff_SL / _DL, ModEwaldFunc.F90:86-180, the
 //     same tables as hi/lo) is evaluated with Dekker's float-float product
 //     and sum, and 1/r by rsqrtf, an FP32 Newton step and a float-float
@@ -32,10 +31,14 @@
 // targets share their colatitudes and pair up about the meridian, so per point
 // pair (class) and column j the theta part U_j, D_j (4 terms each) is computed
 // once for the ring, and a point takes the 4 terms of the phi part from the
-// columns j and j + 1.  About 500 packed instructions of interpolation a point
-// against 900 with 16 terms, and 0.4 KB of loads against 1.7 KB.  256 cells,
-// SL+DL: 6.5 -> 4.8 ms against one warp per target, the FP32D matvec 10.66 -> 8.89.
-//
+// columns j and j + 1; the two points of a class run as the halves of packed
+// FP32x2 operations.  256 cells, SL+DL: 6.5 -> 3.5 ms against one warp per
+// target with 16-term sums (the FP32D matvec 10.63 -> 7.62 ms); of that 4.8 ->
+// 3.9 by loading a quad's U and D slots in turn (32 registers of node values
+// instead of 64, no spills), -> 3.5 by the fused 6-operation sums (Dot2).
+// ncu at 64 cells: FMA pipe 56%, L1 data pipe 56%, issue 44% at 16 warps an
+// SM (registers); measured and not kept: three blocks an SM (80 registers,
+// spills: 3.8), two classes between barriers (3.9 against 3.9), loads past L1.
 // Data layout.  Per row i and slot d (u, u_th, u_ph, u_thph) the 12 values x
 // (relative to the cell centre), f and g density sets and a3 (three
 // components each) are stored as three quads in column order; a quad's hi and
@@ -53,16 +56,14 @@
 namespace {
 
 constexpr int FF_ROW = 12;   // 32-byte entries of a node: 4 slots x 3 quads
-constexpr int FF_CHUNK = 2;  // classes between two barriers: the rows' entries are loaded once for both
 
 // A class of patch points (RingClass) in hi/lo parts, each weight as the
 // operands (h, h, l, l): the theta weights of (u, u', u_th, u'_th), per side
 // the phi weights of (U_j, U_j+1, D_j, D_j+1).
 struct FFClass {
   int i1, j[2], pad;
-  float4 x[4], y[2][4];
-  float2 w, pad2;
-};
+  float4 x[4], y[2][4], w;  // w: quadrature weights (h, l) of the sides; a point without mirror image stands
+};                          // on both sides, with weight 0 on the second
 static_assert(sizeof(FFClass) % 16 == 0, "vector loads of the weights");
 
 // ---------------------------------------------------------------------------
@@ -70,47 +71,12 @@ static_assert(sizeof(FFClass) % 16 == 0, "vector loads of the weights");
 struct ff {
   float h, l;
 };
-__device__ __forceinline__ ff two_sum(float a, float b) {
-  const float s = __fadd_rn(a, b);
-  const float bb = __fsub_rn(s, a);
-  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
-}
-__device__ __forceinline__ ff fast_two_sum(float a, float b) {  // |a| >= |b| or a == 0
-  const float s = __fadd_rn(a, b);
-  return {s, __fsub_rn(b, __fsub_rn(s, a))};
-}
-__device__ __forceinline__ ff ff_norm(ff a) { return fast_two_sum(a.h, a.l); }
-__device__ __forceinline__ ff ff_add(ff a, ff b) {
-  ff s = two_sum(a.h, b.h);
-  return fast_two_sum(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
-}
-__device__ __forceinline__ ff ff_sub(ff a, ff b) {
-  ff s = two_sum(a.h, -b.h);
-  return fast_two_sum(s.h, __fadd_rn(s.l, __fsub_rn(a.l, b.l)));
-}
-// product without the final renormalisation: |l| stays ~2^-23 |h|
-__device__ __forceinline__ ff ff_mul(ff a, ff b) {
-  const float p = __fmul_rn(a.h, b.h);
-  float e = fmaf(a.h, b.h, -p);
-  e = fmaf(a.h, b.l, e);
-  e = fmaf(a.l, b.h, e);
-  return {p, e};
-}
 __device__ __forceinline__ bool ff_ge(ff a, ff b) { return a.h > b.h || (a.h == b.h && a.l >= b.l); }
-
-// lazy accumulator: hi parts summed exactly, errors and lo parts in FP32
-struct ffacc {
-  float s, c;
-  __device__ __forceinline__ void add(ff v) {
-    const ff t = two_sum(s, v.h);
-    s = t.h;
-    c = __fadd_rn(c, __fadd_rn(t.l, v.l));
-  }
-};
 
 // one 32-byte read-only load (hi quad, lo quad of one node)
 __device__ __forceinline__ void ld8(const float4* p, float4& h, float4& l) {
   asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+
       : "=f"(h.x), "=f"(h.y), "=f"(h.z), "=f"(h.w), "=f"(l.x), "=f"(l.y), "=f"(l.z), "=f"(l.w)
       : "l"(p));
 }
@@ -124,32 +90,33 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
   return *reinterpret_cast<float2*>(&d);
 }
 
-// Compensated dot-product accumulator for two values sharing a weight.
+// Compensated dot-product accumulator for two values sharing a weight:
+// s + c += w v with the weight's stored operands (h, h, l, l).
 struct Dot2 {
   float2 s, c;
-  // s + c += w * v with w = (wh, wl), v = (vh, vl) per half; nwh = -wh.
-  // FAST: s has been kept above every product in magnitude (FastTwoSum)
-  template <bool FAST>
-  __device__ __forceinline__ void add(float2 wh, float2 nwh, float2 wl, float2 vh, float2 vl) {
-    const float2 p = __fmul2_rn(wh, vh);
-    const float2 ne = __ffma2_rn(nwh, vh, p);  // p - wh vh: minus the product's rounding error
-    const float2 t = __fadd2_rn(s, p);
-    float2 err;
-    if (FAST) {
-      err = sub2(p, sub2(t, s));
-    } else {
-      const float2 bb = sub2(t, s);
-      err = __fadd2_rn(sub2(s, sub2(t, bb)), sub2(p, bb));
-    }
-    s = t;
-    c = __ffma2_rn(wh, vl, c);
-    c = __ffma2_rn(wl, vh, c);
-    c = __fadd2_rn(c, sub2(err, ne));
-  }
-  // FAST with the weight's stored operands (h, h, l, l)
+  // FAST: s has been kept at off/2 .. 3 off/2 with |w v| <= off/2, so the fused
+  // t = RN(s + wh vh) leaves t - s exact, and wh vh - (t - s), rounded once, is
+  // what t lost: 6 operations where a separate product and FastTwoSum take 9
   template <bool FAST>
   __device__ __forceinline__ void add(float4 w, float2 vh, float2 vl) {
-    add<FAST>(make_float2(w.x, w.y), make_float2(-w.x, -w.y), make_float2(w.z, w.w), vh, vl);
+    const float2 wh = make_float2(w.x, w.y), wl = make_float2(w.z, w.w);
+    if (FAST) {
+      const float2 t = __ffma2_rn(wh, vh, s);
+      const float2 lost = __ffma2_rn(wh, vh, sub2(s, t));
+      s = t;
+      c = __ffma2_rn(wh, vl, c);
+      c = __ffma2_rn(wl, vh, c);
+      c = __fadd2_rn(c, lost);
+    } else {
+      const float2 np = __fmul2_rn(make_float2(-w.x, -w.y), vh);  // minus the product
+      const float2 e = __ffma2_rn(wh, vh, np);
+      const float2 t = sub2(s, np), bb = sub2(t, s);
+      const float2 err = sub2(sub2(s, sub2(t, bb)), __fadd2_rn(np, bb));
+      s = t;
+      c = __ffma2_rn(wh, vl, c);
+      c = __ffma2_rn(wl, vh, c);
+      c = __fadd2_rn(c, __fadd2_rn(err, e));
+    }
   }
 };
 
@@ -161,7 +128,7 @@ struct FFArgs {
   const FFClass* cls;   // [latitude][NC]
   const float4* thi;    // target positions relative to the cell centre, hi
   const float4* tlo;    // and lo
-  const float4* tab;    // [3][EWALD_NTAB]: {T_i hi, T_i lo, (T_i+1 - T_i) hi, lo}
+  const float4* tab;    // [EWALD_NTAB][3]: {T_i hi, T_i lo, (T_i+1 - T_i) hi, lo}
   const uint4* bnd;     // [set x f g a3][cell]: max |u|, |u_th|, |u_ph|, |u_thph| (float bits)
   float hq1, hq2;       // derivative weight-sum bounds: h_th / 4, h_ph / 4
   const int* celltype;
@@ -170,16 +137,53 @@ struct FFArgs {
   ff rc2, r_eps, ntab_over_rc;
 };
 
-__device__ __forceinline__ ff ld_ff(float2 v) { return {v.x, v.y}; }
-
-// T + D f1 for table t at index it
-__device__ __forceinline__ ff tab_lerp(const float4* tab, int t, int it, ff f1) {
-  const float4 e = __ldg(tab + (size_t)t * EWALD_NTAB + it);
-  return ff_add({e.x, e.y}, ff_mul({e.z, e.w}, f1));
+// float-float arithmetic on two points at once (packed FP32x2)
+struct ff2 {
+  float2 h, l;
+};
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ ff2 two_sum2(float2 a, float2 b) {
+  const float2 s = __fadd2_rn(a, b), bb = sub2(s, a);
+  return {s, __fadd2_rn(sub2(a, sub2(s, bb)), sub2(b, bb))};
 }
-
-__device__ __forceinline__ ff dot3(const ff* a, const ff* b) {
-  return ff_add(ff_add(ff_mul(a[0], b[0]), ff_mul(a[1], b[1])), ff_mul(a[2], b[2]));
+__device__ __forceinline__ ff2 fast_two_sum2(float2 a, float2 b) {  // |a| >= |b| or a == 0, per half
+  const float2 s = __fadd2_rn(a, b);
+  return {s, sub2(b, sub2(s, a))};
+}
+// a + b without the final renormalisation
+__device__ __forceinline__ ff2 add2(ff2 a, ff2 b) {
+  const ff2 s = two_sum2(a.h, b.h);
+  return {s.h, __fadd2_rn(s.l, __fadd2_rn(a.l, b.l))};
+}
+// product without the final renormalisation: |l| stays ~2^-23 |h|
+__device__ __forceinline__ ff2 mul2(ff2 a, ff2 b) {
+  const float2 p = __fmul2_rn(a.h, b.h);
+  float2 e = __ffma2_rn(a.h, b.h, neg2(p));
+  e = __ffma2_rn(a.h, b.l, e);
+  e = __ffma2_rn(a.l, b.h, e);
+  return {p, e};
+}
+// compensated dot product, not renormalised
+__device__ __forceinline__ ff2 dot3(const ff2* a, const ff2* b) {
+  ff2 r = mul2(a[0], b[0]);
+#pragma unroll
+  for (int k = 1; k < 3; ++k) {
+    const float2 p = __fmul2_rn(a[k].h, b[k].h), e = __ffma2_rn(a[k].h, b[k].h, neg2(p));
+    const ff2 t = two_sum2(r.h, p);
+    r.h = t.h;
+    r.l = __ffma2_rn(a[k].h, b[k].l, r.l);
+    r.l = __ffma2_rn(a[k].l, b[k].h, r.l);
+    r.l = __fadd2_rn(r.l, __fadd2_rn(t.l, e));
+  }
+  return r;
+}
+__device__ __forceinline__ ff2 both(ff a) { return {make_float2(a.h, a.h), make_float2(a.l, a.l)}; }
+// T + D f1 for table t at the indices ia, ib (|D f1| <= |T|), not renormalised
+__device__ __forceinline__ ff2 tab_lerp(const float4* tab, int t, int ia, int ib, ff2 f1) {
+  const float4 a = __ldg(tab + 3 * ia + t), b = __ldg(tab + 3 * ib + t);
+  const ff2 p = mul2({make_float2(a.z, b.z), make_float2(a.w, b.w)}, f1);
+  const ff2 r = fast_two_sum2(make_float2(a.x, b.x), p.h);
+  return {r.h, __fadd2_rn(r.l, __fadd2_rn(make_float2(a.y, b.y), p.l))};
 }
 
 // The pairs of values: (x.x x.y) (x.z f.x) (f.y f.z) (g.x g.y) (g.z a.x) (a.y a.z),
@@ -227,89 +231,116 @@ __device__ __forceinline__ void cell_offsets(const FFArgs& a, int cell, FFCell& 
 __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
 
-// RBC_SingInt's loop body at interpolated values v (s and c of the 6 pairs)
-// for a target at xi: c1 and c2 terms added to the sums acc (stride st).
+__device__ __forceinline__ ff2 vx(const Dot2& a, const Dot2& b) {
+  return {make_float2(a.s.x, b.s.x), make_float2(a.c.x, b.c.x)};
+}
+__device__ __forceinline__ ff2 vy(const Dot2& a, const Dot2& b) {
+  return {make_float2(a.s.y, b.s.y), make_float2(a.c.y, b.c.y)};
+}
+__device__ __forceinline__ ff2 norm2(ff2 a) { return fast_two_sum2(a.h, a.l); }
+// v - t for the targets' positions ta, tb (h, l)
+__device__ __forceinline__ ff2 from_target(ff2 v, float2 ta, float2 tb) {
+  v = norm2(v);
+  const ff2 s = two_sum2(v.h, make_float2(-ta.x, -tb.x));
+  return fast_two_sum2(s.h, __fadd2_rn(s.l, sub2(v.l, make_float2(ta.y, tb.y))));
+}
+// whether a patch point at squared distance (h, l) counts: not rr >= rc
+// (ModRbcSingInt.F90:65), not zero, not NaN
+__device__ __forceinline__ bool in_range(const FFArgs& a, float h, float l) {
+  return h > 0.f && (h < a.rc2.h || (h == a.rc2.h && l < a.rc2.l));
+}
+__device__ __forceinline__ int table_index(float h, float l) {
+  const float fi = floorf(h);
+  return (int)(h == fi && l < 0.f ? fi - 1.f : fi);
+}
+
+// RBC_SingInt's loop body for the two points of a class, interpolated values
+// A and B (s and c of the 6 pairs): their c1 and c2 terms added to the sums
+// accA and accB (stride st) of the targets at tA and tB (stride st).
 template <bool SL, bool DL>
-__device__ __forceinline__ void patch_point(const FFArgs& a, const Dot2* d2, const ff* xi, ff c2m, ff wq, float2* acc,
-                                            int st) {
-  ff xx[3], F[3], G[3], A[3];
-  xx[0] = ff_sub(fast_two_sum(d2[0].s.x, d2[0].c.x), xi[0]);
-  xx[1] = ff_sub(fast_two_sum(d2[0].s.y, d2[0].c.y), xi[1]);
-  xx[2] = ff_sub(fast_two_sum(d2[1].s.x, d2[1].c.x), xi[2]);
-  if (SL) {
-    F[0] = fast_two_sum(d2[1].s.y, d2[1].c.y);
-    F[1] = fast_two_sum(d2[2].s.x, d2[2].c.x);
-    F[2] = fast_two_sum(d2[2].s.y, d2[2].c.y);
-  }
+__device__ __forceinline__ void patch_points(const FFArgs& a, const Dot2* A, const Dot2* B, const float2* tA,
+                                             const float2* tB, ff c2m, float4 wq, float2* accA, float2* accB, int st) {
+  ff2 xx[3], F[3], Gv[3], N[3];
+  xx[0] = from_target(vx(A[0], B[0]), tA[0], tB[0]);
+  xx[1] = from_target(vy(A[0], B[0]), tA[st], tB[st]);
+  xx[2] = from_target(vx(A[1], B[1]), tA[2 * st], tB[2 * st]);
+  if (SL) { F[0] = vy(A[1], B[1]); F[1] = vx(A[2], B[2]); F[2] = vy(A[2], B[2]); }
   if (DL) {
-    G[0] = fast_two_sum(d2[3].s.x, d2[3].c.x);
-    G[1] = fast_two_sum(d2[3].s.y, d2[3].c.y);
-    G[2] = fast_two_sum(d2[4].s.x, d2[4].c.x);
-    A[0] = fast_two_sum(d2[4].s.y, d2[4].c.y);
-    A[1] = fast_two_sum(d2[5].s.x, d2[5].c.x);
-    A[2] = fast_two_sum(d2[5].s.y, d2[5].c.y);
+    Gv[0] = vx(A[3], B[3]); Gv[1] = vy(A[3], B[3]); Gv[2] = vx(A[4], B[4]);
+    // xx . a3 cancels to the surface's curvature times r^2: normalised
+    N[0] = norm2(vy(A[4], B[4])); N[1] = norm2(vx(A[5], B[5])); N[2] = norm2(vy(A[5], B[5]));
   }
-  const ff r2 = ff_add(ff_add(ff_mul(xx[0], xx[0]), ff_mul(xx[1], xx[1])), ff_mul(xx[2], xx[2]));
-  if (ff_ge(r2, a.rc2)) return;  // rr >= rc (ModRbcSingInt.F90:65)
-  if (!(r2.h > 0.f)) return;
+  ff2 r2 = norm2(dot3(xx, xx));
+  bool oka = in_range(a, r2.h.x, r2.l.x), okb = in_range(a, r2.h.y, r2.l.y);
+  r2.h = make_float2(oka ? r2.h.x : 1.f, okb ? r2.h.y : 1.f);
+  r2.l = make_float2(oka ? r2.l.x : 0.f, okb ? r2.l.y : 0.f);
   // 1/r: rsqrtf, an FP32 Newton step, a float-float Newton step
-  float y = rsqrtf(r2.h);
-  y = y * fmaf(-0.5f * r2.h, y * y, 1.5f);
-  const float y2 = __fmul_rn(y, y), y2e = fmaf(y, y, -y2);
-  const float t0 = __fmul_rn(r2.h, y2);
-  const float t1 = fmaf(r2.h, y2, -t0) + fmaf(r2.h, y2e, r2.l * y2);
-  const float eps = __fsub_rn(__fsub_rn(1.f, t0), t1);  // 1 - r2 y^2
-  const ff ir = fast_two_sum(y, 0.5f * y * eps);
-  const ff rv = ff_norm(ff_mul(r2, ir));
-  // EwaldCoeff_SL / _DL share the table position; below r_eps or beyond
-  // the table both are zero
-  if (!ff_ge(rv, a.r_eps)) return;
-  const ff sp = ff_norm(ff_mul(rv, a.ntab_over_rc));
-  float fi = floorf(sp.h);
-  if (sp.h == fi && sp.l < 0.f) fi -= 1.f;
-  const int it = (int)fi;
-  if (it < 0 || it >= EWALD_NTAB) return;
-  const ff f1 = two_sum(__fsub_rn(sp.h, fi), sp.l);
-  const ff ir2 = ff_mul(ir, ir);
-  ff cx = {0.f, 0.f}, cf = {0.f, 0.f};  // dv += cx xx + cf f
+  const float2 half = make_float2(0.5f, 0.5f);
+  float2 y = make_float2(rsqrtf(r2.h.x), rsqrtf(r2.h.y));
+  const float2 hr = __fmul2_rn(make_float2(-0.5f, -0.5f), r2.h);
+  y = __fmul2_rn(y, __ffma2_rn(hr, __fmul2_rn(y, y), make_float2(1.5f, 1.5f)));
+  const float2 y2 = __fmul2_rn(y, y), y2e = __ffma2_rn(y, y, neg2(y2));
+  const float2 t0 = __fmul2_rn(r2.h, y2);
+  const float2 t1 = __fadd2_rn(__ffma2_rn(r2.h, y2, neg2(t0)), __ffma2_rn(r2.h, y2e, __fmul2_rn(r2.l, y2)));
+  const float2 eps = sub2(sub2(make_float2(1.f, 1.f), t0), t1);  // 1 - r2 y^2
+  const ff2 ir = fast_two_sum2(y, __fmul2_rn(__fmul2_rn(half, y), eps));
+  const ff2 rv = norm2(mul2(r2, ir));
+  // EwaldCoeff_SL / _DL share the table position; below r_eps or beyond the
+  // table both are zero
+  const ff2 sp = norm2(mul2(rv, both(a.ntab_over_rc)));
+  const int ia = table_index(sp.h.x, sp.l.x), ib = table_index(sp.h.y, sp.l.y);
+  oka = oka && ff_ge({rv.h.x, rv.l.x}, a.r_eps) && (unsigned)ia < (unsigned)EWALD_NTAB;
+  okb = okb && ff_ge({rv.h.y, rv.l.y}, a.r_eps) && (unsigned)ib < (unsigned)EWALD_NTAB;
+  const int ja = oka ? ia : 0, jb = okb ? ib : 0;
+  // sp.h - ia is 0 or at least an ulp of sp.h
+  const ff2 f1 = fast_two_sum2(sub2(sp.h, make_float2((float)ia, (float)ib)), sp.l);
+  const ff2 ir2 = mul2(ir, ir);
+  const ff2 w = {make_float2(wq.x, wq.z), make_float2(wq.y, wq.w)};
+  ff2 cx, cf;  // dv += cx xx + cf f
   if (SL) {
-    const ff cs1 = tab_lerp(a.tab, 0, it, f1), cs2 = tab_lerp(a.tab, 1, it, f1);
-    const ff c1ir = ff_mul(cs1, ir);
-    const ff EA = ff_mul(ff_add(c1ir, cs2), ir2), EB = ff_sub(c1ir, cs2);
+    const ff2 cs1 = tab_lerp(a.tab, 0, ja, jb, f1), cs2 = tab_lerp(a.tab, 1, ja, jb, f1);
+    const ff2 c1ir = mul2(cs1, ir);
+    const ff2 EA = mul2(add2(c1ir, cs2), ir2), EB = add2(c1ir, {neg2(cs2.h), neg2(cs2.l)});
     // c1 wq (EA xx (xx . f) + EB f)
-    const ff sw = ff_mul(a.c1, wq);
-    cx = ff_mul(sw, ff_mul(EA, dot3(xx, F)));
-    cf = ff_mul(sw, EB);
+    const ff2 sw = mul2(both(a.c1), w);
+    cx = mul2(sw, mul2(EA, dot3(xx, F)));
+    cf = mul2(sw, EB);
   }
   if (DL) {
     // c2 Bcoef wq EA xx (xx . g)(xx . a3), EA = cd / r^5
-    const ff cd = tab_lerp(a.tab, 2, it, f1);
-    const ff EA = ff_mul(cd, ff_mul(ir2, ff_mul(ir2, ir)));
-    const ff t = ff_mul(ff_mul(ff_mul(c2m, wq), EA), ff_mul(dot3(xx, G), dot3(xx, A)));
-    cx = SL ? ff_add(cx, t) : t;
+    const ff2 cd = tab_lerp(a.tab, 2, ja, jb, f1);
+    const ff2 EA = mul2(cd, mul2(ir2, mul2(ir2, ir)));
+    const ff2 t = mul2(mul2(mul2(both(c2m), w), EA), mul2(dot3(xx, Gv), dot3(xx, N)));
+    cx = SL ? add2(cx, t) : t;
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const float2 z = acc[k * st];
-    ffacc s = {z.x, z.y};
-    s.add(ff_mul(cx, xx[k]));
-    if (SL) s.add(ff_mul(cf, F[k]));
-    acc[k * st] = make_float2(s.s, s.c);
+    const float2 za = accA[k * st], zb = accB[k * st];
+    ff2 v = mul2(cx, xx[k]);
+    ff2 s = two_sum2(make_float2(za.x, zb.x), v.h);
+    float2 c = __fadd2_rn(make_float2(za.y, zb.y), __fadd2_rn(s.l, v.l));
+    if (SL) {
+      v = mul2(cf, F[k]);
+      s = two_sum2(s.h, v.h);
+      c = __fadd2_rn(c, __fadd2_rn(s.l, v.l));
+    }
+    if (oka) accA[k * st] = make_float2(s.h.x, c.x);
+    if (okb) accB[k * st] = make_float2(s.h.y, c.y);
   }
 }
 
 // One block: a ring of G cells, thread = column (cols = G nlon; more than 256
-// columns: several a thread).  Per chunk of FF_CHUNK classes the theta parts
-// go to shared memory, then every column evaluates the points in the interval
-// [j, j + 1]: of the targets j - j[0] and j - j[1] (mod nlon), whose sums lie
-// in shared memory, a side each, so no two threads meet between two barriers.
+// columns: several a thread).  Per class the theta parts go to shared memory,
+// then every column evaluates the points in the interval [j, j + 1]: of the
+// targets j - j[0] and j - j[1] (mod nlon), whose sums lie in shared memory, a
+// side each, so no two threads meet between two barriers.
 template <bool SL, bool DL>
 __global__ void __launch_bounds__(256, 2) k_self_ff(FFArgs a) {
   constexpr int NP = DL ? (SL ? 6 : 5) : 3;  // pairs kept; without SL the pair (f.y f.z) is left out
   extern __shared__ __align__(16) unsigned char smem_ff[];
   const int nlon = a.nlon, cols = a.G * nlon;
-  float4* ex = reinterpret_cast<float4*>(smem_ff);            // [FF_CHUNK][NP][U, D][cols]: (s, s, c, c)
-  FFCell* sC = reinterpret_cast<FFCell*>(ex + (size_t)FF_CHUNK * NP * 2 * cols);  // [G]
+  float4* ex = reinterpret_cast<float4*>(smem_ff);            // [2][NP][U, D][cols]: (s, s, c, c)
+  FFCell* sC = reinterpret_cast<FFCell*>(ex + (size_t)4 * NP * cols);  // [G]
   float2* acc = reinterpret_cast<float2*>(sC + a.G);          // [2 sides][3][cols]
   float2* sT = acc + 6 * cols;                                // [3][cols] target positions
   int b = blockIdx.x;
@@ -327,107 +358,89 @@ __global__ void __launch_bounds__(256, 2) k_self_ff(FFArgs a) {
   __syncthreads();
   const int k0 = (int)((long long)a.NC * part / a.parts), k1 = (int)((long long)a.NC * (part + 1) / a.parts);
   const FFClass* cls = a.cls + (size_t)ring * a.NC;
-  for (int kb = k0; kb < k1; kb += FF_CHUNK) {
+  for (int k = k0; k < k1; ++k) {
+    const FFClass& c = cls[k];
+    float4* buf = ex + (size_t)((k & 1) * NP * 2) * cols;
+    const int i1 = c.i1, i2 = i1 + 1 == a.m ? 0 : i1 + 1;
     for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
       const int lc = t / nlon, j = t - lc * nlon;
       const FFCell& C = sC[lc];
       const float4* rc = a.rec + 2 * ((size_t)(cell0 + lc) * a.m * FF_ROW * nlon + j);
+      const float4 w0 = __ldg(c.x), w1 = __ldg(c.x + 1), w2 = __ldg(c.x + 2), w3 = __ldg(c.x + 3);
 #pragma unroll
-      for (int q = 0; q < (DL ? 3 : 2); ++q) {
-        float4 rh[8], rl[8];  // row i1: slots 0..3, row i1 + 1: slots 0..3
-        int have = -1;
+      for (int qh = 0; qh < (DL ? 6 : 4); ++qh) {
+        const int q = qh >> 1, h = qh & 1;  // quad; 0: U from the slots u, u_th, 1: D from u_ph, u_thph
+        float4 rh[4], rl[4];                // slots 2h, 2h + 1 of row i1, then of row i2
 #pragma unroll
-        for (int kk = 0; kk < FF_CHUNK; ++kk) {
-          if (kb + kk >= k1) break;
-          const FFClass& c = cls[kb + kk];
-          if (c.i1 != have) {
-            have = c.i1;
-            const int i2 = have + 1 == a.m ? 0 : have + 1;
+        for (int d = 0; d < 2; ++d) {
+          ld8(rc + 2 * (size_t)((i1 * FF_ROW + 3 * (2 * h + d) + q) * nlon), rh[d], rl[d]);
+          ld8(rc + 2 * (size_t)((i2 * FF_ROW + 3 * (2 * h + d) + q) * nlon), rh[2 + d], rl[2 + d]);
+        }
 #pragma unroll
-            for (int d = 0; d < 4; ++d) {
-              ld8(rc + 2 * (size_t)((have * FF_ROW + 3 * d + q) * nlon), rh[d], rl[d]);
-              ld8(rc + 2 * (size_t)((i2 * FF_ROW + 3 * d + q) * nlon), rh[4 + d], rl[4 + d]);
-            }
+        for (int e = 0; e < 2; ++e) {
+          const int P = 2 * q + e;
+          if ((!DL && P >= 3) || (!SL && P == 2)) continue;
+          const int S = (!SL && P > 2) ? P - 1 : P;
+          auto vh = [&](int i) { return e ? hi2(rh[i]) : lo2(rh[i]); };
+          auto vl = [&](int i) { return e ? hi2(rl[i]) : lo2(rl[i]); };
+          const float2 off = h ? C.d[P] : C.u[P];
+          Dot2 d;
+          d.s = off; d.c = make_float2(0.f, 0.f);
+          d.add<true>(w2, vh(1), vl(1));
+          d.add<true>(w3, vh(3), vl(3));
+          if (h == 0 && P < FF_XPAIRS) {  // off/2 <= s <= 3 off/2: the subtraction is exact
+            d.s = sub2(d.s, off);
+            d.add<false>(w0, vh(0), vl(0));
+            d.add<false>(w1, vh(2), vl(2));
+          } else {
+            d.add<true>(w0, vh(0), vl(0));
+            d.add<true>(w1, vh(2), vl(2));
+            d.s = sub2(d.s, off);
           }
-          const float4 w0 = __ldg(c.x), w1 = __ldg(c.x + 1), w2 = __ldg(c.x + 2), w3 = __ldg(c.x + 3);
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int P = 2 * q + e;
-            if ((!DL && P >= 3) || (!SL && P == 2)) continue;
-            const int S = (!SL && P > 2) ? P - 1 : P;
-            auto vh = [&](int i) { return e ? hi2(rh[i]) : lo2(rh[i]); };
-            auto vl = [&](int i) { return e ? hi2(rl[i]) : lo2(rl[i]); };
-            Dot2 U, D;
-            const float2 ou = C.u[P], od = C.d[P];
-            U.s = ou; U.c = make_float2(0.f, 0.f);
-            U.add<true>(w2, vh(1), vl(1));
-            U.add<true>(w3, vh(5), vl(5));
-            if (P < FF_XPAIRS) {  // off/2 <= s <= 3 off/2: the subtraction is exact
-              U.s = sub2(U.s, ou);
-              U.add<false>(w0, vh(0), vl(0));
-              U.add<false>(w1, vh(4), vl(4));
-            } else {
-              U.add<true>(w0, vh(0), vl(0));
-              U.add<true>(w1, vh(4), vl(4));
-              U.s = sub2(U.s, ou);
-            }
-            D.s = od; D.c = make_float2(0.f, 0.f);
-            D.add<true>(w2, vh(3), vl(3));
-            D.add<true>(w3, vh(7), vl(7));
-            D.add<true>(w0, vh(2), vl(2));
-            D.add<true>(w1, vh(6), vl(6));
-            D.s = sub2(D.s, od);
-            float4* o = ex + (size_t)((kk * NP + S) * 2) * cols + t;
-            o[0] = make_float4(U.s.x, U.s.y, U.c.x, U.c.y);
-            o[cols] = make_float4(D.s.x, D.s.y, D.c.x, D.c.y);
-          }
+          buf[(size_t)(2 * S + h) * cols + t] = make_float4(d.s.x, d.s.y, d.c.x, d.c.y);
         }
       }
     }
+    // one barrier a class: the next class's values go to the other buffer, and
+    // nobody is past this barrier before the previous class's sums are in
     __syncthreads();
-#pragma unroll 1
-    for (int kk = 0; kk < FF_CHUNK && kb + kk < k1; ++kk) {
-      const FFClass& c = cls[kb + kk];
-      for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
-        const int lc = t / nlon, j = t - lc * nlon, base = t - j;
-        const int tn = j + 1 == nlon ? base : t + 1;
-        const FFCell& C = sC[lc];
-#pragma unroll 1
+    for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
+      const int lc = t / nlon, j = t - lc * nlon, base = t - j;
+      const int tn = j + 1 == nlon ? base : t + 1;
+      const FFCell& C = sC[lc];
+      const int qa = base + (j >= c.j[0] ? j - c.j[0] : j - c.j[0] + nlon);  // the targets' columns
+      const int qb = base + (j >= c.j[1] ? j - c.j[1] : j - c.j[1] + nlon);
+      Dot2 da[FF_PAIRS], db[FF_PAIRS];
+#pragma unroll
+      for (int P = 0; P < FF_PAIRS; ++P) {
+        if ((!DL && P >= 3) || (!SL && P == 2)) continue;
+        const int S = (!SL && P > 2) ? P - 1 : P;
+        const float4* o = buf + (size_t)(2 * S) * cols;
+        const float4 D0 = o[cols + t], D1 = o[cols + tn], U0 = o[t], U1 = o[tn];
+        const float2 off = C.p[P];
+#pragma unroll
         for (int side = 0; side < 2; ++side) {
-          const int js = c.j[side];
-          if (js < 0) break;  // the points on the meridian have no mirror image
-          const int q = base + (j >= js ? j - js : j - js + nlon);  // the target's column
           const float4* y = c.y[side];
           const float4 w0 = __ldg(y), w1 = __ldg(y + 1), w2 = __ldg(y + 2), w3 = __ldg(y + 3);
-          Dot2 d2[FF_PAIRS];
-#pragma unroll
-          for (int P = 0; P < FF_PAIRS; ++P) {
-            if ((!DL && P >= 3) || (!SL && P == 2)) continue;
-            const int S = (!SL && P > 2) ? P - 1 : P;
-            const float4* o = ex + (size_t)((kk * NP + S) * 2) * cols;
-            const float4 D0 = o[cols + t], D1 = o[cols + tn], U0 = o[t], U1 = o[tn];
-            const float2 off = C.p[P];
-            Dot2& d = d2[P];
-            d.s = off; d.c = make_float2(0.f, 0.f);
-            d.add<true>(w2, lo2(D0), hi2(D0));
-            d.add<true>(w3, lo2(D1), hi2(D1));
-            if (P < FF_XPAIRS) {
-              d.s = sub2(d.s, off);
-              d.add<false>(w0, lo2(U0), hi2(U0));
-              d.add<false>(w1, lo2(U1), hi2(U1));
-            } else {
-              d.add<true>(w0, lo2(U0), hi2(U0));
-              d.add<true>(w1, lo2(U1), hi2(U1));
-              d.s = sub2(d.s, off);
-            }
+          Dot2& d = side ? db[P] : da[P];
+          d.s = off; d.c = make_float2(0.f, 0.f);
+          d.add<true>(w2, lo2(D0), hi2(D0));
+          d.add<true>(w3, lo2(D1), hi2(D1));
+          if (P < FF_XPAIRS) {
+            d.s = sub2(d.s, off);
+            d.add<false>(w0, lo2(U0), hi2(U0));
+            d.add<false>(w1, lo2(U1), hi2(U1));
+          } else {
+            d.add<true>(w0, lo2(U0), hi2(U0));
+            d.add<true>(w1, lo2(U1), hi2(U1));
+            d.s = sub2(d.s, off);
           }
-          const ff xi[3] = {ld_ff(sT[q]), ld_ff(sT[cols + q]), ld_ff(sT[2 * cols + q])};
-          patch_point<SL, DL>(a, d2, xi, ld_ff(C.c2m), ld_ff(__ldg(&c.w)), acc + 3 * side * cols + q, cols);
         }
       }
-      __syncthreads();  // the next class's sums may meet these
+      patch_points<SL, DL>(a, da, db, sT + qa, sT + qb, {C.c2m.x, C.c2m.y}, __ldg(&c.w), acc + qa, acc + 3 * cols + qb, cols);
     }
   }
+  __syncthreads();
   for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
     const int lc = t / nlon, j = t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
     const double iA = 1.0 / a.tA[p];
@@ -440,11 +453,24 @@ __global__ void __launch_bounds__(256, 2) k_self_ff(FFArgs a) {
   }
 }
 
-// hi/lo split of an FP64 value
-__device__ __forceinline__ void split(double v, float* h, float* l) {
-  const float hv = (float)v;
-  *h = hv;
-  *l = (float)(v - (double)hv);
+// hi/lo split of an FP64 value, both parts rounded to nearest.  In integer
+// arithmetic where both parts are normal: the conversions run on the FP64 pipe.
+__device__ __forceinline__ void split(double v, float& h, float& l) {
+  const unsigned long long b = __double_as_longlong(v);
+  const int e = (int)(b >> 52) & 0x7ff;  // |v| in [2^(e-1023), 2^(e-1022))
+  if (e >= 1023 - 70 && e < 1023 + 120) {
+    // hi: 24 of the 53 bits, rounded by the addition's carry; the remainder
+    // of the 29 bits below as a signed integer in units of 2^(e-1075)
+    const unsigned long long r = b + (1ull << 28);
+    h = __int_as_float((int)((b >> 32) & 0x80000000u) | ((((int)(r >> 52) & 0x7ff) - 1023 + 127) << 23) |
+                       ((int)(r >> 29) & 0x7fffff));
+    const int low = (int)(r & 0x1fffffff) - (1 << 28);
+    const float u = __int_as_float((e - 1075 + 127) << 23);
+    l = (float)low * (b >> 63 ? -u : u);
+  } else {
+    h = (float)v;
+    l = (float)(v - (double)h);
+  }
 }
 
 // Node records of the spline sets named in `sets` (bit 0 x, 1 f, 2 g, 3 a3):
@@ -456,12 +482,9 @@ __global__ void __launch_bounds__(128) k_ff_rec(int ncell, int m, int n, const d
                                                 const double* __restrict__ xc, float* __restrict__ out,
                                                 unsigned* __restrict__ bnd, int sets) {
   __shared__ double s[4][16][4][SPL_NODE];  // set, column, row, value
-  __shared__ unsigned smax[16];
   const int nti = (m + 3) / 4, ntj = (n + 15) / 16;
   const int jt = blockIdx.x % ntj, it = (blockIdx.x / ntj) % nti, cell = blockIdx.x / (ntj * nti);
   const int src[4] = {SPL_X, SPL_F, SPL_G, SPL_A3};
-  if (threadIdx.x < 16) smax[threadIdx.x] = 0;
-  __syncthreads();
   for (int k = 0; k < 4; ++k) {
     if (!(sets & (1 << k))) continue;
     const double* in = spl + ((size_t)cell * SPL_NSET + src[k]) * (size_t)m * n * SPL_NODE;
@@ -469,16 +492,30 @@ __global__ void __launch_bounds__(128) k_ff_rec(int ncell, int m, int n, const d
       const int q = e % SPL_NODE, r = (e / SPL_NODE) % 4, c = e / (4 * SPL_NODE);
       const int j = 16 * jt + c, i = 4 * it + r;
       double v = 0.;
-      if (j < n && i < m) v = in[((size_t)j * m + i) * SPL_NODE + q];
-      if (k == 0 && q < 3 && j < n && i < m) v -= xc[3 * cell + q];
+      if (j < n && i < m) {
+        v = in[((size_t)j * m + i) * SPL_NODE + q];
+        if (k == 0 && q < 3) v -= xc[3 * cell + q];
+      }
       s[k][c][r][q] = v;
-      const unsigned mx = __float_as_uint(__double2float_ru(fabs(v)));
-      atomicMax(&smax[4 * k + q / 3], mx);
     }
   }
   __syncthreads();
-  if (threadIdx.x < 16 && (sets & (1 << (threadIdx.x / 4))))
-    atomicMax(bnd + ((size_t)(threadIdx.x / 4) * ncell + cell) * 4 + threadIdx.x % 4, smax[threadIdx.x]);
+  {  // 8 threads per (set, slot): the largest magnitude, compared as integers
+    const int k = threadIdx.x >> 5, d = (threadIdx.x >> 3) & 3, o = threadIdx.x & 7;
+    unsigned long long mx = 0;
+    if (sets & (1 << k))
+      for (int node = o; node < 64; node += 8)
+        for (int c = 0; c < 3; ++c) {
+          const unsigned long long v = __double_as_longlong(s[k][node >> 2][node & 3][3 * d + c]) & 0x7fffffffffffffffull;
+          mx = v > mx ? v : mx;
+        }
+    for (int w = 4; w > 0; w >>= 1) {
+      const unsigned long long v = __shfl_xor_sync(0xffffffffu, mx, w);
+      mx = v > mx ? v : mx;
+    }
+    if (o == 0 && (sets & (1 << k)))
+      atomicMax(bnd + ((size_t)k * ncell + cell) * 4 + d, __float_as_uint(__double2float_ru(__longlong_as_double(mx))));
+  }
   for (int e = threadIdx.x; e < 4 * FF_ROW * 16; e += blockDim.x) {
     const int c = e % 16, dq = (e / 16) % FF_ROW, r = e / (16 * FF_ROW);
     const int j = 16 * jt + c, i = 4 * it + r;
@@ -486,11 +523,12 @@ __global__ void __launch_bounds__(128) k_ff_rec(int ncell, int m, int n, const d
     float* o = out + 8 * ((((size_t)cell * m + i) * FF_ROW + dq) * n + j);
     float h[4], l[4];
     int have = 0;
+#pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int val = 4 * (dq % 3) + k, set = val / 3;
       h[k] = l[k] = 0.f;
       if (!(sets & (1 << set))) continue;
-      split(s[set][c][r][3 * (dq / 3) + val % 3], h + k, l + k);
+      split(s[set][c][r][3 * (dq / 3) + val % 3], h[k], l[k]);
       have |= 1 << k;
     }
     if (have == 15) {
@@ -520,7 +558,7 @@ rbc3d_status self_ff_tables(rbc3d_ctx* ctx, const std::vector<double>& c1, const
     for (int i = 0; i < N; ++i) {
       const double v = (*src[k])[i], d = (*src[k])[i + 1] - v;
       const ff a = hsplit(v), b = hsplit(d);
-      t[(size_t)k * N + i] = make_float4(a.h, a.l, b.h, b.l);
+      t[3 * (size_t)i + k] = make_float4(a.h, a.l, b.h, b.l);
     }
   CUDA_TRY(ctx->ff_tab.upload(t.data(), t.size(), ctx->st));
   CUDA_TRY(cudaStreamSynchronize(ctx->st));
@@ -537,14 +575,15 @@ rbc3d_status self_ff_grid(rbc3d_ctx* ctx, const std::vector<RingClass>& R) {
   for (size_t i = 0; i < R.size(); ++i) {
     const RingClass& r = R[i];
     FFClass& c = C[i];
-    c.i1 = r.i1; c.j[0] = r.j[0]; c.j[1] = r.j[1]; c.pad = 0;
+    const bool two = r.j[1] >= 0;
+    c.i1 = r.i1; c.j[0] = r.j[0]; c.j[1] = r.j[two]; c.pad = 0;
     c.x[0] = op(1. - r.x[0]); c.x[1] = op(r.x[0]); c.x[2] = op(r.x[1]); c.x[3] = op(r.x[2]);
     for (int s = 0; s < 2; ++s) {
-      c.y[s][0] = op(1. - r.y[s][0]); c.y[s][1] = op(r.y[s][0]); c.y[s][2] = op(r.y[s][1]); c.y[s][3] = op(r.y[s][2]);
+      const double* y = r.y[s && two];
+      c.y[s][0] = op(1. - y[0]); c.y[s][1] = op(y[0]); c.y[s][2] = op(y[1]); c.y[s][3] = op(y[2]);
     }
     const ff w = hsplit(r.w);
-    c.w = make_float2(w.h, w.l);
-    c.pad2 = make_float2(0.f, 0.f);
+    c.w = make_float4(w.h, w.l, two ? w.h : 0.f, two ? w.l : 0.f);
   }
   CUDA_TRY(ctx->ff_cls.upload(reinterpret_cast<const char*>(C.data()), C.size() * sizeof(FFClass), ctx->st));
   CUDA_TRY(cudaStreamSynchronize(ctx->st));
@@ -590,7 +629,7 @@ rbc3d_status run_self_ff(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   const int np = dl ? (sl ? 6 : 5) : 3;
   auto smem = [&](int G) {
     const size_t cols = (size_t)G * ctx->nlon;
-    return sizeof(float4) * FF_CHUNK * np * 2 * cols + sizeof(FFCell) * G + sizeof(float2) * 9 * cols;
+    return sizeof(float4) * 4 * np * cols + sizeof(FFCell) * G + sizeof(float2) * 9 * cols;
   };
   // a ring wider than shared memory holds (about 500 columns) goes to the FP64 patch
   if (smem(1) > 227 * 1024) return run_self_corr(ctx, tlist, sl ? c1 : 0., dl ? c2 : 0.);
