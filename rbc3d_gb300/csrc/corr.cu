@@ -26,10 +26,9 @@ struct CorrArgs {
   int ncell, nlat, nlon, m;
   SplGrid G;  // Spline_Create constants of the (2 nlat, nlon) spline grid
   double rc2;
-  unsigned long long* queue;  // k_near's item counter
-  const int* list;            // k_near: items to process (indices), or null for all
-  long long list_start;       // k_near over a list: its first entry (the staged pass takes those before)
-  int stage_cap;              // the staged pass: entries it takes from the list's head
+  unsigned long long* queue;  // counters of the staged pass (NQ_*); k_near: its item counter
+  const int* list;            // items to process (indices), or null for all
+  int stage_cap;              // the staged pass: corrected items it has room for
   const float* rep;           // k_near_replay: x and a3 node values in FP32, 24 floats a node
   const unsigned long long* nlist;
   const double* th;
@@ -161,115 +160,120 @@ __device__ __forceinline__ void patch_point(double st0, double ct0, double phi0,
   phiG = p - floor(p * RBC3D_I_2PI) * RBC3D_TWO_PI;
 }
 
-// PolarPatch_Map (ModPolarPatch.F90:218-244)
-__device__ __forceinline__ void patch_map(double th0, double phi0, double dth, double dphi, double& th, double& phi) {
-  double st0 = sin(th0), ct0 = cos(th0), sp0 = sin(phi0), cp0 = cos(phi0);
-  double s1[3] = {ct0 * cp0, ct0 * sp0, -st0};
-  double s2[3] = {-sp0, cp0, 0.};
-  double x0[3] = {st0 * cp0, st0 * sp0, ct0};
-  double x[3] = {sin(dth) * cos(dphi), sin(dth) * sin(dphi), cos(dth)};
-  double y[3];
-  for (int c = 0; c < 3; ++c) y[c] = x[0] * s1[c] + x[1] * s2[c] + x[2] * x0[c];
-  double nrm = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
-  for (int c = 0; c < 3; ++c) y[c] /= nrm;
-  y[2] = fmax(-1., fmin(1., y[2]));
-  th = acos(y[2]);
-  phi = atan2(y[1], y[0]);
-  if (phi < 0) phi += RBC3D_TWO_PI;
-}
+// Spline_FindProjection (ModSpline.F90:203-269), a half-warp per target (both
+// halves may hold the same one; all 32 lanes take part).  QuadFit_2D fits
+// 1, px, py, px^2, px py, py^2 to the squared distances at 16 points on two
+// circles of radius h/2 and h and at the centre; in the variables px/h, py/h
+// those points never change, and on 8 equispaced azimuths the odd terms, px py,
+// px^2 - py^2 and (1, px^2 + py^2) are orthogonal, so the normal equations
+// (ModBasicMath.F90:234-284) are solved once and for all: five weighted sums
+// of the distances less the centre's.  An iteration takes about 600 FP64
+// instructions for two targets, against 1600 for one with 27 sums, a Cholesky
+// factorisation and the angles' sines anew (see run_near_corr).
+__device__ __forceinline__ void sincos_r(double x, double* s, double* c) { sincos(x, s, c); }
+__device__ __forceinline__ void sincos_r(float x, float* s, float* c) { sincosf(x, s, c); }
+__device__ __forceinline__ double acos_r(double x) { return acos(x); }
+__device__ __forceinline__ float acos_r(float x) { return acosf(x); }
+__device__ __forceinline__ double atan2_r(double y, double x) { return atan2(y, x); }
+__device__ __forceinline__ float atan2_r(float y, float x) { return atan2f(y, x); }
 
-// dposv on the 6x6 normal equations (upper Cholesky); leaves b unchanged when
-// the matrix is not positive definite, as LAPACK does for info > 0.
-__device__ void chol6(const double* A /*21 packed upper, row-major a<=b*/, double* b) {
-  double U[6][6];
-  double M[6][6];
-  int p = 0;
-  for (int i = 0; i < 6; ++i)
-    for (int j = i; j < 6; ++j) { M[i][j] = A[p]; M[j][i] = A[p]; ++p; }
-  for (int j = 0; j < 6; ++j) {
-    double s = M[j][j];
-    for (int k = 0; k < j; ++k) s -= U[k][j] * U[k][j];
-    if (!(s > 0)) return;
-    U[j][j] = sqrt(s);
-    for (int i = j + 1; i < 6; ++i) {
-      double t = M[j][i];
-      for (int k = 0; k < j; ++k) t -= U[k][j] * U[k][i];
-      U[j][i] = t / U[j][j];
+// A lane's fit point: azimuth and radii of the three levels, and its weights
+// in the fit of u = px/h, v = py/h, uv, u^2 - v^2 and u^2 + v^2.
+template <typename R>
+struct ProjLane {
+  R cph, sph, sL[3], cL[3], wu, wv, wuv, wd, wr;
+  __device__ __forceinline__ void init(double h0) {
+    const int k = threadIdx.x & 15;
+    const double r = 0.5 * (k % 2 + 1), a = (k / 2) * RBC3D_TWO_PI / 8;
+    double s, c;
+    sincos(a, &s, &c);
+    const double u = r * c, v = r * s;
+    cph = (R)c; sph = (R)s;
+    // sums over the points: u^2 5, (uv)^2 17/16, (u^2 - v^2)^2 17/4, and of
+    // r^2 10, r^4 8.5 over 17 points
+    wu = (R)(u / 5); wv = (R)(v / 5); wuv = (R)(u * v / 1.0625); wd = (R)((u * u - v * v) / 4.25);
+    wr = (R)((r * r - 10. / 17) / (8.5 - 100. / 17));
+    for (int l = 0; l < 3; ++l, h0 *= 0.5) {
+      sincos(r * h0, &s, &c);
+      sL[l] = (R)s; cL[l] = (R)c;
     }
   }
-  double y[6];
-  for (int i = 0; i < 6; ++i) {
-    double t = b[i];
-    for (int k = 0; k < i; ++k) t -= U[k][i] * y[k];
-    y[i] = t / U[i][i];
-  }
-  for (int i = 5; i >= 0; --i) {
-    double t = y[i];
-    for (int k = i + 1; k < 6; ++k) t -= U[i][k] * b[k];
-    b[i] = t / U[i][i];
-  }
+};
+template <typename R>
+__device__ __forceinline__ R half_sum(R v) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-// Spline_FindProjection, warp-cooperative.  All lanes return the same result.
-__device__ void find_projection(const double* sx, int m, int n, const double* xt, double& th0, double& phi0,
-                                double* x0) {
-  const int lane = threadIdx.x & 31;
-  SplW W;
-  spline_weights(th0, phi0, m, n, W);
-  spline_eval(sx, W, 3, x0);
-  double h = fmax(RBC3D_TWO_PI / m, RBC3D_TWO_PI / n);
-  for (int iter = 0; iter < 3; ++iter) {
-    double px = 0, py = 0, d2 = 0;
-    bool on = lane <= 16;
-    if (lane < 16) {
-      int ith = lane % 2, iphi = lane / 2;
-      double thL = (ith + 1) * h / 2;
-      double phL = iphi * RBC3D_TWO_PI / 8;
-      double thP, phP;
-      patch_point(sin(th0), cos(th0), phi0, sin(thL), cos(thL), cos(phL), sin(phL), thP, phP);
-      px = thL * cos(phL);
-      py = thL * sin(phL);
-      double xx[3];
-      spline_weights(thP, phP, m, n, W);
-      spline_eval(sx, W, 3, xx);
-      for (int k = 0; k < 3; ++k) xx[k] -= xt[k];
-      d2 = xx[0] * xx[0] + xx[1] * xx[1] + xx[2] * xx[2];
-    } else if (lane == 16) {
-      double xx[3];
-      spline_weights(th0, phi0, m, n, W);
-      spline_eval(sx, W, 3, xx);
-      for (int k = 0; k < 3; ++k) xx[k] -= xt[k];
-      d2 = xx[0] * xx[0] + xx[1] * xx[1] + xx[2] * xx[2];
-    }
-    double d2c = __shfl_sync(0xffffffffu, d2, 16);
-    double u[6] = {on ? 1. : 0., px, py, px * px, px * py, py * py};
-    double A[21], b[6];
-    int p = 0;
-    for (int i = 0; i < 6; ++i)
-      for (int j = i; j < 6; ++j) A[p++] = warp_sum(u[i] * u[j]);
-    for (int i = 0; i < 6; ++i) b[i] = warp_sum(u[i] * d2);
-    chol6(A, b);
+// eval(theta, phi, x): the surface point.  h0: the first level's radius.
+template <typename R, class Eval>
+__device__ __forceinline__ void find_projection(const ProjLane<R>& P, R h0, const R* xt, R& th0, R& phi0, R* x0,
+                                                const Eval& eval) {
+  const R two_pi = (R)RBC3D_TWO_PI, i2pi = (R)RBC3D_I_2PI;
+  auto dist2 = [&](const R* x) {
+    const R a = x[0] - xt[0], b = x[1] - xt[1], c = x[2] - xt[2];
+    return a * a + b * b + c * c;
+  };
+  R st0, ct0, sp0, cp0;
+  sincos_r(th0, &st0, &ct0);
+  sincos_r(phi0, &sp0, &cp0);
+  eval(th0, phi0, x0);
+  R d2c = dist2(x0), h = h0;
+  bool live = true;
+#pragma unroll 1
+  for (int it = 0; it < 3; ++it, h *= (R)0.5) {
+    // the lane's point of PolarPatch_Build (ModPolarPatch.F90:99-148)
+    const R sL = it == 0 ? P.sL[0] : it == 1 ? P.sL[1] : P.sL[2], cL = it == 0 ? P.cL[0] : it == 1 ? P.cL[1] : P.cL[2];
+    const R q0 = sL * P.cph, q1 = sL * P.sph;
+    const R y2 = fmax((R)-1, fmin((R)1, ct0 * cL - st0 * q0));
+    const R p = atan2_r(q1, ct0 * q0 + st0 * cL) + phi0;
+    R xp[3];
+    eval(acos_r(y2), p - floor(p * i2pi) * two_pi, xp);
+    const R d = dist2(xp) - d2c;
+    const R b1 = half_sum(P.wu * d), b2 = half_sum(P.wv * d), b4 = half_sum(P.wuv * d), bd = half_sum(P.wd * d),
+            br = half_sum(P.wr * d);
     // Min_Quad_2D
-    double l11 = 2. * b[3], l12 = b[4], l22 = 2. * b[5];
-    double det = l11 * l22 - l12 * l12;
-    double xm0 = 0., xm1 = 0.;
+    const R l11 = 2 * (br + bd), l22 = 2 * (br - bd), det = l11 * l22 - b4 * b4;
+    R m0 = 0, m1 = 0;
     if (det > 0) {
-      double idet = 1. / det;
-      xm0 = idet * (l22 * (-b[1]) - l12 * (-b[2]));
-      xm1 = idet * (-l12 * (-b[1]) + l11 * (-b[2]));
+      const R id = h / det;
+      m0 = id * (b4 * b2 - l22 * b1);
+      m1 = id * (b4 * b1 - l11 * b2);
     }
-    double thMinL = sqrt(xm0 * xm0 + xm1 * xm1), phiMinL = atan2(xm1, xm0);
-    double thMin, phiMin, xMin[3];
-    patch_map(th0, phi0, thMinL, phiMinL, thMin, phiMin);
-    spline_weights(thMin, phiMin, m, n, W);
-    spline_eval(sx, W, 3, xMin);
-    double e0 = xMin[0] - xt[0], e1 = xMin[1] - xt[1], e2 = xMin[2] - xt[2];
-    double d2Min = e0 * e0 + e1 * e1 + e2 * e2;
-    if (d2Min > d2c) break;
-    th0 = thMin; phi0 = phiMin;
-    for (int k = 0; k < 3; ++k) x0[k] = xMin[k];
-    h = 0.5 * h;
+    // PolarPatch_Map (ModPolarPatch.F90:218-244) of the minimum
+    const R r = sqrt(m0 * m0 + m1 * m1);
+    R sr, cr;
+    sincos_r(r, &sr, &cr);
+    const R sc = r > 0 ? sr / r : (R)1;
+    const R a = sc * m0, b = sc * m1, e = ct0 * a + st0 * cr;
+    const R yx = e * cp0 - b * sp0, yy = e * sp0 + b * cp0, yz = fmax((R)-1, fmin((R)1, ct0 * cr - st0 * a));
+    const R thM = acos_r(yz);
+    R phM = atan2_r(yy, yx), xM[3];
+    if (phM < 0) phM += two_pi;
+    eval(thM, phM, xM);
+    const R d2 = dist2(xM);
+    live = live && !(d2 > d2c);
+    if (live) {
+      th0 = thM; phi0 = phM; d2c = d2;
+      for (int k = 0; k < 3; ++k) x0[k] = xM[k];
+      ct0 = yz;
+      st0 = sqrt(yx * yx + yy * yy);
+      cp0 = st0 > 0 ? yx / st0 : (R)1;
+      sp0 = st0 > 0 ? yy / st0 : (R)0;
+    }
+    if (!__any_sync(0xffffffffu, live)) break;
   }
+}
+
+// FP64, from the spline table sx of the target's cell
+__device__ __forceinline__ void project64(const ProjLane<double>& P, const double* sx, const SplGrid& G,
+                                          const double* xt, double& th0, double& phi0, double* x0) {
+  find_projection(P, fmax(G.hx, G.hy), xt, th0, phi0, x0, [&](double th, double ph, double* x) {
+    SplW W;
+    spline_weights_g(th, ph, G, W);
+    spline_eval(sx, W, 3, x);
+  });
 }
 
 // RBC_NearSingInt_Subtract: lane = latitude row of PolarPatch_FindPoints
@@ -330,9 +334,10 @@ __device__ void near_subtract(const CorrArgs& a, int cell, double c1, double c2,
   for (int k = 0; k < 3; ++k) dv[k] = warp_sum(dv[k]);
 }
 
-// RBC_NearSingInt_ReAdd: nrad = 16, nazm = 32, lane = azimuth
+// RBC_NearSingInt_ReAdd: nrad = 16, nazm = 32, lane = azimuth; the radial
+// points [r0, r1)
 __device__ void near_readd(const CorrArgs& a, int cell, double c1, double c2, const double* xi, const double* x0,
-                           double th0, double phi0, double radPat, double* dv) {
+                           double th0, double phi0, double radPat, double* dv, int r0 = 0, int r1 = 16) {
   const int lane = threadIdx.x & 31;
   const int nrad = 16, nazm = 32;
   double d = sqrt((xi[0] - x0[0]) * (xi[0] - x0[0]) + (xi[1] - x0[1]) * (xi[1] - x0[1]) +
@@ -377,7 +382,7 @@ __device__ void near_readd(const CorrArgs& a, int cell, double c1, double c2, co
     rwt = rwt * mask64(a.T, rth / radPat);
   }
   double acc[3] = {0, 0, 0};
-  for (int irad = 0; irad < nrad; ++irad) {
+  for (int irad = r0; irad < r1; ++irad) {
     const double wt = __shfl_sync(0xffffffffu, rwt, irad);
     const double sthP = __shfl_sync(0xffffffffu, rs, irad), cthP = __shfl_sync(0xffffffffu, rc, irad);
     double thG, phG;
@@ -428,24 +433,7 @@ __device__ __forceinline__ void spline_weights32(float x, float y, int m, int n,
   cy[2] = hy * t * (1.f + t * (-2.f + t)); cy[3] = hy * t * t * (-1.f + t);
   n11 = i1 + m * j1; n12 = i1 + m * j2; n21 = i2 + m * j1; n22 = i2 + m * j2;
 }
-__device__ __forceinline__ void spline_eval32(const double* __restrict__ spl, float th, float ph, int m, int n,
-                                              float* f) {
-  int n11, n12, n21, n22;
-  float cx[4], cy[4];
-  spline_weights32(th, ph, m, n, n11, n12, n21, n22, cx, cy);
-  const double* a = spl + (size_t)n11 * SPL_NODE;
-  const double* b = spl + (size_t)n12 * SPL_NODE;
-  const double* c = spl + (size_t)n21 * SPL_NODE;
-  const double* d = spl + (size_t)n22 * SPL_NODE;
-  for (int l = 0; l < 3; ++l) {
-    float r0 = (float)a[l] * cy[0] + (float)b[l] * cy[1] + (float)a[6 + l] * cy[2] + (float)b[6 + l] * cy[3];
-    float r1 = (float)c[l] * cy[0] + (float)d[l] * cy[1] + (float)c[6 + l] * cy[2] + (float)d[6 + l] * cy[3];
-    float r2 = (float)a[3 + l] * cy[0] + (float)b[3 + l] * cy[1] + (float)a[9 + l] * cy[2] + (float)b[9 + l] * cy[3];
-    float r3 = (float)c[3 + l] * cy[0] + (float)d[3 + l] * cy[1] + (float)c[9 + l] * cy[2] + (float)d[9 + l] * cy[3];
-    f[l] = cx[0] * r0 + cx[1] * r1 + cx[2] * r2 + cx[3] * r3;
-  }
-}
-// the same from the replay's FP32 node records (24 floats a node: the x
+// Spline_Interp from the replay's FP32 node records (24 floats a node: the x
 // slots' 12 values, then a3's; off 0 for x, 12 for a3), with no conversions
 __device__ __forceinline__ void spline_eval32f(const float* __restrict__ rec, int off, float th, float ph, int m,
                                                int n, float* f) {
@@ -464,103 +452,14 @@ __device__ __forceinline__ void spline_eval32f(const float* __restrict__ rec, in
     f[l] = cx[0] * r0 + cx[1] * r1 + cx[2] * r2 + cx[3] * r3;
   }
 }
-__device__ __forceinline__ float warp_sumf_(float v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-// Returns the projection's signed distance a3(x0).(xt - x0) in FP32, from
-// the cell's FP32 node records (x at offset 0, a3 at 12).
-__device__ float projection_dist32(const float* rc, int m, int n, const double* xtd, double th0d, double phi0d) {
-  const int lane = threadIdx.x & 31;
-  const float TWO_PI_F = (float)RBC3D_TWO_PI;
-  float xt[3] = {(float)xtd[0], (float)xtd[1], (float)xtd[2]};
-  float th0 = (float)th0d, phi0 = (float)phi0d;
-  float x0[3];
-  spline_eval32f(rc, 0, th0, phi0, m, n, x0);
-  float h = fmaxf(TWO_PI_F / m, TWO_PI_F / n);
-  for (int iter = 0; iter < 3; ++iter) {
-    float px = 0, py = 0, d2 = 0;
-    float st0 = sinf(th0), ct0 = cosf(th0);
-    if (lane < 16) {
-      int ith = lane % 2, iphi = lane / 2;
-      float thL = (ith + 1) * h / 2;
-      float phL = iphi * TWO_PI_F / 8;
-      float sth = sinf(thL), cth = cosf(thL), cph = cosf(phL), sph = sinf(phL);
-      float q0 = sth * cph, q1 = sth * sph, q2 = cth;
-      float y0 = ct0 * q0 + st0 * q2, y1 = q1, y2 = fmaxf(-1.f, fminf(1.f, -st0 * q0 + ct0 * q2));
-      float thP = acosf(y2), pp = atan2f(y1, y0) + phi0;
-      float phP = pp - floorf(pp / TWO_PI_F) * TWO_PI_F;
-      px = thL * cph;
-      py = thL * sph;
-      float xx[3];
-      spline_eval32f(rc, 0, thP, phP, m, n, xx);
-      d2 = (xx[0] - xt[0]) * (xx[0] - xt[0]) + (xx[1] - xt[1]) * (xx[1] - xt[1]) + (xx[2] - xt[2]) * (xx[2] - xt[2]);
-    } else if (lane == 16) {
-      float xx[3];
-      spline_eval32f(rc, 0, th0, phi0, m, n, xx);
-      d2 = (xx[0] - xt[0]) * (xx[0] - xt[0]) + (xx[1] - xt[1]) * (xx[1] - xt[1]) + (xx[2] - xt[2]) * (xx[2] - xt[2]);
-    }
-    float d2c = __shfl_sync(0xffffffffu, d2, 16);
-    float u[6] = {lane <= 16 ? 1.f : 0.f, px, py, px * px, px * py, py * py};
-    float M[6][6], b[6];
-    for (int i = 0; i < 6; ++i)
-      for (int j = i; j < 6; ++j) { M[i][j] = warp_sumf_(u[i] * u[j]); M[j][i] = M[i][j]; }
-    for (int i = 0; i < 6; ++i) b[i] = warp_sumf_(u[i] * d2);
-    // Cholesky
-    float U[6][6];
-    bool ok = true;
-    for (int j = 0; j < 6 && ok; ++j) {
-      float s = M[j][j];
-      for (int k = 0; k < j; ++k) s -= U[k][j] * U[k][j];
-      if (!(s > 0)) { ok = false; break; }
-      U[j][j] = sqrtf(s);
-      for (int i = j + 1; i < 6; ++i) {
-        float t = M[j][i];
-        for (int k = 0; k < j; ++k) t -= U[k][j] * U[k][i];
-        U[j][i] = t / U[j][j];
-      }
-    }
-    if (ok) {
-      float y[6];
-      for (int i = 0; i < 6; ++i) {
-        float t = b[i];
-        for (int k = 0; k < i; ++k) t -= U[k][i] * y[k];
-        y[i] = t / U[i][i];
-      }
-      for (int i = 5; i >= 0; --i) {
-        float t = y[i];
-        for (int k = i + 1; k < 6; ++k) t -= U[i][k] * b[k];
-        b[i] = t / U[i][i];
-      }
-    }
-    float l11 = 2.f * b[3], l12 = b[4], l22 = 2.f * b[5];
-    float det = l11 * l22 - l12 * l12;
-    float xm0 = 0.f, xm1 = 0.f;
-    if (det > 0) {
-      float idet = 1.f / det;
-      xm0 = idet * (l22 * (-b[1]) - l12 * (-b[2]));
-      xm1 = idet * (-l12 * (-b[1]) + l11 * (-b[2]));
-    }
-    float dth = sqrtf(xm0 * xm0 + xm1 * xm1), dph = atan2f(xm1, xm0);
-    float sp0 = sinf(phi0), cp0 = cosf(phi0);
-    float s1[3] = {ct0 * cp0, ct0 * sp0, -st0}, s2[3] = {-sp0, cp0, 0.f}, e0[3] = {st0 * cp0, st0 * sp0, ct0};
-    float qx[3] = {sinf(dth) * cosf(dph), sinf(dth) * sinf(dph), cosf(dth)};
-    float yv[3];
-    for (int c = 0; c < 3; ++c) yv[c] = qx[0] * s1[c] + qx[1] * s2[c] + qx[2] * e0[c];
-    float nr = sqrtf(yv[0] * yv[0] + yv[1] * yv[1] + yv[2] * yv[2]);
-    yv[2] = fmaxf(-1.f, fminf(1.f, yv[2] / nr));
-    float thMin = acosf(yv[2]), phiMin = atan2f(yv[1] / nr, yv[0] / nr);
-    if (phiMin < 0) phiMin += TWO_PI_F;
-    float xMin[3];
-    spline_eval32f(rc, 0, thMin, phiMin, m, n, xMin);
-    float d2Min = (xMin[0] - xt[0]) * (xMin[0] - xt[0]) + (xMin[1] - xt[1]) * (xMin[1] - xt[1]) +
-                  (xMin[2] - xt[2]) * (xMin[2] - xt[2]);
-    if (d2Min > d2c) break;
-    th0 = thMin; phi0 = phiMin;
-    for (int k = 0; k < 3; ++k) x0[k] = xMin[k];
-    h = 0.5f * h;
-  }
-  float a30[3];
+// The projection's signed distance a3(x0).(xt - x0) in FP32, from the cell's
+// FP32 node records (x at offset 0, a3 at 12); a half-warp per target.
+__device__ __forceinline__ float projection_dist32(const ProjLane<float>& P, const float* rc, int m, int n,
+                                                   const double* xtd, double th0d, double phi0d) {
+  const float xt[3] = {(float)xtd[0], (float)xtd[1], (float)xtd[2]};
+  float th0 = (float)th0d, phi0 = (float)phi0d, x0[3], a30[3];
+  find_projection(P, fmaxf((float)(RBC3D_TWO_PI / m), (float)(RBC3D_TWO_PI / n)), xt, th0, phi0, x0,
+                  [&](float th, float ph, float* x) { spline_eval32f(rc, 0, th, ph, m, n, x); });
   spline_eval32f(rc, 12, th0, phi0, m, n, a30);
   return a30[0] * (xt[0] - x0[0]) + a30[1] * (xt[1] - x0[1]) + a30[2] * (xt[2] - x0[2]);
 }
@@ -601,48 +500,48 @@ __global__ void k_near_screen(CorrArgs a, int* __restrict__ out, unsigned long l
   out[atomicAdd(nout, 1ull)] = (int)i;
 }
 
-// stage 2 (one warp per listed candidate): the FP32 replay of the projection;
+// stage 2 (a half-warp per listed candidate): the FP32 replay of the projection;
 // candidates within 2.3*meshSize are listed for the FP64 stage.
 __global__ void __launch_bounds__(128) k_near_replay(CorrArgs a, const int* __restrict__ in,
                                                      const unsigned long long* __restrict__ nin,
                                                      int* __restrict__ out, unsigned long long* __restrict__ nout) {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, half = lane >> 4;
   const long long n = (long long)*nin;
   const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n; w += nw) {
-    const int idx = in[w];
+  ProjLane<float> P;
+  P.init(fmax(a.G.hx, a.G.hy));
+  for (long long w = 2 * ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); w < n; w += 2 * nw) {
+    const bool on = w + half < n;
+    const int idx = in[on ? w + half : w];
     const int4 item = a.items[idx];
     const int cell = item.y - 1;
     double x0[3], xt[3];
     size_t q0;
     item_geometry(a, item, x0, xt, q0);
     const double msz = a.meshSize[cell];
-    const float d32 = projection_dist32(a.rep + (size_t)cell * a.m * a.nlon * 24, a.m, a.nlon, xt, a.th[item.z],
+    const float d32 = projection_dist32(P, a.rep + (size_t)cell * a.m * a.nlon * 24, a.m, a.nlon, xt, a.th[item.z],
                                         a.phi[item.w]);
-    if ((double)d32 > 2.3 * msz) continue;
-    if (lane == 0) out[atomicAdd(nout, 1ull)] = idx;
+    if (on && (lane & 15) == 0 && !((double)d32 > 2.3 * msz)) out[atomicAdd(nout, 1ull)] = idx;
   }
 }
 
+// RBC_NearSingInt with one warp per item: the verification of the screens
+// (every candidate), and what the staged pass below had no room for.
 __global__ void __launch_bounds__(128) k_near(CorrArgs a) {
   const int lane = threadIdx.x & 31;
   unsigned long long nitem = a.list ? *a.nlist : *a.nitems;
   if (nitem > (unsigned long long)a.cap) nitem = a.cap;
-  // warps take items from a shared counter (the grid is one resident wave):
-  // corrected items cost ~100x screened ones, so a static split leaves a tail
-  // items per counter update: 4 over the full candidate list; 1 over the short
-  // list of the FP32 modes, so its few expensive items spread over all SMs
-  const int GRAB = a.list ? 1 : 4;
-  long long it = 0, it_end = 0;
+  if (nitem == 0) return;
+  ProjLane<double> PL;
+  PL.init(fmax(a.G.hx, a.G.hy));
+  ProjLane<float> PF;
+  if (a.screen) PF.init(fmax(a.G.hx, a.G.hy));
+  // warps take items from a shared counter (the grid is one resident wave)
   for (;;) {
-    if (it == it_end) {
-      unsigned long long g0 = 0;
-      if (lane == 0) g0 = atomicAdd(a.queue, (unsigned long long)GRAB);
-      it = (long long)__shfl_sync(0xffffffffu, g0, 0);
-      it_end = it + GRAB;
-    }
-    if (it + a.list_start >= (long long)nitem) break;
-    const long long cur = a.list_start + it++;
+    unsigned long long g0 = 0;
+    if (lane == 0) g0 = atomicAdd(a.queue, 1ull);
+    const long long cur = (long long)__shfl_sync(0xffffffffu, g0, 0);
+    if (cur >= (long long)nitem) break;
     int4 item = a.items[a.list ? a.list[cur] : cur];
     int t = item.x, cell = item.y - 1, ilat0 = item.z, ilon0 = item.w;
     if (cell < 0 || cell >= a.ncell) continue;
@@ -668,14 +567,14 @@ __global__ void __launch_bounds__(128) k_near(CorrArgs a) {
       // (2) FP32 replay of the projection, margin 0.3*meshSize
       else {
         if (lane == 0) atomicAdd(a.cnt + 8, 1ull);
-        if ((double)projection_dist32(a.rep + (size_t)cell * a.m * a.nlon * 24, a.m, a.nlon, xt, th0, phi0) >
+        if ((double)projection_dist32(PF, a.rep + (size_t)cell * a.m * a.nlon * 24, a.m, a.nlon, xt, th0, phi0) >
             2.3 * msz)
           skip = true;
       }
       if (skip && !a.verify) continue;
     }
-    if (lane == 0) atomicAdd(a.cnt + 9, 1ull);
-    find_projection(sx, a.m, a.nlon, xt, th0, phi0, x0);
+    if (lane == 0 && !a.list) atomicAdd(a.cnt + 9, 1ull);  // a listed item was counted by k_near_proj
+    project64(PL, sx, a.G, xt, th0, phi0, x0);
     const double c1 = a.c1, c2 = a.c2 * a.Bc[a.celltype[cell]];
     SplW W;
     double a30[3];
@@ -683,7 +582,7 @@ __global__ void __launch_bounds__(128) k_near(CorrArgs a) {
     spline_eval(set_ptr(a, cell, SPL_A3), W, 3, a30);
     double dist = a30[0] * (xt[0] - x0[0]) + a30[1] * (xt[1] - x0[1]) + a30[2] * (xt[2] - x0[2]);
     if (dist > 2 * msz) continue;
-    if (lane == 0) {
+    if (lane == 0 && !a.list) {
       atomicAdd(a.cnt + 3, 1ull);
       if (skip) atomicAdd(a.cnt + 6, 1ull);  // a screened item that needs a correction
     }
@@ -715,138 +614,159 @@ __global__ void __launch_bounds__(128) k_near(CorrArgs a) {
   }
 }
 
-// The FP32 modes' FP64 pass over their short list, staged so that its work
-// spreads evenly over the SMs: with one warp per item the pass waited on its
-// slowest items.  (1) k_near_proj, one warp per item: the projection and the
-// correction test; (2) k_near_units, one warp per quadrature (the first
-// re-adds of every item, then the second ones, then the subtracts), each
-// keeping its warp sum; (3) k_near_fin, one thread per item: the combination
-// of RBC_NearSingInt (ModRbcSingInt.F90:103-160) in the order k_near uses, so the
-// sums are k_near's.  Entries past its capacity (NEAR_STAGE_CAP, or less when
-// RBC3D_NEAR_STAGE_CAP asks for it) go through k_near.
+// The FP64 pass (over every candidate in the FP64 mode, over the short list of
+// the FP32 modes), staged so that its work spreads evenly over the SMs: with
+// one warp per item the pass waited on its slowest items.  (1) k_near_proj, a
+// half-warp per item: the projection and the correction test; the corrected
+// items' plans are listed; (2) k_near_units, one warp per quarter of a re-add
+// (the first re-adds of every item, then the second ones) or per subtract,
+// each keeping its warp sum; (3) k_near_fin, one thread per item: the
+// combination of RBC_NearSingInt (ModRbcSingInt.F90:103-160).  Corrected items
+// past its capacity (NEAR_STAGE_CAP, or less when RBC3D_NEAR_STAGE_CAP asks for
+// it) go through k_near.
 struct NearPlan {
   double th0, phi0, x0[3], xt[3], a30[3], dist, dist1;
-  int t, cell, two, ok;
+  int t, cell, two, pad;
 };
 static_assert(sizeof(NearPlan) <= 16 * sizeof(double), "plan slot");
+constexpr int NEAR_QUART = 4;                     // parts of a re-add
+constexpr int NEAR_PART = 3 * (2 * NEAR_QUART + 1);  // doubles a plan: subtract, first and second re-add
+
+// counters of the staged pass (near_queue): projection queue, unit queue, plans, overflow, k_near's queue
+enum { NQ_PROJ = 0, NQ_UNIT = 1, NQ_PLAN = 2, NQ_OVER = 3, NQ_REST = 4, NQ_N = 5 };
 
 __device__ __forceinline__ long long near_stage_count(const CorrArgs& a) {
-  unsigned long long n = *a.nlist;
-  if (n > (unsigned long long)a.cap) n = a.cap;
-  if (n > (unsigned long long)a.stage_cap) n = a.stage_cap;
-  return (long long)n;
+  const unsigned long long n = a.queue[NQ_PLAN];
+  return (long long)(n > (unsigned long long)a.stage_cap ? (unsigned long long)a.stage_cap : n);
 }
 
-__global__ void __launch_bounds__(128) k_near_proj(CorrArgs a, NearPlan* __restrict__ plan) {
-  const int lane = threadIdx.x & 31;
-  const long long n = near_stage_count(a);
+__global__ void __launch_bounds__(128) k_near_proj(CorrArgs a, NearPlan* __restrict__ plan, int* __restrict__ over) {
+  const int lane = threadIdx.x & 31, half = lane >> 4;
+  unsigned long long nn = a.list ? *a.nlist : *a.nitems;
+  const long long n = (long long)(nn > (unsigned long long)a.cap ? (unsigned long long)a.cap : nn);
+  ProjLane<double> PL;
+  PL.init(fmax(a.G.hx, a.G.hy));
+  unsigned done = 0, hits = 0;
   for (;;) {
     unsigned long long g0 = 0;
-    if (lane == 0) g0 = atomicAdd(a.queue, 1ull);
-    const long long cur = (long long)__shfl_sync(0xffffffffu, g0, 0);
-    if (cur >= n) break;
-    NearPlan P{};
-    const int4 item = a.items[a.list[cur]];
-    const int t = item.x, cell = item.y - 1, ilat0 = item.z, ilon0 = item.w;
-    if (cell >= 0 && cell < a.ncell) {
-      double th0 = a.th[ilat0], phi0 = a.phi[ilon0];
-      const size_t q0 = (size_t)cell * a.nlat * a.nlon + (size_t)ilon0 * a.nlat + ilat0;
-      double x0[3], xt[3];
-      for (int k = 0; k < 3; ++k) {
-        x0[k] = a.x[q0 + (size_t)k * a.npt];
-        double xx = a.tx[t + (size_t)k * a.nt] - x0[k];
-        xx = xx - round(xx * a.iL[k]) * a.L[k];
-        xt[k] = x0[k] + xx;
-      }
-      if (lane == 0) atomicAdd(a.cnt + 9, 1ull);
-      find_projection(set_ptr(a, cell, SPL_X), a.m, a.nlon, xt, th0, phi0, x0);
-      SplW W;
-      double a30[3];
-      spline_weights(th0, phi0, a.m, a.nlon, W);
-      spline_eval(set_ptr(a, cell, SPL_A3), W, 3, a30);
-      const double dist = a30[0] * (xt[0] - x0[0]) + a30[1] * (xt[1] - x0[1]) + a30[2] * (xt[2] - x0[2]);
-      if (!(dist > 2 * a.meshSize[cell])) {
-        if (lane == 0) atomicAdd(a.cnt + 3, 1ull);
-        const double sizePat = a.radius * sqrt(a.area[cell] / (4 * RBC3D_PI));
-        P.dist = dist;
-        P.dist1 = copysign(fabs(0.01 * sizePat), dist);
-        P.two = fabs(dist) < fabs(P.dist1) ? 1 : 0;
-        P.th0 = th0;
-        P.phi0 = phi0;
-        for (int k = 0; k < 3; ++k) {
-          P.x0[k] = x0[k];
-          P.xt[k] = xt[k];
-          P.a30[k] = a30[k];
-        }
-        P.t = t;
-        P.cell = cell;
-        P.ok = 1;
-      }
+    if (lane == 0) g0 = atomicAdd(a.queue + NQ_PROJ, 2ull);
+    const long long base = (long long)__shfl_sync(0xffffffffu, g0, 0);
+    if (base >= n) break;
+    bool on = base + half < n;
+    const long long cur = on ? base + half : base;
+    const int idx = a.list ? a.list[cur] : (int)cur;
+    const int4 item = a.items[idx];
+    int cell = item.y - 1;
+    if (cell < 0 || cell >= a.ncell) { on = false; cell = 0; }
+    double th0 = a.th[item.z], phi0 = a.phi[item.w];
+    const size_t q0 = (size_t)cell * a.nlat * a.nlon + (size_t)item.w * a.nlat + item.z;
+    double x0[3], xt[3];
+    for (int k = 0; k < 3; ++k) {
+      x0[k] = a.x[q0 + (size_t)k * a.npt];
+      double xx = a.tx[item.x + (size_t)k * a.nt] - x0[k];
+      xx = xx - round(xx * a.iL[k]) * a.L[k];
+      xt[k] = x0[k] + xx;
     }
-    if (lane == 0) plan[cur] = P;
+    project64(PL, set_ptr(a, cell, SPL_X), a.G, xt, th0, phi0, x0);
+    SplW W;
+    double a30[3];
+    spline_weights_g(th0, phi0, a.G, W);
+    spline_eval(set_ptr(a, cell, SPL_A3), W, 3, a30);
+    const double dist = a30[0] * (xt[0] - x0[0]) + a30[1] * (xt[1] - x0[1]) + a30[2] * (xt[2] - x0[2]);
+    if (!on || (lane & 15)) continue;
+    ++done;
+    if (dist > 2 * a.meshSize[cell]) continue;
+    ++hits;
+    const unsigned long long pos = atomicAdd(a.queue + NQ_PLAN, 1ull);
+    if (pos >= (unsigned long long)a.stage_cap) {
+      over[atomicAdd(a.queue + NQ_OVER, 1ull)] = idx;
+      continue;
+    }
+    NearPlan P;
+    const double sizePat = a.radius * sqrt(a.area[cell] / (4 * RBC3D_PI));
+    P.dist = dist;
+    P.dist1 = copysign(fabs(0.01 * sizePat), dist);
+    P.two = fabs(dist) < fabs(P.dist1) ? 1 : 0;
+    P.th0 = th0;
+    P.phi0 = phi0;
+    for (int k = 0; k < 3; ++k) {
+      P.x0[k] = x0[k];
+      P.xt[k] = xt[k];
+      P.a30[k] = a30[k];
+    }
+    P.t = item.x;
+    P.cell = cell;
+    P.pad = 0;
+    plan[pos] = P;
   }
+  if (done) atomicAdd(a.cnt + 9, (unsigned long long)done);
+  if (hits) atomicAdd(a.cnt + 3, (unsigned long long)hits);
 }
 
 __global__ void __launch_bounds__(128) k_near_units(CorrArgs a, const NearPlan* __restrict__ plan,
-                                                    double* __restrict__ part, unsigned long long* __restrict__ queue) {
+                                                    double* __restrict__ part) {
   const int lane = threadIdx.x & 31;
   const long long n = near_stage_count(a);
+  if (n == 0) return;
   for (;;) {
     unsigned long long g0 = 0;
-    if (lane == 0) g0 = atomicAdd(queue, 1ull);
+    if (lane == 0) g0 = atomicAdd(a.queue + NQ_UNIT, 1ull);
     const long long u = (long long)__shfl_sync(0xffffffffu, g0, 0);
-    if (u >= 3 * n) break;
+    if (u >= (2 * NEAR_QUART + 1) * n) break;
     const long long i = u % n;
-    // kind 0: re-add at xt (at xi1 when the target is within dist1);
-    // kind 1: re-add at x0 (only then); kind 2: subtract
-    const int kind = (int)(u / n);
+    // slot < NEAR_QUART: re-add at xt (at xi1 when the target is within
+    // dist1); then re-add at x0 (only then); last the subtract
+    const int slot = (int)(u / n), second = slot >= NEAR_QUART, q = slot - second * NEAR_QUART;
     const NearPlan P = plan[i];
-    if (!P.ok || (kind == 1 && !P.two)) continue;
     const double c2 = a.c2 * a.Bc[a.celltype[P.cell]];
     double dv[3];
-    if (kind == 0) {
-      double xi1[3];
-      for (int k = 0; k < 3; ++k) xi1[k] = P.x0[k] + P.dist1 * P.a30[k];
-      near_readd(a, P.cell, a.c1, c2, P.two ? xi1 : P.xt, P.x0, P.th0, P.phi0, a.radius, dv);
-    } else if (kind == 1) {
-      near_readd(a, P.cell, a.c1, c2, P.x0, P.x0, P.th0, P.phi0, a.radius, dv);
-    } else {
+    if (slot == 2 * NEAR_QUART) {
       near_subtract(a, P.cell, a.c1, c2, P.xt, P.th0, P.phi0, a.radius, a.rthr, dv);
+    } else {
+      if (second && !P.two) continue;
+      double xi[3];
+      for (int k = 0; k < 3; ++k) xi[k] = second ? P.x0[k] : P.two ? P.x0[k] + P.dist1 * P.a30[k] : P.xt[k];
+      near_readd(a, P.cell, a.c1, c2, xi, P.x0, P.th0, P.phi0, a.radius, dv, 16 / NEAR_QUART * q,
+                 16 / NEAR_QUART * (q + 1));
     }
-    if (lane == 0) {
-      const int o = kind == 2 ? 0 : (kind == 0 ? 3 : 6);
-      for (int k = 0; k < 3; ++k) part[9 * i + o + k] = dv[k];
-    }
+    if (lane == 0)
+      for (int k = 0; k < 3; ++k) part[NEAR_PART * i + 3 * slot + k] = dv[k];
   }
 }
 
 __global__ void k_near_fin(CorrArgs a, const NearPlan* __restrict__ plan, const double* __restrict__ part) {
   const long long n = near_stage_count(a);
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const NearPlan& P = plan[i];
-  if (!P.ok) return;
-  const double* S = part + 9 * i;
-  double dv[3] = {S[0], S[1], S[2]};
-  if (!P.two) {
-    for (int k = 0; k < 3; ++k) dv[k] += S[3 + k];
-  } else {
-    const double c2 = a.c2 * a.Bc[a.celltype[P.cell]];
-    double dv1[3] = {S[3], S[4], S[5]}, dv0[3] = {S[6], S[7], S[8]};
-    if (c2 != 0.) {
-      SplW W;
-      double dJ0[3], g0[3];
-      spline_weights(P.th0, P.phi0, a.m, a.nlon, W);
-      spline_eval(set_ptr(a, P.cell, SPL_DJ), W, 1, dJ0);
-      spline_eval(set_ptr(a, P.cell, SPL_G), W, 3, g0);
-      for (int k = 0; k < 3; ++k) g0[k] = g0[k] / dJ0[0];
-      for (int k = 0; k < 3; ++k)
-        dv0[k] = (P.dist > 0) ? dv0[k] + c2 * 4 * RBC3D_PI * g0[k] : dv0[k] - c2 * 4 * RBC3D_PI * g0[k];
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const NearPlan& P = plan[i];
+    const double* S = part + NEAR_PART * i;
+    double dv[3], dv1[3], dv0[3];
+    for (int k = 0; k < 3; ++k) {
+      dv[k] = S[6 * NEAR_QUART + k];
+      dv1[k] = dv0[k] = 0.;
+      for (int q = 0; q < NEAR_QUART; ++q) {
+        dv1[k] += S[3 * q + k];
+        if (P.two) dv0[k] += S[3 * (NEAR_QUART + q) + k];
+      }
     }
-    for (int k = 0; k < 3; ++k) dv[k] += dv0[k] + P.dist / P.dist1 * (dv1[k] - dv0[k]);
+    if (!P.two) {
+      for (int k = 0; k < 3; ++k) dv[k] += dv1[k];
+    } else {
+      const double c2 = a.c2 * a.Bc[a.celltype[P.cell]];
+      if (c2 != 0.) {
+        SplW W;
+        double dJ0[3], g0[3];
+        spline_weights(P.th0, P.phi0, a.m, a.nlon, W);
+        spline_eval(set_ptr(a, P.cell, SPL_DJ), W, 1, dJ0);
+        spline_eval(set_ptr(a, P.cell, SPL_G), W, 3, g0);
+        for (int k = 0; k < 3; ++k) g0[k] = g0[k] / dJ0[0];
+        for (int k = 0; k < 3; ++k)
+          dv0[k] = (P.dist > 0) ? dv0[k] + c2 * 4 * RBC3D_PI * g0[k] : dv0[k] - c2 * 4 * RBC3D_PI * g0[k];
+      }
+      for (int k = 0; k < 3; ++k) dv[k] += dv0[k] + P.dist / P.dist1 * (dv1[k] - dv0[k]);
+    }
+    const double iA = 1.0 / a.tA[P.t];
+    for (int k = 0; k < 3; ++k) atomicAdd(a.v + P.t + (size_t)k * a.nt, dv[k] * iA);
   }
-  const double iA = 1.0 / a.tA[P.t];
-  for (int k = 0; k < 3; ++k) atomicAdd(a.v + P.t + (size_t)k * a.nt, dv[k] * iA);
 }
 
 // The FP32 replay's node records: x and a3 of every spline node in FP32,
@@ -869,6 +789,7 @@ __global__ void k_rep_rec(long long nn, int per, const double* __restrict__ spl,
 // InterCellRepulsion (ModRepulsion.F90:270-402): one warp per cell point.
 struct RepArgs {
   int n, nv, nlat, nlon, m;
+  SplGrid G;
   const double* x;      // cell points, point layout (3 x n)
   const double* sx;     // sorted source positions (3 x n)
   const int4* smeta;    // (surf 1-based, ilat, ilon, point index)
@@ -942,7 +863,10 @@ __global__ void __launch_bounds__(128) k_inter_rep(RepArgs a) {
     }
     double th0 = a.th[m.y], phi0 = a.phi[m.z];
     const double* sx = a.spl + ((size_t)cell0 * SPL_NSET + SPL_X) * (size_t)a.m * a.nlon * SPL_NODE;
-    find_projection(sx, a.m, a.nlon, xtar, th0, phi0, x1);
+    const SplGrid G = a.G;
+    ProjLane<double> PL;
+    PL.init(fmax(G.hx, G.hy));
+    project64(PL, sx, G, xtar, th0, phi0, x1);
     double d2 = 0;
     for (int d = 0; d < 3; ++d) d2 += (xtar[d] - x1[d]) * (xtar[d] - x1[d]);
     dist1 = sqrt(d2);
@@ -1081,7 +1005,7 @@ rbc3d_status run_near_corr(rbc3d_ctx* ctx, int tlist, double c1, double c2, int 
   // FP32 modes: pairs closer than rthr were left out of the FP32 pair sum and
   // are added back by the FP64 pass (-1: the FP64 plain form left nothing out)
   a.rthr = (prec != RBC3D_FP64) ? near_rthr_now(ctx) : -1.0;
-  a.verify = ctx->verify_screen ? 1 : 0;
+  a.verify = a.screen && ctx->verify_screen ? 1 : 0;
   a.list = nullptr;
   a.nlist = nullptr;
   int nsm = 0, per_sm = 0;
@@ -1098,7 +1022,7 @@ rbc3d_status run_near_corr(rbc3d_ctx* ctx, int tlist, double c1, double c2, int 
     a.rep = ctx->rep_rec.p;
   }
   if (a.screen && !a.verify) {
-    // FP32 modes: geometric screen per thread, FP32 replay per warp, then the
+    // geometric screen per thread, FP32 replay per warp, then the
     // FP64 pass on what is left (counters: dcnt[8] replays, dcnt[10] listed)
     CUDA_TRY(ctx->near_l1.alloc(std::max(ctx->items_cap, 1)));
     CUDA_TRY(ctx->near_l2.alloc(std::max(ctx->items_cap, 1)));
@@ -1109,27 +1033,26 @@ rbc3d_status run_near_corr(rbc3d_ctx* ctx, int tlist, double c1, double c2, int 
     a.list = ctx->near_l2.p;
     a.nlist = ctx->dcnt.p + 10;
   }
-  CUDA_TRY(ctx->near_queue.alloc(2));
-  CUDA_TRY(cudaMemsetAsync(ctx->near_queue.p, 0, 2 * sizeof(unsigned long long), ctx->st));
+  CUDA_TRY(ctx->near_queue.alloc(NQ_N));
+  CUDA_TRY(cudaMemsetAsync(ctx->near_queue.p, 0, NQ_N * sizeof(unsigned long long), ctx->st));
   a.queue = ctx->near_queue.p;
-  a.list_start = 0;
   a.stage_cap = std::max(0, std::min(ctx->near_stage_cap, NEAR_STAGE_CAP));
-  if (a.list && a.stage_cap > 0) {  // the staged pass over the list's first stage_cap entries
-    CUDA_TRY(ctx->near_plan.alloc((size_t)a.stage_cap * 16));
-    CUDA_TRY(ctx->near_part.alloc((size_t)a.stage_cap * 9));
+  if (!a.verify) {  // the staged pass; k_near takes the corrected items past its capacity
+    CUDA_TRY(ctx->near_l1.alloc(std::max(ctx->items_cap, 1)));  // the screen's list is done with
+    CUDA_TRY(ctx->near_plan.alloc((size_t)std::max(a.stage_cap, 1) * 16));
+    CUDA_TRY(ctx->near_part.alloc((size_t)std::max(a.stage_cap, 1) * NEAR_PART));
     NearPlan* plan = reinterpret_cast<NearPlan*>(ctx->near_plan.p);
     int ps = 0, us = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k_near_proj, 128, 0));
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&us, k_near_units, 128, 0));
-    { k_near_proj<<<nsm * std::max(ps, 1), 128, 0, ctx->st>>>(a, plan); ++ctx->launches; }
-    { k_near_units<<<nsm * std::max(us, 1), 128, 0, ctx->st>>>(a, plan, ctx->near_part.p, ctx->near_queue.p + 1);
-      ++ctx->launches; }
-    { k_near_fin<<<(a.stage_cap + 127) / 128, 128, 0, ctx->st>>>(a, plan, ctx->near_part.p); ++ctx->launches; }
+    { k_near_proj<<<nsm * std::max(ps, 1), 128, 0, ctx->st>>>(a, plan, ctx->near_l1.p); ++ctx->launches; }
+    { k_near_units<<<nsm * std::max(us, 1), 128, 0, ctx->st>>>(a, plan, ctx->near_part.p); ++ctx->launches; }
+    { k_near_fin<<<nsm, 128, 0, ctx->st>>>(a, plan, ctx->near_part.p); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
-    // entries past the staged pass's capacity: k_near from there
-    a.list_start = a.stage_cap;
-    CUDA_TRY(cudaMemsetAsync(ctx->near_queue.p, 0, sizeof(unsigned long long), ctx->st));
+    a.list = ctx->near_l1.p;
+    a.nlist = ctx->near_queue.p + NQ_OVER;
   }
+  a.queue = ctx->near_queue.p + NQ_REST;
   CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_near, 128, 0));
   { k_near<<<nsm * std::max(per_sm, 1), 128, 0, ctx->st>>>(a); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());
@@ -1150,6 +1073,7 @@ extern "C" rbc3d_status rbc3d_inter_cell_repulsion(rbc3d_ctx* ctx, double epsDis
   if (W.nele > 0 && !W.cstart.p) return ctx_fail(ctx, RBC3D_ERR_STATE, "inter_cell_repulsion: wall lists not built");
   RepArgs a;
   a.n = n; a.nv = ctx->nlat * ctx->nlon; a.nlat = ctx->nlat; a.nlon = ctx->nlon; a.m = ctx->m;
+  a.G = spl_grid(ctx->m, ctx->nlon);
   a.x = ctx->x.p; a.sx = ctx->s_x.p; a.smeta = ctx->s_meta.p; a.cs = ctx->s_cstart.p; a.ce = ctx->s_cend.p;
   a.spl = ctx->spl.p; a.th = ctx->th.p; a.phi = ctx->phi.p;
   for (int d = 0; d < 3; ++d) { a.Nc[d] = ctx->hg.Nc[d]; a.L[d] = ctx->prm.Lb[d]; a.iL[d] = ctx->iLb[d]; }
