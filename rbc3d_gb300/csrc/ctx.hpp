@@ -232,10 +232,10 @@ struct rbc3d_ctx {
   WallState wall;
   WallSpec wspec;
 
-  // FP32M self patch: FP32 node records, per-(latitude, patch point) weights,
-  // target positions relative to the cell centre (hi/lo)
-  DBuf<float> mix_rec, mix_pw;
-  DBuf<char> mix_w;
+  // FP32M self patch: FP32 node records, the ring classes, target positions
+  // relative to the cell centre (hi/lo)
+  DBuf<float> mix_rec;
+  DBuf<char> mix_cls;
   DBuf<float4> mix_thi, mix_tlo;
   int mix_sets = 0;  // current FP32M node-record parts: bit 0 geometry, 1 f, 2 g
   bool phi_uniform = false;
@@ -355,8 +355,7 @@ rbc3d_status self_ring_tables(rbc3d_ctx* ctx, const std::vector<double>& c1, con
 rbc3d_status run_self_ring(rbc3d_ctx* ctx, int tlist, double c1, double c2);
 
 // selfmix.cu
-rbc3d_status self_mixed_grid(rbc3d_ctx* ctx, const std::vector<double>& thG, const std::vector<double>& phiA,
-                             const std::vector<double>& pw);
+rbc3d_status self_mixed_grid(rbc3d_ctx* ctx, const std::vector<RingClass>& R);
 rbc3d_status self_mixed_geom(rbc3d_ctx* ctx);
 rbc3d_status self_mixed_density(rbc3d_ctx* ctx, bool f, bool g);
 rbc3d_status run_self_mixed(rbc3d_ctx* ctx, int tlist, double c1, double c2);

@@ -5,19 +5,19 @@
 // The only cancellation-prone quantity of the patch quadrature is the
 // separation xx = x(patch point) - x(target), as small as 1e-2 for the first
 // radial ring.  Positions are stored relative to each cell's centre as FP32
-// (hi, lo) pairs computed in FP64, and each stencil node's offset from the
-// target, (X_hi - t_hi) + (X_lo - t_lo), is formed before the bicubic
-// weights are applied, so xx carries ~1e-7 relative error instead of the
-// ~1e-5 of plain FP32 positions.  Densities, normals, weights and the Ewald
-// kernel are FP32 (erfc as exp(-x^2) t Q(t), the fit of fit_erfcx),
-// accumulated with Kahan compensation per target.  Node records are read
-// as float4.  erfc is exp(-x^2) t Q(t) with the fitted
-// polynomial of fit_erfcx (pair.cu).
+// (hi, lo) pairs computed in FP64, and the stencil's values enter as offsets
+// (X_hi - T_hi) + (X_lo - T_lo) from nearby target positions, formed before any
+// weight is applied, so xx carries ~1e-7 relative error instead of the ~1e-5 of
+// plain FP32 positions.  Densities, normals, weights and the Ewald kernel are
+// FP32 (erfc as exp(-x^2) t Q(t), the fit of fit_erfcx, pair.cu), accumulated
+// with Kahan compensation per target.
 //
-// Patch geometry: the bicubic weights of patch point q of a target at
-// latitude ilat0 depend only on (ilat0, q); longitudes shift the stencil by
-// whole grid columns (phiG = atan2(...) + phi0 with phi0 on the grid), so they
-// are tabulated once per grid.
+// By latitude rings, as selfring.cu and selfff.cu: per point pair (class) of a
+// ring and column j the theta part once, relative to the ring's target T_j of
+// that column; a point of target q takes it from the columns j and j + 1 with
+// T_j - T_q and T_j+1 - T_q added.  About 240 packed instructions for the two
+// points of a class and 0.4 KB of loads a point, against 300 scalar ones and
+// 0.8 KB a point with one warp per target and 16-term sums, bound by L1.
 #include <cmath>
 #include <vector>
 
@@ -27,14 +27,17 @@ namespace {
 
 inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
-// Node record (52 floats = 13 float4): x hi(3) lo(3) u1(3) u2(3) u12(3) |
-// a3 u u1 u2 u12 (12) | FdetJ (12) | GdetJ (12) | pad(1)
-constexpr int REC = 52;
-constexpr int OFF_X = 0, OFF_A3 = 15, OFF_F = 27, OFF_G = 39;
+// Node record: 13 float4 in column order, [cell][row][MIX_ROW][column]: slot d (u,
+// u_th, u_ph, u_thph) has the 12 values x, f, g, a3 in quads 3 d .. 3 d + 2 (x
+// of slot u: the hi parts relative to the cell centre), quad 12 the lo parts.
+constexpr int MIX_ROW = 13;
 
-struct SelfW {
-  int i1, j1b;
-  float cx[4], cy[4];
+// A class of patch points (RingClass): theta weights of (u, u', u_th, u'_th),
+// per side the phi weights of (U_j, U_j+1, D_j, D_j+1), the sides' quadrature
+// weights (0 for a point without mirror image, which stands on both sides).
+struct MixClass {
+  int i1, j[2], pad;
+  float x[4], y[2][4], w[2], pad2[2];
 };
 
 // mean of each cell's grid points (x SoA, 3 x npt)
@@ -56,44 +59,45 @@ __global__ void k_cell_mean(int nv, long long npt, const double* __restrict__ x,
   }
 }
 
-__global__ void k_mix_geom(int ncell, int m, int n, const double* __restrict__ spl, const double* __restrict__ xc,
-                           float* __restrict__ out) {
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long per = (long long)m * n;
-  if (idx >= (long long)ncell * per) return;
-  int cell = (int)(idx / per);
-  int node = (int)(idx - (long long)cell * per);
-  const double* sx = spl + (((size_t)cell * SPL_NSET + SPL_X) * per + node) * SPL_NODE;
-  const double* sa = spl + (((size_t)cell * SPL_NSET + SPL_A3) * per + node) * SPL_NODE;
-  float* o = out + ((size_t)cell * per + node) * REC;
-  for (int k = 0; k < 3; ++k) {
-    double r = sx[k] - xc[3 * cell + k];
-    float h = (float)r;
-    o[OFF_X + k] = h;
-    o[OFF_X + 3 + k] = (float)(r - (double)h);
-    o[OFF_X + 6 + k] = (float)sx[3 + k];   // u1
-    o[OFF_X + 9 + k] = (float)sx[6 + k];   // u2
-    o[OFF_X + 12 + k] = (float)sx[9 + k];  // u12
+// Node records of the sets in `sets` (bit 0 x and a3, 1 f, 2 g): a block takes
+// 4 rows x 16 columns of one cell through shared memory (the tables are in row
+// order, the records in column order).
+__global__ void __launch_bounds__(128) k_mix_rec(int m, int n, const double* __restrict__ spl,
+                                                 const double* __restrict__ xc, float* __restrict__ out, int sets) {
+  __shared__ float s[4][16][4][SPL_NODE];  // set x f g a3, column, row, value
+  __shared__ float lo[16][4][3];
+  const int nti = (m + 3) / 4, ntj = (n + 15) / 16;
+  const int jt = blockIdx.x % ntj, it = (blockIdx.x / ntj) % nti, cell = blockIdx.x / (ntj * nti);
+  const int src[4] = {SPL_X, SPL_F, SPL_G, SPL_A3}, bit[4] = {1, 2, 4, 1};
+  for (int k = 0; k < 4; ++k) {
+    if (!(sets & bit[k])) continue;
+    const double* in = spl + ((size_t)cell * SPL_NSET + src[k]) * (size_t)m * n * SPL_NODE;
+    for (int e = threadIdx.x; e < 16 * 4 * SPL_NODE; e += blockDim.x) {
+      const int q = e % SPL_NODE, r = (e / SPL_NODE) % 4, c = e / (4 * SPL_NODE);
+      const int j = 16 * jt + c, i = 4 * it + r;
+      if (j >= n || i >= m) continue;
+      double v = in[((size_t)j * m + i) * SPL_NODE + q];
+      if (k == 0 && q < 3) {
+        v -= xc[3 * cell + q];
+        lo[c][r][q] = (float)(v - (double)(float)v);
+      }
+      s[k][c][r][q] = (float)v;
+    }
   }
-  for (int k = 0; k < 12; ++k) o[OFF_A3 + k] = (float)sa[k];
-  o[REC - 1] = 0.f;
-}
-
-__global__ void k_mix_dens(int ncell, int m, int n, const double* __restrict__ spl, float* __restrict__ out, int do_f,
-                           int do_g) {
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long per = (long long)m * n;
-  if (idx >= (long long)ncell * per) return;
-  int cell = (int)(idx / per);
-  int node = (int)(idx - (long long)cell * per);
-  float* o = out + ((size_t)cell * per + node) * REC;
-  if (do_f) {
-    const double* s = spl + (((size_t)cell * SPL_NSET + SPL_F) * per + node) * SPL_NODE;
-    for (int k = 0; k < 12; ++k) o[OFF_F + k] = (float)s[k];
-  }
-  if (do_g) {
-    const double* s = spl + (((size_t)cell * SPL_NSET + SPL_G) * per + node) * SPL_NODE;
-    for (int k = 0; k < 12; ++k) o[OFF_G + k] = (float)s[k];
+  __syncthreads();
+  for (int e = threadIdx.x; e < 4 * MIX_ROW * 16; e += blockDim.x) {
+    const int c = e % 16, dq = (e / 16) % MIX_ROW, r = e / (16 * MIX_ROW);
+    const int j = 16 * jt + c, i = 4 * it + r;
+    if (j >= n || i >= m) continue;
+    float* o = out + 4 * ((((size_t)cell * m + i) * MIX_ROW + dq) * n + j);
+    for (int k = 0; k < 4; ++k) {
+      if (dq == 12) {
+        if (sets & 1) o[k] = k < 3 ? lo[c][r][k] : 0.f;
+        continue;
+      }
+      const int val = 4 * (dq % 3) + k, set = val / 3;
+      if (sets & bit[set]) o[k] = s[set][c][r][3 * (dq / 3) + val % 3];
+    }
   }
 }
 
@@ -121,12 +125,11 @@ __global__ void k_mix_targets(int npt, int nlat, int nlon, int m, const double* 
 }
 
 struct MixArgs {
-  int nt, ncell, nlat, nlon, m, NQ, nrad;
+  int nt, ncell, nlat, nlon, m, NC, G, parts;
   const double* tA;
   double* v;
-  const float* rec;
-  const SelfW* W;
-  const float* pw;
+  const float4* rec;
+  const MixClass* cls;  // [latitude][NC]
   const float4* thi;
   const float4* tlo;
   const int* celltype;
@@ -136,134 +139,189 @@ struct MixArgs {
   float erfcx_q[ERFCX_DEG + 1];
 };
 
-// The 13 float4 of a node record in registers (only those the terms need).
-template <bool DL>
-__device__ __forceinline__ void load_rec(const float* r, float* v) {
-  const float4* r4 = reinterpret_cast<const float4*>(r);
-#pragma unroll
-  for (int i = 0; i < REC / 4; ++i) {
-    // SL needs x (floats 0-14) and F (27-38): float4 0-3 and 6-9
-    if (!DL && (i == 4 || i == 5 || i >= 10)) continue;
-    const float4 q = __ldg(r4 + i);
-    v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
-  }
-}
+__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// one warp per target; warps of a block walk one latitude ring so that
-// neighbouring warps share most stencil nodes in L1
-template <bool DL>
-__global__ void __launch_bounds__(256) k_self_mix(MixArgs a) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int nv = a.nlat * a.nlon;
-  if (w >= a.ncell * nv) return;
-  const int cell = w / nv, rr = w - cell * nv;
-  const int ilon0 = rr % a.nlon, ilat0 = rr / a.nlon;
-  const int p = cell * nv + ilon0 * a.nlat + ilat0;
-  const float c1 = a.c1;
-  const float c2m = DL ? (float)(a.c2 * a.B[a.celltype[cell]]) : 0.f;
-  const float4 th4 = a.thi[p], tl4 = a.tlo[p];
-  const float th_[3] = {th4.x, th4.y, th4.z}, tl_[3] = {tl4.x, tl4.y, tl4.z};
-  const float* base = a.rec + (size_t)cell * a.m * a.nlon * REC;
-  Kahan3 acc;
-  acc.zero();
-  for (int q = lane; q < a.NQ; q += 32) {
-    const SelfW e = a.W[ilat0 * a.NQ + q];
-    const int irad = q % a.nrad;
-    int j1 = e.j1b + ilon0;
-    j1 = imod(j1, a.nlon);
-    const int j2 = (j1 + 1 == a.nlon) ? 0 : j1 + 1;
-    const int i1 = e.i1, i2 = (i1 + 1 == a.m) ? 0 : i1 + 1;
-    const int nodes[4] = {i1 + a.m * j1, i1 + a.m * j2, i2 + a.m * j1, i2 + a.m * j2};
-    // weights of (u, u1, u2, u12) per node (Spline_Interp, ModSpline.F90:172-185)
-    const float wu[4] = {e.cx[0] * e.cy[0], e.cx[0] * e.cy[1], e.cx[1] * e.cy[0], e.cx[1] * e.cy[1]};
-    const float w1[4] = {e.cx[2] * e.cy[0], e.cx[2] * e.cy[1], e.cx[3] * e.cy[0], e.cx[3] * e.cy[1]};
-    const float w2[4] = {e.cx[0] * e.cy[2], e.cx[0] * e.cy[3], e.cx[1] * e.cy[2], e.cx[1] * e.cy[3]};
-    const float w12[4] = {e.cx[2] * e.cy[2], e.cx[2] * e.cy[3], e.cx[3] * e.cy[2], e.cx[3] * e.cy[3]};
-    float xx[3] = {0, 0, 0}, F[3] = {0, 0, 0}, G[3] = {0, 0, 0}, A3[3] = {0, 0, 0};
+// One block: a ring of G cells, thread = column (cols = G nlon; more than 256
+// columns: several a thread); values in pairs (x.x x.y) (x.z f.x) (f.y f.z)
+// (g.x g.y) (g.z a.x) (a.y a.z).  One barrier a class: the theta parts
+// alternate between two buffers; the targets' sums lie in shared memory, a side
+// each, so no two threads meet between two barriers.
+template <bool SL, bool DL>
+__global__ void __launch_bounds__(256, 3) k_self_mix(MixArgs a) {
+  constexpr int NP = DL ? (SL ? 6 : 5) : 3;  // pairs kept; without SL (f.y f.z) is left out
+  extern __shared__ __align__(16) unsigned char smem_mix[];
+  const int nlon = a.nlon, cols = a.G * nlon;
+  float4* ex = reinterpret_cast<float4*>(smem_mix);              // [2][NP][cols]: U pair, D pair
+  float2* acc = reinterpret_cast<float2*>(ex + 2 * NP * cols);   // [2 sides][3][cols]: Kahan sum and error
+  float2* sT = acc + 6 * cols;                                   // [3][cols]: target position hi, lo
+  int b = blockIdx.x;
+  const int part = b % a.parts; b /= a.parts;
+  const int ring = b % a.nlat, cell0 = (b / a.nlat) * a.G;
+  const int ncol = min(a.G, a.ncell - cell0) * nlon, nv = a.nlat * nlon;
+  for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
+    const int lc = t / nlon, j = t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
+    const float4 h = a.thi[p], l = a.tlo[p];
+    sT[t] = make_float2(h.x, l.x); sT[cols + t] = make_float2(h.y, l.y); sT[2 * cols + t] = make_float2(h.z, l.z);
+    for (int k = 0; k < 6; ++k) acc[k * cols + t] = make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+  const int k0 = (int)((long long)a.NC * part / a.parts), k1 = (int)((long long)a.NC * (part + 1) / a.parts);
+  const MixClass* cls = a.cls + (size_t)ring * a.NC;
+  for (int kc = k0; kc < k1; ++kc) {
+    const MixClass& c = cls[kc];
+    float4* buf = ex + (size_t)((kc & 1) * NP) * cols;
+    const int i1 = c.i1, i2 = i1 + 1 == a.m ? 0 : i1 + 1;
+    for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
+      const int lc = t / nlon, j = t - lc * nlon;
+      const float4* r1 = a.rec + ((size_t)(cell0 + lc) * a.m + i1) * MIX_ROW * nlon + j;
+      const float4* r2 = a.rec + ((size_t)(cell0 + lc) * a.m + i2) * MIX_ROW * nlon + j;
+      const float4 w = *reinterpret_cast<const float4*>(c.x);
+      const float2 w0 = dup(w.x), w1 = dup(w.y), w2 = dup(w.z), w3 = dup(w.w);
+      const float2 T0 = sT[t], T1 = sT[cols + t], T2 = sT[2 * cols + t];
+      const float4 l1 = __ldg(r1 + 12 * nlon), l2 = __ldg(r2 + 12 * nlon);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float v[REC];
-      load_rec<DL>(base + (size_t)nodes[k] * REC, v);
+      for (int q = 0; q < (DL ? 3 : 2); ++q) {
+        float4 p[4], r[4];  // the quad's slots of row i1 and of row i2
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float d = __fadd_rn(__fsub_rn(v[OFF_X + c], th_[c]), __fsub_rn(v[OFF_X + 3 + c], tl_[c]));
-        xx[c] += wu[k] * d + w1[k] * v[OFF_X + 6 + c] + w2[k] * v[OFF_X + 9 + c] + w12[k] * v[OFF_X + 12 + c];
-        F[c] += wu[k] * v[OFF_F + c] + w1[k] * v[OFF_F + 3 + c] + w2[k] * v[OFF_F + 6 + c] + w12[k] * v[OFF_F + 9 + c];
-        if (DL) {
-          G[c] += wu[k] * v[OFF_G + c] + w1[k] * v[OFF_G + 3 + c] + w2[k] * v[OFF_G + 6 + c] +
-                  w12[k] * v[OFF_G + 9 + c];
-          A3[c] += wu[k] * v[OFF_A3 + c] + w1[k] * v[OFF_A3 + 3 + c] + w2[k] * v[OFF_A3 + 6 + c] +
-                   w12[k] * v[OFF_A3 + 9 + c];
+        for (int d = 0; d < 4; ++d) { p[d] = __ldg(r1 + (3 * d + q) * nlon); r[d] = __ldg(r2 + (3 * d + q) * nlon); }
+        if (q == 0) {  // x as offsets from T_j (f.x passes unchanged)
+          const float2 hxy = make_float2(T0.x, T1.x), lxy = make_float2(T0.y, T1.y);
+          float2 v = __fadd2_rn(sub2(make_float2(p[0].x, p[0].y), hxy), sub2(make_float2(l1.x, l1.y), lxy));
+          p[0].x = v.x; p[0].y = v.y;
+          v = __fadd2_rn(sub2(make_float2(r[0].x, r[0].y), hxy), sub2(make_float2(l2.x, l2.y), lxy));
+          r[0].x = v.x; r[0].y = v.y;
+          p[0].z = __fadd_rn(__fsub_rn(p[0].z, T2.x), __fsub_rn(l1.z, T2.y));
+          r[0].z = __fadd_rn(__fsub_rn(r[0].z, T2.x), __fsub_rn(l2.z, T2.y));
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int P = 2 * q + e;
+          if ((!DL && P >= 3) || (!SL && P == 2)) continue;
+          const int S = (!SL && P > 2) ? P - 1 : P;
+          auto lo = [&](const float4& v) { return e ? make_float2(v.z, v.w) : make_float2(v.x, v.y); };
+          const float2 U = fma2(w3, lo(r[1]), fma2(w2, lo(p[1]), fma2(w1, lo(r[0]), mul2(w0, lo(p[0])))));
+          const float2 D = fma2(w3, lo(r[3]), fma2(w2, lo(p[3]), fma2(w1, lo(r[2]), mul2(w0, lo(p[2])))));
+          buf[(size_t)S * cols + t] = make_float4(U.x, U.y, D.x, D.y);
         }
       }
     }
-    const float r2 = xx[0] * xx[0] + xx[1] * xx[1] + xx[2] * xx[2];
-    if (r2 >= a.rc2) continue;  // rr >= rc (ModRbcSingInt.F90:65)
-    const float rinv = rsqrtf(r2), rv = r2 * rinv, ir2 = rinv * rinv;
-    const float st = rv * a.sqpa, ex = __expf(-st * st);
-    // erfc(st) = exp(-st^2) t Q(t), t = 1/(1 + st/2) (fit_erfcx)
-    const float tq = __fdividef(1.f, fmaf(0.5f, st, 1.f));
-    float Qp = a.erfcx_q[ERFCX_DEG];
+    __syncthreads();
+    for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
+      const int lc = t / nlon, j = t - lc * nlon, base = t - j;
+      const int tn = j + 1 == nlon ? base : t + 1;
+      const int qs[2] = {base + (j >= c.j[0] ? j - c.j[0] : j - c.j[0] + nlon),
+                         base + (j >= c.j[1] ? j - c.j[1] : j - c.j[1] + nlon)};
+      float2 val[2][6];
+      {
+        float2 Tj[3], Tn[3];
 #pragma unroll
-    for (int k = ERFCX_DEG - 1; k >= 0; --k) Qp = fmaf(Qp, tq, a.erfcx_q[k]);
-    const float e1 = ex * (tq * Qp), e2 = a.two_isqa * ex;
-    const float wq = a.pw[irad];
-    float v0 = 0.f, v1 = 0.f, v2 = 0.f;
-    if (c1 != 0.f) {
-      const float A = (e1 * rinv + e2) * ir2, Bc = e1 * rinv - e2;
-      const float f0 = wq * F[0], f1 = wq * F[1], f2 = wq * F[2];
-      const float d = xx[0] * f0 + xx[1] * f1 + xx[2] * f2;
-      v0 = c1 * (A * xx[0] * d + Bc * f0);
-      v1 = c1 * (A * xx[1] * d + Bc * f1);
-      v2 = c1 * (A * xx[2] * d + Bc * f2);
+        for (int k = 0; k < 3; ++k) { Tj[k] = sT[k * cols + t]; Tn[k] = sT[k * cols + tn]; }
+#pragma unroll
+        for (int P = 0; P < 6; ++P) {
+          if ((!DL && P >= 3) || (!SL && P == 2)) continue;
+          const int S = (!SL && P > 2) ? P - 1 : P;
+          const float4 A = buf[(size_t)S * cols + t], B = buf[(size_t)S * cols + tn];
+#pragma unroll
+          for (int side = 0; side < 2; ++side) {
+            const float4 y = *reinterpret_cast<const float4*>(c.y[side]);
+            float2 U0 = make_float2(A.x, A.y), U1 = make_float2(B.x, B.y);
+            if (P < 2) {  // x: offsets from T_q
+              const int q = qs[side];
+              const float2 a0 = sT[2 * P * cols + q], z = make_float2(0.f, 0.f);
+              const float2 a1 = P == 0 ? sT[cols + q] : z, j1 = P == 0 ? Tj[1] : z, n1 = P == 0 ? Tn[1] : z;
+              U0 = __fadd2_rn(U0, __fadd2_rn(sub2(make_float2(Tj[2 * P].x, j1.x), make_float2(a0.x, a1.x)),
+                                             sub2(make_float2(Tj[2 * P].y, j1.y), make_float2(a0.y, a1.y))));
+              U1 = __fadd2_rn(U1, __fadd2_rn(sub2(make_float2(Tn[2 * P].x, n1.x), make_float2(a0.x, a1.x)),
+                                             sub2(make_float2(Tn[2 * P].y, n1.y), make_float2(a0.y, a1.y))));
+            }
+            val[side][P] = fma2(dup(y.w), make_float2(B.z, B.w),
+                                fma2(dup(y.z), make_float2(A.z, A.w), fma2(dup(y.y), U1, mul2(dup(y.x), U0))));
+          }
+        }
+      }
+      // both points at once: x = side 0, y = side 1
+      auto vx = [&](int P) { return make_float2(val[0][P].x, val[1][P].x); };
+      auto vy = [&](int P) { return make_float2(val[0][P].y, val[1][P].y); };
+      const float2 xx = vx(0), yy = vy(0), zz = vx(1);
+      float2 r2 = fma2(xx, xx, fma2(yy, yy, mul2(zz, zz)));
+      const bool ok[2] = {r2.x < a.rc2, r2.y < a.rc2};  // not rr >= rc (ModRbcSingInt.F90:65)
+      r2 = make_float2(ok[0] ? r2.x : 1.f, ok[1] ? r2.y : 1.f);
+      const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y)), ir2 = mul2(ri, ri);
+      const float2 st = mul2(mul2(r2, ri), dup(a.sqpa));
+      const float2 exn = make_float2(__expf(-st.x * st.x), __expf(-st.y * st.y));
+      // erfc(st) = exp(-st^2) t Q(t), t = 1/(1 + st/2) (fit_erfcx)
+      const float2 den = fma2(dup(0.5f), st, dup(1.f)), tq = make_float2(__fdividef(1.f, den.x), __fdividef(1.f, den.y));
+      float2 Q = dup(a.erfcx_q[ERFCX_DEG]);
+#pragma unroll
+      for (int k = ERFCX_DEG - 1; k >= 0; --k) Q = fma2(Q, tq, dup(a.erfcx_q[k]));
+      const float2 e1 = mul2(exn, mul2(tq, Q)), wq = *reinterpret_cast<const float2*>(c.w);
+      float2 cx, cf;  // dv = cx xx + cf f
+      if (SL) {
+        const float2 e1r = mul2(e1, ri), e2 = mul2(dup(a.two_isqa), exn), sw = mul2(dup(a.c1), wq);
+        const float2 d = fma2(xx, vy(1), fma2(yy, vx(2), mul2(zz, vy(2))));
+        cx = mul2(mul2(sw, mul2(__fadd2_rn(e1r, e2), ir2)), d);
+        cf = mul2(sw, sub2(e1r, e2));
+      }
+      if (DL) {
+        const float c2m = (float)(a.c2 * a.B[a.celltype[cell0 + lc]]);
+        const float2 cdl = mul2(dup(a.m8_ispi), fma2(exn, mul2(st, fma2(st, st, dup(1.5f))), mul2(dup(a.q75_spi), e1)));
+        const float2 Ad = mul2(mul2(mul2(cdl, ir2), ir2), ri);
+        const float2 dg = fma2(xx, vx(3), fma2(yy, vy(3), mul2(zz, vx(4))));
+        const float2 da = fma2(xx, vy(4), fma2(yy, vx(5), mul2(zz, vy(5))));
+        const float2 tt = mul2(mul2(mul2(dup(c2m), wq), Ad), mul2(dg, da));
+        cx = SL ? __fadd2_rn(cx, tt) : tt;
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        float2 v = mul2(cx, k == 0 ? xx : k == 1 ? yy : zz);
+        if (SL) v = fma2(cf, k == 0 ? vy(1) : k == 1 ? vx(2) : vy(2), v);
+        float2* s0 = acc + k * cols + qs[0];
+        float2* s1 = acc + (3 + k) * cols + qs[1];
+        const float2 z0 = *s0, z1 = *s1;  // (sum, error)
+        const float2 sum = make_float2(z0.x, z1.x), y = sub2(v, make_float2(z0.y, z1.y));
+        const float2 n = __fadd2_rn(sum, y), err = sub2(sub2(n, sum), y);
+        if (ok[0]) *s0 = make_float2(n.x, err.x);
+        if (ok[1]) *s1 = make_float2(n.y, err.y);
+      }
     }
-    if (DL) {
-      const float cdl = a.m8_ispi * (ex * (st * (1.5f + st * st)) + a.q75_spi * e1);
-      const float Ad = cdl * ir2 * ir2 * rinv;
-      const float dg = wq * (xx[0] * G[0] + xx[1] * G[1] + xx[2] * G[2]);
-      const float da = xx[0] * A3[0] + xx[1] * A3[1] + xx[2] * A3[2];
-      const float t = c2m * Ad * dg * da;
-      v0 += t * xx[0]; v1 += t * xx[1]; v2 += t * xx[2];
-    }
-    acc.add(0, v0);
-    acc.add(1, v1);
-    acc.add(2, v2);
   }
-  double dv[3];
-  for (int k = 0; k < 3; ++k) dv[k] = warp_sum((double)acc.s[k] - (double)acc.c[k]);
-  if (lane == 0) {
-    double iA = 1.0 / a.tA[p];
-    for (int k = 0; k < 3; ++k) a.v[p + (size_t)k * a.nt] += dv[k] * iA;
+  __syncthreads();
+  for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
+    const int lc = t / nlon, j = t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
+    const double iA = 1.0 / a.tA[p];
+    for (int k = 0; k < 3; ++k) {
+      const float2 z0 = acc[k * cols + t], z1 = acc[(3 + k) * cols + t];
+      const double dv = (((double)z0.x - (double)z0.y) + ((double)z1.x - (double)z1.y)) * iA;
+      if (a.parts == 1) a.v[p + (size_t)k * a.nt] += dv;
+      else atomicAdd(a.v + p + (size_t)k * a.nt, dv);
+    }
   }
 }
 
 }  // namespace
 
-// Patch weights per (target latitude, patch point): from thG and the atan2
-// part of phiG of RbcPolarPatch_Create.
-rbc3d_status self_mixed_grid(rbc3d_ctx* ctx, const std::vector<double>& thG, const std::vector<double>& phiA,
-                             const std::vector<double>& pw) {
-  const int NQ = ctx->nrad * ctx->nazm, m = ctx->m, n = ctx->nlon;
-  const double ihx = m / RBC3D_TWO_PI, ihy = n / RBC3D_TWO_PI;
-  const double hx = RBC3D_TWO_PI / m, hy = RBC3D_TWO_PI / n;
-  std::vector<SelfW> W((size_t)ctx->nlat * NQ);
-  for (size_t i = 0; i < W.size(); ++i) {
-    double x = thG[i] * ihx, y = phiA[i] * ihy;
-    int i1 = (int)std::floor(x), j1 = (int)std::floor(y);
-    double s = x - i1, t = y - j1;
-    SelfW e;
-    e.i1 = ((i1 % m) + m) % m;
-    e.j1b = j1;
-    e.cx[0] = (float)(1 + s * s * (-3. + 2. * s)); e.cx[1] = (float)(s * s * (3. - 2. * s));
-    e.cx[2] = (float)(hx * s * (1. + s * (-2. + s))); e.cx[3] = (float)(hx * s * s * (-1. + s));
-    e.cy[0] = (float)(1 + t * t * (-3. + 2. * t)); e.cy[1] = (float)(t * t * (3. - 2. * t));
-    e.cy[2] = (float)(hy * t * (1. + t * (-2. + t))); e.cy[3] = (float)(hy * t * t * (-1. + t));
-    W[i] = e;
+// The ring classes in FP32.
+rbc3d_status self_mixed_grid(rbc3d_ctx* ctx, const std::vector<RingClass>& R) {
+  std::vector<MixClass> C(R.size());
+  for (size_t i = 0; i < R.size(); ++i) {
+    const RingClass& r = R[i];
+    const bool two = r.j[1] >= 0;
+    MixClass c{};
+    c.i1 = r.i1; c.j[0] = r.j[0]; c.j[1] = r.j[two];
+    c.x[0] = (float)(1. - r.x[0]);
+    for (int k = 0; k < 3; ++k) c.x[1 + k] = (float)r.x[k];
+    for (int s = 0; s < 2; ++s) {
+      const double* y = r.y[s && two];
+      c.y[s][0] = (float)(1. - y[0]);
+      for (int k = 0; k < 3; ++k) c.y[s][1 + k] = (float)y[k];
+    }
+    c.w[0] = (float)r.w; c.w[1] = two ? (float)r.w : 0.f;
+    C[i] = c;
   }
-  std::vector<float> pwf(pw.begin(), pw.end());
-  CUDA_TRY(ctx->mix_w.upload((const char*)W.data(), W.size() * sizeof(SelfW), ctx->st));
-  CUDA_TRY(ctx->mix_pw.upload(pwf.data(), pwf.size(), ctx->st));
+  CUDA_TRY(ctx->mix_cls.upload((const char*)C.data(), C.size() * sizeof(MixClass), ctx->st));
   CUDA_TRY(cudaStreamSynchronize(ctx->st));
   return RBC3D_OK;
 }
@@ -298,32 +356,36 @@ rbc3d_status self_mixed_density(rbc3d_ctx* ctx, bool f, bool g) {
 rbc3d_status run_self_mixed(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   TargetSet& t = ctx->tl[tlist];
   if (tlist != RBC3D_TLIST_RBC || t.n == 0 || ctx->ncell == 0) return RBC3D_OK;
+  const bool sl = c1 != 0 && ctx->has_f, dl = c2 != 0 && ctx->has_g;
+  if (!sl && !dl) return RBC3D_OK;
+  const int np = dl ? (sl ? 6 : 5) : 3;
+  auto smem = [&](int G) {
+    const size_t cols = (size_t)G * ctx->nlon;
+    return sizeof(float4) * 2 * np * cols + sizeof(float2) * 9 * cols;
+  };
+  // a ring wider than shared memory holds (about 850 columns) goes to the FP64 patch
+  if (smem(1) > 227 * 1024) return run_self_corr(ctx, tlist, sl ? c1 : 0., dl ? c2 : 0.);
   // FP32 node records of the current geometry and densities (bit 0 geometry, 1 f, 2 g)
-  const long long per = (long long)ctx->m * ctx->nlon;
-  if (!ctx->mix_rec.p || ctx->mix_rec.n < (size_t)ctx->ncell * per * REC) {
-    CUDA_TRY(ctx->mix_rec.alloc((size_t)ctx->ncell * per * REC));
+  const size_t per = 4 * (size_t)ctx->m * ctx->nlon * MIX_ROW;
+  if (!ctx->mix_rec.p || ctx->mix_rec.n < ctx->ncell * per) {
+    CUDA_TRY(ctx->mix_rec.alloc(ctx->ncell * per));
     ctx->mix_sets = 0;
   }
-  if (!(ctx->mix_sets & 1)) {
-    { k_mix_geom<<<nblk(ctx->ncell * per, 256), 256, 0, ctx->st>>>(ctx->ncell, ctx->m, ctx->nlon, ctx->spl.p,
-                                                                    ctx->mix_xc.p, ctx->mix_rec.p); ++ctx->launches; }
-    ctx->mix_sets |= 1;
+  const int build = (1 | (sl ? 2 : 0) | (dl ? 4 : 0)) & ~ctx->mix_sets;
+  if (build) {
+    const long long nb = (long long)ctx->ncell * ((ctx->m + 3) / 4) * ((ctx->nlon + 15) / 16);
+    { k_mix_rec<<<(int)nb, 128, 0, ctx->st>>>(ctx->m, ctx->nlon, ctx->spl.p, ctx->mix_xc.p, ctx->mix_rec.p, build); ++ctx->launches; }
+    CUDA_TRY(cudaGetLastError());
+    ctx->mix_sets |= build;
   }
-  const bool df = ctx->has_f && !(ctx->mix_sets & 2), dg = ctx->has_g && !(ctx->mix_sets & 4);
-  if (df || dg) {
-    { k_mix_dens<<<nblk(ctx->ncell * per, 256), 256, 0, ctx->st>>>(ctx->ncell, ctx->m, ctx->nlon, ctx->spl.p,
-                                                                    ctx->mix_rec.p, df, dg); ++ctx->launches; }
-    ctx->mix_sets |= (df ? 2 : 0) | (dg ? 4 : 0);
-  }
-  CUDA_TRY(cudaGetLastError());
   MixArgs a;
   a.nt = t.n; a.ncell = ctx->ncell; a.nlat = ctx->nlat; a.nlon = ctx->nlon; a.m = ctx->m;
-  a.NQ = ctx->nrad * ctx->nazm; a.nrad = ctx->nrad;
-  a.tA = t.Acoef.p; a.v = t.v.p; a.rec = ctx->mix_rec.p; a.W = (const SelfW*)ctx->mix_w.p; a.pw = ctx->mix_pw.p;
+  a.tA = t.Acoef.p; a.v = t.v.p; a.rec = reinterpret_cast<const float4*>(ctx->mix_rec.p);
+  a.cls = reinterpret_cast<const MixClass*>(ctx->mix_cls.p);
   a.thi = ctx->mix_thi.p; a.tlo = ctx->mix_tlo.p; a.celltype = ctx->celltype.p;
   for (int l = 0; l < RBC3D_MAX_CELLTYPES; ++l) a.B[l] = ctx->Bcoef[l];
-  a.c1 = (float)((c1 != 0 && ctx->has_f) ? c1 : 0.0);
-  a.c2 = (float)((c2 != 0 && ctx->has_g) ? c2 : 0.0);
+  a.c1 = (float)c1;
+  a.c2 = (float)c2;
   a.rc2 = (float)(ctx->prm.rc * ctx->prm.rc);
   a.sqpa = (float)std::sqrt(RBC3D_PI / ctx->prm.alpha);
   a.two_isqa = (float)(2.0 / std::sqrt(ctx->prm.alpha));
@@ -331,9 +393,21 @@ rbc3d_status run_self_mixed(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   a.q75_spi = (float)(0.75 * std::sqrt(RBC3D_PI));
   erfcx_coeffs(ctx);
   for (int k = 0; k <= ERFCX_DEG; ++k) a.erfcx_q[k] = ctx->erfcx_q[k];
-  long long threads = (long long)t.n * 32;
-  if (a.c2 != 0.f) { k_self_mix<true><<<(int)((threads + 255) / 256), 256, 0, ctx->st>>>(a); ++ctx->launches; }
-  else { k_self_mix<false><<<(int)((threads + 255) / 256), 256, 0, ctx->st>>>(a); ++ctx->launches; }
-  CUDA_TRY(cudaGetLastError());
-  return RBC3D_OK;
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
+  a.NC = ctx->nrad * (ctx->nazm / 2 + 1);
+  a.G = ring_cells(ctx->ncell, ctx->nlon);
+  const int blocks = (ctx->ncell + a.G - 1) / a.G * ctx->nlat, thr = std::min(256, (a.G * ctx->nlon + 31) / 32 * 32);
+  a.parts = ring_parts(a.NC, blocks, nsm);
+  const size_t bytes = smem(a.G);
+  auto launch = [&](auto kern) -> rbc3d_status {
+    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    kern<<<blocks * a.parts, thr, bytes, ctx->st>>>(a);
+    ++ctx->launches;
+    CUDA_TRY(cudaGetLastError());
+    return RBC3D_OK;
+  };
+  if (sl && dl) return launch(k_self_mix<true, true>);
+  if (sl) return launch(k_self_mix<true, false>);
+  return launch(k_self_mix<false, true>);
 }
