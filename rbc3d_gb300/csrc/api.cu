@@ -450,6 +450,12 @@ rbc3d_status rbc3d_create(const rbc3d_params* prm, rbc3d_ctx** out) {
   T.sl_c1 = ctx->t_sl1.p; T.sl_c2 = ctx->t_sl2.p; T.dl_c1 = ctx->t_dl.p; T.mask = ctx->t_mask.p;
   T.sl32 = ctx->t_sl32.p; T.dl32 = ctx->t_dl32.p; T.mask32 = ctx->t_mask32.p;
   T.rc = rc; T.r_eps = 1.e-3 * std::sqrt(alpha / RBC3D_PI); T.ntab_over_rc = N / rc;
+  {
+    const double e2 = T.r_eps * T.r_eps, rc2 = rc * rc;
+    std::memcpy(&T.eps2b, &e2, 8);
+    std::memcpy(&T.rc2b, &rc2, 8);
+    T.tab6 = ctx->ring_tab.p;
+  }
   T.rc_f = (float)rc; T.r_eps_f = (float)T.r_eps; T.ntab_over_rc_f = (float)(N / rc);
   // cell list
   for (int d = 0; d < 3; ++d) {

@@ -29,7 +29,49 @@ struct Tables {
   const float2* mask32;
   double rc, r_eps, ntab_over_rc;
   float rc_f, r_eps_f, ntab_over_rc_f;
+  // the FP64 tables entry by entry as (value, step to the next): c1, dc1, c2,
+  // dc2, dl, ddl; the bits of r_eps^2 and rc^2
+  const double* tab6;
+  long long eps2b, rc2b;
 };
+
+// 1/sqrt(x) for a positive, normal x: the hardware's approximation and one
+// step of third order (y <- y + y e (1/2 + 3/8 e), e = 1 - x y^2).
+__device__ __forceinline__ double rsqrt_step(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// EwaldCoeff_SL / EwaldCoeff_DL (ModEwaldFunc.F90:86-180) from a squared
+// distance: EA, EB, ED with v = EA (x.f) x + EB f + ED (x.g)(x.n) x.  False where
+// they are zero or not evaluated: below r_eps, from rc on, NaN (positive
+// doubles order as their bits).  No FP64 division, comparison or conversion:
+// the table position is floored by a downward-rounded sum with 1.5 2^52.
+template <bool SL, bool DL>
+__device__ __forceinline__ bool ewald_coef64(const Tables& T, double r2, double& EA, double& EB, double& ED) {
+  const long long bits = __double_as_longlong(r2);
+  if (bits < T.eps2b || bits >= T.rc2b) return false;
+  const double ir = rsqrt_step(r2), rr = r2 * ir;
+  const double magic = 6755399441055744.0;
+  const double ft = __fma_rd(rr, T.ntab_over_rc, magic);
+  const int it = __double2loint(ft);
+  if ((unsigned)it >= (unsigned)EWALD_NTAB) return false;
+  const double f1 = fma(rr, T.ntab_over_rc, magic - ft), ir2 = ir * ir;
+  const double2* tb = reinterpret_cast<const double2*>(T.tab6) + 3 * it;
+  if (SL) {
+    const double2 t1 = __ldg(tb), t2 = __ldg(tb + 1);
+    const double c1ir = fma(t1.y, f1, t1.x) * ir, c2 = fma(t2.y, f1, t2.x);
+    EA = (c1ir + c2) * ir2;
+    EB = c1ir - c2;
+  }
+  if (DL) {
+    const double2 t3 = __ldg(tb + 2);
+    ED = fma(t3.y, f1, t3.x) * (ir2 * ir2 * ir);
+  }
+  return true;
+}
 
 // ---------------------------------------------------------------------------
 // EwaldCoeff_SL / EwaldCoeff_DL (ModEwaldFunc.F90:86-180), FP64.
@@ -43,39 +85,6 @@ __device__ __forceinline__ void ewald_sl64(const Tables& T, double r, double& A,
   double ir = 1. / r, ir2 = ir * ir;
   A = c1 * ir * ir2 + c2 * ir2;
   B = c1 * ir - c2;
-}
-// The same with 1/r supplied (from rsqrt of r^2, 1 ulp) and the table index as
-// r * (NTAB/rc): no FP64 division.
-// Callers pass r = r2 * rsqrt(r2), which is NaN for r2 = 0 (a target that is
-// its own source): !(r >= r_eps) catches it, and the index is range-checked.
-__device__ __forceinline__ void ewald_sl64r(const Tables& T, double r, double ir, double& A, double& B) {
-  if (!(r >= T.r_eps)) { A = 0.; B = 0.; return; }
-  double s = r * T.ntab_over_rc;
-  int i = (int)floor(s);
-  if (i < 0 || i >= EWALD_NTAB) { A = 0.; B = 0.; return; }
-  double c1 = __ldg(T.sl_c1 + i) * (i + 1 - s) + __ldg(T.sl_c1 + i + 1) * (s - i);
-  double c2 = __ldg(T.sl_c2 + i) * (i + 1 - s) + __ldg(T.sl_c2 + i + 1) * (s - i);
-  double ir2 = ir * ir;
-  A = c1 * ir * ir2 + c2 * ir2;
-  B = c1 * ir - c2;
-}
-__device__ __forceinline__ double ewald_dl64r(const Tables& T, double r, double ir) {
-  if (!(r >= T.r_eps)) return 0.;
-  double s = r * T.ntab_over_rc;
-  int i = (int)floor(s);
-  if (i < 0 || i >= EWALD_NTAB) return 0.;
-  double c1 = __ldg(T.dl_c1 + i) * (i + 1 - s) + __ldg(T.dl_c1 + i + 1) * (s - i);
-  double ir2 = ir * ir;
-  return c1 * (ir2 * ir2 * ir);
-}
-__device__ __forceinline__ double ewald_dl64(const Tables& T, double r) {
-  if (r < T.r_eps) return 0.;
-  double s = EWALD_NTAB * r / T.rc;
-  int i = (int)floor(s);
-  if (i >= EWALD_NTAB) return 0.;
-  double c1 = __ldg(T.dl_c1 + i) * (i + 1 - s) + __ldg(T.dl_c1 + i + 1) * (s - i);
-  double r2 = r * r;
-  return c1 / (r2 * r2 * r);
 }
 // MaskFunc (ModBasicMath.F90:351-379), FP64
 __device__ __forceinline__ double mask64(const Tables& T, double x) {

@@ -50,10 +50,8 @@ struct TargetSet {
   DBuf<int4> meta;      // (surf, ilat, ilon, 0); surf 1-based, -1 for raw
   DBuf<int> order;      // sorted position -> target index
   DBuf<int> cstart, cend;
-  DBuf<int4> units;     // (hash cell, first sorted position, count, 0): up to TILE targets (FP64 pair sums)
-  int nunits = 0;
-  DBuf<int4> wunits;    // the same with up to 32 targets, one per warp (FP32 pair sums)
-  int nwunits = 0;
+  DBuf<int4> units;     // (hash cell, first sorted position, count, 0): up to 32 / sub targets, a warp each
+  int nunits = 0, sub = 1;
   bool sorted = false;
   DBuf<double> v;       // 3n accumulator of the current matvec
   DBuf<double> v2;      // 3n accumulator of the stages on the side stream
@@ -206,6 +204,7 @@ struct rbc3d_ctx {
   DBuf<int> s_inv;              // point -> sorted source position
   int s_ntiles = 0;
   DBuf<unsigned long long> near_queue;  // work counter of the near-singular kernel
+  DBuf<double> s_rec64;         // FP64 pair-sum records (12 doubles a source)
   DBuf<double> dBcoef;                  // Bcoef per cell type on the device
   DBuf<char> ring_cls;                  // patch-point classes per latitude (RingClass)
   DBuf<double> ring_tab, ring_rec;      // FP64 patch: Ewald tables with steps, node values in column order

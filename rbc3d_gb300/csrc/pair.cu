@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "ctx.hpp"
@@ -38,24 +39,38 @@ namespace {
 
 constexpr int TILE = 128;
 
+// Sort keys: the hash cell; for targets (MORTON) followed by the place in the
+// cell's 8 x 8 x 8 sub-cells along the Morton curve, so that the targets of a
+// warp lie together and its box reaches few sources.
+constexpr int MORTON_BITS = 9;
+template <bool MORTON>
 __global__ void k_hash_keys(int n, const double* __restrict__ x, int Nc0, int Nc1, int Nc2, double s0, double s1,
                             double s2, int* __restrict__ key, int* __restrict__ idx) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   // HashTable_Index, ModHashTable.F90:67-94 (single node): modulo(floor(x*Nc/L), Nc)
-  int i1 = imod((int)floor(x[p] * s0), Nc0);
-  int i2 = imod((int)floor(x[p + n] * s1), Nc1);
-  int i3 = imod((int)floor(x[p + 2 * (size_t)n] * s2), Nc2);
-  key[p] = i1 + Nc0 * (i2 + Nc1 * i3);
+  const double u[3] = {x[p] * s0, x[p + n] * s1, x[p + 2 * (size_t)n] * s2};
+  const double f[3] = {floor(u[0]), floor(u[1]), floor(u[2])};
+  const int cell = imod((int)f[0], Nc0) + Nc0 * (imod((int)f[1], Nc1) + Nc1 * imod((int)f[2], Nc2));
+  if (MORTON) {
+    int m = 0;
+    for (int d = 0; d < 3; ++d) {
+      const int i = min(7, max(0, (int)(8.f * (float)(u[d] - f[d]))));
+      m |= (i & 1) << d | (i & 2) << (d + 2) | (i & 4) << (d + 4);
+    }
+    key[p] = cell << MORTON_BITS | m;
+  } else {
+    key[p] = cell;
+  }
   idx[p] = p;
 }
 
-__global__ void k_cell_ranges(int n, const int* __restrict__ key, int* __restrict__ cs, int* __restrict__ ce) {
+__global__ void k_cell_ranges(int n, int shift, const int* __restrict__ key, int* __restrict__ cs, int* __restrict__ ce) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
-  int k = key[p];
-  if (p == 0 || key[p - 1] != k) cs[k] = p;
-  if (p == n - 1 || key[p + 1] != k) ce[k] = p + 1;
+  int k = key[p] >> shift;
+  if (p == 0 || key[p - 1] >> shift != k) cs[k] = p;
+  if (p == n - 1 || key[p + 1] >> shift != k) ce[k] = p + 1;
 }
 
 // Lists built on the device from sorted cell ranges (no host round trip).
@@ -245,12 +260,34 @@ __global__ void k_own_records(int n, int nlat, int nv, const double* __restrict_
 
 // c1 f dS and c2 g dS Bcoef of the sorted sources in FP32 (per call).
 __global__ void k_src_dens4(int n, double c1, double c2, const double* __restrict__ sf, const double* __restrict__ sg,
-                            int do_g, float4* __restrict__ F, float4* __restrict__ Gv) {
+                            int do_f, int do_g, float4* __restrict__ F, float4* __restrict__ Gv) {
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
-  F[q] = make_float4((float)(c1 * sf[q]), (float)(c1 * sf[q + n]), (float)(c1 * sf[q + 2 * (size_t)n]), 0.f);
+  F[q] = do_f ? make_float4((float)(c1 * sf[q]), (float)(c1 * sf[q + n]), (float)(c1 * sf[q + 2 * (size_t)n]), 0.f)
+              : make_float4(0.f, 0.f, 0.f, 0.f);
   if (do_g)
     Gv[q] = make_float4((float)(c2 * sg[q]), (float)(c2 * sg[q + n]), (float)(c2 * sg[q + 2 * (size_t)n]), 0.f);
+}
+
+// FP64 records of the sorted sources, 12 doubles each: position relative to
+// the source's hash-cell centre, c1 f dS, c2 g dS Bcoef, a3 (per call).
+__global__ void k_src_rec64(int n, double c1, double c2, const double* __restrict__ sx, const double* __restrict__ sf,
+                            const double* __restrict__ sg, const double* __restrict__ sa3, int Nc0, int Nc1, int Nc2,
+                            double h0, double h1, double h2, double L0, double L1, double L2, int do_f, int do_g,
+                            double* __restrict__ rec) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  const int Nc[3] = {Nc0, Nc1, Nc2};
+  const double h[3] = {h0, h1, h2}, L[3] = {L0, L1, L2};
+  double* o = rec + 12 * (size_t)q;
+  for (int k = 0; k < 3; ++k) {
+    const double x = sx[q + (size_t)k * n];
+    const int c = imod((int)floor(x * (Nc[k] / L[k])), Nc[k]);  // HashTable_Index
+    o[k] = min_image(x - (c + 0.5) * h[k], L[k], 1.0 / L[k]);
+    o[3 + k] = do_f ? c1 * sf[q + (size_t)k * n] : 0.;
+    o[6 + k] = do_g ? c2 * sg[q + (size_t)k * n] : 0.;
+    o[9 + k] = sa3[q + (size_t)k * n];
+  }
 }
 
 // SourceList_UpdateDensity (ModSourceList.F90:160-189): f*dS, g*dS with
@@ -285,15 +322,10 @@ struct PairArgs {
   const int4* tmeta;
   const int* torder;
   const int4* units;
-  int nunits;  // k_pair32: warp units
+  int nunits;
   double* v;  // 3*nt accumulator
   // sources (sorted)
   int ns;
-  const double* sx;
-  const double* sf;
-  const double* sg;
-  const double* sa3;
-  const int4* smeta;
   const int* cs;
   const int* ce;
   // FP32 source records (sorted order) and tile boxes
@@ -318,9 +350,9 @@ struct PairArgs {
   const float* mtab32;   // 1 - mask in FP32
   double radius, inv_radius;
   float inv_radius_f, chord2_max;
-  double c1, c2;
-  float c1f, c2f;
   double rc2;
+  const double* rec64;  // FP64 source records
+  const double* px;     // the points' positions (k_pair_own64)
   float rc2_f, reps2_f;
   float rc2_loose;  // (rc + 1e-3)^2: hi-part reject threshold of the FP32 pair kernel
   float rthr2_f;  // FP32 path: cross-surface pairs closer than this are left to the FP64 near-singular pass
@@ -332,8 +364,8 @@ struct PairArgs {
   int4* items;
   int cap;
   unsigned long long* cnt;  // [0] items, [1] pairs, [2] overflow
-  // own-cell pairs of the FP32 modes (cell targets, same-cell weight table):
-  // k_pair_own32 takes them and k_pair32 skips same-surface sources
+  // own-cell pairs (cell targets, same-cell weight table): the dense pass takes
+  // them and k_pair skips same-surface sources
   int own_split;
   const float4* op0;  // per point (point order): (x, y, z) hi relative to its cell's first point, id bits
   const float4* op1;  // lo
@@ -356,14 +388,6 @@ struct NbrList {
     if (n < RBC3D_NBR_MAX) { surf[n] = s; idx[n] = id; d2[n] = d; ++n; }
     else overflow = 1;
   }
-};
-
-// Shared-memory source tile of the FP64 pair kernel
-struct TileD {
-  double x[TILE], y[TILE], z[TILE];
-  double fx[TILE], fy[TILE], fz[TILE], gx[TILE], gy[TILE], gz[TILE];
-  double ax[TILE], ay[TILE], az[TILE];
-  int surf[TILE], ilat[TILE], ilon[TILE];
 };
 
 // Box-to-box distance test of the tile culling: true if every point of box
@@ -395,41 +419,7 @@ __device__ __forceinline__ void two_diff(float a, float b, float& s, float& e) {
   e = (a - (s + bb)) + (bb - b);
 }
 
-// Target and tile bounding boxes of the culling, shared by both precisions.
-struct CullBoxes {
-  float3 wlo, whi;  // this warp's targets
-  float3 clo, chi;  // the CTA's targets
-};
-
-__device__ __forceinline__ CullBoxes cull_boxes(bool active, float tx, float ty, float tz, float3 (*wb)[2]) {
-  const float big = 3.0e38f;
-  CullBoxes b;
-  b.wlo = active ? make_float3(tx, ty, tz) : make_float3(big, big, big);
-  b.whi = active ? make_float3(tx, ty, tz) : make_float3(-big, -big, -big);
-  warp_minmax(b.wlo, b.whi);
-  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0) { wb[w][0] = b.wlo; wb[w][1] = b.whi; }
-  __syncthreads();
-  b.clo = wb[0][0]; b.chi = wb[0][1];
-  for (int k = 1; k < nw; ++k) {
-    b.clo.x = fminf(b.clo.x, wb[k][0].x); b.clo.y = fminf(b.clo.y, wb[k][0].y); b.clo.z = fminf(b.clo.z, wb[k][0].z);
-    b.chi.x = fmaxf(b.chi.x, wb[k][1].x); b.chi.y = fmaxf(b.chi.y, wb[k][1].y); b.chi.z = fmaxf(b.chi.z, wb[k][1].z);
-  }
-  return b;
-}
-
 __device__ __forceinline__ float3 f3sub(float3 a, float3 d) { return make_float3(a.x - d.x, a.y - d.y, a.z - d.z); }
-
-// Per-warp source chunk in structure-of-arrays form, so that two consecutive
-// sources' components load as one float2 for the packed FP32x2 arithmetic.
-template <bool DL>
-struct ChunkX2 {
-  float hx[32], hy[32], hz[32], lx[32], ly[32], lz[32];
-  float fx[32], fy[32], fz[32];
-  float gx[DL ? 32 : 2], gy[DL ? 32 : 2], gz[DL ? 32 : 2];
-  float ax[DL ? 32 : 2], ay[DL ? 32 : 2], az[DL ? 32 : 2];
-  int surf[32], id[32];
-};
 
 __device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }
 __device__ __forceinline__ float2 ld2(const float* p, int j) { return *reinterpret_cast<const float2*>(p + j); }
@@ -439,7 +429,7 @@ __device__ __forceinline__ float2 ld2(const float* p, int j) { return *reinterpr
 // packed FP32x2 arithmetic: the Stokeslet term A (x.f) x + B f and the
 // stresslet factor Adl of (x.g)(x.n) x, for squared distances r2 (a pair of
 // weight 0 enters with r^2 = 1, harmless).
-template <bool DL>
+template <bool SL, bool DL>
 __device__ __forceinline__ void ewald_coef2(const PairArgs& a, float2 r2, float wa, float wb, float2& A, float2& B,
                                             float2& Adl) {
   const float2 sqpa2 = f2(a.sqpa_f, a.sqpa_f), half2 = f2(0.5f, 0.5f), one2 = f2(1.f, 1.f);
@@ -456,9 +446,11 @@ __device__ __forceinline__ void ewald_coef2(const PairArgs& a, float2 r2, float 
   for (int k = ERFCX_DEG - 1; k >= 0; --k) Q = __ffma2_rn(Q, tq, f2(a.erfcx_q[k], a.erfcx_q[k]));
   const float2 c1 = __fmul2_rn(ex, __fmul2_rn(tq, Q)), c2 = __fmul2_rn(tisqa2, ex);
   const float2 ir2 = __fmul2_rn(rinv, rinv);
-  const float2 c1r = __fmul2_rn(c1, rinv);
-  A = __fmul2_rn(__fadd2_rn(c1r, c2), ir2);
-  B = __fadd2_rn(c1r, f2(-c2.x, -c2.y));
+  if (SL) {
+    const float2 c1r = __fmul2_rn(c1, rinv);
+    A = __fmul2_rn(__fadd2_rn(c1r, c2), ir2);
+    B = __fadd2_rn(c1r, f2(-c2.x, -c2.y));
+  }
   if (DL) {
     const float2 st2 = __fmul2_rn(st, st);
     const float2 cdl = __fmul2_rn(f2(a.m8_ispi_f, a.m8_ispi_f),
@@ -468,91 +460,98 @@ __device__ __forceinline__ void ewald_coef2(const PairArgs& a, float2 r2, float 
   }
 }
 
-// A (x.f) x + B f + Adl (x.g)(x.n) x for two pairs (DL: the last term)
-template <bool DL>
+// A (x.f) x + B f + Adl (x.g)(x.n) x for two pairs (SL: the first two terms, DL: the last)
+template <bool SL, bool DL>
 __device__ __forceinline__ void ewald_apply2(float2 xx, float2 yy, float2 zz, float2 A, float2 B, float2 Adl,
                                              float2 fx, float2 fy, float2 fz, float2 gx, float2 gy, float2 gz,
                                              float2 nx, float2 ny, float2 nz, float2& vx, float2& vy, float2& vz) {
-  const float2 Ad = __fmul2_rn(A, __ffma2_rn(xx, fx, __ffma2_rn(yy, fy, __fmul2_rn(zz, fz))));
-  vx = __ffma2_rn(Ad, xx, __fmul2_rn(B, fx));
-  vy = __ffma2_rn(Ad, yy, __fmul2_rn(B, fy));
-  vz = __ffma2_rn(Ad, zz, __fmul2_rn(B, fz));
+  if (SL) {
+    const float2 Ad = __fmul2_rn(A, __ffma2_rn(xx, fx, __ffma2_rn(yy, fy, __fmul2_rn(zz, fz))));
+    vx = __ffma2_rn(Ad, xx, __fmul2_rn(B, fx));
+    vy = __ffma2_rn(Ad, yy, __fmul2_rn(B, fy));
+    vz = __ffma2_rn(Ad, zz, __fmul2_rn(B, fz));
+  }
   if (DL) {
     const float2 dg = __ffma2_rn(xx, gx, __ffma2_rn(yy, gy, __fmul2_rn(zz, gz)));
     const float2 da = __ffma2_rn(xx, nx, __ffma2_rn(yy, ny, __fmul2_rn(zz, nz)));
     const float2 t = __fmul2_rn(__fmul2_rn(Adl, dg), da);
-    vx = __ffma2_rn(t, xx, vx);
-    vy = __ffma2_rn(t, yy, vy);
-    vz = __ffma2_rn(t, zz, vz);
+    vx = SL ? __ffma2_rn(t, xx, vx) : __fmul2_rn(t, xx);
+    vy = SL ? __ffma2_rn(t, yy, vy) : __fmul2_rn(t, yy);
+    vz = SL ? __ffma2_rn(t, zz, vz) : __fmul2_rn(t, zz);
   }
 }
 
-// The Ewald real-space kernels of two sources at once added to (cx, cy, cz)
-// with the weights wa, wb: pair vectors (xx, yy, zz) with squares r2, the
-// sources' c1 f dS (f*), c2 g dS Bcoef (g*) and normals (n*).
-template <bool DL>
-__device__ __forceinline__ void ewald_pair2(const PairArgs& a, float2 xx, float2 yy, float2 zz, float2 r2, float wa,
-                                            float wb, float2 fx, float2 fy, float2 fz, float2 gx, float2 gy, float2 gz,
-                                            float2 nx, float2 ny, float2 nz, float& cx, float& cy, float& cz) {
-  float2 A, B, Adl, vx, vy, vz;
-  ewald_coef2<DL>(a, r2, wa, wb, A, B, Adl);
-  ewald_apply2<DL>(xx, yy, zz, A, B, Adl, fx, fy, fz, gx, gy, gz, nx, ny, nz, vx, vy, vz);
-  cx = fmaf(wb, vx.y, fmaf(wa, vx.x, cx));
-  cy = fmaf(wb, vy.y, fmaf(wa, vy.x, cy));
-  cz = fmaf(wb, vz.y, fmaf(wa, vz.x, cz));
+// A warp's tile of up to TILE sources.  FP32: records of NQ float4 (hi
+// coordinates and surface, lo coordinates and grid index, f, g, a3), read by
+// lanes at sources of their own with 16-byte loads.  FP64: the FP32 hi
+// coordinates of the tests and the FP64 values as a structure of arrays.
+template <int NQ>
+struct WarpTile32 {
+  float4 r[TILE][NQ];
+};
+struct WarpTile64 {
+  float4 p0[TILE];
+  int id[TILE];
+  double v[12][TILE];  // xyz, f, g, a3
+};
+template <typename R, bool SL, bool DL>
+constexpr size_t warp_tile_bytes() {
+  return sizeof(R) == 8 ? sizeof(WarpTile64) : sizeof(WarpTile32<2 + SL + 2 * DL>);
 }
 
-// FP32 real-space pair sums (EwaldCoeff_SL / EwaldCoeff_DL of ModEwaldFunc
-// over the 27 neighbour hash cells, AddIntOnRbcs ModIntOnRbcs.F90:25-160).
-// One CTA per (hash cell, up to TILE targets).  Sources carry FP32 hi/lo
-// coordinates relative to their own cell centre; per neighbour cell the
-// targets are shifted into that frame with an error-free difference, so the
-// pair vector keeps full FP32 accuracy however far from the origin the cells
-// are.  Source tiles (TILE consecutive sources of a cell) whose bounding box
-// is farther than rc from the CTA's targets are not loaded, and a warp skips
-// a loaded tile that is out of its own targets' reach.
-// Each warp stages its own 32-source chunks (no block barrier).  The inner
-// loop runs over pairs of sources: the geometric tests, weights and
-// neighbour bookkeeping stay per source and in source order; the Ewald
-// kernels of both sources run in packed FP32x2 arithmetic (__ffma2_rn /
-// __fmul2_rn / __fadd2_rn, round-to-nearest like the scalar operations), a
-// source that does not contribute entering with weight 0 and a harmless
-// r^2 = 1 (4.20 -> 3.96 ms against the one-source loop on the 256-cell
-// workload).  Eight 128-thread blocks per SM (64 registers a thread, 132
-// bytes of spills): with the own-cell pairs taken by k_pair_own32 this
-// kernel runs a little longer than at six blocks (80 registers), but the
-// PME spread beside it gets its SMs sooner (the FP32D matvec 10.62 -> 10.52
-// ms on the 256-cell workload; four, five and seven blocks: 10.65, 10.61,
-// 10.58).  Before the own-cell split, six blocks against the unbounded 96
-// registers: 3.58 against 3.76 ms alone; Estrin's scheme for the fitted erfc
-// polynomial measured slower.
-template <bool DL>
-__global__ void __launch_bounds__(TILE, 8) k_pair32(PairArgs a) {
-  __shared__ __align__(16) ChunkX2<DL> s_ch[TILE / 32];
+// Real-space pair sums (EwaldCoeff_SL / EwaldCoeff_DL of ModEwaldFunc over the
+// 27 neighbour hash cells, AddIntOnRbcs ModIntOnRbcs.F90:25-160), one warp per
+// unit of up to 32/SUB targets of one hash cell, SUB lanes per target.
+//
+// FP32: sources carry hi/lo coordinates relative to their own cell centre; per
+// neighbour cell the targets are shifted into that frame with an error-free
+// difference, so the pair vector keeps full FP32 accuracy however far from the
+// origin the cells are; two sources at once in packed FP32x2 arithmetic, plain
+// sums per 32-source chunk, Kahan-compensated across them.  FP64 (the plain form):
+// the same frames in FP64, reference table arithmetic.
+//
+// Per tile (TILE consecutive sources of a cell; tiles and 32-source chunks
+// whose bounding box is out of the warp's reach are skipped) a lane tests all
+// its sources in FP32 (with a margin) and collects the survivors as bits; then
+// the lanes pop their own bits, so a step evaluates a pair in every lane that
+// has one left.  Before, all lanes walked the same sources and about 7 of 32
+// had a pair to evaluate.  FP64 is bound by its pipe, FP32 by issue.
+//
+// SUB = 4: four lanes share a target, each with one 32-source chunk of the
+// tile, and merge sums and neighbour lists at the end: a quarter of the serial
+// work per warp where there are few targets (see pair_sub).
+template <typename R, bool SL, bool DL, int SUB>
+__global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs a) {
+  constexpr bool F64 = sizeof(R) == 8;
+  extern __shared__ __align__(16) unsigned char smem_pair[];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int wu = blockIdx.x * (TILE / 32) + wid;  // this warp's unit
   if (wu >= a.nunits) return;
   const int4 unit = a.units[wu];
   if (unit.z == 0) return;  // the empty tail
-  const int cell = unit.x;
-  const bool active = lane < unit.z;
+  constexpr int NQ = 2 + SL + 2 * DL;
+  unsigned char* tile = smem_pair + wid * warp_tile_bytes<R, SL, DL>();
+  WarpTile32<NQ>& C = *reinterpret_cast<WarpTile32<NQ>*>(tile);  // FP32
+  WarpTile64& D = *reinterpret_cast<WarpTile64*>(tile);          // FP64
+  const int cell = unit.x, sub = lane % SUB;
+  const bool active = lane / SUB < unit.z;
   const int ci = cell % a.Nc[0], cj = (cell / a.Nc[0]) % a.Nc[1], ck = cell / (a.Nc[0] * a.Nc[1]);
   const double c0[3] = {(ci + 0.5) * a.h[0], (cj + 0.5) * a.h[1], (ck + 0.5) * a.h[2]};
-  int ti = active ? a.torder[unit.y + lane] : 0;
+  const int ti = active ? a.torder[unit.y + lane / SUB] : 0;
+  double t64[3] = {0, 0, 0};
   float th_[3] = {0, 0, 0}, tl_[3] = {0, 0, 0};
-  float4 ui = make_float4(0, 0, 0, 0);
   int surf_i = -2, tlat = 0, tlon = 0;
+  bool grid = false;
   if (active) {
     for (int k = 0; k < 3; ++k) {
-      double r = min_image(a.tx[ti + (size_t)k * a.nt] - c0[k], a.L[k], a.iL[k]);
-      th_[k] = (float)r;
-      tl_[k] = (float)(r - (double)th_[k]);
+      t64[k] = min_image(a.tx[ti + (size_t)k * a.nt] - c0[k], a.L[k], a.iL[k]);
+      th_[k] = (float)t64[k];
+      tl_[k] = (float)(t64[k] - (double)th_[k]);
     }
-    int4 m = a.tmeta[ti];
+    const int4 m = a.tmeta[ti];
     surf_i = m.x;
-    if (m.y >= 0) { ui = a.usph[m.y + a.nlat * m.z]; tlat = m.y; tlon = m.z; }
+    if (m.y >= 0) { tlat = m.y; tlon = m.z; grid = true; }
   }
-  const float* mrow = a.mtab32 ? a.mtab32 + (size_t)tlat * a.nlat * a.nhalf : nullptr;
   float3 wlo0, whi0;
   {
     const float big = 3.0e38f;
@@ -560,15 +559,15 @@ __global__ void __launch_bounds__(TILE, 8) k_pair32(PairArgs a) {
     whi0 = active ? make_float3(th_[0], th_[1], th_[2]) : make_float3(-big, -big, -big);
     warp_minmax(wlo0, whi0);
   }
-  ChunkX2<DL>& C = s_ch[wid];
   Kahan3 acc;
   acc.zero();
+  double acc64[3] = {0, 0, 0};
   NbrList L;
   L.n = 0; L.overflow = 0;
   int run_surf = -3, run_id = -1;
-  float run_d2 = 3.4e38f;
+  R run_d2 = (R)3.4e38f;
   unsigned npairs = 0;  // < 2^32 pairs per target
-  // own-cell pairs left to k_pair_own32: the warp's surface when all its
+  // own-cell pairs left to the dense pass: the warp's surface when all its
   // targets share one (whole tiles and chunks of it are skipped), else -7
   int wsurf = -7;
   if (a.own_split) {
@@ -576,21 +575,27 @@ __global__ void __launch_bounds__(TILE, 8) k_pair32(PairArgs a) {
     wsurf = __all_sync(0xffffffffu, !active || surf_i == s0) ? s0 : -7;
   }
 
-  // per-source bookkeeping in source order: neighbour-surface runs, the pair
-  // count, the weight (0 when the pair does not contribute here)
-  // (the closest point per other surface: runs of accepted pairs of one
-  // surface, each run's minimum merged into L by surface, so sources that
-  // are out of reach need no bookkeeping)
-  auto weight = [&](int sj, int idj, float r2, bool ok, int qglob) -> float {
-    if (!ok) return 0.f;
-    ++npairs;
-    float wgt = 1.f;
-    if (sj == surf_i && mrow) {
+  // 1 - MaskFunc of a pair on one cell
+  auto same_weight = [&](int idj, int q) -> R {
+    if (F64) {
+      double m = 0.;
+      if (a.mtab64) {
+        int dl = abs((idj >> 16) - tlon);
+        dl = min(dl, a.nlon - dl);
+        m = __ldg(a.mtab64 + ((size_t)tlat * a.nlat + (idj & 0xffff)) * a.nhalf + dl);
+      } else if (grid) {
+        const double dth = dist_on_sphere(a.th[tlat], a.phi[tlon], a.th[idj & 0xffff], a.phi[idj >> 16]);
+        m = mask64(a.T, dth * a.inv_radius);
+      }
+      return (R)(1. - m);
+    }
+    float w = 1.f;
+    if (a.mtab32) {
       int dl = abs((idj >> 16) - tlon);
       dl = min(dl, a.nlon - dl);
-      wgt = __ldg(mrow + (idj & 0xffff) * a.nhalf + dl);
-    } else if (sj == surf_i) {
-      const float4 u = a.su[qglob];
+      w = __ldg(a.mtab32 + (size_t)tlat * a.nlat * a.nhalf + (idj & 0xffff) * a.nhalf + dl);
+    } else if (grid) {
+      const float4 u = a.su[q], ui = a.usph[tlat + a.nlat * tlon];
       const float ex = ui.x - u.x, ey = ui.y - u.y, ez = ui.z - u.z;
       const float ch2 = ex * ex + ey * ey + ez * ez;
       if (ch2 < a.chord2_max) {
@@ -599,19 +604,27 @@ __global__ void __launch_bounds__(TILE, 8) k_pair32(PairArgs a) {
         const int i = (int)sx;
         if (i < MASK_NTAB) {
           const float2 e = __ldg(a.T.mask32 + i);
-          wgt = 1.f - (e.x + (sx - (float)i) * e.y);
+          w = 1.f - (e.x + (sx - (float)i) * e.y);
         }
       }
-    } else if (a.collect) {
+    }
+    return (R)w;
+  };
+  // bookkeeping of a source within rc (sorted index q), in source order: pair
+  // count, neighbour-surface runs (each run's closest point merged into L by
+  // surface), the weight (FP32: 0 for pairs left to the near-singular pass)
+  auto weight = [&](int sj, int idj, int q, R r2) -> R {
+    ++npairs;
+    if (sj == surf_i) return same_weight(idj, q);
+    if (a.collect) {
       if (sj != run_surf) {
-        if (run_id >= 0) L.insert(run_surf, run_id, run_d2);
-        run_surf = sj; run_id = -1; run_d2 = 3.4e38f;
+        if (run_id >= 0) L.insert(run_surf, run_id, (float)run_d2);
+        run_surf = sj; run_id = -1; run_d2 = (R)3.4e38f;
       }
       if (r2 < run_d2) { run_d2 = r2; run_id = idj; }
-      if (r2 < a.rthr2_f) return 0.f;
+      if (!F64 && r2 < (R)a.rthr2_f) return (R)0;
     }
-    if (r2 < a.reps2_f) return 0.f;
-    return wgt;
+    return (R)1;
   };
 
   for (int nb = 0; nb < 27; ++nb) {
@@ -622,134 +635,197 @@ __global__ void __launch_bounds__(TILE, 8) k_pair32(PairArgs a) {
     if (sbeg >= send) continue;
     const double d64[3] = {dx * a.h[0], dy * a.h[1], dz * a.h[2]};
     const float3 dh = make_float3((float)d64[0], (float)d64[1], (float)d64[2]);
-    const float3 dl = make_float3((float)(d64[0] - (double)dh.x), (float)(d64[1] - (double)dh.y),
-                                  (float)(d64[2] - (double)dh.z));
-    float tsh[3], tsl[3];
+    float tsh[3], tsl[3];  // the target in the neighbour's frame
     {
-      float e;
-      two_diff(th_[0], dh.x, tsh[0], e); tsl[0] = (tl_[0] - dl.x) + e;
-      two_diff(th_[1], dh.y, tsh[1], e); tsl[1] = (tl_[1] - dl.y) + e;
-      two_diff(th_[2], dh.z, tsh[2], e); tsl[2] = (tl_[2] - dl.z) + e;
+      const float dl[3] = {(float)(d64[0] - (double)dh.x), (float)(d64[1] - (double)dh.y), (float)(d64[2] - (double)dh.z)};
+      const float d3[3] = {dh.x, dh.y, dh.z};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        float e;
+        two_diff(th_[k], d3[k], tsh[k], e);
+        tsl[k] = (tl_[k] - dl[k]) + e;
+      }
     }
-    const float2 nth0 = f2(-tsh[0], -tsh[0]), nth1 = f2(-tsh[1], -tsh[1]), nth2 = f2(-tsh[2], -tsh[2]);
-    const float2 ntl0 = f2(-tsl[0], -tsl[0]), ntl1 = f2(-tsl[1], -tsl[1]), ntl2 = f2(-tsl[2], -tsl[2]);
+    const double tn[3] = {t64[0] - d64[0], t64[1] - d64[1], t64[2] - d64[2]};
     const float3 wlo = f3sub(wlo0, dh), whi = f3sub(whi0, dh);
-    const int t0 = a.toff[ncell];
-    for (int base = sbeg, tt = t0; base < send; base += TILE, ++tt) {
+    for (int base = sbeg, tt = a.toff[ncell], cc = a.coff[ncell]; base < send; base += TILE, ++tt, cc += TILE / 32) {
       const float4 blo = a.tbox[2 * tt], bhi = a.tbox[2 * tt + 1];
       if (boxes_apart(wlo, whi, make_float3(blo.x, blo.y, blo.z), make_float3(bhi.x, bhi.y, bhi.z), a.rc2_f)) continue;
       if (__float_as_int(blo.w) == wsurf && __float_as_int(bhi.w) == wsurf) continue;  // own cell only
-      const int tend = min(base + TILE, send);
-      for (int cb = base, cc = a.coff[ncell] + (base - sbeg) / 32; cb < tend; cb += 32, ++cc) {
-        {
-          const float4 clo4 = a.cbox[2 * cc], chi4 = a.cbox[2 * cc + 1];
-          if (boxes_apart(wlo, whi, make_float3(clo4.x, clo4.y, clo4.z), make_float3(chi4.x, chi4.y, chi4.z), a.rc2_f))
-            continue;  // uniform over the warp
-          if (__float_as_int(clo4.w) == wsurf && __float_as_int(chi4.w) == wsurf) continue;  // own cell only
+      const int cnt = min(TILE, send - base);
+      unsigned live = 0;  // chunks within reach (uniform over the warp)
+#pragma unroll
+      for (int w = 0; w < TILE / 32; ++w) {
+        if (32 * w >= cnt) break;
+        const float4 clo = a.cbox[2 * (cc + w)], chi = a.cbox[2 * (cc + w) + 1];
+        if (!boxes_apart(wlo, whi, make_float3(clo.x, clo.y, clo.z), make_float3(chi.x, chi.y, chi.z), a.rc2_f) &&
+            !(__float_as_int(clo.w) == wsurf && __float_as_int(chi.w) == wsurf))
+          live |= 1u << w;
+      }
+      if (!live) continue;
+      __syncwarp();
+#pragma unroll
+      for (int w = 0; w < TILE / 32; ++w) {
+        const int j = 32 * w + lane;
+        if (!(live & (1u << w))) continue;
+        if (j >= cnt) {  // padding: out of every target's reach
+          const float4 far = make_float4(1.0e18f, 0.f, 0.f, __int_as_float(-9));
+          if constexpr (F64) D.p0[j] = far;
+          else C.r[j][0] = far;
+          continue;
         }
-        const int cnt = min(32, tend - cb);
-        __syncwarp();
-        if (lane < cnt) {
-          const int q = cb + lane;
-          const float4 p0 = a.sp0[q], p1 = a.sp1[q], f = a.sF4[q];
-          C.hx[lane] = p0.x; C.hy[lane] = p0.y; C.hz[lane] = p0.z; C.surf[lane] = __float_as_int(p0.w);
-          C.lx[lane] = p1.x; C.ly[lane] = p1.y; C.lz[lane] = p1.z; C.id[lane] = __float_as_int(p1.w);
-          C.fx[lane] = f.x; C.fy[lane] = f.y; C.fz[lane] = f.z;
-          if (DL) {
-            const float4 g = a.sG4[q], an = a.sa4[q];
-            C.gx[lane] = g.x; C.gy[lane] = g.y; C.gz[lane] = g.z;
-            C.ax[lane] = an.x; C.ay[lane] = an.y; C.az[lane] = an.z;
+        const int q = base + j;
+        const float4 p0 = a.sp0[q], p1 = a.sp1[q];
+        if constexpr (F64) {
+          D.p0[j] = p0;
+          D.id[j] = __float_as_int(p1.w);
+          const double2* r = reinterpret_cast<const double2*>(a.rec64) + 6 * (size_t)q;
+#pragma unroll
+          for (int k = 0; k < 6; ++k) {
+            if ((!SL && (k == 2)) || (!DL && k >= 3)) continue;  // values 4, 5 (f) or 6.. (g, a3) unused
+            const double2 v = r[k];
+            D.v[2 * k][j] = v.x; D.v[2 * k + 1][j] = v.y;
           }
+        } else {
+          C.r[j][0] = p0;
+          C.r[j][1] = p1;
+          if (SL) C.r[j][2] = a.sF4[q];
+          if (DL) { C.r[j][2 + SL] = a.sG4[q]; C.r[j][3 + SL] = a.sa4[q]; }
         }
-        __syncwarp();
-        if (!active) continue;
-        float cx = 0.f, cy = 0.f, cz = 0.f;
-        int j = 0;
-        for (; j + 2 <= cnt; j += 2) {
-          // hi parts of both sources, reject when both are out of reach
-          const float2 hx = __fadd2_rn(ld2(C.hx, j), nth0), hy = __fadd2_rn(ld2(C.hy, j), nth1),
-                       hz = __fadd2_rn(ld2(C.hz, j), nth2);
-          const float2 h2 = __ffma2_rn(hx, hx, __ffma2_rn(hy, hy, __fmul2_rn(hz, hz)));
-          const int sa = C.surf[j], sb = C.surf[j + 1];
-          bool oka = h2.x <= a.rc2_loose && !(a.own_split && sa == surf_i);
-          bool okb = h2.y <= a.rc2_loose && !(a.own_split && sb == surf_i);
-          if (!(oka || okb)) continue;
-          const float2 xx = __fadd2_rn(hx, __fadd2_rn(ld2(C.lx, j), ntl0));
-          const float2 yy = __fadd2_rn(hy, __fadd2_rn(ld2(C.ly, j), ntl1));
-          const float2 zz = __fadd2_rn(hz, __fadd2_rn(ld2(C.lz, j), ntl2));
+      }
+      __syncwarp();
+      // the lane's candidates: bits of TILE/32/SUB words
+      constexpr int NW = TILE / 32 / SUB;
+      unsigned bits[NW];
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        bits[w] = 0;
+        const int word = SUB == 1 ? w : w * SUB + sub;
+        if (!active || !(live & (1u << word))) continue;
+        unsigned m = 0;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) {
+          const float4 p = F64 ? D.p0[32 * word + j] : C.r[32 * word + j][0];
+          const float hx = p.x - tsh[0], hy = p.y - tsh[1], hz = p.z - tsh[2];
+          const float h2 = fmaf(hx, hx, fmaf(hy, hy, hz * hz));
+          if (h2 <= a.rc2_loose && !(a.own_split && __float_as_int(p.w) == surf_i)) m |= 1u << j;
+        }
+        bits[w] = m;
+      }
+      // a step: every lane that has a bit left evaluates its next source (FP32:
+      // its next two of one chunk)
+      int w = 0;
+      unsigned m = bits[0];
+      float cx = 0.f, cy = 0.f, cz = 0.f;
+      for (;;) {
+        if (NW > 1 && m == 0 && w < NW - 1) {  // the lane's next chunk
+          acc.add(0, cx); acc.add(1, cy); acc.add(2, cz);
+          cx = cy = cz = 0.f;
+#pragma unroll
+          for (int k = 1; k < NW; ++k)
+            if (m == 0 && w < k) { w = k; m = bits[k]; }
+        }
+        if (!__any_sync(0xffffffffu, m != 0)) break;
+        if (m == 0) continue;
+        const int j0 = 32 * (SUB == 1 ? w : w * SUB + sub);
+        const int ja = j0 + __ffs(m) - 1;
+        m &= m - 1;
+        if constexpr (F64) {
+          const double x = D.v[0][ja] - tn[0], y = D.v[1][ja] - tn[1], z = D.v[2][ja] - tn[2];
+          const double r2 = fma(x, x, fma(y, y, z * z));
+          if (r2 > a.rc2) continue;
+          const double wt = weight(__float_as_int(D.p0[ja].w), D.id[ja], base + ja, r2);
+          double EA, EB, ED;
+          if (!ewald_coef64<SL, DL>(a.T, r2, EA, EB, ED)) continue;
+          double t = 0., b = 0.;
+          if (SL) { t = EA * fma(x, D.v[3][ja], fma(y, D.v[4][ja], z * D.v[5][ja])); b = wt * EB; }
+          if (DL) {
+            const double dg = fma(x, D.v[6][ja], fma(y, D.v[7][ja], z * D.v[8][ja]));
+            const double da = fma(x, D.v[9][ja], fma(y, D.v[10][ja], z * D.v[11][ja]));
+            t = fma(ED * dg, da, t);
+          }
+          t *= wt;
+          acc64[0] = fma(t, x, acc64[0]); acc64[1] = fma(t, y, acc64[1]); acc64[2] = fma(t, z, acc64[2]);
+          if (SL) {
+            acc64[0] = fma(b, D.v[3][ja], acc64[0]); acc64[1] = fma(b, D.v[4][ja], acc64[1]);
+            acc64[2] = fma(b, D.v[5][ja], acc64[2]);
+          }
+        } else {
+          const bool two = m != 0;
+          const int jb = two ? j0 + __ffs(m) - 1 : ja;
+          m &= m - 1;  // 0 stays 0
+          const float4 pa = C.r[ja][0], pb = C.r[jb][0], la = C.r[ja][1], lb = C.r[jb][1];
+          const float2 xx = __fadd2_rn(f2(pa.x - tsh[0], pb.x - tsh[0]), f2(la.x - tsl[0], lb.x - tsl[0]));
+          const float2 yy = __fadd2_rn(f2(pa.y - tsh[1], pb.y - tsh[1]), f2(la.y - tsl[1], lb.y - tsl[1]));
+          const float2 zz = __fadd2_rn(f2(pa.z - tsh[2], pb.z - tsh[2]), f2(la.z - tsl[2], lb.z - tsl[2]));
           const float2 r2 = __ffma2_rn(xx, xx, __ffma2_rn(yy, yy, __fmul2_rn(zz, zz)));
-          oka = oka && r2.x <= a.rc2_f;
-          okb = okb && r2.y <= a.rc2_f;
-          const float wa = weight(sa, C.id[j], r2.x, oka, cb + j);
-          const float wb = weight(sb, C.id[j + 1], r2.y, okb, cb + j + 1);
+          float wa = 0.f, wb = 0.f;
+          if (r2.x <= a.rc2_f) {
+            wa = weight(__float_as_int(pa.w), __float_as_int(la.w), base + ja, r2.x);
+            if (r2.x < a.reps2_f) wa = 0.f;
+          }
+          if (two && r2.y <= a.rc2_f) {
+            wb = weight(__float_as_int(pb.w), __float_as_int(lb.w), base + jb, r2.y);
+            if (r2.y < a.reps2_f) wb = 0.f;
+          }
           if (wa == 0.f && wb == 0.f) continue;
           const float2 z2 = f2(0.f, 0.f);
-          ewald_pair2<DL>(a, xx, yy, zz, r2, wa, wb, ld2(C.fx, j), ld2(C.fy, j), ld2(C.fz, j),
-                          DL ? ld2(C.gx, j) : z2, DL ? ld2(C.gy, j) : z2, DL ? ld2(C.gz, j) : z2,
-                          DL ? ld2(C.ax, j) : z2, DL ? ld2(C.ay, j) : z2, DL ? ld2(C.az, j) : z2, cx, cy, cz);
-        }
-        if (j < cnt) {  // the odd last source
-          const float hx = C.hx[j] - tsh[0], hy = C.hy[j] - tsh[1], hz = C.hz[j] - tsh[2];
-          bool ok = hx * hx + hy * hy + hz * hz <= a.rc2_loose && !(a.own_split && C.surf[j] == surf_i);
-          float xx = 0.f, yy = 0.f, zz = 0.f, r2 = 0.f;
-          if (ok) {
-            xx = __fadd_rn(hx, C.lx[j] - tsl[0]);
-            yy = __fadd_rn(hy, C.ly[j] - tsl[1]);
-            zz = __fadd_rn(hz, C.lz[j] - tsl[2]);
-            r2 = xx * xx + yy * yy + zz * zz;
-            ok = r2 <= a.rc2_f;
+          float2 A, B, Adl, vx, vy, vz, fx = z2, fy = z2, fz = z2, gx = z2, gy = z2, gz = z2, nx = z2, ny = z2, nz = z2;
+          if (SL) {
+            const float4 u = C.r[ja][2], v = C.r[jb][2];
+            fx = f2(u.x, v.x); fy = f2(u.y, v.y); fz = f2(u.z, v.z);
           }
-          const float w = weight(C.surf[j], C.id[j], r2, ok, cb + j);
-          if (w != 0.f) {
-            const float rinv = rsqrtf(r2);
-            const float r = r2 * rinv;
-            const float st = r * a.sqpa_f;
-            const float ex = __expf(-st * st);
-            const float tq = __fdividef(1.f, fmaf(0.5f, st, 1.f));
-            float Q = a.erfcx_q[ERFCX_DEG];
-#pragma unroll
-            for (int k = ERFCX_DEG - 1; k >= 0; --k) Q = fmaf(Q, tq, a.erfcx_q[k]);
-            const float c1 = ex * (tq * Q), c2 = a.two_isqa_f * ex;
-            const float ir2 = rinv * rinv;
-            const float A = (c1 * rinv + c2) * ir2;
-            const float B = c1 * rinv - c2;
-            const float fx = C.fx[j], fy = C.fy[j], fz = C.fz[j];
-            const float Ad = A * (xx * fx + yy * fy + zz * fz);
-            float vx = Ad * xx + B * fx, vy = Ad * yy + B * fy, vz = Ad * zz + B * fz;
-            if (DL) {
-              const float cdl = a.m8_ispi_f * (ex * (st * (1.5f + st * st)) + a.q75_spi_f * c1);
-              const float Adl = cdl * ir2 * ir2 * rinv;
-              const float t = Adl * (xx * C.gx[j] + yy * C.gy[j] + zz * C.gz[j]) *
-                              (xx * C.ax[j] + yy * C.ay[j] + zz * C.az[j]);
-              vx += t * xx; vy += t * yy; vz += t * zz;
-            }
-            cx = fmaf(w, vx, cx);
-            cy = fmaf(w, vy, cy);
-            cz = fmaf(w, vz, cz);
+          if (DL) {
+            const float4 u = C.r[ja][2 + SL], v = C.r[jb][2 + SL], s = C.r[ja][3 + SL], t = C.r[jb][3 + SL];
+            gx = f2(u.x, v.x); gy = f2(u.y, v.y); gz = f2(u.z, v.z);
+            nx = f2(s.x, t.x); ny = f2(s.y, t.y); nz = f2(s.z, t.z);
           }
+          ewald_coef2<SL, DL>(a, r2, wa, wb, A, B, Adl);
+          ewald_apply2<SL, DL>(xx, yy, zz, A, B, Adl, fx, fy, fz, gx, gy, gz, nx, ny, nz, vx, vy, vz);
+          cx = fmaf(wb, vx.y, fmaf(wa, vx.x, cx));
+          cy = fmaf(wb, vy.y, fmaf(wa, vy.x, cy));
+          cz = fmaf(wb, vz.y, fmaf(wa, vz.x, cz));
         }
-        acc.add(0, cx);
-        acc.add(1, cy);
-        acc.add(2, cz);
-        if (a.collect && run_id >= 0) { L.insert(run_surf, run_id, run_d2); }
-        run_surf = -3; run_id = -1; run_d2 = 3.4e38f;
+      }
+      if (!F64) { acc.add(0, cx); acc.add(1, cy); acc.add(2, cz); }
+    }
+  }
+  if (run_id >= 0) L.insert(run_surf, run_id, (float)run_d2);
+  double sum[3];
+  for (int k = 0; k < 3; ++k) sum[k] = F64 ? acc64[k] : (double)acc.s[k] - (double)acc.c[k];
+  if (SUB > 1) {
+    // the target's lanes: their sums, and their neighbour lists into lane 0's
+    for (int o = 1; o < SUB; o <<= 1)
+      for (int k = 0; k < 3; ++k) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+    if (a.collect) {
+      L.overflow = __any_sync(0xffffffffu, L.overflow);
+      for (int r = 1; r < SUB; ++r) {
+        const int src = (lane & ~(SUB - 1)) + r;
+        const int nr = __shfl_sync(0xffffffffu, L.n, src);
+        const int most = __reduce_max_sync(0xffffffffu, nr);
+        for (int e = 0; e < most; ++e) {
+          const int k = min(e, RBC3D_NBR_MAX - 1);
+          const int sj = __shfl_sync(0xffffffffu, L.surf[k], src), id = __shfl_sync(0xffffffffu, L.idx[k], src);
+          const float d = __shfl_sync(0xffffffffu, L.d2[k], src);
+          if (sub == 0 && e < nr) L.insert(sj, id, d);
+        }
       }
     }
   }
-  if (active) {
-    double iA = 1.0 / a.tA[ti];
-    for (int k = 0; k < 3; ++k) a.v[ti + (size_t)k * a.nt] += ((double)acc.s[k] - (double)acc.c[k]) * iA;
+  if (active && sub == 0) {
+    const double iA = 1.0 / a.tA[ti];
+    for (int k = 0; k < 3; ++k) a.v[ti + (size_t)k * a.nt] += sum[k] * iA;
     if (a.collect) {
       if (L.overflow) atomicAdd(a.cnt + 2, 1ull);
       for (int e = 0; e < L.n; ++e) {
-        unsigned long long pos = atomicAdd(a.cnt + 0, 1ull);
+        const unsigned long long pos = atomicAdd(a.cnt + 0, 1ull);
         if (pos < (unsigned long long)a.cap) a.items[pos] = make_int4(ti, L.surf[e], L.idx[e] & 0xffff, L.idx[e] >> 16);
       }
     }
   }
   unsigned long long np = npairs;
   for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(0xffffffffu, np, o);
-  if ((tid & 31) == 0 && np) atomicAdd(a.cnt + 1, np);
+  if (lane == 0 && np) atomicAdd(a.cnt + 1, np);
 }
 
 // Own-cell pairs of the FP32 modes: the pairs of AddIntOnRbcs whose source
@@ -771,7 +847,7 @@ __global__ void __launch_bounds__(TILE, 8) k_pair32(PairArgs a) {
 // the same stream.  The target tile's at most (OWN_TILE - 1) / nlon + 2
 // latitude rings' rows of the weight table sit in shared memory.
 constexpr int OWN_TILE = 128;
-template <bool DL>
+template <bool SL, bool DL>
 __global__ void __launch_bounds__(OWN_TILE) k_pair_own32(PairArgs a) {
   __shared__ __align__(16) float s_src[15][OWN_TILE];  // hi xyz, lo xyz, f xyz, g xyz, normal xyz
   __shared__ __align__(16) int s_id[OWN_TILE];
@@ -862,8 +938,8 @@ __global__ void __launch_bounds__(OWN_TILE) k_pair_own32(PairArgs a) {
       }
       if (wa != 0.f || wb != 0.f) {
         float2 A, B, Adl, vx, vy, vz;
-        ewald_coef2<DL>(a, r2, wa, wb, A, B, Adl);
-        ewald_apply2<DL>(xx, yy, zz, A, B, Adl, ld2(s_src[6], j), ld2(s_src[7], j), ld2(s_src[8], j),
+        ewald_coef2<SL, DL>(a, r2, wa, wb, A, B, Adl);
+        ewald_apply2<SL, DL>(xx, yy, zz, A, B, Adl, ld2(s_src[6], j), ld2(s_src[7], j), ld2(s_src[8], j),
                          DL ? ld2(s_src[9], j) : z2, DL ? ld2(s_src[10], j) : z2, DL ? ld2(s_src[11], j) : z2,
                          DL ? ld2(s_src[12], j) : z2, DL ? ld2(s_src[13], j) : z2, DL ? ld2(s_src[14], j) : z2, vx,
                          vy, vz);
@@ -871,7 +947,7 @@ __global__ void __launch_bounds__(OWN_TILE) k_pair_own32(PairArgs a) {
         cy = fmaf(wb, vy.y, fmaf(wa, vy.x, cy));
         cz = fmaf(wb, vz.y, fmaf(wa, vz.x, cz));
         if (!diag) {  // pair (j, i): the vector is -x, so only the stresslet term changes sign
-          ewald_apply2<DL>(xx, yy, zz, A, B, Adl, tfx, tfy, tfz, tgx, tgy, tgz, tnx, tny, tnz, vx, vy, vz);
+          ewald_apply2<SL, DL>(xx, yy, zz, A, B, Adl, tfx, tfy, tfz, tgx, tgy, tgz, tnx, tny, tnz, vx, vy, vz);
           const float2 w2 = f2(wa, wb);
           float2* rx = reinterpret_cast<float2*>(&s_rev[wid][0][j]);
           float2* ry = reinterpret_cast<float2*>(&s_rev[wid][1][j]);
@@ -908,123 +984,127 @@ __global__ void __launch_bounds__(OWN_TILE) k_pair_own32(PairArgs a) {
   if ((tid & 31) == 0 && np) atomicAdd(a.cnt + 1, np);
 }
 
-// FP64 plain form: the same traversal with the reference arithmetic.
-template <bool DL>
-__global__ void __launch_bounds__(TILE) k_pair64(PairArgs a) {
-  __shared__ TileD sm;
-  __shared__ float3 wb[TILE / 32][2];
-  const int4 unit = a.units[blockIdx.x];
-  if (unit.z == 0) return;  // an empty entry past the end of the unit list
-  const int cell = unit.x;
-  const int tid = threadIdx.x;
-  const bool active = tid < unit.z;
-  const int ci = cell % a.Nc[0], cj = (cell / a.Nc[0]) % a.Nc[1], ck = cell / (a.Nc[0] * a.Nc[1]);
-  const double c0[3] = {(ci + 0.5) * a.h[0], (cj + 0.5) * a.h[1], (ck + 0.5) * a.h[2]};
-  int ti = active ? a.torder[unit.y + tid] : 0;
-  double t_[3] = {0, 0, 0};
-  int surf_i = -2, tlat = 0, tlon = 0;
-  double th_i = 0, phi_i = 0;
-  if (active) {
-    for (int k = 0; k < 3; ++k) t_[k] = min_image(a.tx[ti + (size_t)k * a.nt] - c0[k], a.L[k], a.iL[k]);
-    int4 m = a.tmeta[ti];
-    surf_i = m.x;
-    if (m.y >= 0) { th_i = a.th[m.y]; phi_i = a.phi[m.z]; tlat = m.y; tlon = m.z; }
+// The same in FP64: one source a step (at step s lane l takes source
+// (l + s) mod OWN_TILE), coefficients by the reference's tables.  Bound by the
+// FP64 pipe: about 66 instructions for both orders of a pair, against 75 and
+// more for each order in the cell-list walk.
+template <bool SL, bool DL>
+__global__ void __launch_bounds__(OWN_TILE) k_pair_own64(PairArgs a) {
+  __shared__ double s_src[12][OWN_TILE];  // xyz (relative to the cell's first point), f, g, normal
+  __shared__ int s_id[OWN_TILE];
+  __shared__ double s_rev[OWN_TILE / 32][3][OWN_TILE];  // per warp: the sources' sums
+  extern __shared__ double s_mask64[];  // rows lat0.. of the table, nlat * nhalf each
+  const int nlat = a.nlat, nlon = a.nlon, nv = nlat * nlon, rowlen = nlat * a.nhalf;
+  const int ntile = (nv + OWN_TILE - 1) / OWN_TILE, npt = ntile * (ntile + 1) / 2;
+  const int cell = blockIdx.x / npt;
+  int r = blockIdx.x - cell * npt, T = 0;
+  while (r >= ntile - T) { r -= ntile - T; ++T; }
+  const int S = T + r;
+  const bool diag = S == T;
+  const int tid = threadIdx.x, wid = tid >> 5;
+  const int k = T * OWN_TILE + tid;
+  const bool active = k < nv;
+  const int tlat = active ? k / nlon : 0, tlon = active ? k - tlat * nlon : 0;
+  const int lat0 = T * OWN_TILE / nlon;
+  const int nrow = min(nlat - 1, (T * OWN_TILE + OWN_TILE - 1) / nlon) - lat0 + 1;
+  for (int i = tid; i < nrow * rowlen; i += OWN_TILE) s_mask64[i] = a.mtab64[(size_t)lat0 * rowlen + i];
+  const int p = cell * nv + tlon * nlat + tlat, first = cell * nv;
+  auto relative = [&](int point, int c) {
+    return min_image(a.px[point + (size_t)c * a.ns] - a.px[first + (size_t)c * a.ns], a.L[c], a.iL[c]);
+  };
+  const int js = S * OWN_TILE + tid;
+  int ps = 0;
+  if (js < nv) {
+    const int sl = js / nlon;
+    ps = cell * nv + (js - sl * nlon) * nlat + sl;
+    const double* rec = a.rec64 + 12 * (size_t)a.sinv[ps];
+    for (int c = 0; c < 3; ++c) s_src[c][tid] = relative(ps, c);
+    for (int c = 3; c < 12; ++c)
+      if ((SL && c < 6) || (DL && c >= 6)) s_src[c][tid] = rec[c];
+    s_id[tid] = sl | ((js - sl * nlon) << 16);
+  } else {  // padding: a source beyond rc of every target
+    for (int c = 0; c < 12; ++c) s_src[c][tid] = 0.;
+    s_src[0][tid] = 1.0e18;
+    s_id[tid] = 0;
   }
-  // the same tile culling as the FP32 form (boxes in FP32 with a margin)
-  const CullBoxes cb = cull_boxes(active, (float)t_[0], (float)t_[1], (float)t_[2], wb);
+  for (int w = 0; w < OWN_TILE / 32; ++w)
+    for (int c = 0; c < 3; ++c) s_rev[w][c][tid] = 0.;
+  double tx[3] = {0, 0, 0}, tf[3] = {0, 0, 0}, tg[3] = {0, 0, 0}, tn[3] = {0, 0, 0};
+  if (active) {
+    const double* rec = a.rec64 + 12 * (size_t)a.sinv[p];
+    for (int c = 0; c < 3; ++c) {
+      tx[c] = relative(p, c);
+      if (SL) tf[c] = rec[3 + c];
+      if (DL) { tg[c] = rec[6 + c]; tn[c] = rec[9 + c]; }
+    }
+  }
+  __syncthreads();
+  const double* mrow = s_mask64 + (tlat - lat0) * rowlen;
   double acc[3] = {0, 0, 0};
-  NbrList L;
-  L.n = 0; L.overflow = 0;
-  int run_surf = -3, run_id = -1;
-  double run_d = 1e300;
-  unsigned long long npairs = 0;
-
-  for (int nb = 0; nb < 27; ++nb) {
-    int dx = nb % 3 - 1, dy = (nb / 3) % 3 - 1, dz = nb / 9 - 1;
-    int ni = imod(ci + dx, a.Nc[0]), nj = imod(cj + dy, a.Nc[1]), nk = imod(ck + dz, a.Nc[2]);
-    int ncell = ni + a.Nc[0] * (nj + a.Nc[1] * nk);
-    int sbeg = a.cs[ncell], send = a.ce[ncell];
-    const float3 dh = make_float3((float)(dx * a.h[0]), (float)(dy * a.h[1]), (float)(dz * a.h[2]));
-    const float3 wlo = f3sub(cb.wlo, dh), whi = f3sub(cb.whi, dh);
-    const float3 clo = f3sub(cb.clo, dh), chi = f3sub(cb.chi, dh);
-    for (int base = sbeg, tt = a.toff[ncell]; base < send; base += TILE, ++tt) {
-      const float4 blo = a.tbox[2 * tt], bhi = a.tbox[2 * tt + 1];
-      const float3 bl = make_float3(blo.x, blo.y, blo.z), bh = make_float3(bhi.x, bhi.y, bhi.z);
-      if (boxes_apart(clo, chi, bl, bh, a.rc2_f)) continue;  // uniform over the CTA
-      int cnt = min(TILE, send - base);
-      __syncthreads();
-      if (tid < cnt) {
-        int q = base + tid;
-        sm.x[tid] = min_image(a.sx[q] - c0[0], a.L[0], a.iL[0]);
-        sm.y[tid] = min_image(a.sx[q + a.ns] - c0[1], a.L[1], a.iL[1]);
-        sm.z[tid] = min_image(a.sx[q + 2 * (size_t)a.ns] - c0[2], a.L[2], a.iL[2]);
-        sm.fx[tid] = a.sf[q]; sm.fy[tid] = a.sf[q + a.ns]; sm.fz[tid] = a.sf[q + 2 * (size_t)a.ns];
+  unsigned npairs = 0;
+  for (int step = 0; step < OWN_TILE; ++step) {
+    if (active) {
+      const int j = (tid + step) & (OWN_TILE - 1);
+      const double x = s_src[0][j] - tx[0], y = s_src[1][j] - tx[1], z = s_src[2][j] - tx[2];
+      const double r2 = fma(x, x, fma(y, y, z * z));
+      npairs += r2 <= a.rc2 ? (diag ? 1u : 2u) : 0u;
+      double EA, EB, ED;
+      if (ewald_coef64<SL, DL>(a.T, r2, EA, EB, ED)) {
+        const int id = s_id[j];
+        int dl = abs((id >> 16) - tlon);
+        dl = min(dl, nlon - dl);
+        const double wt = 1. - mrow[(id & 0xffff) * a.nhalf + dl];
+        double t = 0., u = 0., b = 0., dg, da;
+        if (SL) {
+          EA *= wt;
+          b = wt * EB;
+          t = EA * fma(x, s_src[3][j], fma(y, s_src[4][j], z * s_src[5][j]));
+        }
         if (DL) {
-          sm.gx[tid] = a.sg[q]; sm.gy[tid] = a.sg[q + a.ns]; sm.gz[tid] = a.sg[q + 2 * (size_t)a.ns];
-          sm.ax[tid] = a.sa3[q]; sm.ay[tid] = a.sa3[q + a.ns]; sm.az[tid] = a.sa3[q + 2 * (size_t)a.ns];
+          ED *= wt;
+          dg = fma(x, s_src[6][j], fma(y, s_src[7][j], z * s_src[8][j]));
+          da = fma(x, s_src[9][j], fma(y, s_src[10][j], z * s_src[11][j]));
+          t = fma(ED * dg, da, t);
         }
-        int4 m = a.smeta[q];
-        sm.surf[tid] = m.x; sm.ilat[tid] = m.y; sm.ilon[tid] = m.z;
-      }
-      __syncthreads();
-      if (active && !boxes_apart(wlo, whi, bl, bh, a.rc2_f)) {
-        for (int j = 0; j < cnt; ++j) {
-          const int sj = sm.surf[j];
-          if (a.collect && sj != run_surf) {
-            if (run_id >= 0) L.insert(run_surf, run_id, (float)run_d);
-            run_surf = sj; run_id = -1; run_d = 1e300;
-          }
-          double xx = sm.x[j] - t_[0], yy = sm.y[j] - t_[1], zz = sm.z[j] - t_[2];
-          const double r2 = xx * xx + yy * yy + zz * zz;
-          if (r2 > a.rc2) continue;  // the square root only for pairs inside the cutoff
-          const double ir = rsqrt(r2), rr = r2 > 0. ? r2 * ir : 0.;
-          ++npairs;
-          double mask = 0.;
-          if (sj == surf_i && a.mtab64) {
-            int dl = abs(sm.ilon[j] - tlon);
-            dl = min(dl, a.nlon - dl);
-            mask = __ldg(a.mtab64 + ((size_t)tlat * a.nlat + sm.ilat[j]) * a.nhalf + dl);
-          } else if (sj == surf_i) {
-            double dth = dist_on_sphere(th_i, phi_i, a.th[sm.ilat[j]], a.phi[sm.ilon[j]]);
-            mask = mask64(a.T, dth * a.inv_radius);
-          } else if (a.collect) {
-            if (rr < run_d) { run_d = rr; run_id = sm.ilat[j] | (sm.ilon[j] << 16); }
-          }
-          double EA, EB;
-          ewald_sl64r(a.T, rr, ir, EA, EB);
-          double s1 = (1. - mask) * a.c1;
-          double d = xx * sm.fx[j] + yy * sm.fy[j] + zz * sm.fz[j];
-          acc[0] += s1 * (EA * xx * d + EB * sm.fx[j]);
-          acc[1] += s1 * (EA * yy * d + EB * sm.fy[j]);
-          acc[2] += s1 * (EA * zz * d + EB * sm.fz[j]);
+        acc[0] = fma(t, x, acc[0]); acc[1] = fma(t, y, acc[1]); acc[2] = fma(t, z, acc[2]);
+        if (SL) {
+          acc[0] = fma(b, s_src[3][j], acc[0]); acc[1] = fma(b, s_src[4][j], acc[1]); acc[2] = fma(b, s_src[5][j], acc[2]);
+        }
+        if (!diag) {  // pair (j, i): the vector is -x, so only the stresslet term changes sign
+          if (SL) u = EA * fma(x, tf[0], fma(y, tf[1], z * tf[2]));
           if (DL) {
-            double EAd = ewald_dl64r(a.T, rr, ir);
-            double dg = xx * sm.gx[j] + yy * sm.gy[j] + zz * sm.gz[j];
-            double da = xx * sm.ax[j] + yy * sm.ay[j] + zz * sm.az[j];
-            double s2 = (1. - mask) * a.c2;
-            acc[0] += s2 * (EAd * xx * dg * da);
-            acc[1] += s2 * (EAd * yy * dg * da);
-            acc[2] += s2 * (EAd * zz * dg * da);
+            dg = fma(x, tg[0], fma(y, tg[1], z * tg[2]));
+            da = fma(x, tn[0], fma(y, tn[1], z * tn[2]));
+            u = fma(-ED * dg, da, u);
+          }
+          const double xs[3] = {x, y, z};
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            double v = fma(u, xs[c], s_rev[wid][c][j]);
+            if (SL) v = fma(b, tf[c], v);
+            s_rev[wid][c][j] = v;
           }
         }
-        if (a.collect && run_id >= 0) L.insert(run_surf, run_id, (float)run_d);
-        run_surf = -3; run_id = -1; run_d = 1e300;
       }
     }
+    __syncwarp();  // the lanes' per-warp sums of this step are written before the next step's
   }
+  __syncthreads();
   if (active) {
-    double iA = 1.0 / a.tA[ti];
-    for (int k = 0; k < 3; ++k) a.v[ti + (size_t)k * a.nt] += acc[k] * iA;
-    if (a.collect) {
-      if (L.overflow) atomicAdd(a.cnt + 2, 1ull);
-      for (int e = 0; e < L.n; ++e) {
-        unsigned long long pos = atomicAdd(a.cnt + 0, 1ull);
-        if (pos < (unsigned long long)a.cap) a.items[pos] = make_int4(ti, L.surf[e], L.idx[e] & 0xffff, L.idx[e] >> 16);
-      }
+    const double iA = 1.0 / a.tA[p];
+    for (int c = 0; c < 3; ++c) atomicAdd(a.v + p + (size_t)c * a.nt, acc[c] * iA);
+  }
+  if (!diag && js < nv) {
+    const double iA = 1.0 / a.tA[ps];
+    for (int c = 0; c < 3; ++c) {
+      double sum = 0.;
+      for (int w = 0; w < OWN_TILE / 32; ++w) sum += s_rev[w][c][tid];
+      atomicAdd(a.v + ps + (size_t)c * a.nt, sum * iA);
     }
   }
-  for (int o = 16; o > 0; o >>= 1) npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
-  if ((tid & 31) == 0 && npairs) atomicAdd(a.cnt + 1, npairs);
+  unsigned long long np = npairs;
+  for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(0xffffffffu, np, o);
+  if ((tid & 31) == 0 && np) atomicAdd(a.cnt + 1, np);
 }
 
 // AddLinearInt (ModIntOnRbcs.F90:162-201): xvint = sum Bcoef * x * (g.a3) dS
@@ -1052,21 +1132,31 @@ __global__ void k_linear_add(int nt, const double* __restrict__ tA, const double
 
 inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
-rbc3d_status sort_points(rbc3d_ctx* ctx, int n, const double* x_dev, DBuf<int>& order, DBuf<int>& cs, DBuf<int>& ce) {
+rbc3d_status sort_points(rbc3d_ctx* ctx, int n, const double* x_dev, DBuf<int>& order, DBuf<int>& cs, DBuf<int>& ce,
+                         bool targets = false) {
   const HashGrid& hg = ctx->hg;
   DBuf<int>&key = ctx->sort_key, &key2 = ctx->sort_key2, &idx = ctx->sort_idx;
   CUDA_TRY(key.alloc(n)); CUDA_TRY(key2.alloc(n)); CUDA_TRY(idx.alloc(n)); CUDA_TRY(order.alloc(n));
   CUDA_TRY(cs.alloc(hg.ncells)); CUDA_TRY(ce.alloc(hg.ncells));
-  { k_hash_keys<<<nblk(n, 256), 256, 0, ctx->st>>>(n, x_dev, hg.Nc[0], hg.Nc[1], hg.Nc[2], hg.Nc[0] / hg.L[0],
-                                                  hg.Nc[1] / hg.L[1], hg.Nc[2] / hg.L[2], key.p, idx.p); ++ctx->launches; }
+  int bits = 1;
+  while ((1ll << bits) < hg.ncells) ++bits;
+  const bool morton = targets && bits + MORTON_BITS < 31;
+  const int shift = morton ? MORTON_BITS : 0;
+  auto keys = [&](auto kern) {
+    kern<<<nblk(n, 256), 256, 0, ctx->st>>>(n, x_dev, hg.Nc[0], hg.Nc[1], hg.Nc[2], hg.Nc[0] / hg.L[0],
+                                            hg.Nc[1] / hg.L[1], hg.Nc[2] / hg.L[2], key.p, idx.p);
+    ++ctx->launches;
+  };
+  if (morton) keys(k_hash_keys<true>);
+  else keys(k_hash_keys<false>);
   size_t tmp = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, tmp, key.p, key2.p, idx.p, order.p, n, 0, 32, ctx->st);
+  cub::DeviceRadixSort::SortPairs(nullptr, tmp, key.p, key2.p, idx.p, order.p, n, 0, bits + shift, ctx->st);
   DBuf<char>& tbuf = ctx->sort_tmp;
   CUDA_TRY(tbuf.alloc(tmp + 1));
-  CUDA_TRY(cub::DeviceRadixSort::SortPairs(tbuf.p, tmp, key.p, key2.p, idx.p, order.p, n, 0, 32, ctx->st));
+  CUDA_TRY(cub::DeviceRadixSort::SortPairs(tbuf.p, tmp, key.p, key2.p, idx.p, order.p, n, 0, bits + shift, ctx->st));
   CUDA_TRY(cudaMemsetAsync(cs.p, 0, sizeof(int) * hg.ncells, ctx->st));
   CUDA_TRY(cudaMemsetAsync(ce.p, 0, sizeof(int) * hg.ncells, ctx->st));
-  { k_cell_ranges<<<nblk(n, 256), 256, 0, ctx->st>>>(n, key2.p, cs.p, ce.p); ++ctx->launches; }
+  { k_cell_ranges<<<nblk(n, 256), 256, 0, ctx->st>>>(n, shift, key2.p, cs.p, ce.p); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());
   return RBC3D_OK;
 }
@@ -1111,11 +1201,16 @@ rbc3d_status fill_units(rbc3d_ctx* ctx, const DBuf<int>& cs, const DBuf<int>& ce
   return RBC3D_OK;
 }
 
+// Lanes per target of the pair sums.  Few targets: with one lane each the
+// longest warps set the time.  FP32D, pair stage alone and whole matvec, one
+// lane / four: 8 cells (10,000 targets) 653 / 325 us and 918 / 609; 64 cells
+// (80,000) 1197 / 883 and 2242 / 2052; 128 cells 1775 / 1693 but 4061 / 4313
+// (the wider walk holds up the mesh beside it); 256 cells 2702 / 3029.  FP64,
+// 64 cells: 13.2 / 11.2 ms; 256 cells: 42.3 / 42.2.
+int pair_sub(int n) { return n <= 100000 ? 4 : 1; }
+
 rbc3d_status make_units(rbc3d_ctx* ctx, TargetSet& t, const DBuf<int>& cs, const DBuf<int>& ce) {
   const int nc = ctx->hg.ncells;
-  // capacity: every non-empty cell gives at most count / tile + 1 units
-  const int cap = nc + (t.n + TILE - 1) / TILE, wcap = nc + (t.n + 31) / 32;
-  rbc3d_status s;
   // sources per cell: the source list's ranges (or the targets' own when
   // there is no source list)
   const bool src = ctx->npt > 0 && ctx->s_cstart.p;
@@ -1126,14 +1221,12 @@ rbc3d_status make_units(rbc3d_ctx* ctx, TargetSet& t, const DBuf<int>& cs, const
     CUDA_TRY(cudaMemsetAsync(ctx->unit_zero.p, 0, sizeof(int) * nc, ctx->st));
     ss = se = ctx->unit_zero.p;
   }
-  // block units (FP64 pair sums: the block shares its source tiles) and
-  // warp units (FP32 pair sums: each warp stages its own chunks, so a block's
-  // warps may come from different cells and none idles)
-  if ((s = fill_units(ctx, cs, ce, ss, se, TILE, cap, t.units))) return s;
-  if ((s = fill_units(ctx, cs, ce, ss, se, 32, wcap, t.wunits))) return s;
+  t.sub = pair_sub(t.n);
+  const int tile = 32 / t.sub;
+  // capacity: every non-empty cell gives at most count / tile + 1 units
+  const int cap = nc + (t.n + tile - 1) / tile;
   t.nunits = cap;
-  t.nwunits = wcap;
-  return RBC3D_OK;
+  return fill_units(ctx, cs, ce, ss, se, tile, cap, t.units);
 }
 
 }  // namespace
@@ -1266,7 +1359,7 @@ rbc3d_status sort_targets(rbc3d_ctx* ctx, int tlist) {
     CUDA_TRY(cudaMemcpyAsync(t.cstart.p, ctx->s_cstart.p, sizeof(int) * ctx->hg.ncells, cudaMemcpyDeviceToDevice, ctx->st));
     CUDA_TRY(cudaMemcpyAsync(t.cend.p, ctx->s_cend.p, sizeof(int) * ctx->hg.ncells, cudaMemcpyDeviceToDevice, ctx->st));
   } else {
-    if ((s = sort_points(ctx, t.n, t.x.p, t.order, t.cstart, t.cend))) return s;
+    if ((s = sort_points(ctx, t.n, t.x.p, t.order, t.cstart, t.cend, true))) return s;
   }
   if ((s = make_units(ctx, t, t.cstart, t.cend))) return s;
   t.sorted = true;
@@ -1280,12 +1373,11 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
   rbc3d_status s = sort_targets(ctx, tlist);
   if (s) return s;
   PairArgs a;
-  a.nt = t.n; a.tx = t.x.p; a.tA = t.Acoef.p; a.tmeta = t.meta.p; a.torder = t.order.p; a.units = t.units.p; a.v = t.v.p;
-  a.ns = ctx->npt; a.sx = ctx->s_x.p; a.sf = ctx->s_f.p; a.sg = ctx->s_g.p; a.sa3 = ctx->s_a3.p; a.smeta = ctx->s_meta.p;
-  a.cs = ctx->s_cstart.p; a.ce = ctx->s_cend.p;
+  a.nt = t.n; a.tx = t.x.p; a.tA = t.Acoef.p; a.tmeta = t.meta.p; a.torder = t.order.p; a.v = t.v.p;
+  a.units = t.units.p; a.nunits = t.nunits;
+  a.ns = ctx->npt; a.cs = ctx->s_cstart.p; a.ce = ctx->s_cend.p;
   a.sp0 = ctx->s_p0.p; a.sp1 = ctx->s_p1.p; a.su = ctx->s_u4.p; a.sa4 = ctx->s_a4.p;
-  a.sF4 = ctx->s_F4.p; a.sG4 = ctx->s_G4.p; a.toff = ctx->s_toff.p; a.tbox = ctx->s_tbox.p;
-  a.coff = ctx->s_coff.p; a.cbox = ctx->s_cbox.p;
+  a.toff = ctx->s_toff.p; a.tbox = ctx->s_tbox.p; a.coff = ctx->s_coff.p; a.cbox = ctx->s_cbox.p;
   for (int d = 0; d < 3; ++d) { a.Nc[d] = ctx->hg.Nc[d]; a.h[d] = ctx->hg.h[d]; a.L[d] = ctx->hg.L[d]; a.iL[d] = ctx->iLb[d]; }
   a.th = ctx->th.p; a.phi = ctx->phi.p; a.usph = ctx->usph.p; a.nlat = ctx->nlat;
   a.nlon = ctx->nlon; a.nhalf = ctx->nlon / 2 + 1;
@@ -1294,8 +1386,8 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
   a.radius = ctx->radius; a.inv_radius = 1.0 / ctx->radius; a.inv_radius_f = (float)(1.0 / ctx->radius);
   double cm = 2.0 * sin(0.5 * ctx->radius) * (1.0 + 1e-6);
   a.chord2_max = (float)(cm * cm);
-  a.c1 = c1; a.c2 = c2; a.c1f = (float)c1; a.c2f = (float)c2;
   a.rc2 = ctx->prm.rc * ctx->prm.rc; a.rc2_f = (float)a.rc2;
+  a.px = ctx->x.p;
   a.rc2_loose = (float)((ctx->prm.rc + 1e-3) * (ctx->prm.rc + 1e-3)); a.reps2_f = (float)(ctx->T.r_eps * ctx->T.r_eps);
   const double rthr = near_rthr_now(ctx);
   a.rthr2_f = (float)(rthr * rthr);
@@ -1308,45 +1400,58 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
   a.T = ctx->T;
   a.collect = collect_nbr ? 1 : 0;
   a.items = ctx->items.p; a.cap = ctx->items_cap; a.cnt = ctx->dcnt.p;
-  bool dl = (c2 != 0.0) && ctx->has_g;
-  if (prec != RBC3D_FP64) {
-    CUDA_TRY(ctx->s_F4.alloc(ctx->npt));
-    if (dl) CUDA_TRY(ctx->s_G4.alloc(ctx->npt));
-    a.sF4 = ctx->s_F4.p; a.sG4 = ctx->s_G4.p;
-    { k_src_dens4<<<nblk(ctx->npt, 256), 256, 0, ctx->st>>>(ctx->npt, c1, c2, ctx->s_f.p, ctx->s_g.p, dl ? 1 : 0,
-                                                             ctx->s_F4.p, ctx->s_G4.p); ++ctx->launches; }
-    a.units = t.wunits.p;
-    a.nunits = t.nwunits;
-    // own-cell pairs of the cell targets by the dense pass when the
-    // same-cell weights come from the table (uniform longitudes)
-    const int nrow = std::min(ctx->nlat, (OWN_TILE - 1) / std::max(ctx->nlon, 1) + 2);
-    const size_t own_sm = sizeof(float) * (size_t)nrow * ctx->nlat * a.nhalf;
-    const bool own = tlist == RBC3D_TLIST_RBC && a.mtab32 && t.n == ctx->npt && ctx->s_op0.p && own_sm <= 160 * 1024;
-    a.own_split = own ? 1 : 0;
-    a.op0 = ctx->s_op0.p; a.op1 = ctx->s_op1.p; a.sinv = ctx->s_inv.p;
-    const int nb = (t.nwunits + TILE / 32 - 1) / (TILE / 32);
-    if (dl) { k_pair32<true><<<nb, TILE, 0, ctx->st>>>(a); ++ctx->launches; }
-    else { k_pair32<false><<<nb, TILE, 0, ctx->st>>>(a); ++ctx->launches; }
-    if (own) {
-      const int nv = ctx->nlat * ctx->nlon, nt = (nv + OWN_TILE - 1) / OWN_TILE, nbo = ctx->ncell * (nt * (nt + 1) / 2);
-      if (dl) {
-        if (own_sm > 48 * 1024)
-          CUDA_TRY(cudaFuncSetAttribute(k_pair_own32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)own_sm));
-        k_pair_own32<true><<<nbo, OWN_TILE, own_sm, ctx->st>>>(a);
-      } else {
-        if (own_sm > 48 * 1024)
-          CUDA_TRY(cudaFuncSetAttribute(k_pair_own32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)own_sm));
-        k_pair_own32<false><<<nbo, OWN_TILE, own_sm, ctx->st>>>(a);
-      }
-      ++ctx->launches;
-    }
+  const bool dl = c2 != 0.0 && ctx->has_g, sl = c1 != 0.0 && ctx->has_f;
+  const int n = ctx->npt, nb = (t.nunits + TILE / 32 - 1) / (TILE / 32);
+  const HashGrid& hg = ctx->hg;
+  // own-cell pairs of the cell targets by the dense pass when the same-cell
+  // weights come from the table (uniform longitudes)
+  const bool f64 = prec == RBC3D_FP64;
+  const int nrow = std::min(ctx->nlat, (OWN_TILE - 1) / std::max(ctx->nlon, 1) + 2);
+  const size_t own_sm = (f64 ? sizeof(double) : sizeof(float)) * (size_t)nrow * ctx->nlat * a.nhalf;
+  const bool own = tlist == RBC3D_TLIST_RBC && a.mtab32 && t.n == n && ctx->s_op0.p && own_sm <= 160 * 1024;
+  a.own_split = own ? 1 : 0;
+  a.op0 = ctx->s_op0.p; a.op1 = ctx->s_op1.p; a.sinv = ctx->s_inv.p;
+  if (f64) {
+    CUDA_TRY(ctx->s_rec64.alloc(12 * (size_t)n));
+    a.rec64 = ctx->s_rec64.p;
+    { k_src_rec64<<<nblk(n, 256), 256, 0, ctx->st>>>(n, c1, c2, ctx->s_x.p, ctx->s_f.p, ctx->s_g.p, ctx->s_a3.p, hg.Nc[0],
+                                                     hg.Nc[1], hg.Nc[2], hg.h[0], hg.h[1], hg.h[2], hg.L[0], hg.L[1],
+                                                     hg.L[2], sl, dl, ctx->s_rec64.p); ++ctx->launches; }
   } else {
-    a.own_split = 0;
-    if (dl) { k_pair64<true><<<t.nunits, TILE, 0, ctx->st>>>(a); ++ctx->launches; }
-    else { k_pair64<false><<<t.nunits, TILE, 0, ctx->st>>>(a); ++ctx->launches; }
+    CUDA_TRY(ctx->s_F4.alloc(n));
+    if (dl) CUDA_TRY(ctx->s_G4.alloc(n));
+    a.sF4 = ctx->s_F4.p; a.sG4 = ctx->s_G4.p;
+    { k_src_dens4<<<nblk(n, 256), 256, 0, ctx->st>>>(n, c1, c2, ctx->s_f.p, ctx->s_g.p, sl, dl,
+                                                     ctx->s_F4.p, ctx->s_G4.p); ++ctx->launches; }
   }
-  CUDA_TRY(cudaGetLastError());
-  return RBC3D_OK;
+  auto launch = [&](auto kern, int blocks, size_t bytes) -> rbc3d_status {
+    // (static and dynamic shared memory together may pass the 48 KB that need no opt-in)
+    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    kern<<<blocks, TILE, bytes, ctx->st>>>(a);
+    ++ctx->launches;
+    CUDA_TRY(cudaGetLastError());
+    return RBC3D_OK;
+  };
+  auto pairs = [&](auto R, auto SL, auto DL) -> rbc3d_status {
+    using T = decltype(R);
+    const size_t bytes = TILE / 32 * warp_tile_bytes<T, SL.value, DL.value>();
+    if (t.sub == 4) return launch(k_pair<T, SL.value, DL.value, 4>, nb, bytes);
+    return launch(k_pair<T, SL.value, DL.value, 1>, nb, bytes);
+  };
+  auto own_pairs = [&](auto R, auto SL, auto DL) -> rbc3d_status {
+    const int nt = (ctx->nlat * ctx->nlon + OWN_TILE - 1) / OWN_TILE, blocks = ctx->ncell * (nt * (nt + 1) / 2);
+    if (sizeof(R) == 8) return launch(k_pair_own64<SL.value, DL.value>, blocks, own_sm);
+    return launch(k_pair_own32<SL.value, DL.value>, blocks, own_sm);
+  };
+  const std::true_type yes{};
+  const std::false_type no{};
+  auto run = [&](auto R) -> rbc3d_status {
+    // without a density the walk still counts pairs and lists neighbours: as the single layer of zeros
+    rbc3d_status e = sl && dl ? pairs(R, yes, yes) : dl ? pairs(R, no, yes) : pairs(R, yes, no);
+    if (e || !own) return e;
+    return sl && dl ? own_pairs(R, yes, yes) : dl ? own_pairs(R, no, yes) : own_pairs(R, yes, no);
+  };
+  return f64 ? run(0.0) : run(0.f);
 }
 
 rbc3d_status run_linear(rbc3d_ctx* ctx, int tlist, double c2) {

@@ -30,7 +30,6 @@
 // u_th, u_ph, u'_ph - u_ph, u_thph, values x, f, g, a3.
 #include <algorithm>
 #include <cmath>
-#include <cstring>
 #include <vector>
 
 #include "ctx.hpp"
@@ -50,9 +49,8 @@ struct RingArgs {
   double* v;
   const int* celltype;
   const double* Bc;
-  const double* tab;  // per Ewald table entry: c1, dc1, c2, dc2, dl, ddl (value and step to the next)
-  double c1, c2, ntab_over_rc;
-  long long eps2, rc2;  // bits of r_eps^2 and rc^2: positive doubles order as their bits
+  Tables T;
+  double c1, c2;
 };
 
 // Node values of the sets in `sets` (bit 0 x, 1 f, 2 g, 3 a3) in column order;
@@ -85,15 +83,6 @@ __global__ void __launch_bounds__(128) k_ring_rec(int m, int n, const double* __
     if (sl == 1 || sl == 4) v = s[r + 1][c][q] - v;
     rec[(((size_t)cell * m + i) * RSLOT * RVAL + (size_t)sl * RVAL + 3 * set + k) * n + j] = v;
   }
-}
-
-// 1/sqrt(x) for a positive, normal x: the hardware's approximation and one
-// step of third order (y <- y + y e (1/2 + 3/8 e), e = 1 - x y^2).
-__device__ __forceinline__ double rsqrt_step(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 template <bool SL, bool DL>
@@ -164,31 +153,17 @@ __global__ void __launch_bounds__(256, 1) k_self_ring(RingArgs a) {
       for (int v = 0; v < NV; ++v) p[v] = fma(y3, E[v], fma(y2, D[v], fma(y1, dU[v], U[v])));
       for (int k = 0; k < 3; ++k) p[k] -= sT[k * W + q];
       const double r2 = fma(p[0], p[0], fma(p[1], p[1], p[2] * p[2]));
-      // rr >= rc (ModRbcSingInt.F90:65) and rr < r_eps contribute nothing, nor does a NaN
-      const long long bits = __double_as_longlong(r2);
-      if (bits < a.eps2 || bits >= a.rc2) continue;
-      const double ir = rsqrt_step(r2), rr = r2 * ir;
-      // table position: floor by the downward-rounded sum with 1.5 2^52
-      const double magic = 6755399441055744.0;
-      const double ft = __fma_rd(rr, a.ntab_over_rc, magic);
-      const int it = __double2loint(ft);
-      if ((unsigned)it >= (unsigned)EWALD_NTAB) continue;
-      const double f1 = fma(rr, a.ntab_over_rc, magic - ft);
-      const double2* tb = reinterpret_cast<const double2*>(a.tab) + 3 * it;
-      const double ir2 = ir * ir;
+      double EA, EB, ED;
+      if (!ewald_coef64<SL, DL>(a.T, r2, EA, EB, ED)) continue;  // rr >= rc: ModRbcSingInt.F90:65
       double cx = 0., cf = 0.;  // dv = cx xx + cf f
       if (SL) {
-        const double2 t1 = __ldg(tb), t2 = __ldg(tb + 1);
-        const double c1ir = fma(t1.y, f1, t1.x) * ir, cs2 = fma(t2.y, f1, t2.x);
-        cx = w1 * ((c1ir + cs2) * ir2) * fma(p[0], p[OF], fma(p[1], p[OF + 1], p[2] * p[OF + 2]));
-        cf = w1 * (c1ir - cs2);
+        cx = w1 * EA * fma(p[0], p[OF], fma(p[1], p[OF + 1], p[2] * p[OF + 2]));
+        cf = w1 * EB;
       }
       if (DL && c2m != 0.) {
-        const double2 t3 = __ldg(tb + 2);
-        const double EA = w2 * fma(t3.y, f1, t3.x) * (ir2 * ir2 * ir);
         const double dg = fma(p[0], p[OG], fma(p[1], p[OG + 1], p[2] * p[OG + 2]));
         const double da = fma(p[0], p[OA], fma(p[1], p[OA + 1], p[2] * p[OA + 2]));
-        cx = fma(EA * dg, da, cx);
+        cx = fma(w2 * ED * dg, da, cx);
       }
       double* s = acc + 3 * side * W + q;
 #pragma unroll
@@ -317,11 +292,8 @@ rbc3d_status run_self_ring(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   a.parts = ring_parts(a.NC, blocks, nsm);
   a.rec = ctx->ring_rec.p; a.cls = reinterpret_cast<const RingClass*>(ctx->ring_cls.p); a.spl = ctx->spl.p;
   a.th = ctx->th.p; a.phi = ctx->phi.p; a.tA = t.Acoef.p; a.v = t.v.p; a.celltype = ctx->celltype.p; a.Bc = ctx->dBcoef.p;
-  a.tab = ctx->ring_tab.p;
-  a.c1 = c1; a.c2 = c2; a.ntab_over_rc = ctx->T.ntab_over_rc;
-  const double e2 = ctx->T.r_eps * ctx->T.r_eps, rc2 = ctx->prm.rc * ctx->prm.rc;
-  std::memcpy(&a.eps2, &e2, 8);
-  std::memcpy(&a.rc2, &rc2, 8);
+  a.T = ctx->T;
+  a.c1 = c1; a.c2 = c2;
   auto launch = [&](auto kern, int nv) -> rbc3d_status {
     const size_t bytes = sizeof(double) * (size_t)thr * (2 * nv + 9);
     CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
