@@ -90,6 +90,10 @@ struct PmeState {
   DBuf<float> vel32;       // 3*G velocity grid
   DBuf<double> vel64;
   DBuf<double> bbx, bby, bbz;
+  DBuf<float2> infl32;     // influence factors per half-spectrum entry, wave numbers per axis
+  DBuf<double2> infl64;
+  DBuf<float> wave32;
+  DBuf<double> wave64;
   cufftHandle r2c32_3 = 0, r2c32_12 = 0, c2r32_3 = 0;
   cufftHandle r2c64_3 = 0, r2c64_12 = 0, c2r64_3 = 0;
   bool planned32 = false, planned64 = false;
@@ -200,11 +204,11 @@ struct rbc3d_ctx {
   DBuf<float4> s_p0, s_p1, s_u4, s_a4, s_F4, s_G4;
   DBuf<int> s_toff, s_coff;
   DBuf<float4> s_tbox, s_cbox;  // per 128-source tile and per 32-source chunk
+  DBuf<double> s_rec64;         // FP64 pair-sum records (12 doubles a source)
   DBuf<float4> s_op0, s_op1;    // own-cell pair records in point order (k_pair_own32)
   DBuf<int> s_inv;              // point -> sorted source position
   int s_ntiles = 0;
   DBuf<unsigned long long> near_queue;  // work counter of the near-singular kernel
-  DBuf<double> s_rec64;         // FP64 pair-sum records (12 doubles a source)
   DBuf<double> dBcoef;                  // Bcoef per cell type on the device
   DBuf<char> ring_cls;                  // patch-point classes per latitude (RingClass)
   DBuf<double> ring_tab, ring_rec;      // FP64 patch: Ewald tables with steps, node values in column order

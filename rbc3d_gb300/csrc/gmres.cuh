@@ -77,20 +77,36 @@ __global__ void k_axpby(int n, double a, const double* __restrict__ x, double b,
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = a * x[i] + b * y[i];
 }
-// Givens / Hessenberg step for column k (single thread).  H column-major with
-// leading dimension ldh = restart+1.  Writes |g_{k+1}| to res.
-__global__ void k_givens(int k, int ldh, double* H, const double* hcol, double hn, double* cs, double* sn,
-                         double* g, double* res) {
-  if (threadIdx.x || blockIdx.x) return;
+// Givens / Hessenberg step for column k (one block).  H column-major with
+// leading dimension ldh = restart+1.  Writes |g_{k+1}| to res.  The rotations
+// are a serial chain; it runs over blocks of kGivens columns in shared memory
+// (from global memory each step waited for its loads: 17 us a step at 100
+// columns).
+constexpr int kGivens = 128;
+__global__ void __launch_bounds__(kGivens) k_givens(int k, int ldh, double* H, const double* hcol, double hn, double* cs,
+                                                    double* sn, double* g, double* res) {
+  __shared__ double sc[kGivens], ss[kGivens], sh[kGivens + 1];
   double* c = H + (size_t)ldh * k;
-  for (int j = 0; j <= k; ++j) c[j] = hcol[j];
-  c[k + 1] = hn;
-  for (int j = 0; j < k; ++j) {
-    double a = c[j], b = c[j + 1];
-    c[j] = cs[j] * a + sn[j] * b;
-    c[j + 1] = -sn[j] * a + cs[j] * b;
+  double a = 0, b = 0;  // thread 0: the running entry
+  for (int j0 = 0; j0 < k; j0 += kGivens) {
+    const int n = min(kGivens, k - j0), t = threadIdx.x;
+    if (t < n) { sc[t] = cs[j0 + t]; ss[t] = sn[j0 + t]; sh[t] = hcol[j0 + t + 1]; }
+    __syncthreads();
+    if (t == 0) {
+      if (j0 == 0) a = hcol[0];
+      for (int j = 0; j < n; ++j) {
+        b = sh[j];
+        sh[j] = sc[j] * a + ss[j] * b;
+        a = -ss[j] * a + sc[j] * b;
+      }
+    }
+    __syncthreads();
+    if (t < n) c[j0 + t] = sh[t];
+    __syncthreads();
   }
-  double a = c[k], b = c[k + 1];
+  if (threadIdx.x) return;
+  if (k == 0) a = hcol[0];
+  b = hn;
   double den = sqrt(a * a + b * b);
   cs[k] = den > 0 ? a / den : 1.;
   sn[k] = den > 0 ? b / den : 0.;
@@ -100,12 +116,14 @@ __global__ void k_givens(int k, int ldh, double* H, const double* hcol, double h
   g[k] = cs[k] * g[k];
   *res = fabs(g[k + 1]);
 }
-__global__ void k_backsolve(int k, int ldh, const double* H, const double* g, double* y) {
-  if (threadIdx.x || blockIdx.x) return;
+// Back substitution by one warp, a row at a time (its sum over the lanes).
+__global__ void __launch_bounds__(32) k_backsolve(int k, int ldh, const double* H, const double* g, double* y) {
   for (int i = k - 1; i >= 0; --i) {
-    double s = g[i];
-    for (int j = i + 1; j < k; ++j) s -= H[i + (size_t)ldh * j] * y[j];
-    y[i] = s / H[i + (size_t)ldh * i];
+    double s = 0;
+    for (int j = i + 1 + threadIdx.x; j < k; j += 32) s += H[i + (size_t)ldh * j] * y[j];
+    s = warp_sum(s);
+    if (threadIdx.x == 0) y[i] = (g[i] - s) / H[i + (size_t)ldh * i];
+    __syncwarp();
   }
 }
 __global__ void k_xupdate(int n, int k, const double* __restrict__ V, size_t ld, const double* __restrict__ y,
@@ -190,14 +208,14 @@ rbc3d_status gmres_cycles(rbc3d_ctx* ctx, int n, MV&& matvec, const double* b, d
       { k_orth<<<gm_nblk(n, 256), 256, 0, ctx->st>>>(n, k + 1, V.p, ld, hcol.p, w.p); ++ctx->launches; }
       double hn = dev_norm(ctx, n, w.p, tmp.p);
       if (hn > 0) { k_axpby<<<gm_nblk(n, 256), 256, 0, ctx->st>>>(n, 1.0 / hn, w.p, 0.0, V.p + (k + 1) * ld); ++ctx->launches; }
-      { k_givens<<<1, 1, 0, ctx->st>>>(k, R + 1, H.p, hcol.p, hn, cs.p, sn.p, g.p, tmp.p + R + 1); ++ctx->launches; }
+      { k_givens<<<1, kGivens, 0, ctx->st>>>(k, R + 1, H.p, hcol.p, hn, cs.p, sn.p, g.p, tmp.p + R + 1); ++ctx->launches; }
       double res = 0;
       CUDA_TRY(cudaMemcpyAsync(&res, tmp.p + R + 1, sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
       CUDA_TRY(cudaStreamSynchronize(ctx->st));
       ++its;
       if (res <= ttol || hn == 0) { ++k; conv = true; break; }
     }
-    { k_backsolve<<<1, 1, 0, ctx->st>>>(k, R + 1, H.p, g.p, yv.p); ++ctx->launches; }
+    { k_backsolve<<<1, 32, 0, ctx->st>>>(k, R + 1, H.p, g.p, yv.p); ++ctx->launches; }
     if (pc.active()) {  // x += M (V y)
       CUDA_TRY(cudaMemsetAsync(u.p, 0, sizeof(double) * n, ctx->st));
       { k_xupdate<<<gm_nblk(n, 256), 256, 0, ctx->st>>>(n, k, V.p, ld, yv.p, u.p); ++ctx->launches; }

@@ -77,6 +77,18 @@ __device__ __forceinline__ void weights(double x, double ih, int P, int& imin, R
 
 constexpr int SPREAD_TILE = 8;     // grid nodes per tile edge
 constexpr int SPREAD_CHUNK = 256;  // sources per CTA at most
+// Sources up to which the spread goes to the grid without boxes (k_spread_direct;
+// FP32, three planes): a box costs its clearing and flushing whatever it holds
+// (4,608 wall elements in FP64: 128 / 42 us; FP32, 10,000 sources and 12 planes
+// alone 151 / 71 us but the matvec beside it 597 / 718; 320,000: 813 / 1385).
+// FP64 always: its boxes fill an SM's shared memory with one block (12 planes,
+// 5,000 sources 547 / 80 us, 80,000 1504 / 968, 320,000 4982 / 3797).
+constexpr int DIRECT_SL = 32768;
+// Targets up to which a warp gathers one (k_gather_warp), FP32 and FP64: few
+// threads of 648 loads each leave the GPU empty.  us, thread / warp: FP32 10,000
+// targets 40 / 19, 30,000 43 / 35, 80,000 62 / 79; FP64 2,352 103 / 26, 20,000
+// 93 / 190.
+constexpr int GATHER_WARP32 = 40000, GATHER_WARP64 = 8192;
 
 struct TileArgs {
   int ntile[3];        // tiles per axis
@@ -214,6 +226,44 @@ __global__ void __launch_bounds__(128) k_spread_tile(SpreadArgs a, TileArgs t, c
   }
 }
 
+// The same without the boxes, a warp per source with its lanes over the P^3
+// nodes, one global atomic a node and plane: see launch_spread.
+template <typename R>
+__global__ void __launch_bounds__(128) k_spread_direct(SpreadArgs a, const int* __restrict__ perm, R* __restrict__ grid) {
+  __shared__ R sw[4][3][8], sv[4][12];
+  __shared__ int si[4][3][8];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, s = blockIdx.x * 4 + wid, P = a.P;
+  if (s >= a.n) return;
+  const int p = perm[s];  // tile order: neighbouring warps meet in L2
+  if (lane < 3) {
+    R w[8];
+    int m;
+    weights<R>(a.x[p + (size_t)lane * a.n], a.ih[lane], P, m, w);
+    int g = imod(m, a.N[lane]);
+    const int stride = lane == 1 ? a.N[0] : 1;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      sw[wid][lane][q] = w[q];
+      si[wid][lane][q] = g * stride;
+      g = g + 1 == a.N[lane] ? 0 : g + 1;
+    }
+  } else if (lane >= 8 && lane < 20) {
+    const int c = lane - 8;
+    R v = 0;
+    if (c < 3 && a.sl) v = (R)(a.c1 * a.f[p + (size_t)c * a.n]);
+    if (c >= 3 && a.dl) v = (R)(a.c2 * (a.g[p + (size_t)((c - 3) % 3) * a.n] * a.a3[p + (size_t)((c - 3) / 3) * a.n]));
+    sv[wid][c] = v;
+  }
+  __syncwarp();
+  const int P2 = P * P, c0 = a.sl ? 0 : 3, c1 = a.dl ? 12 : 3;
+  for (int e = lane; e < P2 * P; e += 32) {
+    const int k = e / P2, r = e - k * P2, j = r / P, i = r - j * P;
+    const R w = sw[wid][0][i] * sw[wid][1][j] * sw[wid][2][k];
+    R* q = grid + (size_t)a.N[0] * a.N[1] * si[wid][2][k] + si[wid][1][j] + si[wid][0][i];
+    for (int c = c0; c < c1; ++c) atomicAdd(q + (size_t)c * a.G, w * sv[wid][c]);
+  }
+}
+
 // Wall centroid sources (ModPME.F90:104-131): x = mean of the vertices,
 // f = mean vertex density * element area.
 __global__ void k_wall_sources(int nele, int nvert, const int* __restrict__ e2v, const double* __restrict__ x,
@@ -240,34 +290,54 @@ struct InflArgs {
   const double* bbz;
 };
 
+// The wave numbers (per axis) and the two factors of the influence at every
+// half-spectrum entry, from FP64: t.x = 2 pi alpha^2 / V phi1 bb, t.y = 4 pi
+// alpha / V phi0 bb with the B-spline factor bb (0 at the origin).  They depend
+// on the box and the mesh only: computed in every transform they cost an FP64
+// exponential, a square root and three products an entry (103 us of a 1.3 ms
+// wall product on a 96 x 96 x 64 mesh in FP64, 87 us on 128^3 in FP32).
 template <typename R, typename CT>
-__device__ __forceinline__ void influence(const InflArgs& a, const CT* __restrict__ F, int i, int j, int k, CT* out) {
-  size_t q = (size_t)i + (size_t)a.NH * (j + (size_t)a.N2 * k);
-  if (i == 0 && j == 0 && k == 0) {
-    for (int d = 0; d < 3; ++d) { out[d].x = 0; out[d].y = 0; }
-    return;
+__global__ void k_influence_table(InflArgs a, CT* __restrict__ tab, R* __restrict__ q) {
+  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int n[3] = {a.NH, a.N2, a.N3};
+  if (idx < (size_t)(n[0] + n[1] + n[2])) {
+    const int d = idx < (size_t)n[0] ? 0 : idx < (size_t)(n[0] + n[1]) ? 1 : 2;
+    const int k = (int)idx - (d > 0 ? n[0] : 0) - (d > 1 ? n[1] : 0);
+    q[idx] = (R)(d == 0 ? k * a.iL[0] : d == 1 ? ((k < a.N2 / 2) ? k : k - a.N2) * a.iL[1]
+                                               : ((2 * k <= a.N3) ? k : k - a.N3) * a.iL[2]);
   }
-  R qv[3];
-  qv[0] = (R)(i * a.iL[0]);
-  qv[1] = (R)((j < a.N2 / 2) ? j * a.iL[1] : (j - a.N2) * a.iL[1]);
-  qv[2] = (R)((2 * k <= a.N3) ? k * a.iL[2] : (k - a.N3) * a.iL[2]);
-  const R PI_ = (R)RBC3D_PI;
-  const R alpha = (R)a.alpha;
-  R sq = (R)sqrt(RBC3D_PI * a.alpha);
-  R qt[3] = {sq * qv[0], sq * qv[1], sq * qv[2]};
-  R q2 = qv[0] * qv[0] + qv[1] * qv[1] + qv[2] * qv[2];
-  R q2t = PI_ * alpha * q2;
-  R e = exp(-q2t);
-  R phi0 = e / q2t, phi1 = (e + phi0) / q2t;
+  if (idx >= a.GC) return;
+  const int i = (int)(idx % a.NH), j = (int)((idx / a.NH) % a.N2), k = (int)(idx / ((size_t)a.NH * a.N2));
+  double t0 = 0., t1 = 0.;
+  if (idx > 0) {
+    const double qx = i * a.iL[0], qy = ((j < a.N2 / 2) ? j : j - a.N2) * a.iL[1],
+                 qz = ((2 * k <= a.N3) ? k : k - a.N3) * a.iL[2];
+    const double q2t = RBC3D_PI * a.alpha * (qx * qx + qy * qy + qz * qz);
+    const double e = exp(-q2t), phi0 = e / q2t, phi1 = (e + phi0) / q2t, bb = a.bbx[i] * a.bby[j] * a.bbz[k];
+    t1 = 2. * a.alpha / a.vol * phi1 * bb * RBC3D_PI * a.alpha;
+    t0 = 4. * RBC3D_PI * a.alpha / a.vol * phi0 * bb;
+  }
+  CT t;
+  t.x = (R)t1;
+  t.y = (R)t0;
+  tab[idx] = t;
+}
+
+template <typename R, typename CT>
+__device__ __forceinline__ void influence(const InflArgs& a, const CT* __restrict__ F, const CT* __restrict__ tab,
+                                          const R* __restrict__ qa, int i, int j, int k, CT* out) {
+  const size_t q = (size_t)i + (size_t)a.NH * (j + (size_t)a.N2 * k);
+  const CT t = tab[q];
+  const R qv[3] = {qa[i], qa[a.NH + j], qa[a.NH + a.N2 + k]};
+  const R q2 = qv[0] * qv[0] + qv[1] * qv[1] + qv[2] * qv[2];
   R vr[3] = {0, 0, 0}, vi[3] = {0, 0, 0};
-  if (a.sl) {
+  if (a.sl) {  // 2 alpha / V phi1 (q2t F - qt (qt . F)), qt = sqrt(pi alpha) q
     CT Fv[3] = {F[q], F[q + a.GC], F[q + 2 * a.GC]};
-    R qfr = qt[0] * Fv[0].x + qt[1] * Fv[1].x + qt[2] * Fv[2].x;
-    R qfi = qt[0] * Fv[0].y + qt[1] * Fv[1].y + qt[2] * Fv[2].y;
-    R s = (R)2 * alpha / (R)a.vol * phi1;
+    const R qfr = qv[0] * Fv[0].x + qv[1] * Fv[1].x + qv[2] * Fv[2].x;
+    const R qfi = qv[0] * Fv[0].y + qv[1] * Fv[1].y + qv[2] * Fv[2].y;
     for (int d = 0; d < 3; ++d) {
-      vr[d] += s * (q2t * Fv[d].x - qt[d] * qfr);
-      vi[d] += s * (q2t * Fv[d].y - qt[d] * qfi);
+      vr[d] += t.x * (q2 * Fv[d].x - qv[d] * qfr);
+      vi[d] += t.x * (q2 * Fv[d].y - qv[d] * qfi);
     }
   }
   if (a.dl) {
@@ -282,8 +352,7 @@ __device__ __forceinline__ void influence(const InflArgs& a, const CT* __restric
       qTqr += qv[aa] * tr_;
       qTqi += qv[aa] * ti_;
     }
-    R s0 = (R)4 * PI_ * alpha / (R)a.vol * phi0;
-    R s1 = (R)8 * PI_ * PI_ * alpha * alpha / (R)a.vol * phi1;
+    const R s0 = t.y, s1 = (R)(4 * RBC3D_PI) * t.x;  // 8 pi^2 alpha^2 / V phi1
     for (int d = 0; d < 3; ++d) {
       R wr = qv[d] * trr + (qv[0] * T[0][d].x + qv[1] * T[1][d].x + qv[2] * T[2][d].x) +
              (T[d][0].x * qv[0] + T[d][1].x * qv[1] + T[d][2].x * qv[2]);
@@ -296,24 +365,25 @@ __device__ __forceinline__ void influence(const InflArgs& a, const CT* __restric
       vi[d] -= ti_;
     }
   }
-  R bb = (R)(a.bbx[i] * a.bby[j] * a.bbz[k]);
-  for (int d = 0; d < 3; ++d) { out[d].x = bb * vr[d]; out[d].y = bb * vi[d]; }
+  const bool origin = i == 0 && j == 0 && k == 0;
+  for (int d = 0; d < 3; ++d) { out[d].x = origin ? (R)0 : vr[d]; out[d].y = origin ? (R)0 : vi[d]; }
 }
 
 template <typename R, typename CT>
-__global__ void k_influence(InflArgs a, const CT* __restrict__ F, CT* __restrict__ V) {
+__global__ void k_influence(InflArgs a, const CT* __restrict__ tab, const R* __restrict__ qa, const CT* __restrict__ F,
+                            CT* __restrict__ V) {
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= a.GC) return;
   int i = (int)(idx % a.NH);
   int j = (int)((idx / a.NH) % a.N2);
   int k = (int)(idx / ((size_t)a.NH * a.N2));
   CT out[3];
-  influence<R, CT>(a, F, i, j, k, out);
+  influence<R, CT>(a, F, tab, qa, i, j, k, out);
   if (i == 0 || 2 * i == a.N1) {
     // Hermitian part of the kx = 0 / Nx/2 planes
     CT op[3];
     int jp = (a.N2 - j) % a.N2, kp = (a.N3 - k) % a.N3;
-    influence<R, CT>(a, F, i, jp, kp, op);
+    influence<R, CT>(a, F, tab, qa, i, jp, kp, op);
     for (int d = 0; d < 3; ++d) {
       out[d].x = (R)0.5 * (out[d].x + op[d].x);
       out[d].y = (R)0.5 * (out[d].y - op[d].y);
@@ -361,6 +431,47 @@ __global__ void k_gather(GatherArgs a, const R* __restrict__ vel) {
   }
   double iA = 1.0 / a.A[p];
   for (int d = 0; d < 3; ++d) a.v[p + (size_t)d * a.n] += (double)dv[d] * iA;
+}
+
+// The same with a warp per target, lanes over its P^3 nodes (a row of P nodes
+// is contiguous): see pme_gather.
+template <typename R>
+__global__ void __launch_bounds__(128) k_gather_warp(GatherArgs a, const R* __restrict__ vel) {
+  __shared__ R sw[4][3][8];
+  __shared__ int si[4][3][8];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, p = blockIdx.x * 4 + wid, P = a.P;
+  if (p >= a.n) return;
+  if (lane < 3) {
+    R w[8];
+    int m;
+    weights<R>(a.x[p + (size_t)lane * a.n], a.ih[lane], P, m, w);
+    int g = imod(m, a.N[lane]);
+    const int stride = lane == 1 ? a.N[0] : 1;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      sw[wid][lane][q] = w[q];
+      si[wid][lane][q] = g * stride;
+      g = g + 1 == a.N[lane] ? 0 : g + 1;
+    }
+  }
+  __syncwarp();
+  R dv[3] = {0, 0, 0};
+  const int P2 = P * P;
+  for (int e = lane; e < P2 * P; e += 32) {
+    const int k = e / P2, r = e - k * P2, j = r / P, i = r - j * P;
+    const R w = sw[wid][0][i] * (sw[wid][1][j] * sw[wid][2][k]);
+    const size_t q = (size_t)a.N[0] * a.N[1] * si[wid][2][k] + si[wid][1][j] + si[wid][0][i];
+    dv[0] += w * __ldg(vel + q);
+    dv[1] += w * __ldg(vel + q + a.G);
+    dv[2] += w * __ldg(vel + q + 2 * a.G);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    for (int d = 0; d < 3; ++d) dv[d] += __shfl_xor_sync(0xffffffffu, dv[d], o);
+  if (lane < 3) {
+    const double v = (double)(lane == 0 ? dv[0] : lane == 1 ? dv[1] : dv[2]);
+    a.v[p + (size_t)lane * a.n] += v * (1.0 / a.A[p]);
+  }
 }
 
 rbc3d_status make_plans(rbc3d_ctx* ctx, int prec) {
@@ -552,7 +663,12 @@ rbc3d_status launch_spread_p(rbc3d_ctx* ctx, const SpreadArgs& a, const SpreadPl
 template <typename R>
 rbc3d_status launch_spread(rbc3d_ctx* ctx, const SpreadArgs& a, const SpreadPlan& pl, R* grid) {
   if (pl.nchunk == 0) return RBC3D_OK;
-  switch (a.P) {
+  if (sizeof(R) == 8 || (!a.dl && a.n <= DIRECT_SL)) {
+    { k_spread_direct<R><<<nblk(a.n, 4), 128, 0, ctx->st>>>(a, pl.perm.p, grid); ++ctx->launches; }
+    CUDA_TRY(cudaGetLastError());
+    return RBC3D_OK;
+  }
+  if constexpr (sizeof(R) == 4) switch (a.P) {
     case 2: return launch_spread_p<R, 2>(ctx, a, pl, grid);
     case 3: return launch_spread_p<R, 3>(ctx, a, pl, grid);
     case 4: return launch_spread_p<R, 4>(ctx, a, pl, grid);
@@ -561,6 +677,7 @@ rbc3d_status launch_spread(rbc3d_ctx* ctx, const SpreadArgs& a, const SpreadPlan
     case 7: return launch_spread_p<R, 7>(ctx, a, pl, grid);
     default: return launch_spread_p<R, 8>(ctx, a, pl, grid);  // P <= 8 checked at rbc3d_create
   }
+  return RBC3D_OK;
 }
 
 // The cell sources' spread plan (tile binning of the sorted positions), built
@@ -630,6 +747,7 @@ rbc3d_status pme_transform(rbc3d_ctx* ctx) {
   a.alpha = ctx->prm.alpha; a.vol = ctx->prm.Lb[0] * ctx->prm.Lb[1] * ctx->prm.Lb[2];
   a.sl = P.sl; a.dl = P.dl;
   a.bbx = P.bbx.p; a.bby = P.bby.p; a.bbz = P.bbz.p;
+  const size_t nwave = (size_t)P.NH + P.N2 + P.N3;
   // the transforms run on the context's current stream (the matvec may put PME on its side stream)
   if (P.prec == RBC3D_FP32C) {
     cufftSetStream(P.r2c32_3, ctx->st); cufftSetStream(P.r2c32_12, ctx->st); cufftSetStream(P.c2r32_3, ctx->st);
@@ -640,14 +758,22 @@ rbc3d_status pme_transform(rbc3d_ctx* ctx) {
     CUDA_TRY(P.spec32.alloc(12 * P.GC)); CUDA_TRY(P.vspec32.alloc(3 * P.GC)); CUDA_TRY(P.vel32.alloc(3 * P.G));
     if (P.dl) { if (cufftExecR2C(P.r2c32_12, P.grid32.p, (cufftComplex*)P.spec32.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecR2C"); }
     else if (cufftExecR2C(P.r2c32_3, P.grid32.p, (cufftComplex*)P.spec32.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecR2C");
-    { k_influence<float, float2><<<nblk(P.GC, 256), 256, 0, ctx->st>>>(a, P.spec32.p, P.vspec32.p); ++ctx->launches; }
+    if (!P.infl32.p) {
+      CUDA_TRY(P.infl32.alloc(P.GC)); CUDA_TRY(P.wave32.alloc(nwave));
+      { k_influence_table<float, float2><<<nblk(std::max(P.GC, nwave), 256), 256, 0, ctx->st>>>(a, P.infl32.p, P.wave32.p); ++ctx->launches; }
+    }
+    { k_influence<float, float2><<<nblk(P.GC, 256), 256, 0, ctx->st>>>(a, P.infl32.p, P.wave32.p, P.spec32.p, P.vspec32.p); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
     if (cufftExecC2R(P.c2r32_3, (cufftComplex*)P.vspec32.p, P.vel32.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecC2R");
   } else {
     CUDA_TRY(P.spec64.alloc(12 * P.GC)); CUDA_TRY(P.vspec64.alloc(3 * P.GC)); CUDA_TRY(P.vel64.alloc(3 * P.G));
     if (P.dl) { if (cufftExecD2Z(P.r2c64_12, P.grid64.p, (cufftDoubleComplex*)P.spec64.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecD2Z"); }
     else if (cufftExecD2Z(P.r2c64_3, P.grid64.p, (cufftDoubleComplex*)P.spec64.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecD2Z");
-    { k_influence<double, double2><<<nblk(P.GC, 256), 256, 0, ctx->st>>>(a, P.spec64.p, P.vspec64.p); ++ctx->launches; }
+    if (!P.infl64.p) {
+      CUDA_TRY(P.infl64.alloc(P.GC)); CUDA_TRY(P.wave64.alloc(nwave));
+      { k_influence_table<double, double2><<<nblk(std::max(P.GC, nwave), 256), 256, 0, ctx->st>>>(a, P.infl64.p, P.wave64.p); ++ctx->launches; }
+    }
+    { k_influence<double, double2><<<nblk(P.GC, 256), 256, 0, ctx->st>>>(a, P.infl64.p, P.wave64.p, P.spec64.p, P.vspec64.p); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
     if (cufftExecZ2D(P.c2r64_3, (cufftDoubleComplex*)P.vspec64.p, P.vel64.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecZ2D");
   }
@@ -664,8 +790,12 @@ rbc3d_status pme_gather(rbc3d_ctx* ctx, int tlist) {
   a.n = t.n; a.x = t.x.p; a.A = t.Acoef.p; a.v = t.v.p;
   for (int d = 0; d < 3; ++d) { a.N[d] = ctx->prm.Nb[d]; a.ih[d] = ctx->prm.Nb[d] / ctx->prm.Lb[d]; }
   a.P = ctx->prm.P; a.G = P.G;
-  if (P.prec == RBC3D_FP32C) { k_gather<float><<<nblk(a.n, 128), 128, 0, ctx->st>>>(a, P.vel32.p); ++ctx->launches; }
-  else { k_gather<double><<<nblk(a.n, 128), 128, 0, ctx->st>>>(a, P.vel64.p); ++ctx->launches; }
+  const bool f32 = P.prec == RBC3D_FP32C, warp = a.n <= (f32 ? GATHER_WARP32 : GATHER_WARP64);
+  if (f32 && warp) k_gather_warp<float><<<nblk(a.n, 4), 128, 0, ctx->st>>>(a, P.vel32.p);
+  else if (f32) k_gather<float><<<nblk(a.n, 128), 128, 0, ctx->st>>>(a, P.vel32.p);
+  else if (warp) k_gather_warp<double><<<nblk(a.n, 4), 128, 0, ctx->st>>>(a, P.vel64.p);
+  else k_gather<double><<<nblk(a.n, 128), 128, 0, ctx->st>>>(a, P.vel64.p);
+  ++ctx->launches;
   CUDA_TRY(cudaGetLastError());
   return RBC3D_OK;
 }
