@@ -90,7 +90,7 @@ struct PmeState {
   DBuf<float> vel32;       // 3*G velocity grid
   DBuf<double> vel64;
   DBuf<double> bbx, bby, bbz;
-  DBuf<float2> infl32;     // influence factors per half-spectrum entry, wave numbers per axis
+  DBuf<float> infl32;      // influence factors per half-spectrum entry, wave numbers per axis
   DBuf<double2> infl64;
   DBuf<float> wave32;
   DBuf<double> wave64;

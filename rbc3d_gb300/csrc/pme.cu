@@ -77,18 +77,11 @@ __device__ __forceinline__ void weights(double x, double ih, int P, int& imin, R
 
 constexpr int SPREAD_TILE = 8;     // grid nodes per tile edge
 constexpr int SPREAD_CHUNK = 256;  // sources per CTA at most
-// Sources up to which the spread goes to the grid without boxes (k_spread_direct;
-// FP32, three planes): a box costs its clearing and flushing whatever it holds
-// (4,608 wall elements in FP64: 128 / 42 us; FP32, 10,000 sources and 12 planes
-// alone 151 / 71 us but the matvec beside it 597 / 718; 320,000: 813 / 1385).
-// FP64 always: its boxes fill an SM's shared memory with one block (12 planes,
-// 5,000 sources 547 / 80 us, 80,000 1504 / 968, 320,000 4982 / 3797).
-constexpr int DIRECT_SL = 32768;
-// Targets up to which a warp gathers one (k_gather_warp), FP32 and FP64: few
-// threads of 648 loads each leave the GPU empty.  us, thread / warp: FP32 10,000
-// targets 40 / 19, 30,000 43 / 35, 80,000 62 / 79; FP64 2,352 103 / 26, 20,000
-// 93 / 190.
-constexpr int GATHER_WARP32 = 40000, GATHER_WARP64 = 8192;
+// FP64 targets up to which a warp gathers one (k_gather_warp): few threads of
+// 648 loads each leave the GPU empty (us, thread / warp: 2,352 targets 103 / 26,
+// 20,000 93 / 190).  In FP32 the order of the 216 terms decides the rounding
+// (1e-7 of the velocities), and it stays one thread's.
+constexpr int GATHER_WARP64 = 8192;
 
 struct TileArgs {
   int ntile[3];        // tiles per axis
@@ -285,19 +278,28 @@ struct InflArgs {
   double iL[3];
   double alpha, vol;
   int sl, dl;
+  float sqpa;  // sqrt(pi alpha)
   const double* bbx;
   const double* bby;
   const double* bbz;
 };
 
-// The wave numbers (per axis) and the two factors of the influence at every
-// half-spectrum entry, from FP64: t.x = 2 pi alpha^2 / V phi1 bb, t.y = 4 pi
-// alpha / V phi0 bb with the B-spline factor bb (0 at the origin).  They depend
-// on the box and the mesh only: computed in every transform they cost an FP64
-// exponential, a square root and three products an entry (103 us of a 1.3 ms
-// wall product on a 96 x 96 x 64 mesh in FP64, 87 us on 128^3 in FP32).
-template <typename R, typename CT>
-__global__ void k_influence_table(InflArgs a, CT* __restrict__ tab, R* __restrict__ q) {
+// Per half-spectrum entry what the influence takes from FP64, and the wave
+// numbers per axis.  FP64: t.x = 2 pi alpha^2 / V phi1 bb, t.y = 4 pi alpha / V
+// phi0 bb (bb the B-spline factor; 0 at the origin); FP32: bb alone, the rest
+// stays FP32 arithmetic.  They depend on the box and the mesh only: computed in
+// every transform they cost FP64 exponentials and divisions, in FP32 the FP64
+// wave numbers, a square root and bb (103 us of a 1.3 ms wall product on a 96 x
+// 96 x 64 mesh in FP64, 87 us on 128^3 in FP32).
+template <typename R>
+struct Infl;
+template <>
+struct Infl<float> { typedef float T; };
+template <>
+struct Infl<double> { typedef double2 T; };
+
+template <typename R>
+__global__ void k_influence_table(InflArgs a, typename Infl<R>::T* __restrict__ tab, R* __restrict__ q) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int n[3] = {a.NH, a.N2, a.N3};
   if (idx < (size_t)(n[0] + n[1] + n[2])) {
@@ -308,36 +310,62 @@ __global__ void k_influence_table(InflArgs a, CT* __restrict__ tab, R* __restric
   }
   if (idx >= a.GC) return;
   const int i = (int)(idx % a.NH), j = (int)((idx / a.NH) % a.N2), k = (int)(idx / ((size_t)a.NH * a.N2));
-  double t0 = 0., t1 = 0.;
-  if (idx > 0) {
-    const double qx = i * a.iL[0], qy = ((j < a.N2 / 2) ? j : j - a.N2) * a.iL[1],
-                 qz = ((2 * k <= a.N3) ? k : k - a.N3) * a.iL[2];
-    const double q2t = RBC3D_PI * a.alpha * (qx * qx + qy * qy + qz * qz);
-    const double e = exp(-q2t), phi0 = e / q2t, phi1 = (e + phi0) / q2t, bb = a.bbx[i] * a.bby[j] * a.bbz[k];
-    t1 = 2. * a.alpha / a.vol * phi1 * bb * RBC3D_PI * a.alpha;
-    t0 = 4. * RBC3D_PI * a.alpha / a.vol * phi0 * bb;
+  const double bb = a.bbx[i] * a.bby[j] * a.bbz[k];
+  if constexpr (sizeof(R) == 4) {
+    tab[idx] = (float)bb;
+  } else {
+    double t0 = 0., t1 = 0.;
+    if (idx > 0) {
+      const double qx = i * a.iL[0], qy = ((j < a.N2 / 2) ? j : j - a.N2) * a.iL[1],
+                   qz = ((2 * k <= a.N3) ? k : k - a.N3) * a.iL[2];
+      const double q2t = RBC3D_PI * a.alpha * (qx * qx + qy * qy + qz * qz);
+      const double e = exp(-q2t), phi0 = e / q2t, phi1 = (e + phi0) / q2t;
+      t1 = 2. * a.alpha / a.vol * phi1 * bb * RBC3D_PI * a.alpha;
+      t0 = 4. * RBC3D_PI * a.alpha / a.vol * phi0 * bb;
+    }
+    tab[idx] = make_double2(t1, t0);
   }
-  CT t;
-  t.x = (R)t1;
-  t.y = (R)t0;
-  tab[idx] = t;
 }
 
 template <typename R, typename CT>
-__device__ __forceinline__ void influence(const InflArgs& a, const CT* __restrict__ F, const CT* __restrict__ tab,
-                                          const R* __restrict__ qa, int i, int j, int k, CT* out) {
+__device__ __forceinline__ void influence(const InflArgs& a, const CT* __restrict__ F,
+                                          const typename Infl<R>::T* __restrict__ tab, const R* __restrict__ qa, int i,
+                                          int j, int k, CT* out) {
   const size_t q = (size_t)i + (size_t)a.NH * (j + (size_t)a.N2 * k);
-  const CT t = tab[q];
+  if (i == 0 && j == 0 && k == 0) {
+    for (int d = 0; d < 3; ++d) { out[d].x = 0; out[d].y = 0; }
+    return;
+  }
   const R qv[3] = {qa[i], qa[a.NH + j], qa[a.NH + a.N2 + k]};
   const R q2 = qv[0] * qv[0] + qv[1] * qv[1] + qv[2] * qv[2];
+  // SL: sl (ql2 F - qt (qt . F)); DL: s0, s1; the sums' factor
+  R sl, ql2, qt[3], s0, s1, fac;
+  if constexpr (sizeof(R) == 4) {
+    const R PI_ = (R)RBC3D_PI, alpha = (R)a.alpha, sq = a.sqpa;
+    for (int d = 0; d < 3; ++d) qt[d] = sq * qv[d];
+    ql2 = PI_ * alpha * q2;
+    const R e = exp(-ql2), phi0 = e / ql2, phi1 = (e + phi0) / ql2;
+    sl = (R)2 * alpha / (R)a.vol * phi1;
+    s0 = (R)4 * PI_ * alpha / (R)a.vol * phi0;
+    s1 = (R)8 * PI_ * PI_ * alpha * alpha / (R)a.vol * phi1;
+    fac = tab[q];
+  } else {
+    const double2 t = tab[q];
+    for (int d = 0; d < 3; ++d) qt[d] = qv[d];
+    ql2 = q2;
+    sl = t.x;
+    s0 = t.y;
+    s1 = 4 * RBC3D_PI * t.x;
+    fac = 1;
+  }
   R vr[3] = {0, 0, 0}, vi[3] = {0, 0, 0};
-  if (a.sl) {  // 2 alpha / V phi1 (q2t F - qt (qt . F)), qt = sqrt(pi alpha) q
+  if (a.sl) {
     CT Fv[3] = {F[q], F[q + a.GC], F[q + 2 * a.GC]};
-    const R qfr = qv[0] * Fv[0].x + qv[1] * Fv[1].x + qv[2] * Fv[2].x;
-    const R qfi = qv[0] * Fv[0].y + qv[1] * Fv[1].y + qv[2] * Fv[2].y;
+    R qfr = qt[0] * Fv[0].x + qt[1] * Fv[1].x + qt[2] * Fv[2].x;
+    R qfi = qt[0] * Fv[0].y + qt[1] * Fv[1].y + qt[2] * Fv[2].y;
     for (int d = 0; d < 3; ++d) {
-      vr[d] += t.x * (q2 * Fv[d].x - qv[d] * qfr);
-      vi[d] += t.x * (q2 * Fv[d].y - qv[d] * qfi);
+      vr[d] += sl * (ql2 * Fv[d].x - qt[d] * qfr);
+      vi[d] += sl * (ql2 * Fv[d].y - qt[d] * qfi);
     }
   }
   if (a.dl) {
@@ -352,7 +380,6 @@ __device__ __forceinline__ void influence(const InflArgs& a, const CT* __restric
       qTqr += qv[aa] * tr_;
       qTqi += qv[aa] * ti_;
     }
-    const R s0 = t.y, s1 = (R)(4 * RBC3D_PI) * t.x;  // 8 pi^2 alpha^2 / V phi1
     for (int d = 0; d < 3; ++d) {
       R wr = qv[d] * trr + (qv[0] * T[0][d].x + qv[1] * T[1][d].x + qv[2] * T[2][d].x) +
              (T[d][0].x * qv[0] + T[d][1].x * qv[1] + T[d][2].x * qv[2]);
@@ -365,12 +392,11 @@ __device__ __forceinline__ void influence(const InflArgs& a, const CT* __restric
       vi[d] -= ti_;
     }
   }
-  const bool origin = i == 0 && j == 0 && k == 0;
-  for (int d = 0; d < 3; ++d) { out[d].x = origin ? (R)0 : vr[d]; out[d].y = origin ? (R)0 : vi[d]; }
+  for (int d = 0; d < 3; ++d) { out[d].x = fac * vr[d]; out[d].y = fac * vi[d]; }
 }
 
 template <typename R, typename CT>
-__global__ void k_influence(InflArgs a, const CT* __restrict__ tab, const R* __restrict__ qa, const CT* __restrict__ F,
+__global__ void k_influence(InflArgs a, const typename Infl<R>::T* __restrict__ tab, const R* __restrict__ qa, const CT* __restrict__ F,
                             CT* __restrict__ V) {
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= a.GC) return;
@@ -433,18 +459,17 @@ __global__ void k_gather(GatherArgs a, const R* __restrict__ vel) {
   for (int d = 0; d < 3; ++d) a.v[p + (size_t)d * a.n] += (double)dv[d] * iA;
 }
 
-// The same with a warp per target, lanes over its P^3 nodes (a row of P nodes
-// is contiguous): see pme_gather.
-template <typename R>
-__global__ void __launch_bounds__(128) k_gather_warp(GatherArgs a, const R* __restrict__ vel) {
-  __shared__ R sw[4][3][8];
+// The same in FP64 with a warp per target, lanes over its P^3 nodes (a row of P
+// nodes is contiguous): see pme_gather.
+__global__ void __launch_bounds__(128) k_gather_warp(GatherArgs a, const double* __restrict__ vel) {
+  __shared__ double sw[4][3][8];
   __shared__ int si[4][3][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, p = blockIdx.x * 4 + wid, P = a.P;
   if (p >= a.n) return;
   if (lane < 3) {
-    R w[8];
+    double w[8];
     int m;
-    weights<R>(a.x[p + (size_t)lane * a.n], a.ih[lane], P, m, w);
+    weights<double>(a.x[p + (size_t)lane * a.n], a.ih[lane], P, m, w);
     int g = imod(m, a.N[lane]);
     const int stride = lane == 1 ? a.N[0] : 1;
 #pragma unroll
@@ -455,11 +480,11 @@ __global__ void __launch_bounds__(128) k_gather_warp(GatherArgs a, const R* __re
     }
   }
   __syncwarp();
-  R dv[3] = {0, 0, 0};
+  double dv[3] = {0, 0, 0};
   const int P2 = P * P;
   for (int e = lane; e < P2 * P; e += 32) {
     const int k = e / P2, r = e - k * P2, j = r / P, i = r - j * P;
-    const R w = sw[wid][0][i] * (sw[wid][1][j] * sw[wid][2][k]);
+    const double w = sw[wid][0][i] * (sw[wid][1][j] * sw[wid][2][k]);
     const size_t q = (size_t)a.N[0] * a.N[1] * si[wid][2][k] + si[wid][1][j] + si[wid][0][i];
     dv[0] += w * __ldg(vel + q);
     dv[1] += w * __ldg(vel + q + a.G);
@@ -469,7 +494,7 @@ __global__ void __launch_bounds__(128) k_gather_warp(GatherArgs a, const R* __re
   for (int o = 16; o > 0; o >>= 1)
     for (int d = 0; d < 3; ++d) dv[d] += __shfl_xor_sync(0xffffffffu, dv[d], o);
   if (lane < 3) {
-    const double v = (double)(lane == 0 ? dv[0] : lane == 1 ? dv[1] : dv[2]);
+    const double v = lane == 0 ? dv[0] : lane == 1 ? dv[1] : dv[2];
     a.v[p + (size_t)lane * a.n] += v * (1.0 / a.A[p]);
   }
 }
@@ -660,10 +685,17 @@ rbc3d_status launch_spread_p(rbc3d_ctx* ctx, const SpreadArgs& a, const SpreadPl
   }
   return RBC3D_OK;
 }
+// The spread without boxes (k_spread_direct) for wall sources, a dozen a tile: a
+// box costs its clearing and flushing whatever it holds (4,608 elements in FP64:
+// 128 / 42 us); and in FP64 always, whose boxes fill an SM's shared memory with
+// one block (12 planes, 5,000 sources 547 / 80 us, 80,000 1504 / 968, 320,000
+// 4982 / 3797).  Cell sources in FP32 keep the boxes: with all 12 planes the
+// atomics hold up the pair sums beside them (10,000 sources alone 151 / 71 us,
+// the matvec 597 / 718), and their order adds rounding noise.
 template <typename R>
-rbc3d_status launch_spread(rbc3d_ctx* ctx, const SpreadArgs& a, const SpreadPlan& pl, R* grid) {
+rbc3d_status launch_spread(rbc3d_ctx* ctx, const SpreadArgs& a, const SpreadPlan& pl, R* grid, bool walls) {
   if (pl.nchunk == 0) return RBC3D_OK;
-  if (sizeof(R) == 8 || (!a.dl && a.n <= DIRECT_SL)) {
+  if (sizeof(R) == 8 || walls) {
     { k_spread_direct<R><<<nblk(a.n, 4), 128, 0, ctx->st>>>(a, pl.perm.p, grid); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
     return RBC3D_OK;
@@ -717,8 +749,8 @@ rbc3d_status pme_spread(rbc3d_ctx* ctx, double c1, double c2, int cells, int wal
     if (a.sl || a.dl) {
       rbc3d_status s;
       if (!P.cplan.valid && (s = build_spread_plan(ctx, a.n, a.x, a, P.cplan))) return s;
-      s = prec == RBC3D_FP32C ? launch_spread<float>(ctx, a, P.cplan, P.grid32.p)
-                              : launch_spread<double>(ctx, a, P.cplan, P.grid64.p);
+      s = prec == RBC3D_FP32C ? launch_spread<float>(ctx, a, P.cplan, P.grid32.p, false)
+                              : launch_spread<double>(ctx, a, P.cplan, P.grid64.p, false);
       if (s) return s;
     }
   }
@@ -730,8 +762,8 @@ rbc3d_status pme_spread(rbc3d_ctx* ctx, double c1, double c2, int cells, int wal
     a.n = W.nele; a.x = W.src_x.p; a.f = W.src_f.p; a.g = nullptr; a.a3 = nullptr; a.sl = 1; a.dl = 0;
     rbc3d_status s;
     if (!P.wplan.valid && (s = build_spread_plan(ctx, a.n, a.x, a, P.wplan))) return s;
-    s = prec == RBC3D_FP32C ? launch_spread<float>(ctx, a, P.wplan, P.grid32.p)
-                            : launch_spread<double>(ctx, a, P.wplan, P.grid64.p);
+    s = prec == RBC3D_FP32C ? launch_spread<float>(ctx, a, P.wplan, P.grid32.p, true)
+                            : launch_spread<double>(ctx, a, P.wplan, P.grid64.p, true);
     if (s) return s;
   }
   return RBC3D_OK;
@@ -746,6 +778,7 @@ rbc3d_status pme_transform(rbc3d_ctx* ctx) {
   for (int d = 0; d < 3; ++d) a.iL[d] = ctx->iLb[d];
   a.alpha = ctx->prm.alpha; a.vol = ctx->prm.Lb[0] * ctx->prm.Lb[1] * ctx->prm.Lb[2];
   a.sl = P.sl; a.dl = P.dl;
+  a.sqpa = (float)sqrt(RBC3D_PI * a.alpha);
   a.bbx = P.bbx.p; a.bby = P.bby.p; a.bbz = P.bbz.p;
   const size_t nwave = (size_t)P.NH + P.N2 + P.N3;
   // the transforms run on the context's current stream (the matvec may put PME on its side stream)
@@ -760,7 +793,7 @@ rbc3d_status pme_transform(rbc3d_ctx* ctx) {
     else if (cufftExecR2C(P.r2c32_3, P.grid32.p, (cufftComplex*)P.spec32.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecR2C");
     if (!P.infl32.p) {
       CUDA_TRY(P.infl32.alloc(P.GC)); CUDA_TRY(P.wave32.alloc(nwave));
-      { k_influence_table<float, float2><<<nblk(std::max(P.GC, nwave), 256), 256, 0, ctx->st>>>(a, P.infl32.p, P.wave32.p); ++ctx->launches; }
+      { k_influence_table<float><<<nblk(std::max(P.GC, nwave), 256), 256, 0, ctx->st>>>(a, P.infl32.p, P.wave32.p); ++ctx->launches; }
     }
     { k_influence<float, float2><<<nblk(P.GC, 256), 256, 0, ctx->st>>>(a, P.infl32.p, P.wave32.p, P.spec32.p, P.vspec32.p); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
@@ -771,7 +804,7 @@ rbc3d_status pme_transform(rbc3d_ctx* ctx) {
     else if (cufftExecD2Z(P.r2c64_3, P.grid64.p, (cufftDoubleComplex*)P.spec64.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecD2Z");
     if (!P.infl64.p) {
       CUDA_TRY(P.infl64.alloc(P.GC)); CUDA_TRY(P.wave64.alloc(nwave));
-      { k_influence_table<double, double2><<<nblk(std::max(P.GC, nwave), 256), 256, 0, ctx->st>>>(a, P.infl64.p, P.wave64.p); ++ctx->launches; }
+      { k_influence_table<double><<<nblk(std::max(P.GC, nwave), 256), 256, 0, ctx->st>>>(a, P.infl64.p, P.wave64.p); ++ctx->launches; }
     }
     { k_influence<double, double2><<<nblk(P.GC, 256), 256, 0, ctx->st>>>(a, P.infl64.p, P.wave64.p, P.spec64.p, P.vspec64.p); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
@@ -790,10 +823,8 @@ rbc3d_status pme_gather(rbc3d_ctx* ctx, int tlist) {
   a.n = t.n; a.x = t.x.p; a.A = t.Acoef.p; a.v = t.v.p;
   for (int d = 0; d < 3; ++d) { a.N[d] = ctx->prm.Nb[d]; a.ih[d] = ctx->prm.Nb[d] / ctx->prm.Lb[d]; }
   a.P = ctx->prm.P; a.G = P.G;
-  const bool f32 = P.prec == RBC3D_FP32C, warp = a.n <= (f32 ? GATHER_WARP32 : GATHER_WARP64);
-  if (f32 && warp) k_gather_warp<float><<<nblk(a.n, 4), 128, 0, ctx->st>>>(a, P.vel32.p);
-  else if (f32) k_gather<float><<<nblk(a.n, 128), 128, 0, ctx->st>>>(a, P.vel32.p);
-  else if (warp) k_gather_warp<double><<<nblk(a.n, 4), 128, 0, ctx->st>>>(a, P.vel64.p);
+  if (P.prec == RBC3D_FP32C) k_gather<float><<<nblk(a.n, 128), 128, 0, ctx->st>>>(a, P.vel32.p);
+  else if (a.n <= GATHER_WARP64) k_gather_warp<<<nblk(a.n, 4), 128, 0, ctx->st>>>(a, P.vel64.p);
   else k_gather<double><<<nblk(a.n, 128), 128, 0, ctx->st>>>(a, P.vel64.p);
   ++ctx->launches;
   CUDA_TRY(cudaGetLastError());

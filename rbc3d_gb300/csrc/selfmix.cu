@@ -2,22 +2,26 @@
 // the own-cell polar-patch quadrature with FP64-accurate geometry and FP32
 // arithmetic.
 //
-// The only cancellation-prone quantity of the patch quadrature is the
-// separation xx = x(patch point) - x(target), as small as 1e-2 for the first
-// radial ring.  Positions are stored relative to each cell's centre as FP32
-// (hi, lo) pairs computed in FP64, and the stencil's values enter as offsets
-// (X_hi - T_hi) + (X_lo - T_lo) from nearby target positions, formed before any
-// weight is applied, so xx carries ~1e-7 relative error instead of the ~1e-5 of
-// plain FP32 positions.  Densities, normals, weights and the Ewald kernel are
-// FP32 (erfc as exp(-x^2) t Q(t), the fit of fit_erfcx, pair.cu), accumulated
-// with Kahan compensation per target.
+// The cancellation-prone quantities of the patch quadrature are the separation
+// xx = x(patch point) - x(target), as small as 1e-2 for the first radial ring,
+// and its product with the normal.  Positions are stored relative to each
+// cell's centre as FP32 (hi, lo) pairs computed in FP64, and each stencil node's
+// offset from the target, (X_hi - t_hi) + (X_lo - t_lo), is formed before the
+// bicubic weights are applied, so xx carries ~1e-7 relative error instead of
+// the ~1e-5 of plain FP32 positions.  Densities, normals, weights and the Ewald
+// kernel are FP32 (erfc as exp(-x^2) t Q(t), the fit of fit_erfcx, pair.cu),
+// accumulated with Kahan compensation per target.
 //
-// By latitude rings, as selfring.cu and selfff.cu: per point pair (class) of a
-// ring and column j the theta part once, relative to the ring's target T_j of
-// that column; a point of target q takes it from the columns j and j + 1 with
-// T_j - T_q and T_j+1 - T_q added.  About 240 packed instructions for the two
-// points of a class and 0.4 KB of loads a point, against 300 scalar ones and
-// 0.8 KB a point with one warp per target and 16-term sums, bound by L1.
+// By latitude rings, as selfring.cu and selfff.cu: the two points of a class
+// that fall into a column interval share their four stencil nodes, so a thread
+// (column) loads the nodes' positions and normals once for both (their sums
+// keep all 16 terms: any other order moves xx . a3 near the target by its
+// rounding, 2e-6 of the velocities), and the densities go through the theta
+// part computed once per column and class.  0.4 KB of loads a point instead of
+// 0.8 KB with one warp per target, which L1 bound: 256 cells, SL+DL, 3.08 ->
+// 1.72 ms alone (two blocks an SM 1.82).  With the theta part for the positions
+// and normals too, relative to the ring's target, 1.41 ms, but outputs 1.3e-7
+// from these by rounding alone.
 #include <cmath>
 #include <vector>
 
@@ -27,17 +31,19 @@ namespace {
 
 inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
-// Node record: 13 float4 in column order, [cell][row][MIX_ROW][column]: slot d (u,
-// u_th, u_ph, u_thph) has the 12 values x, f, g, a3 in quads 3 d .. 3 d + 2 (x
-// of slot u: the hi parts relative to the cell centre), quad 12 the lo parts.
-constexpr int MIX_ROW = 13;
+// Node record: 13 float4 in column order, [cell][row][MIX_ROW][column]: floats
+// x hi(3) lo(3), a3(3), then u_th, u_ph, u_thph of x (9) and of a3 (9), pad;
+// from quad 7 on f and g (6 floats) of the slots u, u_th, u_ph, u_thph.
+constexpr int MIX_ROW = 13, MIX_XA = 7;
 
-// A class of patch points (RingClass): theta weights of (u, u', u_th, u'_th),
-// per side the phi weights of (U_j, U_j+1, D_j, D_j+1), the sides' quadrature
-// weights (0 for a point without mirror image, which stands on both sides).
+// A class of patch points (RingClass): theta weights of (u, u', u_th, u'_th);
+// per side the phi weights of (U_j, U_j+1, D_j, D_j+1) and, per stencil node
+// (row i1: columns j, j + 1; the next row: j, j + 1), the products for (u,
+// u_th, u_ph, u_thph); the sides' quadrature weights (0 for a point without
+// mirror image, which stands on both sides).
 struct MixClass {
   int i1, j[2], pad;
-  float x[4], y[2][4], w[2], pad2[2];
+  float x[4], y[2][4], n[2][4][4], w[2], pad2[2];
 };
 
 // mean of each cell's grid points (x SoA, 3 x npt)
@@ -64,24 +70,31 @@ __global__ void k_cell_mean(int nv, long long npt, const double* __restrict__ x,
 // order, the records in column order).
 __global__ void __launch_bounds__(128) k_mix_rec(int m, int n, const double* __restrict__ spl,
                                                  const double* __restrict__ xc, float* __restrict__ out, int sets) {
-  __shared__ float s[4][16][4][SPL_NODE];  // set x f g a3, column, row, value
-  __shared__ float lo[16][4][3];
+  __shared__ float s[16][4][4 * MIX_ROW + 1];  // column, row, float of the record
   const int nti = (m + 3) / 4, ntj = (n + 15) / 16;
   const int jt = blockIdx.x % ntj, it = (blockIdx.x / ntj) % nti, cell = blockIdx.x / (ntj * nti);
-  const int src[4] = {SPL_X, SPL_F, SPL_G, SPL_A3}, bit[4] = {1, 2, 4, 1};
+  const int src[4] = {SPL_X, SPL_A3, SPL_F, SPL_G}, bit[4] = {1, 1, 2, 4};
   for (int k = 0; k < 4; ++k) {
     if (!(sets & bit[k])) continue;
     const double* in = spl + ((size_t)cell * SPL_NSET + src[k]) * (size_t)m * n * SPL_NODE;
     for (int e = threadIdx.x; e < 16 * 4 * SPL_NODE; e += blockDim.x) {
-      const int q = e % SPL_NODE, r = (e / SPL_NODE) % 4, c = e / (4 * SPL_NODE);
+      const int q = e % SPL_NODE, r = (e / SPL_NODE) % 4, c = e / (4 * SPL_NODE), d = q / 3, v3 = q % 3;
       const int j = 16 * jt + c, i = 4 * it + r;
       if (j >= n || i >= m) continue;
       double v = in[((size_t)j * m + i) * SPL_NODE + q];
-      if (k == 0 && q < 3) {
-        v -= xc[3 * cell + q];
-        lo[c][r][q] = (float)(v - (double)(float)v);
+      float* o = s[c][r];
+      if (k == 0) {
+        if (d == 0) {
+          v -= xc[3 * cell + v3];
+          o[3 + v3] = (float)(v - (double)(float)v);
+          if (v3 == 0) o[4 * MIX_XA - 1] = 0.f;
+        }
+        o[d == 0 ? v3 : 9 + 3 * (d - 1) + v3] = (float)v;
+      } else if (k == 1) {
+        o[d == 0 ? 6 + v3 : 18 + 3 * (d - 1) + v3] = (float)v;
+      } else {
+        o[4 * MIX_XA + 6 * d + 3 * (k - 2) + v3] = (float)v;
       }
-      s[k][c][r][q] = (float)v;
     }
   }
   __syncthreads();
@@ -91,12 +104,9 @@ __global__ void __launch_bounds__(128) k_mix_rec(int m, int n, const double* __r
     if (j >= n || i >= m) continue;
     float* o = out + 4 * ((((size_t)cell * m + i) * MIX_ROW + dq) * n + j);
     for (int k = 0; k < 4; ++k) {
-      if (dq == 12) {
-        if (sets & 1) o[k] = k < 3 ? lo[c][r][k] : 0.f;
-        continue;
-      }
-      const int val = 4 * (dq % 3) + k, set = val / 3;
-      if (sets & bit[set]) o[k] = s[set][c][r][3 * (dq / 3) + val % 3];
+      const int f = 4 * dq + k;  // the record's float, and the set it belongs to
+      const int b = dq < MIX_XA ? 1 : (f - 4 * MIX_XA) % 6 < 3 ? 2 : 4;
+      if (sets & b) o[k] = s[c][r][f];
     }
   }
 }
@@ -139,24 +149,17 @@ struct MixArgs {
   float erfcx_q[ERFCX_DEG + 1];
 };
 
-__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-
 // One block: a ring of G cells, thread = column (cols = G nlon; more than 256
-// columns: several a thread); values in pairs (x.x x.y) (x.z f.x) (f.y f.z)
-// (g.x g.y) (g.z a.x) (a.y a.z).  One barrier a class: the theta parts
+// columns: several a thread).  One barrier a class: the densities' theta parts
 // alternate between two buffers; the targets' sums lie in shared memory, a side
 // each, so no two threads meet between two barriers.
 template <bool SL, bool DL>
 __global__ void __launch_bounds__(256, 3) k_self_mix(MixArgs a) {
-  constexpr int NP = DL ? (SL ? 6 : 5) : 3;  // pairs kept; without SL (f.y f.z) is left out
   extern __shared__ __align__(16) unsigned char smem_mix[];
   const int nlon = a.nlon, cols = a.G * nlon;
-  float4* ex = reinterpret_cast<float4*>(smem_mix);              // [2][NP][cols]: U pair, D pair
-  float2* acc = reinterpret_cast<float2*>(ex + 2 * NP * cols);   // [2 sides][3][cols]: Kahan sum and error
-  float2* sT = acc + 6 * cols;                                   // [3][cols]: target position hi, lo
+  float4* ex = reinterpret_cast<float4*>(smem_mix);            // [2][3][cols]: (f0 f1) (f2 g0) (g1 g2) of U, D
+  float2* acc = reinterpret_cast<float2*>(ex + 2 * 3 * cols);  // [2 sides][3][cols]: Kahan sum and error
+  float2* sT = acc + 6 * cols;                                 // [3][cols]: target position hi, lo
   int b = blockIdx.x;
   const int part = b % a.parts; b /= a.parts;
   const int ring = b % a.nlat, cell0 = (b / a.nlat) * a.G;
@@ -170,121 +173,122 @@ __global__ void __launch_bounds__(256, 3) k_self_mix(MixArgs a) {
   __syncthreads();
   const int k0 = (int)((long long)a.NC * part / a.parts), k1 = (int)((long long)a.NC * (part + 1) / a.parts);
   const MixClass* cls = a.cls + (size_t)ring * a.NC;
+  const float c1 = a.c1;
   for (int kc = k0; kc < k1; ++kc) {
     const MixClass& c = cls[kc];
-    float4* buf = ex + (size_t)((kc & 1) * NP) * cols;
+    float4* buf = ex + (size_t)((kc & 1) * 3) * cols;
     const int i1 = c.i1, i2 = i1 + 1 == a.m ? 0 : i1 + 1;
     for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
       const int lc = t / nlon, j = t - lc * nlon;
-      const float4* r1 = a.rec + ((size_t)(cell0 + lc) * a.m + i1) * MIX_ROW * nlon + j;
-      const float4* r2 = a.rec + ((size_t)(cell0 + lc) * a.m + i2) * MIX_ROW * nlon + j;
+      const float4* r1 = a.rec + (((size_t)(cell0 + lc) * a.m + i1) * MIX_ROW + MIX_XA) * nlon + j;
+      const float4* r2 = a.rec + (((size_t)(cell0 + lc) * a.m + i2) * MIX_ROW + MIX_XA) * nlon + j;
       const float4 w = *reinterpret_cast<const float4*>(c.x);
-      const float2 w0 = dup(w.x), w1 = dup(w.y), w2 = dup(w.z), w3 = dup(w.w);
-      const float2 T0 = sT[t], T1 = sT[cols + t], T2 = sT[2 * cols + t];
-      const float4 l1 = __ldg(r1 + 12 * nlon), l2 = __ldg(r2 + 12 * nlon);
+      float o[2][6];  // U (slots u, u_th), D (u_ph, u_thph) of f and g
 #pragma unroll
-      for (int q = 0; q < (DL ? 3 : 2); ++q) {
-        float4 p[4], r[4];  // the quad's slots of row i1 and of row i2
+      for (int h = 0; h < 2; ++h) {
+        float p[12], r[12];
 #pragma unroll
-        for (int d = 0; d < 4; ++d) { p[d] = __ldg(r1 + (3 * d + q) * nlon); r[d] = __ldg(r2 + (3 * d + q) * nlon); }
-        if (q == 0) {  // x as offsets from T_j (f.x passes unchanged)
-          const float2 hxy = make_float2(T0.x, T1.x), lxy = make_float2(T0.y, T1.y);
-          float2 v = __fadd2_rn(sub2(make_float2(p[0].x, p[0].y), hxy), sub2(make_float2(l1.x, l1.y), lxy));
-          p[0].x = v.x; p[0].y = v.y;
-          v = __fadd2_rn(sub2(make_float2(r[0].x, r[0].y), hxy), sub2(make_float2(l2.x, l2.y), lxy));
-          r[0].x = v.x; r[0].y = v.y;
-          p[0].z = __fadd_rn(__fsub_rn(p[0].z, T2.x), __fsub_rn(l1.z, T2.y));
-          r[0].z = __fadd_rn(__fsub_rn(r[0].z, T2.x), __fsub_rn(l2.z, T2.y));
+        for (int q = 0; q < 3; ++q) {
+          const float4 u = __ldg(r1 + (3 * h + q) * nlon), v = __ldg(r2 + (3 * h + q) * nlon);
+          p[4 * q] = u.x; p[4 * q + 1] = u.y; p[4 * q + 2] = u.z; p[4 * q + 3] = u.w;
+          r[4 * q] = v.x; r[4 * q + 1] = v.y; r[4 * q + 2] = v.z; r[4 * q + 3] = v.w;
         }
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int P = 2 * q + e;
-          if ((!DL && P >= 3) || (!SL && P == 2)) continue;
-          const int S = (!SL && P > 2) ? P - 1 : P;
-          auto lo = [&](const float4& v) { return e ? make_float2(v.z, v.w) : make_float2(v.x, v.y); };
-          const float2 U = fma2(w3, lo(r[1]), fma2(w2, lo(p[1]), fma2(w1, lo(r[0]), mul2(w0, lo(p[0])))));
-          const float2 D = fma2(w3, lo(r[3]), fma2(w2, lo(p[3]), fma2(w1, lo(r[2]), mul2(w0, lo(p[2])))));
-          buf[(size_t)S * cols + t] = make_float4(U.x, U.y, D.x, D.y);
-        }
+        for (int k = 0; k < 6; ++k) o[h][k] = fmaf(w.w, r[6 + k], fmaf(w.z, p[6 + k], fmaf(w.y, r[k], w.x * p[k])));
       }
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        buf[q * cols + t] = make_float4(o[0][2 * q], o[0][2 * q + 1], o[1][2 * q], o[1][2 * q + 1]);
     }
     __syncthreads();
     for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
-      const int lc = t / nlon, j = t - lc * nlon, base = t - j;
-      const int tn = j + 1 == nlon ? base : t + 1;
+      const int lc = t / nlon, j = t - lc * nlon, base = t - j, jn = j + 1 == nlon ? 0 : j + 1, tn = base + jn;
       const int qs[2] = {base + (j >= c.j[0] ? j - c.j[0] : j - c.j[0] + nlon),
                          base + (j >= c.j[1] ? j - c.j[1] : j - c.j[1] + nlon)};
-      float2 val[2][6];
-      {
-        float2 Tj[3], Tn[3];
+      float xx[2][3], A3[2][3], FG[2][6], th_[2][3], tl_[2][3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) { Tj[k] = sT[k * cols + t]; Tn[k] = sT[k * cols + tn]; }
+      for (int s = 0; s < 2; ++s)
 #pragma unroll
-        for (int P = 0; P < 6; ++P) {
-          if ((!DL && P >= 3) || (!SL && P == 2)) continue;
-          const int S = (!SL && P > 2) ? P - 1 : P;
-          const float4 A = buf[(size_t)S * cols + t], B = buf[(size_t)S * cols + tn];
+        for (int k = 0; k < 3; ++k) {
+          const float2 T = sT[k * cols + qs[s]];
+          th_[s][k] = T.x; tl_[s][k] = T.y;
+          xx[s][k] = 0.f; A3[s][k] = 0.f;
+        }
+      const float4* rows = a.rec + (size_t)(cell0 + lc) * a.m * MIX_ROW * nlon;
 #pragma unroll
-          for (int side = 0; side < 2; ++side) {
-            const float4 y = *reinterpret_cast<const float4*>(c.y[side]);
-            float2 U0 = make_float2(A.x, A.y), U1 = make_float2(B.x, B.y);
-            if (P < 2) {  // x: offsets from T_q
-              const int q = qs[side];
-              const float2 a0 = sT[2 * P * cols + q], z = make_float2(0.f, 0.f);
-              const float2 a1 = P == 0 ? sT[cols + q] : z, j1 = P == 0 ? Tj[1] : z, n1 = P == 0 ? Tn[1] : z;
-              U0 = __fadd2_rn(U0, __fadd2_rn(sub2(make_float2(Tj[2 * P].x, j1.x), make_float2(a0.x, a1.x)),
-                                             sub2(make_float2(Tj[2 * P].y, j1.y), make_float2(a0.y, a1.y))));
-              U1 = __fadd2_rn(U1, __fadd2_rn(sub2(make_float2(Tn[2 * P].x, n1.x), make_float2(a0.x, a1.x)),
-                                             sub2(make_float2(Tn[2 * P].y, n1.y), make_float2(a0.y, a1.y))));
-            }
-            val[side][P] = fma2(dup(y.w), make_float2(B.z, B.w),
-                                fma2(dup(y.z), make_float2(A.z, A.w), fma2(dup(y.y), U1, mul2(dup(y.x), U0))));
+      for (int k = 0; k < 4; ++k) {  // the stencil nodes
+        const float4* r = rows + (size_t)(k < 2 ? i1 : i2) * MIX_ROW * nlon + (k & 1 ? jn : j);
+        float v[4 * MIX_XA];
+#pragma unroll
+        for (int q = 0; q < MIX_XA; ++q) {
+          if (!DL && q >= 5) continue;  // a3's derivatives
+          const float4 u = __ldg(r + q * nlon);
+          v[4 * q] = u.x; v[4 * q + 1] = u.y; v[4 * q + 2] = u.z; v[4 * q + 3] = u.w;
+        }
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          const float4 w = *reinterpret_cast<const float4*>(c.n[s][k]);
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            const float d = __fadd_rn(__fsub_rn(v[e], th_[s][e]), __fsub_rn(v[3 + e], tl_[s][e]));
+            // in this order: it decides the rounding of xx . a3 near the target
+            xx[s][e] = __fadd_rn(xx[s][e], fmaf(w.w, v[15 + e], fmaf(w.z, v[12 + e], fmaf(w.x, d, __fmul_rn(w.y, v[9 + e])))));
+            if (DL)
+              A3[s][e] = __fadd_rn(A3[s][e], fmaf(w.w, v[24 + e], fmaf(w.z, v[21 + e],
+                                                                       fmaf(w.x, v[6 + e], __fmul_rn(w.y, v[18 + e])))));
           }
         }
       }
-      // both points at once: x = side 0, y = side 1
-      auto vx = [&](int P) { return make_float2(val[0][P].x, val[1][P].x); };
-      auto vy = [&](int P) { return make_float2(val[0][P].y, val[1][P].y); };
-      const float2 xx = vx(0), yy = vy(0), zz = vx(1);
-      float2 r2 = fma2(xx, xx, fma2(yy, yy, mul2(zz, zz)));
-      const bool ok[2] = {r2.x < a.rc2, r2.y < a.rc2};  // not rr >= rc (ModRbcSingInt.F90:65)
-      r2 = make_float2(ok[0] ? r2.x : 1.f, ok[1] ? r2.y : 1.f);
-      const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y)), ir2 = mul2(ri, ri);
-      const float2 st = mul2(mul2(r2, ri), dup(a.sqpa));
-      const float2 exn = make_float2(__expf(-st.x * st.x), __expf(-st.y * st.y));
-      // erfc(st) = exp(-st^2) t Q(t), t = 1/(1 + st/2) (fit_erfcx)
-      const float2 den = fma2(dup(0.5f), st, dup(1.f)), tq = make_float2(__fdividef(1.f, den.x), __fdividef(1.f, den.y));
-      float2 Q = dup(a.erfcx_q[ERFCX_DEG]);
 #pragma unroll
-      for (int k = ERFCX_DEG - 1; k >= 0; --k) Q = fma2(Q, tq, dup(a.erfcx_q[k]));
-      const float2 e1 = mul2(exn, mul2(tq, Q)), wq = *reinterpret_cast<const float2*>(c.w);
-      float2 cx, cf;  // dv = cx xx + cf f
-      if (SL) {
-        const float2 e1r = mul2(e1, ri), e2 = mul2(dup(a.two_isqa), exn), sw = mul2(dup(a.c1), wq);
-        const float2 d = fma2(xx, vy(1), fma2(yy, vx(2), mul2(zz, vy(2))));
-        cx = mul2(mul2(sw, mul2(__fadd2_rn(e1r, e2), ir2)), d);
-        cf = mul2(sw, sub2(e1r, e2));
-      }
-      if (DL) {
-        const float c2m = (float)(a.c2 * a.B[a.celltype[cell0 + lc]]);
-        const float2 cdl = mul2(dup(a.m8_ispi), fma2(exn, mul2(st, fma2(st, st, dup(1.5f))), mul2(dup(a.q75_spi), e1)));
-        const float2 Ad = mul2(mul2(mul2(cdl, ir2), ir2), ri);
-        const float2 dg = fma2(xx, vx(3), fma2(yy, vy(3), mul2(zz, vx(4))));
-        const float2 da = fma2(xx, vy(4), fma2(yy, vx(5), mul2(zz, vy(5))));
-        const float2 tt = mul2(mul2(mul2(dup(c2m), wq), Ad), mul2(dg, da));
-        cx = SL ? __fadd2_rn(cx, tt) : tt;
-      }
+      for (int q = 0; q < 3; ++q) {
+        const float4 A = buf[q * cols + t], B = buf[q * cols + tn];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        float2 v = mul2(cx, k == 0 ? xx : k == 1 ? yy : zz);
-        if (SL) v = fma2(cf, k == 0 ? vy(1) : k == 1 ? vx(2) : vy(2), v);
-        float2* s0 = acc + k * cols + qs[0];
-        float2* s1 = acc + (3 + k) * cols + qs[1];
-        const float2 z0 = *s0, z1 = *s1;  // (sum, error)
-        const float2 sum = make_float2(z0.x, z1.x), y = sub2(v, make_float2(z0.y, z1.y));
-        const float2 n = __fadd2_rn(sum, y), err = sub2(sub2(n, sum), y);
-        if (ok[0]) *s0 = make_float2(n.x, err.x);
-        if (ok[1]) *s1 = make_float2(n.y, err.y);
+        for (int s = 0; s < 2; ++s) {
+          const float4 y = *reinterpret_cast<const float4*>(c.y[s]);
+          FG[s][2 * q] = fmaf(y.w, B.z, fmaf(y.z, A.z, fmaf(y.y, B.x, y.x * A.x)));
+          FG[s][2 * q + 1] = fmaf(y.w, B.w, fmaf(y.z, A.w, fmaf(y.y, B.y, y.x * A.y)));
+        }
+      }
+      const float c2m = DL ? (float)(a.c2 * a.B[a.celltype[cell0 + lc]]) : 0.f;
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const float* x = xx[s];
+        const float r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+        if (r2 >= a.rc2) continue;  // rr >= rc (ModRbcSingInt.F90:65)
+        const float rinv = rsqrtf(r2), rv = r2 * rinv, ir2 = rinv * rinv;
+        const float st = rv * a.sqpa, exn = __expf(-st * st);
+        // erfc(st) = exp(-st^2) t Q(t), t = 1/(1 + st/2) (fit_erfcx)
+        const float tq = __fdividef(1.f, fmaf(0.5f, st, 1.f));
+        float Qp = a.erfcx_q[ERFCX_DEG];
+#pragma unroll
+        for (int k = ERFCX_DEG - 1; k >= 0; --k) Qp = fmaf(Qp, tq, a.erfcx_q[k]);
+        const float e1 = exn * (tq * Qp), e2 = a.two_isqa * exn;
+        const float wq = c.w[s];
+        float v0 = 0.f, v1 = 0.f, v2 = 0.f;
+        if (SL) {
+          const float A = (e1 * rinv + e2) * ir2, Bc = e1 * rinv - e2;
+          const float f0 = wq * FG[s][0], f1 = wq * FG[s][1], f2 = wq * FG[s][2];
+          const float d = x[0] * f0 + x[1] * f1 + x[2] * f2;
+          v0 = c1 * (A * x[0] * d + Bc * f0);
+          v1 = c1 * (A * x[1] * d + Bc * f1);
+          v2 = c1 * (A * x[2] * d + Bc * f2);
+        }
+        if (DL) {
+          const float cdl = a.m8_ispi * (exn * (st * (1.5f + st * st)) + a.q75_spi * e1);
+          const float Ad = cdl * ir2 * ir2 * rinv;
+          const float dg = wq * (x[0] * FG[s][3] + x[1] * FG[s][4] + x[2] * FG[s][5]);
+          const float da = fmaf(x[2], A3[s][2], fmaf(x[0], A3[s][0], __fmul_rn(x[1], A3[s][1])));
+          const float tt = c2m * Ad * dg * da;
+          v0 += tt * x[0]; v1 += tt * x[1]; v2 += tt * x[2];
+        }
+        float2* z = acc + 3 * s * cols + qs[s];
+        const float v[3] = {v0, v1, v2};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {  // Kahan: (sum, error)
+          const float2 o = z[k * cols];
+          const float y = __fsub_rn(v[k], o.y), n = __fadd_rn(o.x, y);
+          z[k * cols] = make_float2(n, __fsub_rn(__fsub_rn(n, o.x), y));
+        }
       }
     }
   }
@@ -318,6 +322,11 @@ rbc3d_status self_mixed_grid(rbc3d_ctx* ctx, const std::vector<RingClass>& R) {
       c.y[s][0] = (float)(1. - y[0]);
       for (int k = 0; k < 3; ++k) c.y[s][1 + k] = (float)y[k];
     }
+    for (int s = 0; s < 2; ++s)
+      for (int k = 0; k < 4; ++k) {  // u, u_th, u_ph, u_thph of node (row k / 2, column k % 2)
+        const float xu = c.x[k / 2], xd = c.x[2 + k / 2], yu = c.y[s][k % 2], yd = c.y[s][2 + k % 2];
+        c.n[s][k][0] = xu * yu; c.n[s][k][1] = xd * yu; c.n[s][k][2] = xu * yd; c.n[s][k][3] = xd * yd;
+      }
     c.w[0] = (float)r.w; c.w[1] = two ? (float)r.w : 0.f;
     C[i] = c;
   }
@@ -358,12 +367,11 @@ rbc3d_status run_self_mixed(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   if (tlist != RBC3D_TLIST_RBC || t.n == 0 || ctx->ncell == 0) return RBC3D_OK;
   const bool sl = c1 != 0 && ctx->has_f, dl = c2 != 0 && ctx->has_g;
   if (!sl && !dl) return RBC3D_OK;
-  const int np = dl ? (sl ? 6 : 5) : 3;
   auto smem = [&](int G) {
     const size_t cols = (size_t)G * ctx->nlon;
-    return sizeof(float4) * 2 * np * cols + sizeof(float2) * 9 * cols;
+    return sizeof(float4) * 2 * 3 * cols + sizeof(float2) * 9 * cols;
   };
-  // a ring wider than shared memory holds (about 850 columns) goes to the FP64 patch
+  // a ring wider than shared memory holds (about 1,300 columns) goes to the FP64 patch
   if (smem(1) > 227 * 1024) return run_self_corr(ctx, tlist, sl ? c1 : 0., dl ? c2 : 0.);
   // FP32 node records of the current geometry and densities (bit 0 geometry, 1 f, 2 g)
   const size_t per = 4 * (size_t)ctx->m * ctx->nlon * MIX_ROW;
