@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from rbc3d_gb300 import geometry as G
-from rbc3d_gb300.abi import FP32D, FP64, TERM_CORR, TERM_LINEAR, TERM_REAL, TLIST_RBC, Context
+from rbc3d_gb300.abi import FP32C, FP32D, FP64, TERM_CORR, TERM_LINEAR, TERM_REAL, TLIST_RAW, TLIST_RBC, Context
 
 pytestmark = pytest.mark.gpu
 C = 1 / (4 * math.pi)
@@ -39,3 +39,53 @@ def test_ring_patch_matches_oracle(gpu, oracle, nlat, nlon, ncell):
         assert np.linalg.norm(out - ref) <= 2e-11 * np.linalg.norm(ref), (c1, c2)
     for c in ctx:
         c.close()
+
+
+def test_shifted_longitudes(gpu, oracle):
+    """Longitudes phi(j) = j 2 pi / nlon + 0.3 are not the uniform grid of the
+    ring patch and the dense own-cell pass: the general patch, and own-cell
+    pairs with mask weights in the cell-list walk."""
+    L, ncell = 14.0, 3
+    cells = G.make_cells(np.random.default_rng(3), ncell, [L] * 3, 3.2, nlat=12, nlon=24, with_g=True)
+    cells.phi = cells.phi + 0.3
+    prm = dict(Lb=[L] * 3, alpha=G.alpha_for_cutoff(3.0, 1e-6), rc=3.0, eps=1e-6, Nb=[16] * 3, P=4, nlat=12, nlon=24,
+               ncelltypes=1, viscRat=[5.0])
+    out = []
+    for lib in (oracle, gpu):
+        c = Context(lib, prm)
+        c.set_cells(cells)
+        c.set_cell_density(f=cells.f, g=cells.g, spl_F=cells.spl_F, spl_G=cells.spl_G)
+        out.append(c.matvec(TLIST_RBC, C, C, TERM_REAL | TERM_CORR | TERM_LINEAR, FP64))
+        if lib is gpu:
+            out.append(c.matvec(TLIST_RBC, C, C, TERM_REAL | TERM_CORR | TERM_LINEAR, FP32C))
+        c.close()
+    ref = np.linalg.norm(out[0])
+    assert np.linalg.norm(out[1] - out[0]) <= 1e-11 * ref  # as the uniform grid
+    assert np.linalg.norm(out[2] - out[0]) <= 1e-6 * ref   # FP32 pair sums
+
+
+@pytest.mark.parametrize("n", [1, 7, 33, 8192, 8193])
+def test_few_points(gpu, oracle, n):
+    """Velocities at n free points: units of 8 targets with four lanes each,
+    their remainders, and both gathers of the FP64 mesh part (a warp per target
+    up to 8192)."""
+    L = 14.0
+    rng = np.random.default_rng(n)
+    cells = G.make_cells(rng, 3, [L] * 3, 3.2, nlat=12, nlon=24, with_g=True)
+    prm = dict(Lb=[L] * 3, alpha=G.alpha_for_cutoff(3.0, 1e-6), rc=3.0, eps=1e-6, Nb=[16, 18, 20], P=5, nlat=12, nlon=24,
+               ncelltypes=1, viscRat=[5.0])
+    # at least 0.3 from every surface point: no near-singular item decides on a rounded distance
+    x = rng.uniform(0, L, size=(3, 3 * n + 30))
+    d = x[:, :, None] - cells.x[:, None, :]
+    d -= np.round(d / L) * L
+    x = np.ascontiguousarray(x[:, np.sqrt((d ** 2).sum(0)).min(1) > 0.3][:, :n])
+    out = []
+    for lib in (oracle, gpu):
+        c = Context(lib, prm)
+        c.set_cells(cells)
+        c.set_cell_density(f=cells.f, g=cells.g, spl_F=cells.spl_F, spl_G=cells.spl_G)
+        c.set_raw_targets(x)
+        out.append(c.calc_velocity_field(TLIST_RAW))
+        c.close()
+    # as every FP64 result: rounding of the sums
+    assert x.shape[1] == n and np.linalg.norm(out[1] - out[0]) <= 1e-10 * np.linalg.norm(out[0])
