@@ -4,8 +4,9 @@
 // refinement, Givens rotations, PCNONE, converged when the true residual
 // ||b - A x|| < rtol ||b|| (KSPConvergedDefault); a cycle ends on the Givens
 // estimate and the true residual after the update decides.  The Krylov basis,
-// Hessenberg matrix and rotations stay on the device; one scalar per
-// iteration is read back for the convergence test.
+// Hessenberg matrix and rotations stay on the device; one
+// read-back per iteration (the estimate and the new vector's norm) serves the
+// convergence test.
 #pragma once
 #include <algorithm>
 #include <cmath>
@@ -78,13 +79,14 @@ __global__ void k_axpby(int n, double a, const double* __restrict__ x, double b,
   if (i < n) y[i] = a * x[i] + b * y[i];
 }
 // Givens / Hessenberg step for column k (one block).  H column-major with
-// leading dimension ldh = restart+1.  Writes |g_{k+1}| to res.  The rotations
+// leading dimension ldh = restart+1.  hn2: the squared norm of the new vector.
+// Writes |g_{k+1}| and that norm to res.  The rotations
 // are a serial chain; it runs over blocks of kGivens columns in shared memory
 // (from global memory each step waited for its loads: 17 us a step at 100
 // columns).
 constexpr int kGivens = 128;
-__global__ void __launch_bounds__(kGivens) k_givens(int k, int ldh, double* H, const double* hcol, double hn, double* cs,
-                                                    double* sn, double* g, double* res) {
+__global__ void __launch_bounds__(kGivens) k_givens(int k, int ldh, double* H, const double* hcol, const double* hn2,
+                                                    double* cs, double* sn, double* g, double* res) {
   __shared__ double sc[kGivens], ss[kGivens], sh[kGivens + 1];
   double* c = H + (size_t)ldh * k;
   double a = 0, b = 0;  // thread 0: the running entry
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(kGivens) k_givens(int k, int ldh, double* H, c
   }
   if (threadIdx.x) return;
   if (k == 0) a = hcol[0];
+  const double hn = sqrt(*hn2);
   b = hn;
   double den = sqrt(a * a + b * b);
   cs[k] = den > 0 ? a / den : 1.;
@@ -114,7 +117,14 @@ __global__ void __launch_bounds__(kGivens) k_givens(int k, int ldh, double* H, c
   c[k + 1] = 0.;
   g[k + 1] = -sn[k] * g[k];
   g[k] = cs[k] * g[k];
-  *res = fabs(g[k + 1]);
+  res[0] = fabs(g[k + 1]);
+  res[1] = hn;
+}
+// y = w / sqrt(h2), the next basis vector (y is left alone for h2 = 0)
+__global__ void k_unit(int n, const double* __restrict__ w, const double* __restrict__ h2, double* __restrict__ y) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const double h = sqrt(*h2);
+  if (i < n && h > 0) y[i] = w[i] * (1.0 / h);
 }
 // Back substitution by one warp, a row at a time (its sum over the lanes).
 __global__ void __launch_bounds__(32) k_backsolve(int k, int ldh, const double* H, const double* g, double* y) {
@@ -181,7 +191,7 @@ rbc3d_status gmres_cycles(rbc3d_ctx* ctx, int n, MV&& matvec, const double* b, d
   if (pc.active()) { CUDA_TRY(z.alloc(n)); CUDA_TRY(u.alloc(n)); }
   CUDA_TRY(V.alloc((size_t)(R + 1) * ld)); CUDA_TRY(w.alloc(n));
   CUDA_TRY(H.alloc((size_t)(R + 1) * R)); CUDA_TRY(cs.alloc(R)); CUDA_TRY(sn.alloc(R)); CUDA_TRY(g.alloc(R + 1));
-  CUDA_TRY(hcol.alloc(R + 1)); CUDA_TRY(yv.alloc(R)); CUDA_TRY(tmp.alloc(R + 2));
+  CUDA_TRY(hcol.alloc(R + 1)); CUDA_TRY(yv.alloc(R)); CUDA_TRY(tmp.alloc(R + 3));
   rbc3d_status s;
   auto residual = [&]() -> rbc3d_status {  // r = b - A x
     rbc3d_status e = matvec(x, w.p);
@@ -206,14 +216,14 @@ rbc3d_status gmres_cycles(rbc3d_ctx* ctx, int n, MV&& matvec, const double* b, d
       }
       dev_dots(ctx, n, k + 1, V.p, ld, w.p, hcol.p);
       { k_orth<<<gm_nblk(n, 256), 256, 0, ctx->st>>>(n, k + 1, V.p, ld, hcol.p, w.p); ++ctx->launches; }
-      double hn = dev_norm(ctx, n, w.p, tmp.p);
-      if (hn > 0) { k_axpby<<<gm_nblk(n, 256), 256, 0, ctx->st>>>(n, 1.0 / hn, w.p, 0.0, V.p + (k + 1) * ld); ++ctx->launches; }
-      { k_givens<<<1, kGivens, 0, ctx->st>>>(k, R + 1, H.p, hcol.p, hn, cs.p, sn.p, g.p, tmp.p + R + 1); ++ctx->launches; }
-      double res = 0;
-      CUDA_TRY(cudaMemcpyAsync(&res, tmp.p + R + 1, sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
+      dev_dots(ctx, n, 1, w.p, 0, w.p, tmp.p);
+      { k_unit<<<gm_nblk(n, 256), 256, 0, ctx->st>>>(n, w.p, tmp.p, V.p + (k + 1) * ld); ++ctx->launches; }
+      { k_givens<<<1, kGivens, 0, ctx->st>>>(k, R + 1, H.p, hcol.p, tmp.p, cs.p, sn.p, g.p, tmp.p + R + 1); ++ctx->launches; }
+      double res[2] = {0, 0};  // the residual estimate and the new vector's norm
+      CUDA_TRY(cudaMemcpyAsync(res, tmp.p + R + 1, sizeof(res), cudaMemcpyDeviceToHost, ctx->st));
       CUDA_TRY(cudaStreamSynchronize(ctx->st));
       ++its;
-      if (res <= ttol || hn == 0) { ++k; conv = true; break; }
+      if (res[0] <= ttol || res[1] == 0) { ++k; conv = true; break; }
     }
     { k_backsolve<<<1, 32, 0, ctx->st>>>(k, R + 1, H.p, g.p, yv.p); ++ctx->launches; }
     if (pc.active()) {  // x += M (V y)

@@ -38,6 +38,14 @@
 namespace {
 
 constexpr int TILE = 128;
+// Up to this many targets a block shares a unit (SPLIT of k_pair).  Measured,
+// warps apart -> together (real part, us): FP64 3750 targets 1516 -> 770,
+// 10000 2176 -> 1598, 25000 3909 -> 3676 (the whole matvec 7.06 -> 6.59 ms),
+// 40000 6986 -> 6613 but the matvec 11.58 -> 11.63, 80000 19.48 -> 19.93; FP32
+// 6250 targets 249 -> 168, 10000 325 -> 240 (matvec 600 -> 564), 13750
+// 334 -> 280 but the matvec 663 -> 675, 16250 640 -> 693: blocks that wait for
+// their longest warp hold shared memory that the patch beside them lacks.
+constexpr int PAIR_SPLIT_MAX64 = 24000, PAIR_SPLIT_MAX32 = 12000;
 
 // Sort keys: the hash cell; for targets (MORTON) followed by the place in the
 // cell's 8 x 8 x 8 sub-cells along the Morton curve, so that the targets of a
@@ -520,12 +528,15 @@ constexpr size_t warp_tile_bytes() {
 // SUB = 4: four lanes share a target, each with one 32-source chunk of the
 // tile, and merge sums and neighbour lists at the end: a quarter of the serial
 // work per warp where there are few targets (see pair_sub).
-template <typename R, bool SL, bool DL, int SUB>
+//
+// SPLIT = 4: the four warps of a block share a unit as well, each with every
+// fourth live tile, and merge in the same way.
+template <typename R, bool SL, bool DL, int SUB, int SPLIT>
 __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs a) {
   constexpr bool F64 = sizeof(R) == 8;
   extern __shared__ __align__(16) unsigned char smem_pair[];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int wu = blockIdx.x * (TILE / 32) + wid;  // this warp's unit
+  const int wu = SPLIT > 1 ? blockIdx.x : blockIdx.x * (TILE / 32) + wid;  // this warp's unit
   if (wu >= a.nunits) return;
   const int4 unit = a.units[wu];
   if (unit.z == 0) return;  // the empty tail
@@ -627,6 +638,7 @@ __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs 
     return (R)1;
   };
 
+  int turn = 0;  // SPLIT: live tiles so far, the same for the block's warps
   for (int nb = 0; nb < 27; ++nb) {
     const int dx = nb % 3 - 1, dy = (nb / 3) % 3 - 1, dz = nb / 9 - 1;
     const int ni = imod(ci + dx, a.Nc[0]), nj = imod(cj + dy, a.Nc[1]), nk = imod(ck + dz, a.Nc[2]);
@@ -662,7 +674,7 @@ __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs 
             !(__float_as_int(clo.w) == wsurf && __float_as_int(chi.w) == wsurf))
           live |= 1u << w;
       }
-      if (!live) continue;
+      if (!live || (SPLIT > 1 && (turn++ & (SPLIT - 1)) != wid)) continue;
       __syncwarp();
 #pragma unroll
       for (int w = 0; w < TILE / 32; ++w) {
@@ -812,7 +824,32 @@ __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs 
       }
     }
   }
-  if (active && sub == 0) {
+  if (SPLIT > 1) {
+    // the block's warps: sums and lists of their targets to warp 0
+    constexpr int NT = 32 / SUB;
+    struct Merge {
+      double sum[SPLIT][NT][3];
+      int n[SPLIT][NT], surf[SPLIT][NT][RBC3D_NBR_MAX], idx[SPLIT][NT][RBC3D_NBR_MAX];
+      float d2[SPLIT][NT][RBC3D_NBR_MAX];
+    };
+    static_assert(sizeof(Merge) <= TILE / 32 * warp_tile_bytes<R, SL, DL>(), "fits the tiles' shared memory");
+    __syncthreads();
+    Merge& M = *reinterpret_cast<Merge*>(smem_pair);
+    const int t = lane / SUB;
+    if (wid > 0 && sub == 0) {
+      for (int k = 0; k < 3; ++k) M.sum[wid][t][k] = sum[k];
+      M.n[wid][t] = L.overflow ? -1 : L.n;
+      for (int e = 0; e < L.n; ++e) { M.surf[wid][t][e] = L.surf[e]; M.idx[wid][t][e] = L.idx[e]; M.d2[wid][t][e] = L.d2[e]; }
+    }
+    __syncthreads();
+    if (wid == 0 && sub == 0)
+      for (int r = 1; r < SPLIT; ++r) {
+        for (int k = 0; k < 3; ++k) sum[k] += M.sum[r][t][k];
+        if (M.n[r][t] < 0) L.overflow = 1;
+        for (int e = 0; e < M.n[r][t]; ++e) L.insert(M.surf[r][t][e], M.idx[r][t][e], M.d2[r][t][e]);
+      }
+  }
+  if (active && sub == 0 && (SPLIT == 1 || wid == 0)) {
     const double iA = 1.0 / a.tA[ti];
     for (int k = 0; k < 3; ++k) a.v[ti + (size_t)k * a.nt] += sum[k] * iA;
     if (a.collect) {
@@ -847,6 +884,11 @@ __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs 
 // the same stream.  The target tile's at most (OWN_TILE - 1) / nlon + 2
 // latitude rings' rows of the weight table sit in shared memory.
 constexpr int OWN_TILE = 128;
+// FP64: fewer than this many blocks of 128 points go in tiles of 32 (8 blocks
+// of 4 warps an SM).  FP64 matvec, 128 -> 32 (us): 3 cells (165 blocks)
+// 1761 -> 1533, 3 cells of 12 x 24 839 -> 675, 8 cells 3085 -> 2797, 12 cells
+// 3850 -> 3800, 20 cells (1100) 6596 -> 6589, 64 cells (3520) 19927 -> 20133.
+constexpr int OWN64_BLOCKS = 1216;
 template <bool SL, bool DL>
 __global__ void __launch_bounds__(OWN_TILE) k_pair_own32(PairArgs a) {
   __shared__ __align__(16) float s_src[15][OWN_TILE];  // hi xyz, lo xyz, f xyz, g xyz, normal xyz
@@ -985,34 +1027,35 @@ __global__ void __launch_bounds__(OWN_TILE) k_pair_own32(PairArgs a) {
 }
 
 // The same in FP64: one source a step (at step s lane l takes source
-// (l + s) mod OWN_TILE), coefficients by the reference's tables.  Bound by the
+// (l + s) mod OT), coefficients by the reference's tables.  Bound by the
 // FP64 pipe: about 66 instructions for both orders of a pair, against 75 and
 // more for each order in the cell-list walk.
-template <bool SL, bool DL>
-__global__ void __launch_bounds__(OWN_TILE) k_pair_own64(PairArgs a) {
-  __shared__ double s_src[12][OWN_TILE];  // xyz (relative to the cell's first point), f, g, normal
-  __shared__ int s_id[OWN_TILE];
-  __shared__ double s_rev[OWN_TILE / 32][3][OWN_TILE];  // per warp: the sources' sums
+// Tiles of 32 where 128 would leave SMs short of blocks (OWN64_BLOCKS).
+template <bool SL, bool DL, int OT>
+__global__ void __launch_bounds__(OT) k_pair_own64(PairArgs a) {
+  __shared__ double s_src[12][OT];  // xyz (relative to the cell's first point), f, g, normal
+  __shared__ int s_id[OT];
+  __shared__ double s_rev[OT / 32][3][OT];  // per warp: the sources' sums
   extern __shared__ double s_mask64[];  // rows lat0.. of the table, nlat * nhalf each
   const int nlat = a.nlat, nlon = a.nlon, nv = nlat * nlon, rowlen = nlat * a.nhalf;
-  const int ntile = (nv + OWN_TILE - 1) / OWN_TILE, npt = ntile * (ntile + 1) / 2;
+  const int ntile = (nv + OT - 1) / OT, npt = ntile * (ntile + 1) / 2;
   const int cell = blockIdx.x / npt;
   int r = blockIdx.x - cell * npt, T = 0;
   while (r >= ntile - T) { r -= ntile - T; ++T; }
   const int S = T + r;
   const bool diag = S == T;
   const int tid = threadIdx.x, wid = tid >> 5;
-  const int k = T * OWN_TILE + tid;
+  const int k = T * OT + tid;
   const bool active = k < nv;
   const int tlat = active ? k / nlon : 0, tlon = active ? k - tlat * nlon : 0;
-  const int lat0 = T * OWN_TILE / nlon;
-  const int nrow = min(nlat - 1, (T * OWN_TILE + OWN_TILE - 1) / nlon) - lat0 + 1;
-  for (int i = tid; i < nrow * rowlen; i += OWN_TILE) s_mask64[i] = a.mtab64[(size_t)lat0 * rowlen + i];
+  const int lat0 = T * OT / nlon;
+  const int nrow = min(nlat - 1, (T * OT + OT - 1) / nlon) - lat0 + 1;
+  for (int i = tid; i < nrow * rowlen; i += OT) s_mask64[i] = a.mtab64[(size_t)lat0 * rowlen + i];
   const int p = cell * nv + tlon * nlat + tlat, first = cell * nv;
   auto relative = [&](int point, int c) {
     return min_image(a.px[point + (size_t)c * a.ns] - a.px[first + (size_t)c * a.ns], a.L[c], a.iL[c]);
   };
-  const int js = S * OWN_TILE + tid;
+  const int js = S * OT + tid;
   int ps = 0;
   if (js < nv) {
     const int sl = js / nlon;
@@ -1027,7 +1070,7 @@ __global__ void __launch_bounds__(OWN_TILE) k_pair_own64(PairArgs a) {
     s_src[0][tid] = 1.0e18;
     s_id[tid] = 0;
   }
-  for (int w = 0; w < OWN_TILE / 32; ++w)
+  for (int w = 0; w < OT / 32; ++w)
     for (int c = 0; c < 3; ++c) s_rev[w][c][tid] = 0.;
   double tx[3] = {0, 0, 0}, tf[3] = {0, 0, 0}, tg[3] = {0, 0, 0}, tn[3] = {0, 0, 0};
   if (active) {
@@ -1042,9 +1085,9 @@ __global__ void __launch_bounds__(OWN_TILE) k_pair_own64(PairArgs a) {
   const double* mrow = s_mask64 + (tlat - lat0) * rowlen;
   double acc[3] = {0, 0, 0};
   unsigned npairs = 0;
-  for (int step = 0; step < OWN_TILE; ++step) {
+  for (int step = 0; step < OT; ++step) {
     if (active) {
-      const int j = (tid + step) & (OWN_TILE - 1);
+      const int j = (tid + step) & (OT - 1);
       const double x = s_src[0][j] - tx[0], y = s_src[1][j] - tx[1], z = s_src[2][j] - tx[2];
       const double r2 = fma(x, x, fma(y, y, z * z));
       npairs += r2 <= a.rc2 ? (diag ? 1u : 2u) : 0u;
@@ -1098,7 +1141,7 @@ __global__ void __launch_bounds__(OWN_TILE) k_pair_own64(PairArgs a) {
     const double iA = 1.0 / a.tA[ps];
     for (int c = 0; c < 3; ++c) {
       double sum = 0.;
-      for (int w = 0; w < OWN_TILE / 32; ++w) sum += s_rev[w][c][tid];
+      for (int w = 0; w < OT / 32; ++w) sum += s_rev[w][c][tid];
       atomicAdd(a.v + ps + (size_t)c * a.nt, sum * iA);
     }
   }
@@ -1406,7 +1449,14 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
   // own-cell pairs of the cell targets by the dense pass when the same-cell
   // weights come from the table (uniform longitudes)
   const bool f64 = prec == RBC3D_FP64;
-  const int nrow = std::min(ctx->nlat, (OWN_TILE - 1) / std::max(ctx->nlon, 1) + 2);
+  const int nv = ctx->nlat * ctx->nlon;
+  // FP64 own-cell tiles: 128 points, or 32 where those are under OWN64_BLOCKS
+  auto own_blocks = [&](int tile) {
+    const long long nt = (nv + tile - 1) / tile;
+    return ctx->ncell * (nt * (nt + 1) / 2);
+  };
+  const int own_tile = f64 && own_blocks(OWN_TILE) < OWN64_BLOCKS ? 32 : OWN_TILE;
+  const int nrow = std::min(ctx->nlat, (own_tile - 1) / std::max(ctx->nlon, 1) + 2);
   const size_t own_sm = (f64 ? sizeof(double) : sizeof(float)) * (size_t)nrow * ctx->nlat * a.nhalf;
   const bool own = tlist == RBC3D_TLIST_RBC && a.mtab32 && t.n == n && ctx->s_op0.p && own_sm <= 160 * 1024;
   a.own_split = own ? 1 : 0;
@@ -1424,10 +1474,10 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
     { k_src_dens4<<<nblk(n, 256), 256, 0, ctx->st>>>(n, c1, c2, ctx->s_f.p, ctx->s_g.p, sl, dl,
                                                      ctx->s_F4.p, ctx->s_G4.p); ++ctx->launches; }
   }
-  auto launch = [&](auto kern, int blocks, size_t bytes) -> rbc3d_status {
+  auto launch = [&](auto kern, int blocks, size_t bytes, int threads = TILE) -> rbc3d_status {
     // (static and dynamic shared memory together may pass the 48 KB that need no opt-in)
     CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    kern<<<blocks, TILE, bytes, ctx->st>>>(a);
+    kern<<<blocks, threads, bytes, ctx->st>>>(a);
     ++ctx->launches;
     CUDA_TRY(cudaGetLastError());
     return RBC3D_OK;
@@ -1435,13 +1485,15 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
   auto pairs = [&](auto R, auto SL, auto DL) -> rbc3d_status {
     using T = decltype(R);
     const size_t bytes = TILE / 32 * warp_tile_bytes<T, SL.value, DL.value>();
-    if (t.sub == 4) return launch(k_pair<T, SL.value, DL.value, 4>, nb, bytes);
-    return launch(k_pair<T, SL.value, DL.value, 1>, nb, bytes);
+    if (t.sub == 4 && t.n <= (sizeof(T) == 8 ? PAIR_SPLIT_MAX64 : PAIR_SPLIT_MAX32)) return launch(k_pair<T, SL.value, DL.value, 4, 4>, t.nunits, bytes);
+    if (t.sub == 4) return launch(k_pair<T, SL.value, DL.value, 4, 1>, nb, bytes);
+    return launch(k_pair<T, SL.value, DL.value, 1, 1>, nb, bytes);
   };
   auto own_pairs = [&](auto R, auto SL, auto DL) -> rbc3d_status {
-    const int nt = (ctx->nlat * ctx->nlon + OWN_TILE - 1) / OWN_TILE, blocks = ctx->ncell * (nt * (nt + 1) / 2);
-    if (sizeof(R) == 8) return launch(k_pair_own64<SL.value, DL.value>, blocks, own_sm);
-    return launch(k_pair_own32<SL.value, DL.value>, blocks, own_sm);
+    const int blocks = (int)own_blocks(own_tile);
+    if (sizeof(R) == 4) return launch(k_pair_own32<SL.value, DL.value>, blocks, own_sm);
+    if (own_tile == 32) return launch(k_pair_own64<SL.value, DL.value, 32>, blocks, own_sm, 32);
+    return launch(k_pair_own64<SL.value, DL.value, OWN_TILE>, blocks, own_sm);
   };
   const std::true_type yes{};
   const std::false_type no{};

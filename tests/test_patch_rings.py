@@ -5,6 +5,7 @@ import math
 
 import numpy as np
 import pytest
+from scipy.spatial import cKDTree
 
 from rbc3d_gb300 import geometry as G
 from rbc3d_gb300.abi import FP32C, FP32D, FP64, TERM_CORR, TERM_LINEAR, TERM_REAL, TLIST_RAW, TLIST_RBC, Context
@@ -64,28 +65,30 @@ def test_shifted_longitudes(gpu, oracle):
     assert np.linalg.norm(out[2] - out[0]) <= 1e-6 * ref   # FP32 pair sums
 
 
-@pytest.mark.parametrize("n", [1, 7, 33, 8192, 8193])
-def test_few_points(gpu, oracle, n):
+@pytest.mark.parametrize("n,prec", [(1, FP64), (7, FP64), (33, FP64), (8192, FP64), (8193, FP64), (24000, FP64),
+                                    (24001, FP64), (33, FP32C), (12000, FP32C), (12001, FP32C)])
+def test_few_points(gpu, oracle, n, prec):
     """Velocities at n free points: units of 8 targets with four lanes each,
-    their remainders, and both gathers of the FP64 mesh part (a warp per target
+    their remainders, blocks that share a unit (up to 24000 targets in FP64,
+    12000 in FP32), and both gathers of the FP64 mesh part (a warp per target
     up to 8192)."""
     L = 14.0
     rng = np.random.default_rng(n)
     cells = G.make_cells(rng, 3, [L] * 3, 3.2, nlat=12, nlon=24, with_g=True)
-    prm = dict(Lb=[L] * 3, alpha=G.alpha_for_cutoff(3.0, 1e-6), rc=3.0, eps=1e-6, Nb=[16, 18, 20], P=5, nlat=12, nlon=24,
+    prm = dict(Lb=[L] * 3, alpha=G.alpha_for_cutoff(3.0, 1e-6), rc=3.0, eps=1e-6, Nb=[16, 18, 20], P=6, nlat=12, nlon=24,
                ncelltypes=1, viscRat=[5.0])
     # at least 0.3 from every surface point: no near-singular item decides on a rounded distance
     x = rng.uniform(0, L, size=(3, 3 * n + 30))
-    d = x[:, :, None] - cells.x[:, None, :]
-    d -= np.round(d / L) * L
-    x = np.ascontiguousarray(x[:, np.sqrt((d ** 2).sum(0)).min(1) > 0.3][:, :n])
+    far = cKDTree(cells.x.T % L, boxsize=L).query(x.T)[0] > 0.3
+    x = np.ascontiguousarray(x[:, far][:, :n])
     out = []
     for lib in (oracle, gpu):
         c = Context(lib, prm)
         c.set_cells(cells)
         c.set_cell_density(f=cells.f, g=cells.g, spl_F=cells.spl_F, spl_G=cells.spl_G)
         c.set_raw_targets(x)
-        out.append(c.calc_velocity_field(TLIST_RAW))
+        out.append(c.calc_velocity_field(TLIST_RAW, prec if lib is gpu else FP64))
         c.close()
-    # as every FP64 result: rounding of the sums
-    assert x.shape[1] == n and np.linalg.norm(out[1] - out[0]) <= 1e-10 * np.linalg.norm(out[0])
+    # FP64: rounding of the sums; FP32: of single pairs and of the mesh
+    tol = 1e-10 if prec == FP64 else 2e-6
+    assert x.shape[1] == n and np.linalg.norm(out[1] - out[0]) <= tol * np.linalg.norm(out[0])
