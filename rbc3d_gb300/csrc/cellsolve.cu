@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "ctx.hpp"
+#include "shfold.cuh"
 #include "gmres.cuh"
 
 // Spherepack pbar(m, n, theta) for 0 <= m <= n < L, P[m*L + n]: the standard
@@ -178,113 +179,88 @@ __global__ void k_sh_synth(ShArgs a, const double* __restrict__ cvec, double* __
 // itself: u_ph from m times the sine and cosine parts, u_th from dPE, the
 // FFT_Diff of the pbar samples continued around the great circle (built on
 // the host).  The two halves of the grid hold the same points: node (i >= nlat,
-// j) is the point (M - i, j + N/2) with u_th and u_thph negated, and the
-// columns j and j + N/2 of a row differ only in the sign of the odd-m terms,
-// so the block evaluates the (nlat + 1) x N/2 column pairs once.  Needs an
-// equispaced, even longitude grid (the FFT_Diff axis).
+// j) is the point (M - i, j + N/2) with u_th and u_thph negated.  Needs an
+// equispaced, even longitude grid (the FFT_Diff axis), whose columns go four at
+// a time (shfold.cuh).
+constexpr int SPL_THREADS = 128;
 struct SplArgs {
   int L, nlat, nlon, npt, nvar, set;
   const double* PG;   // pbar at the Gauss rows [i][m][n]
   const double* PE;   // pbar at the equiangular rows i pi / nlat, i <= nlat
   const double* dPE;  // FFT_Diff of pbar along the meridian great circle, same rows
   const double* wf;   // analysis weight per Gauss row
-  const double* cs;   // cos(m phi_j) [m][j]
-  const double* sn;
+  const Fold4* tab;  // fold_table
 };
 
-__global__ void __launch_bounds__(256) k_sh_spline(SplArgs a, const double* __restrict__ v,
-                                                   const double* __restrict__ fac, double* __restrict__ spl) {
+__global__ void __launch_bounds__(SPL_THREADS, 6) k_sh_spline(SplArgs a, const double* __restrict__ v,
+                                                              const double* __restrict__ fac, double* __restrict__ spl) {
   extern __shared__ double sm[];
   const int cell = blockIdx.x / a.nvar, comp = blockIdx.x % a.nvar;
-  const int L = a.L, nlat = a.nlat, nlon = a.nlon, nv = nlat * nlon, R = nlat + 1, N2 = nlon / 2;
+  const int L = a.L, nlat = a.nlat, nlon = a.nlon, nv = nlat * nlon, R = nlat + 1, N2 = nlon / 2, nq = nlon / 4 + 1;
   double* A = sm;               // [m][n]
   double* B = A + L * L;
-  double* Gt = B + L * L;       // [m][r], r <= nlat: G, H, G', H'
+  double* g = B + L * L;        // [i + nlat j]
+  double* C = g + nv;           // [m][i]
+  double* S = C + L * nlat;
+  double* Gt = B + L * L;       // [m][r], r <= nlat, over g, C, S: G, H, G', H'
   double* Ht = Gt + L * R;
   double* Gd = Ht + L * R;
   double* Hd = Gd + L * R;
-  double* g = Hd + L * R;       // [i + nlat j]
-  double* C = g + nv;           // [m][i]
-  double* S = C + L * nlat;
   const size_t base = (size_t)cell * nv;
   for (int r = threadIdx.x; r < nv; r += blockDim.x)
     g[r] = v[base + r + (size_t)comp * a.npt] * (fac ? fac[base + r] : 1.0);
   __syncthreads();
-  // ShAnalGau, longitude part: columns j and j + N/2 paired (cos and sin of
-  // m (phi + pi) are (-1)^m those of m phi)
-  for (int t = threadIdx.x; t < L * nlat; t += blockDim.x) {
-    const int m = t / nlat, i = t % nlat;
-    const double sgn = (m & 1) ? -1.0 : 1.0;
-    double c = 0, s = 0;
-    for (int j = 0; j < N2; ++j) {
-      const double x = g[i + nlat * j] + sgn * g[i + nlat * (j + N2)];
-      c += x * a.cs[m * nlon + j];
-      s += x * a.sn[m * nlon + j];
-    }
-    C[t] = c;
-    S[t] = s;
-  }
+  // ShAnalGau and ShFilter (n < L)
+  fold_columns(nlat, nlon, g);
   __syncthreads();
-  // Legendre part and ShFilter (n < L)
-  for (int t = threadIdx.x; t < L * L; t += blockDim.x) {
-    const int m = t / L, n = t % L;
-    double sa = 0, sb = 0;
-    if (n >= m)
-      for (int i = 0; i < nlat; ++i) {
-        const double p = a.PG[((size_t)i * L + m) * L + n] * a.wf[i];
-        sa += p * C[m * nlat + i];
-        sb -= p * S[m * nlat + i];
-      }
-    A[t] = sa;
-    B[t] = m > 0 ? sb : 0.0;
-  }
+  fold_analysis(L, nlat, nlon, g, a.tab, a.wf, C, S);
+  __syncthreads();
+  legendre_analysis(L, nlat, a.PG, C, S, A, B);
   __syncthreads();
   // G_m, H_m and their theta derivatives on the equiangular rows (the m = 0
   // term of the synthesis carries a factor 1/2)
-  for (int t = threadIdx.x; t < L * R; t += blockDim.x) {
-    const int m = t / R, r = t % R;
-    double gs = 0, hs = 0, gd = 0, hd = 0;
-    for (int n = m; n < L; ++n) {
-      const size_t q = ((size_t)r * L + m) * L + n;
-      const double p = a.PE[q], dp = a.dPE[q];
-      gs += p * A[m * L + n]; hs += p * B[m * L + n];
-      gd += dp * A[m * L + n]; hd += dp * B[m * L + n];
-    }
-    const double h = m == 0 ? 0.5 : 1.0;
-    Gt[t] = h * gs; Ht[t] = h * hs; Gd[t] = h * gd; Hd[t] = h * hd;
-  }
+  legendre_synthesis(L, R, a.PE, a.dPE, A, B, Gt, Ht, Gd, Hd);
   __syncthreads();
   const int M = 2 * nlat;
   double* dst = spl + ((size_t)cell * SPL_NSET + a.set) * (size_t)M * nlon * SPL_NODE;
-  for (int t = threadIdx.x; t < R * N2; t += blockDim.x) {
+  for (int t = threadIdx.x; t < R * nq; t += blockDim.x) {
     const int r = t % R, j = t / R;
-    double e[4] = {0, 0, 0, 0}, o[4] = {0, 0, 0, 0};  // u, u_th, u_ph, u_thph: even and odd m
-    for (int m = 0; m < L; ++m) {
-      const double c = a.cs[m * nlon + j], s = a.sn[m * nlon + j];
+    FoldSum e[4];  // u, u_th, u_ph, u_thph
+    auto term = [&](int m, int odd) {
+      const Fold4 w = a.tab[m * nq + j];
       const double gm = Gt[m * R + r], hm = Ht[m * R + r], gdm = Gd[m * R + r], hdm = Hd[m * R + r];
-      const double w[4] = {gm * c - hm * s, gdm * c - hdm * s, -m * (gm * s + hm * c), -m * (gdm * s + hdm * c)};
-      double* acc = (m & 1) ? o : e;
-      for (int k = 0; k < 4; ++k) acc[k] += w[k];
-    }
-    double p1[4], p2[4];  // the points (r, j) and (r, j + N/2)
-    for (int k = 0; k < 4; ++k) { p1[k] = e[k] + o[k]; p2[k] = e[k] - o[k]; }
-    auto put = [&](int i, int jj, const double* val, double sg) {
+      e[0].c[odd] = fma(gm, w.x, e[0].c[odd]);
+      e[0].s[odd] = fma(hm, w.y, e[0].s[odd]);
+      e[1].c[odd] = fma(gdm, w.x, e[1].c[odd]);
+      e[1].s[odd] = fma(hdm, w.y, e[1].s[odd]);
+      e[2].c[odd] = fma(hm, w.z, e[2].c[odd]);
+      e[2].s[odd] = fma(gm, w.w, e[2].s[odd]);
+      e[3].c[odd] = fma(hdm, w.z, e[3].c[odd]);
+      e[3].s[odd] = fma(gdm, w.w, e[3].s[odd]);
+    };
+    int m = 0;
+    for (; m + 1 < L; m += 2) { term(m, 0); term(m + 1, 1); }
+    if (m < L) term(m, 0);
+    double q[4][4];  // [kind][column]
+    e[0].value(q[0]); e[1].value(q[1]); e[2].dphi(q[2]); e[3].dphi(q[3]);
+    auto put = [&](int i, int jj, int col, double sg) {
       double* d = dst + ((size_t)jj * M + i) * SPL_NODE;
-      d[0 * 3 + comp] = val[0];
-      d[1 * 3 + comp] = sg * val[1];
-      d[2 * 3 + comp] = val[2];
-      d[3 * 3 + comp] = sg * val[3];
+      d[0 * 3 + comp] = q[0][col];
+      d[1 * 3 + comp] = sg * q[1][col];
+      d[2 * 3 + comp] = q[2][col];
+      d[3 * 3 + comp] = sg * q[3][col];
       if (a.nvar == 1)
         for (int kind = 0; kind < 4; ++kind) d[kind * 3 + 1] = d[kind * 3 + 2] = 0.0;
     };
-    if (r < nlat) {
-      put(r, j, p1, 1.0);
-      put(r, j + N2, p2, 1.0);
-    }
-    if (r >= 1) {
-      put(M - r, j + N2, p1, -1.0);
-      put(M - r, j, p2, -1.0);
-    }
+    // node (M - r, column + nlon/2) is the point (r, column)
+    auto column = [&](int jj, int col) {
+      if (r < nlat) put(r, jj, col, 1.0);
+      if (r >= 1) put(M - r, jj < N2 ? jj + N2 : jj - N2, col, -1.0);
+    };
+    column(j, 0);
+    if (j > 0) column(nlon - j, 1);
+    if (2 * j != N2) column(N2 - j, 2);
+    if (j > 0 && 2 * j != N2) column(N2 + j, 3);
   }
 }
 
@@ -334,6 +310,8 @@ rbc3d_status cell_tabs(rbc3d_ctx* ctx, int L, CellSolveTabs& T) {
   CUDA_TRY(T.wf.upload(wf.data(), wf.size(), ctx->st));
   CUDA_TRY(T.cs.upload(cs.data(), cs.size(), ctx->st)); CUDA_TRY(T.sn.upload(sn.data(), sn.size(), ctx->st));
   CUDA_TRY(T.dPE.upload(dPE.data(), dPE.size(), ctx->st));
+  const std::vector<Fold4> fold = fold_table(L, nlon);
+  if (T.equi_lon) CUDA_TRY(T.fold.upload(fold.data(), fold.size(), ctx->st));
   CUDA_TRY(cudaStreamSynchronize(ctx->st));
   T.L = L;
   return RBC3D_OK;
@@ -378,12 +356,12 @@ rbc3d_status build_spline_set(rbc3d_ctx* ctx, const CellSolveTabs& T, const doub
   spl_wait(ctx);  // on the main stream: no other build of the tables still in flight
   SplArgs a;
   a.L = T.L; a.nlat = ctx->nlat; a.nlon = ctx->nlon; a.npt = (int)ctx->npt; a.nvar = nvar; a.set = set;
-  a.PG = T.PG.p; a.PE = T.PE.p; a.dPE = T.dPE.p; a.wf = T.wf.p; a.cs = T.cs.p; a.sn = T.sn.p;
+  a.PG = T.PG.p; a.PE = T.PE.p; a.dPE = T.dPE.p; a.wf = T.wf.p; a.tab = T.fold.p;
   const size_t L = T.L, R = ctx->nlat + 1;
-  const size_t sm = sizeof(double) * (2 * L * L + 4 * L * R + (size_t)ctx->nlat * ctx->nlon + 2 * L * ctx->nlat);
+  const size_t sm = sizeof(double) * (2 * L * L + std::max(4 * L * R, (size_t)ctx->nlat * ctx->nlon + 2 * L * ctx->nlat));
   if (sm > 227 * 1024) return ctx_fail(ctx, RBC3D_ERR_ARG, "spline build: cell grid too large for one block");
   if (sm > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(k_sh_spline, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  { k_sh_spline<<<nvar * ctx->ncell, 256, sm, ctx->st>>>(a, v, fac, ctx->spl.p); ++ctx->launches; }
+  { k_sh_spline<<<nvar * ctx->ncell, SPL_THREADS, sm, ctx->st>>>(a, v, fac, ctx->spl.p); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());
   return RBC3D_OK;
 }

@@ -140,10 +140,15 @@ struct WallSpec {
 // (cellsolve.cu): Gauss and equiangular pbar rows, the meridian FFT_Diff of
 // the equiangular rows, weights, cos / sin(m phi); kept across calls until
 // the grid or L changes.
+struct alignas(16) Fold4 {  // an entry of fold_table (shfold.cuh)
+  double x, y, z, w;
+};
+
 struct ShTabs {
   int L = 0;
   bool equi_lon = false;  // phi equispaced over an even nlon (FFT_Diff's axis)
   DBuf<double> PG, PE, dPE, wf, cs, sn;
+  DBuf<Fold4> fold;       // fold_table (shfold.cuh)
 };
 
 struct rbc3d_ctx {
@@ -256,6 +261,7 @@ struct rbc3d_ctx {
   struct MbState {
     int L = 0;
     DBuf<double> P, DP, wf, cs, sn, sinth;
+    DBuf<Fold4> fold;  // fold_table (shfold.cuh); empty: plain sums
     int nref = 0;
     DBuf<double> ref_ar, ref_b;
     std::vector<double> ES, ED, EB;

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "ctx.hpp"
+#include "shfold.cuh"
 
 namespace {
 
@@ -33,68 +34,88 @@ struct MbArgs {
   const double* wf;  // analysis weight of Gauss row i: wG_i * 2 / nlon
   const double* cs;  // cos(m phi_j) [m][j]
   const double* sn;
+  const Fold4* tab;    // fold_table; 0: longitudes not equispaced or of odd number
 };
+constexpr int MB_THREADS = 128;
 
-// ShAnalGau + ShGradGau of nf fields: F -> Vt = dF/dtheta, Vp = dF/dphi
-__global__ void k_mb_grad(MbArgs a, const double* __restrict__ F, double* __restrict__ Vt, double* __restrict__ Vp) {
+// ShAnalGau + ShGradGau of nf fields: F -> Vt = dF/dtheta, Vp = dF/dphi.
+// FOLD: equispaced longitudes of even number, columns four at a time
+// (shfold.cuh); else the plain sums.
+template <bool FOLD>
+__global__ void __launch_bounds__(MB_THREADS, 6) k_mb_grad(MbArgs a, const double* __restrict__ F, double* __restrict__ Vt,
+                                                           double* __restrict__ Vp) {
   extern __shared__ double sm[];
   const int L = a.L, nlat = a.nlat, nlon = a.nlon, nv = a.nv;
-  double* g = sm;              // nv
+  double* A = sm;              // [m][n]
+  double* B = A + L * L;
+  double* g = B + L * L;       // nv
   double* C = g + nv;          // [m][i]
   double* S = C + L * nlat;
-  double* A = S + L * nlat;    // [m][n]
-  double* B = A + L * L;
-  double* G = B + L * L;       // [i][m]
+  double* G = B + L * L;       // [m][i], over g, C, S
   double* H = G + nlat * L;
   double* Gt = H + nlat * L;
   double* Ht = Gt + nlat * L;
   const size_t base = (size_t)blockIdx.x * nv;
   for (int r = threadIdx.x; r < nv; r += blockDim.x) g[r] = F[base + r];
   __syncthreads();
-  for (int t = threadIdx.x; t < L * nlat; t += blockDim.x) {
-    const int m = t / nlat, i = t % nlat;
-    double c = 0, s = 0;
-    for (int j = 0; j < nlon; ++j) {
-      const double x = g[i + nlat * j];
-      c += x * a.cs[m * nlon + j];
-      s += x * a.sn[m * nlon + j];
-    }
-    C[t] = c;
-    S[t] = s;
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < L * L; t += blockDim.x) {
-    const int m = t / L, n = t % L;
-    double sa = 0, sb = 0;
-    if (n >= m)
-      for (int i = 0; i < nlat; ++i) {
-        const double p = a.P[((size_t)i * L + m) * L + n] * a.wf[i];
-        sa += p * C[m * nlat + i];
-        sb -= p * S[m * nlat + i];
+  if (FOLD) {
+    fold_columns(nlat, nlon, g);
+    __syncthreads();
+    fold_analysis(L, nlat, nlon, g, a.tab, a.wf, C, S);
+  } else {
+    for (int t = threadIdx.x; t < L * nlat; t += blockDim.x) {
+      const int m = t / nlat, i = t % nlat;
+      double c = 0, s = 0;
+      for (int j = 0; j < nlon; ++j) {
+        const double x = g[i + nlat * j];
+        c += x * a.cs[m * nlon + j];
+        s += x * a.sn[m * nlon + j];
       }
-    A[t] = sa;
-    B[t] = sb;
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < nlat * L; t += blockDim.x) {
-    const int i = t / L, m = t % L;
-    double gs = 0, hs = 0, gt = 0, ht = 0;
-    for (int n = m; n < L; ++n) {
-      const size_t q = ((size_t)i * L + m) * L + n;
-      const double p = a.P[q], dp = a.DP[q];
-      gs += p * A[m * L + n]; hs += p * B[m * L + n];
-      gt += dp * A[m * L + n]; ht += dp * B[m * L + n];
+      C[t] = c * a.wf[i];
+      S[t] = s * a.wf[i];
     }
-    G[t] = gs; H[t] = hs; Gt[t] = gt; Ht[t] = ht;
   }
   __syncthreads();
+  legendre_analysis(L, nlat, a.P, C, S, A, B);
+  __syncthreads();
+  legendre_synthesis(L, nlat, a.P, a.DP, A, B, G, H, Gt, Ht);
+  __syncthreads();
+  if (FOLD) {
+    const int N2 = nlon / 2, nq = nlon / 4 + 1;
+    for (int t = threadIdx.x; t < nlat * nq; t += blockDim.x) {
+      const int j = t / nlat, i = t - j * nlat;
+      FoldSum e, f;  // theta and phi derivatives
+      auto term = [&](int m, int odd) {
+        const Fold4 w = a.tab[m * nq + j];
+        e.c[odd] = fma(Gt[m * nlat + i], w.x, e.c[odd]);
+        e.s[odd] = fma(Ht[m * nlat + i], w.y, e.s[odd]);
+        f.c[odd] = fma(H[m * nlat + i], w.z, f.c[odd]);
+        f.s[odd] = fma(G[m * nlat + i], w.w, f.s[odd]);
+      };
+      int m = 0;
+      for (; m + 1 < L; m += 2) { term(m, 0); term(m + 1, 1); }
+      if (m < L) term(m, 0);
+      double vt[4], vp[4];
+      e.value(vt);
+      f.dphi(vp);
+      auto put = [&](int jj, int col) {
+        Vt[base + i + (size_t)nlat * jj] = vt[col];
+        Vp[base + i + (size_t)nlat * jj] = vp[col];
+      };
+      put(j, 0);
+      if (j > 0) put(nlon - j, 1);
+      if (2 * j != N2) put(N2 - j, 2);
+      if (j > 0 && 2 * j != N2) put(N2 + j, 3);
+    }
+    return;
+  }
   for (int r = threadIdx.x; r < nv; r += blockDim.x) {
     const int i = r % nlat, j = r / nlat;
-    double st = 0.5 * Gt[i * L], sp = 0;
+    double st = Gt[i], sp = 0;
     for (int m = 1; m < L; ++m) {
       const double cm = a.cs[m * nlon + j], smv = a.sn[m * nlon + j];
-      st += Gt[i * L + m] * cm - Ht[i * L + m] * smv;
-      sp -= m * (G[i * L + m] * smv + H[i * L + m] * cm);
+      st += Gt[m * nlat + i] * cm - Ht[m * nlat + i] * smv;
+      sp -= m * (G[m * nlat + i] * smv + H[m * nlat + i] * cm);
     }
     Vt[base + r] = st;
     Vp[base + r] = sp;
@@ -417,7 +438,9 @@ void dpbar_table(int L, double theta, const double* P, double* dP) {
     }
 }
 
-size_t grad_smem(int L, int nlat, int nv) { return sizeof(double) * (size_t)(nv + 2 * L * nlat + 2 * L * L + 4 * nlat * L); }
+size_t grad_smem(int L, int nlat, int nv) {
+  return sizeof(double) * (size_t)(2 * L * L + std::max(nv + 2 * L * nlat, 4 * nlat * L));
+}
 
 rbc3d_status mb_tables(rbc3d_ctx* ctx) {
   auto& M = ctx->mb;
@@ -440,19 +463,31 @@ rbc3d_status mb_tables(rbc3d_ctx* ctx) {
   CUDA_TRY(M.wf.upload(wf.data(), wf.size(), ctx->st)); CUDA_TRY(M.cs.upload(cs.data(), cs.size(), ctx->st));
   CUDA_TRY(M.sn.upload(sn.data(), sn.size(), ctx->st)); CUDA_TRY(M.sinth.upload(st.data(), st.size(), ctx->st));
   const size_t sm = grad_smem(L, nlat, nlat * nlon);
-  if (sm > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(k_mb_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (sm > 48 * 1024) {
+    CUDA_TRY(cudaFuncSetAttribute(k_mb_grad<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    CUDA_TRY(cudaFuncSetAttribute(k_mb_grad<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  }
+  bool equi = nlon % 2 == 0;
+  for (int j = 0; j < nlon && equi; ++j)
+    equi = std::fabs(ctx->h_phi[j] - ctx->h_phi[0] - RBC3D_TWO_PI * j / nlon) <= 1e-12;
+  M.fold.release();
+  const std::vector<Fold4> fold = fold_table(L, nlon);
+  if (equi) CUDA_TRY(M.fold.upload(fold.data(), fold.size(), ctx->st));
   M.L = L;
   return RBC3D_OK;
 }
 
 MbArgs mb_args(const rbc3d_ctx* ctx) {
   const auto& M = ctx->mb;
-  return MbArgs{M.L, ctx->nlat, ctx->nlon, ctx->nlat * ctx->nlon, M.P.p, M.DP.p, M.wf.p, M.cs.p, M.sn.p};
+  return MbArgs{M.L, ctx->nlat, ctx->nlon, ctx->nlat * ctx->nlon, M.P.p, M.DP.p, M.wf.p, M.cs.p, M.sn.p,
+                M.fold.p};
 }
 
 void grad(rbc3d_ctx* ctx, int nf, const double* F, double* Vt, double* Vp) {
   const MbArgs a = mb_args(ctx);
-  k_mb_grad<<<nf, 256, grad_smem(a.L, a.nlat, a.nv), ctx->st>>>(a, F, Vt, Vp);
+  const size_t sm = grad_smem(a.L, a.nlat, a.nv);
+  if (a.tab) k_mb_grad<true><<<nf, MB_THREADS, sm, ctx->st>>>(a, F, Vt, Vp);
+  else k_mb_grad<false><<<nf, MB_THREADS, sm, ctx->st>>>(a, F, Vt, Vp);
   ++ctx->launches;
 }
 

@@ -136,14 +136,14 @@ __global__ void k_fill_units(int nc, int tile, int Nc0, int Nc1, int Nc2, const 
       for (int b = 0; b < cnt; b += per, ++u) {
         const int m = min(per, cnt - b);
         units[u] = make_int4(c, cs[c] + b, m, 0);
-        key[u] = nsrc * m;
+        key[u] = nsrc * m + 1;
         idx[u] = u;
       }
     }
   }
   for (int i = off[nc] + c; i < cap; i += gridDim.x * blockDim.x) {
     units[i] = make_int4(0, 0, 0, 0);
-    key[i] = -1;
+    key[i] = 0;
     idx[i] = i;
   }
 }
@@ -1217,7 +1217,7 @@ rbc3d_status scan_counts(rbc3d_ctx* ctx, int nc, const int* cnt, int* off) {
 // The units of `tile` targets at most into `units` (cap entries, the empty
 // tail last): per-cell counts, their scan, the units, a stable sort by work.
 rbc3d_status fill_units(rbc3d_ctx* ctx, const DBuf<int>& cs, const DBuf<int>& ce, const int* ss, const int* se,
-                        int tile, int cap, DBuf<int4>& units) {
+                        int tile, long long nsrc, int cap, DBuf<int4>& units) {
   const int nc = ctx->hg.ncells;
   rbc3d_status s;
   DBuf<int>& cnt = ctx->unit_cnt;
@@ -1233,12 +1233,15 @@ rbc3d_status fill_units(rbc3d_ctx* ctx, const DBuf<int>& cs, const DBuf<int>& ce
                                           ctx->unit_off.p, cap, ctx->unit_tmp.p, key, idx); ++ctx->launches; }
   // heaviest units first, so the last wave holds the light ones; the radix
   // sort is stable, so equal work keeps cell order (as a stable host sort);
-  // the empty tail (key -1) stays last
+  // the empty tail (key 0) stays last.  A key is at most tile times the sources, 24 of 64 bits at
+  // 320,000: three of the sort's passes instead of eight (12 us each).
+  int bits = 1;
+  while (bits < 62 && (1ll << bits) <= (long long)tile * nsrc + 1) ++bits;
   size_t tmp = 0;
-  cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp, key, key + cap, idx, idx + cap, cap, 0, 64, ctx->st);
+  cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp, key, key + cap, idx, idx + cap, cap, 0, bits, ctx->st);
   DBuf<char>& tb = ctx->sort_tmp;
   CUDA_TRY(tb.alloc(tmp + 1));
-  CUDA_TRY(cub::DeviceRadixSort::SortPairsDescending(tb.p, tmp, key, key + cap, idx, idx + cap, cap, 0, 64, ctx->st));
+  CUDA_TRY(cub::DeviceRadixSort::SortPairsDescending(tb.p, tmp, key, key + cap, idx, idx + cap, cap, 0, bits, ctx->st));
   { k_gather_units<<<nblk(cap, 256), 256, 0, ctx->st>>>(cap, idx + cap, ctx->unit_tmp.p, units.p); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());
   return RBC3D_OK;
@@ -1269,7 +1272,7 @@ rbc3d_status make_units(rbc3d_ctx* ctx, TargetSet& t, const DBuf<int>& cs, const
   // capacity: every non-empty cell gives at most count / tile + 1 units
   const int cap = nc + (t.n + tile - 1) / tile;
   t.nunits = cap;
-  return fill_units(ctx, cs, ce, ss, se, tile, cap, t.units);
+  return fill_units(ctx, cs, ce, ss, se, tile, src ? (long long)ctx->npt : 0, cap, t.units);
 }
 
 }  // namespace

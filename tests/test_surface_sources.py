@@ -143,3 +143,44 @@ def test_back_to_back_updates_and_buffer_reuse(gpu):
     v = ctx.matvec(TLIST_RBC, C, C, TERM_ALL, FP64)
     assert np.linalg.norm(v - ref[FP64]) <= 1e-12 * np.linalg.norm(ref[FP64])
     ctx.close()
+
+
+@pytest.mark.parametrize("nlat,nlon,shift", [(12, 24, 0.0), (14, 28, 0.3), (24, 48, 0.0), (25, 50, 0.3), (12, 26, 0.0),
+                                             (12, 24, None)])
+def test_longitude_grids(gpu, oracle, nlat, nlon, shift):
+    """The transforms' longitude sums by fours of columns: sizes with and
+    without a quarter column (nlon / 4), longitudes that start elsewhere, and
+    unequal ones (the plain sums; no spline tables)."""
+    L = 14.0
+    rng = np.random.default_rng(nlat)
+    cells = G.make_cells(rng, 3, [L] * 3, 3.2, nlat=nlat, nlon=nlon, with_g=True)
+    cells.phi = cells.phi + (0.05 * np.sin(cells.phi) if shift is None else shift)
+    prm = dict(Lb=[L] * 3, alpha=G.alpha_for_cutoff(3.0, 1e-6), rc=3.0, eps=1e-6, Nb=[24] * 3, P=6, nlat=nlat, nlon=nlon,
+               ncelltypes=1, viscRat=[5.0])
+    ref, orc = Context(gpu, prm), Context(oracle, prm)
+    geom = []
+    for c in (ref, orc):
+        c.set_cell_grid(cells.th, cells.phi, cells.w)
+        geom.append(c.cell_geometry(cells.x, 3))
+    orc.close()
+    if shift is None:
+        for g, o in zip(*geom):  # the same inexact quadrature
+            assert np.abs(g - o).max() <= 1e-11 * max(1.0, np.abs(o).max())
+        ref.close()
+        return
+    # the surface is a degree-5 expansion: as near to its exact normal and area
+    # element as the oracle's plain sums (2e-12 to 5e-11 by the grid, rounding over sin theta)
+    for k, exact in enumerate((cells.a3, cells.detJ)):
+        err = [np.abs(g[k] - exact).max() for g in geom]
+        assert err[0] <= 1.5 * err[1] + 1e-13
+    hc = host_sources(ref, cells, 8)
+    ref.set_cells(hc)
+    ref.set_cell_density(f=hc.f, g=hc.g, spl_F=hc.spl_F, spl_G=hc.spl_G)
+    dev = Context(gpu, prm)
+    dev.set_cells_x(cells, 8)
+    dev.set_cell_density_x(8, f=cells.f, g=cells.g)
+    a, b = (c.matvec(TLIST_RBC, C, C, TERM_ALL, FP64) for c in (ref, dev))
+    # as test_device_surface_sources_match_host_derivation
+    assert np.linalg.norm(a - b) <= 1e-11 * np.linalg.norm(a)
+    ref.close()
+    dev.close()
