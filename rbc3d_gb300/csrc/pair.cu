@@ -525,9 +525,10 @@ constexpr size_t warp_tile_bytes() {
 // has one left.  Before, all lanes walked the same sources and about 7 of 32
 // had a pair to evaluate.  FP64 is bound by its pipe, FP32 by issue.
 //
-// SUB = 4: four lanes share a target, each with one 32-source chunk of the
-// tile, and merge sums and neighbour lists at the end: a quarter of the serial
-// work per warp where there are few targets (see pair_sub).
+// SUB = 2, 4: that many lanes share a target, each with two or one of the
+// tile's 32-source chunks, and merge sums and neighbour lists at the end: a
+// half or a quarter of the serial work per warp where there are few targets
+// (see pair_sub).
 //
 // SPLIT = 4: the four warps of a block share a unit as well, each with every
 // fourth live tile, and merge in the same way.
@@ -1247,13 +1248,17 @@ rbc3d_status fill_units(rbc3d_ctx* ctx, const DBuf<int>& cs, const DBuf<int>& ce
   return RBC3D_OK;
 }
 
-// Lanes per target of the pair sums.  Few targets: with one lane each the
-// longest warps set the time.  FP32D, pair stage alone and whole matvec, one
-// lane / four: 8 cells (10,000 targets) 653 / 325 us and 918 / 609; 64 cells
-// (80,000) 1197 / 883 and 2242 / 2052; 128 cells 1775 / 1693 but 4061 / 4313
-// (the wider walk holds up the mesh beside it); 256 cells 2702 / 3029.  FP64,
-// 64 cells: 13.2 / 11.2 ms; 256 cells: 42.3 / 42.2.
-int pair_sub(int n) { return n <= 100000 ? 4 : 1; }
+// Lanes per target of the pair sums.  With one lane each and few units the
+// longest warps set the time (256 cells: SMs active 74 % of the kernel's);
+// more lanes a target cost tile walks.  FP32D, pair stage alone and whole
+// matvec (us) with 1 / 2 / 4 lanes: 8 cells (10,000 targets) 653 / - / 325 and
+// 918 / - / 609; 24 cells - / 664 / 529 and - / 1308 / 1164; 40 cells - / 828 /
+// 740 and - / 1588 / 1597; 64 cells 1197 / 874 / 884 and 2242 / 1970 / 2032;
+// 97 cells 1686 / 1175 / - and 3320 / 2970 / -; 128 cells 1744 / 1492 / 1693 and
+// 3983 / 3908 / 4313 (the wider walk holds up the mesh beside it); 160 cells
+// 2073 / 1767 / - but 4887 / 4944 / -; 256 cells 2718 / 2596 / 3029 but 7155 /
+// 7225 / -.  FP64 matvec (ms): 64 cells - / 19.2 / 19.5, 160 cells 50.9 / 50.9.
+int pair_sub(int n) { return n <= 50000 ? 4 : n <= 180000 ? 2 : 1; }
 
 rbc3d_status make_units(rbc3d_ctx* ctx, TargetSet& t, const DBuf<int>& cs, const DBuf<int>& ce) {
   const int nc = ctx->hg.ncells;
@@ -1490,6 +1495,7 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
     const size_t bytes = TILE / 32 * warp_tile_bytes<T, SL.value, DL.value>();
     if (t.sub == 4 && t.n <= (sizeof(T) == 8 ? PAIR_SPLIT_MAX64 : PAIR_SPLIT_MAX32)) return launch(k_pair<T, SL.value, DL.value, 4, 4>, t.nunits, bytes);
     if (t.sub == 4) return launch(k_pair<T, SL.value, DL.value, 4, 1>, nb, bytes);
+    if (t.sub == 2) return launch(k_pair<T, SL.value, DL.value, 2, 1>, nb, bytes);
     return launch(k_pair<T, SL.value, DL.value, 1, 1>, nb, bytes);
   };
   auto own_pairs = [&](auto R, auto SL, auto DL) -> rbc3d_status {

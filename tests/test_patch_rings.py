@@ -66,10 +66,11 @@ def test_shifted_longitudes(gpu, oracle):
 
 
 @pytest.mark.parametrize("n,prec", [(1, FP64), (7, FP64), (33, FP64), (8192, FP64), (8193, FP64), (24000, FP64),
-                                    (24001, FP64), (33, FP32C), (12000, FP32C), (12001, FP32C)])
+                                    (24001, FP64), (50000, FP64), (50001, FP64), (33, FP32C), (12000, FP32C), (12001, FP32C),
+                                    (50001, FP32C), (180001, FP32C)])
 def test_few_points(gpu, oracle, n, prec):
-    """Velocities at n free points: units of 8 targets with four lanes each,
-    their remainders, blocks that share a unit (up to 24000 targets in FP64,
+    """Velocities at n free points: units of 8 targets with four lanes each
+    (of 16 with two above 50000, of 32 above 180000), their remainders, blocks that share a unit (up to 24000 targets in FP64,
     12000 in FP32), and both gathers of the FP64 mesh part (a warp per target
     up to 8192)."""
     L = 14.0
