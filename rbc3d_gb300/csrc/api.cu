@@ -410,6 +410,9 @@ rbc3d_status rbc3d_create(const rbc3d_params* prm, rbc3d_ctx** out) {
     cudaDeviceGetStreamPriorityRange(&lowest, &highest);
     if (cudaStreamCreateWithPriority(&ctx->st, cudaStreamNonBlocking, highest) != cudaSuccess ||
         cudaStreamCreateWithPriority(&ctx->st2, cudaStreamNonBlocking, lowest) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&ctx->st3, cudaStreamNonBlocking, lowest) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_pair, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_own, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_spl, cudaEventDisableTiming) != cudaSuccess ||
@@ -480,10 +483,13 @@ rbc3d_status rbc3d_destroy(rbc3d_ctx* ctx) {
   pme_release(ctx);
   wall_spec_release(ctx);
   if (ctx->st2) cudaStreamSynchronize(ctx->st2);
+  if (ctx->st3) cudaStreamSynchronize(ctx->st3);
   if (ctx->st) cudaStreamSynchronize(ctx->st);
   for (cudaEvent_t e : ctx->evpool) cudaEventDestroy(e);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
+  if (ctx->ev_pair) cudaEventDestroy(ctx->ev_pair);
+  if (ctx->ev_own) cudaEventDestroy(ctx->ev_own);
   if (ctx->ev_spl) cudaEventDestroy(ctx->ev_spl);
   if (ctx->ev_up) cudaEventDestroy(ctx->ev_up);
   if (ctx->ev_rthr) cudaEventDestroy(ctx->ev_rthr);
@@ -491,6 +497,7 @@ rbc3d_status rbc3d_destroy(rbc3d_ctx* ctx) {
   if (ctx->ev_dens) cudaEventDestroy(ctx->ev_dens);
   if (ctx->h_rthr) cudaFreeHost(ctx->h_rthr);
   if (ctx->st2) cudaStreamDestroy(ctx->st2);
+  if (ctx->st3) cudaStreamDestroy(ctx->st3);
   if (ctx->t0) { cudaEventDestroy(ctx->t0); cudaEventDestroy(ctx->t1); }
   cudaStream_t st = ctx->st;
   delete ctx;

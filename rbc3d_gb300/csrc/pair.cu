@@ -852,7 +852,8 @@ __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs 
   }
   if (active && sub == 0 && (SPLIT == 1 || wid == 0)) {
     const double iA = 1.0 / a.tA[ti];
-    for (int k = 0; k < 3; ++k) a.v[ti + (size_t)k * a.nt] += sum[k] * iA;
+    // (beside the own-cell pass)
+    for (int k = 0; k < 3; ++k) atomicAdd(a.v + ti + (size_t)k * a.nt, sum[k] * iA);
     if (a.collect) {
       if (L.overflow) atomicAdd(a.cnt + 2, 1ull);
       for (int e = 0; e < L.n; ++e) {
@@ -1508,9 +1509,27 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
   const std::false_type no{};
   auto run = [&](auto R) -> rbc3d_status {
     // without a density the walk still counts pairs and lists neighbours: as the single layer of zeros
+    // FP32: the own-cell pass on a low-priority stream beside the walk, where it
+    // fills the SMs that the walk's last units leave idle.  After it / beside it
+    // (us): 256 cells pair stage 2700 / 2122, FP32D matvec 7156 / 6936, FP32M
+    // 5502 / 5253; 97 cells 2743 / 2619; 8 cells 558 / 513; 2048 cells 54787 /
+    // 54844.  At the walk's priority 7018 and 5417.  Not in FP64, where the patch
+    // is beside the walk already: 64 cells 19179 / 19644, 8 cells 2815 / 2866.
+    const bool beside = own && !f64 && ctx->st3;
+    if (beside) {
+      CUDA_TRY(cudaEventRecord(ctx->ev_pair, ctx->st));
+      CUDA_TRY(cudaStreamWaitEvent(ctx->st3, ctx->ev_pair, 0));
+    }
     rbc3d_status e = sl && dl ? pairs(R, yes, yes) : dl ? pairs(R, no, yes) : pairs(R, yes, no);
     if (e || !own) return e;
-    return sl && dl ? own_pairs(R, yes, yes) : dl ? own_pairs(R, no, yes) : own_pairs(R, yes, no);
+    if (beside) std::swap(ctx->st, ctx->st3);
+    e = sl && dl ? own_pairs(R, yes, yes) : dl ? own_pairs(R, no, yes) : own_pairs(R, yes, no);
+    if (beside) {
+      std::swap(ctx->st, ctx->st3);
+      CUDA_TRY(cudaEventRecord(ctx->ev_own, ctx->st3));
+      CUDA_TRY(cudaStreamWaitEvent(ctx->st, ctx->ev_own, 0));
+    }
+    return e;
   };
   return f64 ? run(0.0) : run(0.f);
 }
