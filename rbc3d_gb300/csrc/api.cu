@@ -170,6 +170,22 @@ __global__ void k_vadd2(long long n, const double* __restrict__ a, double* __res
   if (i < n) v[i] += a[i];
 }
 
+// The caller's values of finish_add go up beside the kernels where the copy does
+// not hold up the host (page-locked memory).
+rbc3d_status start_add(rbc3d_ctx* ctx, TargetSet& t, const double* v) {
+  const size_t n3 = 3 * (size_t)t.n;
+  cudaPointerAttributes at{};
+  ctx->vadd_up = n3 && ctx->st3 && cudaPointerGetAttributes(&at, v) == cudaSuccess && at.type == cudaMemoryTypeHost;
+  if (!ctx->vadd_up) {
+    cudaGetLastError();  // memory unknown to the driver: an ordinary array
+    return RBC3D_OK;
+  }
+  CUDA_TRY(ctx->vadd.alloc(n3));
+  CUDA_TRY(cudaMemcpyAsync(ctx->vadd.p, v, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->st3));
+  CUDA_TRY(cudaEventRecord(ctx->ev_vup, ctx->st3));
+  return RBC3D_OK;
+}
+
 // v (caller's host array) += the matvec result: the caller's values go up,
 // are added on the device and come back (two copies of 3n doubles, no host loop)
 rbc3d_status finish_add(rbc3d_ctx* ctx, TargetSet& t, double* v) {
@@ -177,7 +193,9 @@ rbc3d_status finish_add(rbc3d_ctx* ctx, TargetSet& t, double* v) {
   if (n3 == 0) return RBC3D_OK;
   DBuf<double>& d = ctx->vadd;
   CUDA_TRY(d.alloc(n3));
-  CUDA_TRY(cudaMemcpyAsync(d.p, v, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->st));
+  if (ctx->vadd_up) CUDA_TRY(cudaStreamWaitEvent(ctx->st, ctx->ev_vup, 0));
+  else CUDA_TRY(cudaMemcpyAsync(d.p, v, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->st));
+  ctx->vadd_up = false;
   { k_vadd2<<<(int)((n3 + 255) / 256), 256, 0, ctx->st>>>((long long)n3, t.v.p, d.p); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(v, d.p, sizeof(double) * n3, cudaMemcpyDeviceToHost, ctx->st));
@@ -250,7 +268,7 @@ rbc3d_status rbcs_dev(rbc3d_ctx* ctx, int which, double c1, double c2, int prec,
   bool corr = (terms & RBC3D_TERM_CORR) != 0;
   rbc3d_status s;
   for (int attempt = 0; attempt < 2; ++attempt) {
-    CUDA_TRY(cudaMemsetAsync(ctx->dcnt.p, 0, sizeof(unsigned long long) * 3, ctx->st));
+    CUDA_TRY(cudaMemsetAsync(ctx->dcnt.p, 0, sizeof(unsigned long long) * 11, ctx->st));  // ([4], [5]: the walls', zeroed there)
     if (terms & RBC3D_TERM_REAL || corr) {
       StageScope sc(ctx, 0);
       if ((s = run_pair_sum(ctx, which, (terms & RBC3D_TERM_REAL) ? c1 : 0.0, (terms & RBC3D_TERM_REAL) ? c2 : 0.0,
@@ -269,9 +287,6 @@ rbc3d_status rbcs_dev(rbc3d_ctx* ctx, int which, double c1, double c2, int prec,
     CUDA_TRY(cudaMemsetAsync(t.v.p, 0, sizeof(double) * 3 * t.n, ctx->st));
   }
   if (corr) {
-    CUDA_TRY(cudaMemsetAsync(ctx->dcnt.p + 3, 0, sizeof(unsigned long long), ctx->st));
-    CUDA_TRY(cudaMemsetAsync(ctx->dcnt.p + 6, 0, sizeof(unsigned long long), ctx->st));
-    CUDA_TRY(cudaMemsetAsync(ctx->dcnt.p + 8, 0, sizeof(unsigned long long) * 3, ctx->st));
     if (self_late) {  // after fork_side: t.v2 is zeroed and PME queued on the side stream
       CUDA_TRY(cudaEventRecord(ctx->ev_fork, ctx->st));
       CUDA_TRY(cudaStreamWaitEvent(ctx->st2, ctx->ev_fork, 0));
@@ -322,13 +337,18 @@ rbc3d_status matvec_dev(rbc3d_ctx* ctx, int which, double c1, double c2, unsigne
   // stream, into their own accumulator, while the main stream does the pair
   // sums, the near-singular pass, the linear term and the walls; the pipes
   // they load differ (FP32 / L1 / FP64 / shared memory), so the kernels share
-  // the SMs.  The side accumulator is added at the join.
-  const bool side = ctx->st2 && which == RBC3D_TLIST_RBC && ctx->npt > 0 && (terms & RBC3D_TERM_CORR) &&
-                    (terms & RBC3D_TERM_PME);
-  // PME joins the shorter stream: the side one when the patch correction is
-  // the short FP32 one (FP32M: 8.5 ms against 9.0 with PME on the main
-  // stream), else the main one after the pair and near passes (FP32C: 52.7
-  // against 53.1 ms)
+  // the SMs.  The side accumulator is added at the join.  Points that are not
+  // the cells' have no patch: PME alone goes beside (FP32D: 20011 points, 64
+  // cells 1999 -> 1706 us, 1000 points, 8 cells 821 -> 613; FP64 7187 -> 6736,
+  // 1416 -> 1332).
+  const bool rbc = which == RBC3D_TLIST_RBC;
+  const bool side = ctx->st2 && t.n > 0 && ctx->npt > 0 && (terms & RBC3D_TERM_CORR) && (terms & RBC3D_TERM_PME);
+  // PME joins the shorter stream: the main one behind the FP64 patch beside
+  // FP32 pair sums (FP32C, 256 cells: pair and near pass 3.3 ms, patch 16.5),
+  // else the side one.  FP64 with PME on the main stream / on the side (us): 3
+  // cells of 12 x 24 702 / 589, 3 cells 1666 / 1490, 8 cells 2904 / 2812, 24
+  // cells 9243 / 8675, 64 cells 19273 / 19385 (19287 with the own-cell pass
+  // beside the walk), 9 cells of 36 x 72 9123 / 9203.
   // The float-float patch (FP32D) loads the FP32 pipe and L1 like the pair
   // sums: next to them it took 15.6 ms against 6.9 alone.  So the side
   // stream runs PME next to the pair sums and then the patch, forked after
@@ -337,11 +357,12 @@ rbc3d_status matvec_dev(rbc3d_ctx* ctx, int which, double c1, double c2, unsigne
   // on a third low-priority stream (the FFTs interleave with the patch) and
   // 13.5 with PME on a third stream of medium priority (it starves the
   // patch).
-  const bool late = side && prec == RBC3D_FP32D;
-  const bool pme_side = prec == RBC3D_FP32M || late;
-  if (side && (s = fork_side(ctx, which, c1, c2, terms, prec, !late, pme_side))) return s;
+  const bool late = side && rbc && prec == RBC3D_FP32D;
+  const bool self_side = side && rbc && !late;
+  const bool pme_side = !rbc || prec != RBC3D_FP32C;
+  if (side && (s = fork_side(ctx, which, c1, c2, terms, prec, self_side, pme_side))) return s;
   if (terms & (RBC3D_TERM_REAL | RBC3D_TERM_CORR | RBC3D_TERM_LINEAR))
-    if ((s = rbcs_dev(ctx, which, c1, c2, prec, terms, side && !late, late))) return s;
+    if ((s = rbcs_dev(ctx, which, c1, c2, prec, terms, self_side, late))) return s;
   if (terms & RBC3D_TERM_WALLS) {
     StageScope sc(ctx, 4);
     if (which == RBC3D_TLIST_WALL) { if ((s = run_wall_self(ctx, c1))) return s; }
@@ -413,6 +434,7 @@ rbc3d_status rbc3d_create(const rbc3d_params* prm, rbc3d_ctx** out) {
         cudaStreamCreateWithPriority(&ctx->st3, cudaStreamNonBlocking, lowest) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_pair, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_own, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_vup, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_spl, cudaEventDisableTiming) != cudaSuccess ||
@@ -490,6 +512,7 @@ rbc3d_status rbc3d_destroy(rbc3d_ctx* ctx) {
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
   if (ctx->ev_pair) cudaEventDestroy(ctx->ev_pair);
   if (ctx->ev_own) cudaEventDestroy(ctx->ev_own);
+  if (ctx->ev_vup) cudaEventDestroy(ctx->ev_vup);
   if (ctx->ev_spl) cudaEventDestroy(ctx->ev_spl);
   if (ctx->ev_up) cudaEventDestroy(ctx->ev_up);
   if (ctx->ev_rthr) cudaEventDestroy(ctx->ev_rthr);
@@ -943,8 +966,13 @@ rbc3d_status rbc3d_pme_add_interp_vel(rbc3d_ctx* ctx, int which, double* v) {
 rbc3d_status rbc3d_matvec(rbc3d_ctx* ctx, int which, double c1, double c2, unsigned terms, int prec, double* v) {
   TargetSet* t = ctx ? tset(ctx, which) : nullptr;
   if (!t || !valid_prec(prec)) return ctx_fail(ctx, RBC3D_ERR_ARG, "matvec");
-  rbc3d_status s = matvec_dev(ctx, which, c1, c2, terms, prec);
-  if (s) return s;
+  rbc3d_status s;
+  if (v && (s = start_add(ctx, *t, v))) return s;
+  if ((s = matvec_dev(ctx, which, c1, c2, terms, prec))) {
+    if (ctx->vadd_up) cudaStreamSynchronize(ctx->st3);  // the caller's array is no longer read
+    ctx->vadd_up = false;
+    return s;
+  }
   if (!v) return RBC3D_OK;  // result stays on the device
   return finish_add(ctx, *t, v);
 }

@@ -160,6 +160,8 @@ struct rbc3d_ctx {
   cudaStream_t st2 = nullptr;  // matvec side stream: self patch and PME next to the pair sums
   cudaStream_t st3 = nullptr;  // the pair sums' own-cell pass, from ev_pair to ev_own
   cudaEvent_t ev_pair = nullptr, ev_own = nullptr;
+  cudaEvent_t ev_vup = nullptr;  // the caller's values are in vadd (vadd_up: on their way, on st3)
+  bool vadd_up = false;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // set_cells_x / set_cell_density_x build the spline tables on the side
   // stream and return; readers on the main stream wait on ev_spl (spl_wait)

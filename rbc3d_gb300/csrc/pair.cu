@@ -1509,13 +1509,14 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
   const std::false_type no{};
   auto run = [&](auto R) -> rbc3d_status {
     // without a density the walk still counts pairs and lists neighbours: as the single layer of zeros
-    // FP32: the own-cell pass on a low-priority stream beside the walk, where it
+    // The own-cell pass on a low-priority stream beside the walk, where it
     // fills the SMs that the walk's last units leave idle.  After it / beside it
     // (us): 256 cells pair stage 2700 / 2122, FP32D matvec 7156 / 6936, FP32M
     // 5502 / 5253; 97 cells 2743 / 2619; 8 cells 558 / 513; 2048 cells 54787 /
-    // 54844.  At the walk's priority 7018 and 5417.  Not in FP64, where the patch
-    // is beside the walk already: 64 cells 19179 / 19644, 8 cells 2815 / 2866.
-    const bool beside = own && !f64 && ctx->st3;
+    // 54844.  At the walk's priority 7018 and 5417.  FP64 with PME on the side
+    // stream: 3 cells 1490 / 1218, 3 cells of 12 x 24 525 / 459, 8 cells 2812 /
+    // 2770, 64 cells 19385 / 19287, 9 cells of 36 x 72 9203 / 9317.
+      const bool beside = own && ctx->st3;
     if (beside) {
       CUDA_TRY(cudaEventRecord(ctx->ev_pair, ctx->st));
       CUDA_TRY(cudaStreamWaitEvent(ctx->st3, ctx->ev_pair, 0));

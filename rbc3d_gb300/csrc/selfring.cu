@@ -297,6 +297,11 @@ rbc3d_status run_self_ring(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   auto launch = [&](auto kern, int nv) -> rbc3d_status {
     const size_t bytes = sizeof(double) * (size_t)thr * (2 * nv + 9);
     CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    // few points: the pair kernels' shared-memory split of the SM, as no block
+    // of another split starts beside this one (3 cells of 12 x 24: matvec 661 ->
+    // 459 us, of 14 x 28 841 -> 617; of 25 x 50 1224 -> 1281, where the L1 counts)
+    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  t.n <= 2000 ? cudaSharedmemCarveoutMaxShared : cudaSharedmemCarveoutDefault));
     kern<<<blocks * a.parts, thr, bytes, ctx->st>>>(a);
     ++ctx->launches;
     CUDA_TRY(cudaGetLastError());
