@@ -229,9 +229,21 @@ rbc3d_status pme_stages(rbc3d_ctx* ctx, int which, double c1, double c2, unsigne
   return pme_gather(ctx, which);
 }
 
-__global__ void k_vadd(long long n, const double* __restrict__ a, double* __restrict__ v) {
+// v += a (+ b, where given)
+__global__ void k_vadd(long long n, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ v) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) v[i] += a[i];
+  if (i < n) v[i] += b ? a[i] + b[i] : a[i];
+}
+
+// The FP32D matvec of many cells has PME on a stream and in an accumulator of
+// its own, so that the late patch need not wait for its transforms: matvec and
+// update with matvec of 256 cells 7211 -> 6986 and 8550 -> 8276 us, 97 cells
+// 2666 -> 2647, 2048 cells 56343 -> 56130; with 64 cells 1933 / 1937, 24 cells
+// 1133 / 1144, 8 cells 540 / 546.  At a higher priority the transforms starve the
+// patch (2048 cells 58046).
+constexpr int PME_STREAM_MIN = 100000;
+bool pme_stream(int which, int prec, int n) {
+  return which == RBC3D_TLIST_RBC && prec == RBC3D_FP32D && n >= PME_STREAM_MIN;
 }
 
 // The own-cell patch correction (with_self) and PME (with_pme) on the side
@@ -241,17 +253,21 @@ rbc3d_status fork_side(rbc3d_ctx* ctx, int which, double c1, double c2, unsigned
   TargetSet& t = ctx->tl[which];
   const double sc1 = ctx->has_f ? c1 : 0.0, sc2 = ctx->has_g ? c2 : 0.0;
   CUDA_TRY(t.v2.alloc(3 * (size_t)std::max(t.n, 1)));
+  const bool own_stream = pme_stream(which, prec, t.n);
+  cudaStream_t& side = own_stream ? ctx->st4 : ctx->st2;
+  DBuf<double>& acc = own_stream ? t.v3 : t.v2;
+  CUDA_TRY(acc.alloc(3 * (size_t)std::max(t.n, 1)));
   CUDA_TRY(cudaEventRecord(ctx->ev_fork, ctx->st));
-  CUDA_TRY(cudaStreamWaitEvent(ctx->st2, ctx->ev_fork, 0));
-  std::swap(ctx->st, ctx->st2);
-  dbuf_swap(t.v, t.v2);
+  CUDA_TRY(cudaStreamWaitEvent(side, ctx->ev_fork, 0));
+  std::swap(ctx->st, side);
+  dbuf_swap(t.v, acc);
   rbc3d_status s = RBC3D_OK;
   if (cudaMemsetAsync(t.v.p, 0, sizeof(double) * 3 * t.n, ctx->st) != cudaSuccess) s = RBC3D_ERR_CUDA;
   if (!s && with_self) s = self_stage(ctx, which, sc1, sc2, prec);
   if (!s && with_pme) s = pme_stages(ctx, which, c1, c2, terms, prec);
-  dbuf_swap(t.v, t.v2);
-  std::swap(ctx->st, ctx->st2);
-  CUDA_TRY(cudaEventRecord(ctx->ev_join, ctx->st2));
+  dbuf_swap(t.v, acc);
+  std::swap(ctx->st, side);
+  CUDA_TRY(cudaEventRecord(own_stream ? ctx->ev_pme : ctx->ev_join, side));
   return s;
 }
 
@@ -287,12 +303,15 @@ rbc3d_status rbcs_dev(rbc3d_ctx* ctx, int which, double c1, double c2, int prec,
     CUDA_TRY(cudaMemsetAsync(t.v.p, 0, sizeof(double) * 3 * t.n, ctx->st));
   }
   if (corr) {
-    if (self_late) {  // after fork_side: t.v2 is zeroed and PME queued on the side stream
+    if (self_late) {  // after fork_side: PME is queued, and t.v2 zeroed where it goes there
       CUDA_TRY(cudaEventRecord(ctx->ev_fork, ctx->st));
       CUDA_TRY(cudaStreamWaitEvent(ctx->st2, ctx->ev_fork, 0));
       std::swap(ctx->st, ctx->st2);
       dbuf_swap(t.v, t.v2);
-      s = self_stage(ctx, which, c1, c2, prec);
+      s = RBC3D_OK;
+      if (pme_stream(which, prec, t.n) && cudaMemsetAsync(t.v.p, 0, sizeof(double) * 3 * t.n, ctx->st) != cudaSuccess)
+        s = RBC3D_ERR_CUDA;
+      if (!s) s = self_stage(ctx, which, c1, c2, prec);
       dbuf_swap(t.v, t.v2);
       std::swap(ctx->st, ctx->st2);
       CUDA_TRY(cudaEventRecord(ctx->ev_join, ctx->st2));
@@ -350,19 +369,20 @@ rbc3d_status matvec_dev(rbc3d_ctx* ctx, int which, double c1, double c2, unsigne
   // cells 9243 / 8675, 64 cells 19273 / 19385 (19287 with the own-cell pass
   // beside the walk), 9 cells of 36 x 72 9123 / 9203.
   // The float-float patch (FP32D) loads the FP32 pipe and L1 like the pair
-  // sums: next to them it took 15.6 ms against 6.9 alone.  So the side
-  // stream runs PME next to the pair sums and then the patch, forked after
-  // them, while the main stream runs the FP64 near-singular pass beside the
-  // end of PME: 12.2 ms, against 13.7 with PME on the main stream, 13.4 with PME
-  // on a third low-priority stream (the FFTs interleave with the patch) and
-  // 13.5 with PME on a third stream of medium priority (it starves the
-  // patch).
+  // sums, so it forks after them, beside the FP64 near-singular pass; PME runs
+  // next to the pair sums.
   const bool late = side && rbc && prec == RBC3D_FP32D;
   const bool self_side = side && rbc && !late;
   const bool pme_side = !rbc || prec != RBC3D_FP32C;
   if (side && (s = fork_side(ctx, which, c1, c2, terms, prec, self_side, pme_side))) return s;
   if (terms & (RBC3D_TERM_REAL | RBC3D_TERM_CORR | RBC3D_TERM_LINEAR))
-    if ((s = rbcs_dev(ctx, which, c1, c2, prec, terms, self_side, late))) return s;
+    if ((s = rbcs_dev(ctx, which, c1, c2, prec, terms, self_side, late))) {
+      if (side) {  // leave nothing in flight beside the main stream
+        cudaStreamSynchronize(ctx->st2);
+        cudaStreamSynchronize(ctx->st4);
+      }
+      return s;
+    }
   if (terms & RBC3D_TERM_WALLS) {
     StageScope sc(ctx, 4);
     if (which == RBC3D_TLIST_WALL) { if ((s = run_wall_self(ctx, c1))) return s; }
@@ -372,7 +392,9 @@ rbc3d_status matvec_dev(rbc3d_ctx* ctx, int which, double c1, double c2, unsigne
   if (side) {
     CUDA_TRY(cudaStreamWaitEvent(ctx->st, ctx->ev_join, 0));
     const long long n3 = 3ll * t.n;
-    { k_vadd<<<nblk(n3, 256), 256, 0, ctx->st>>>(n3, t.v2.p, t.v.p); ++ctx->launches; }
+    const bool third = late && pme_stream(which, prec, t.n);
+    if (third) CUDA_TRY(cudaStreamWaitEvent(ctx->st, ctx->ev_pme, 0));
+    { k_vadd<<<nblk(n3, 256), 256, 0, ctx->st>>>(n3, t.v2.p, third ? t.v3.p : nullptr, t.v.p); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
   } else if (terms & RBC3D_TERM_PME) {
     if ((s = pme_stages(ctx, which, c1, c2, terms, prec))) return s;
@@ -434,6 +456,8 @@ rbc3d_status rbc3d_create(const rbc3d_params* prm, rbc3d_ctx** out) {
         cudaStreamCreateWithPriority(&ctx->st3, cudaStreamNonBlocking, lowest) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_pair, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_own, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->ev_pme, cudaEventDisableTiming) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&ctx->st4, cudaStreamNonBlocking, lowest) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_vup, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
@@ -506,12 +530,14 @@ rbc3d_status rbc3d_destroy(rbc3d_ctx* ctx) {
   wall_spec_release(ctx);
   if (ctx->st2) cudaStreamSynchronize(ctx->st2);
   if (ctx->st3) cudaStreamSynchronize(ctx->st3);
+  if (ctx->st4) cudaStreamSynchronize(ctx->st4);
   if (ctx->st) cudaStreamSynchronize(ctx->st);
   for (cudaEvent_t e : ctx->evpool) cudaEventDestroy(e);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
   if (ctx->ev_pair) cudaEventDestroy(ctx->ev_pair);
   if (ctx->ev_own) cudaEventDestroy(ctx->ev_own);
+  if (ctx->ev_pme) cudaEventDestroy(ctx->ev_pme);
   if (ctx->ev_vup) cudaEventDestroy(ctx->ev_vup);
   if (ctx->ev_spl) cudaEventDestroy(ctx->ev_spl);
   if (ctx->ev_up) cudaEventDestroy(ctx->ev_up);
@@ -521,6 +547,7 @@ rbc3d_status rbc3d_destroy(rbc3d_ctx* ctx) {
   if (ctx->h_rthr) cudaFreeHost(ctx->h_rthr);
   if (ctx->st2) cudaStreamDestroy(ctx->st2);
   if (ctx->st3) cudaStreamDestroy(ctx->st3);
+  if (ctx->st4) cudaStreamDestroy(ctx->st4);
   if (ctx->t0) { cudaEventDestroy(ctx->t0); cudaEventDestroy(ctx->t1); }
   cudaStream_t st = ctx->st;
   delete ctx;
