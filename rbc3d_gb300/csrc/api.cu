@@ -235,15 +235,16 @@ __global__ void k_vadd(long long n, const double* __restrict__ a, const double* 
   if (i < n) v[i] += b ? a[i] + b[i] : a[i];
 }
 
-// The FP32D matvec of many cells has PME on a stream and in an accumulator of
+// The FP32D (FP32M) matvec of many cells has PME on a stream and in an accumulator of
 // its own, so that the late patch need not wait for its transforms: matvec and
 // update with matvec of 256 cells 7211 -> 6986 and 8550 -> 8276 us, 97 cells
 // 2666 -> 2647, 2048 cells 56343 -> 56130; with 64 cells 1933 / 1937, 24 cells
 // 1133 / 1144, 8 cells 540 / 546.  At a higher priority the transforms starve the
 // patch (2048 cells 58046).
 constexpr int PME_STREAM_MIN = 100000;
+bool late_patch(int prec) { return prec == RBC3D_FP32D || prec == RBC3D_FP32M; }
 bool pme_stream(int which, int prec, int n) {
-  return which == RBC3D_TLIST_RBC && prec == RBC3D_FP32D && n >= PME_STREAM_MIN;
+  return which == RBC3D_TLIST_RBC && late_patch(prec) && n >= PME_STREAM_MIN;
 }
 
 // The own-cell patch correction (with_self) and PME (with_pme) on the side
@@ -368,10 +369,12 @@ rbc3d_status matvec_dev(rbc3d_ctx* ctx, int which, double c1, double c2, unsigne
   // cells of 12 x 24 702 / 589, 3 cells 1666 / 1490, 8 cells 2904 / 2812, 24
   // cells 9243 / 8675, 64 cells 19273 / 19385 (19287 with the own-cell pass
   // beside the walk), 9 cells of 36 x 72 9123 / 9203.
-  // The float-float patch (FP32D) loads the FP32 pipe and L1 like the pair
-  // sums, so it forks after them, beside the FP64 near-singular pass; PME runs
-  // next to the pair sums.
-  const bool late = side && rbc && prec == RBC3D_FP32D;
+  // The float-float patch (FP32D) and the mixed one (FP32M) load the FP32 pipe
+  // and L1 like the pair sums, so they fork after them, beside the FP64
+  // near-singular pass; PME runs next to the pair sums.  FP32M with its patch
+  // beside the pair sums / after them: 256 cells 5523 / 5468 us, 1024 cells
+  // 22663 / 22245, 97 cells of 24 x 48 2076 / 2001, 8 cells 524 / 488.
+  const bool late = side && rbc && late_patch(prec);
   const bool self_side = side && rbc && !late;
   const bool pme_side = !rbc || prec != RBC3D_FP32C;
   if (side && (s = fork_side(ctx, which, c1, c2, terms, prec, self_side, pme_side))) return s;
