@@ -330,7 +330,7 @@ class Bench:
         self.ctx.close()
 
 
-def rooflines_of(b, counts, peak32, peak64, hbm_peak, hbm_src, sm_mhz):
+def rooflines_of(b, counts, peak32, peak64, hbm_peak, hbm_src):
     """Per-kernel rooflines from algorithmic work, each stage timed alone."""
     from rbc3d_gb300.abi import FP32C, FP32D, FP32M, TERM_CORR, TERM_LINEAR, TERM_PME, TERM_REAL
     s_c = b.alone(FP32C, TERM_REAL | TERM_CORR | TERM_LINEAR)
@@ -346,10 +346,6 @@ def rooflines_of(b, counts, peak32, peak64, hbm_peak, hbm_src, sm_mhz):
     pairs = counts["pairs_within_rc"]
     pair_fl = pairs * (FLOP_PAIR_SL + FLOP_PAIR_DL)
     self_fl = counts["self_items"] * NQ * FLOP_SELFQ_SLDL
-    # requested L1 load bytes of k_self_ff per patch point: 4 stencil nodes x
-    # 4 slots x 3 quads x 32 B (hi and lo) + 136 B of weights
-    l1_bytes = counts["self_items"] * NQ * (4 * 4 * 3 * 32 + 136)
-    l1_peak = 128.0 * 152 * sm_mhz * 1e6 / 1e9
 
     def fl(name, ms, flops, peak, bound, work):
         a = flops / (ms * 1e-3) / 1e12
@@ -357,14 +353,14 @@ def rooflines_of(b, counts, peak32, peak64, hbm_peak, hbm_src, sm_mhz):
                 "frac": a / peak, "work": work}
 
     r = {
-        "k_pair32": fl("k_pair32 + k_pair_own32 (the pair-sum stage)", s_c["pair"], pair_fl, peak32, "fp32",
+        "k_pair": fl("k_pair + k_pair_own32 (the pair-sum stage)", s_c["pair"], pair_fl, peak32, "fp32",
                        f"{pairs} pairs within rc x {FLOP_PAIR_SL + FLOP_PAIR_DL} flops"),
         "k_self_ff": fl("k_self_ff", s_d["self"], self_fl, peak32, "fp32",
                         f"{counts['self_items']} targets x {NQ} patch points x {FLOP_SELFQ_SLDL} flops of the FP64 "
                         "formula, evaluated in float-float on the FP32 pipe"),
-        "k_self": fl("k_self", s_c["self"], self_fl, peak64, "fp64",
+        "k_self_ring": fl("k_self_ring", s_c["self"], self_fl, peak64, "fp64",
                      f"{counts['self_items']} targets x {NQ} x {FLOP_SELFQ_SLDL} flops"),
-        "k_self_mix": fl("k_self_mix", s_m["self"], self_fl, peak32, "fp32", "the k_self work in FP32"),
+        "k_self_mix": fl("k_self_mix", s_m["self"], self_fl, peak32, "fp32", "the k_self_ring work in FP32"),
         "pme": {"kernel": "k_spread_tile + cuFFT + k_influence + k_gather", "bound": "hbm", "ms": pme_ms,
                 "achieved": pme_bytes / (pme_ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                 "frac": pme_bytes / (pme_ms * 1e-3) / 1e9 / hbm_peak, "peak_source": hbm_src,
@@ -373,15 +369,13 @@ def rooflines_of(b, counts, peak32, peak64, hbm_peak, hbm_src, sm_mhz):
         "note": "stages timed alone on one stream (the matvec runs them on two); FP32 peak = measured FMA chain "
                 "(rbc3d_fma_peak), FP64 likewise",
     }
-    r["k_self_ff"]["l1_request_gbs"] = l1_bytes / (s_d["self"] * 1e-3) / 1e9
-    r["k_self_ff"]["l1_request_frac_of_nominal"] = r["k_self_ff"]["l1_request_gbs"] / l1_peak
     return r, s_d
 
 
 def headline_roofline(r, s_d, targets):
     """The dominant kernel of the FP32D matvec (longest stage timed alone);
     traffic = the ncu bytes per target of that kernel x this launch's targets."""
-    key = "k_self_ff" if s_d["self"] >= s_d["pair"] else "k_pair32"
+    key = "k_self_ff" if s_d["self"] >= s_d["pair"] else "k_pair"
     roof = dict(r[key])
     roof["peak_source"] = "measured FP32 FMA chain over all SMs (rbc3d_fma_peak), same GPU, same run"
     roof["traffic"] = None
@@ -481,8 +475,7 @@ def main():
         hbm_peak, hbm_src = float(mp["hbm_gbs"]), "measured (MEASURED_PEAKS.json)"
     except Exception:
         pass
-    sm_mhz = (clocks or {}).get("sm_mhz") or 2070.0
-    rooflines, s_d = rooflines_of(b, counts, peak32, peak64, hbm_peak, hbm_src, sm_mhz)
+    rooflines, s_d = rooflines_of(b, counts, peak32, peak64, hbm_peak, hbm_src)
     roof = headline_roofline(rooflines, s_d, N)
 
     # ---- CPU baseline on the same inputs (rank 0, N = 1): the oracle on all
@@ -516,7 +509,7 @@ def main():
         vec5 = {n: b5.vector(p) for n, p in (("fp64", FP64), ("fp32c", FP32C), ("fp32m", FP32M), ("fp32d", FP32D))}
         e5 = b5.e2e(FP32D, 5, raw=True)
         e5["floor_ms"] = m5d + e5["h2d_bytes_per_step"] / (e5["h2d_gbs_measured"] * 1e9) * 1e3
-        r5, s5d = rooflines_of(b5, cnt5, peak32, peak64, hbm_peak, hbm_src, sm_mhz)
+        r5, s5d = rooflines_of(b5, cnt5, peak32, peak64, hbm_peak, hbm_src)
         b5.close()
         c5 = {"config": WORKLOADS["C5"], "value": ws * N5 / (m5d * 1e-3), "unit": "targets/s",
               "ms_per_step": m5d, "steps": k5, "warmup": 3, "stages_ms_per_step": st5d, "gpu_launches": l5,

@@ -6,18 +6,16 @@
 // [start, end) ranges per cell.  The same Nc = max(floor(L/rc), 3) cells are
 // used, so a target visits its 27 neighbour cells exactly as the reference.
 //
-// Pair kernels: work units of one target cell's targets (a cell's units
-// equal-sized, heaviest units launched first), each thread owning one
-// target; the 27 neighbour cells are streamed through shared memory.  FP64:
-// one CTA per unit of <= 128 targets, tiles of 128 sources shared by the
-// CTA.  FP32: one warp per unit of <= 32 targets, each warp staging its own
-// 32-source chunks, so the four warps of a CTA may serve different cells
-// (CTA-sized units left 18% of the CTAs' thread slots idle on the 256-cell
-// workload, warp units 5%).  Tiles whose bounding box lies farther than rc
-// from the CTA's (or a warp's) targets are skipped.  FP32 with cell targets:
-// the own-cell pairs (79% of the pairs on the 256-cell workload) go to a
-// dense per-cell pass (k_pair_own32), and k_pair32 skips the target's own
-// surface (whole tiles and chunks when a warp's targets share one surface).
+// Pair kernel (k_pair, both precisions): a warp per work unit, the targets of
+// one hash cell (equal-sized units, heaviest launched first): 32 targets of a
+// lane each, or 16 or 8 of two or four lanes (pair_sub), the block's four warps
+// together on a unit where targets are few (PAIR_SPLIT_MAX*).  A warp stages
+// the tiles of 128 sources of the 27 neighbour cells whose boxes come within
+// rc of its targets, skipping chunks of 32 that do not; every lane marks its
+// candidates in bit lists and evaluates them, so lanes work on sources of
+// their own.  Cell targets: the own cell's pairs (79% of the pairs of dense
+// suspensions) go to a dense pass per cell (k_pair_own32, k_pair_own64), which
+// evaluates a pair once for both points.
 // FP32: sources carry hi/lo FP32
 // coordinates relative to their own cell centre (from FP64, once per
 // position update) and the targets are shifted into each neighbour cell's
@@ -879,11 +877,11 @@ __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs 
 // to its source j (per-warp sums in shared memory; at step s lane l takes
 // the source pair (l + s) mod OWN_TILE/2, so the lanes of a warp touch
 // distinct sources and read consecutive ones).  A diagonal CTA (S = T) takes
-// every ordered pair of its tile one way.  The pair arithmetic is k_pair32's
+// every ordered pair of its tile one way.  The pair arithmetic is k_pair's
 // (ewald_coef2 / ewald_apply2), positions hi/lo FP32 relative to the cell's
 // first point, FP32 sums per 32 sources (Kahan-compensated across them) and
-// per warp, added to the accumulator in FP64 atomically, after k_pair32 on
-// the same stream.  The target tile's at most (OWN_TILE - 1) / nlon + 2
+// per warp, added to the accumulator in FP64 atomically, beside k_pair.
+// The target tile's at most (OWN_TILE - 1) / nlon + 2
 // latitude rings' rows of the weight table sit in shared memory.
 constexpr int OWN_TILE = 128;
 // FP64: fewer than this many blocks of 128 points go in tiles of 32 (8 blocks
