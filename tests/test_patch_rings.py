@@ -8,7 +8,8 @@ import pytest
 from scipy.spatial import cKDTree
 
 from rbc3d_gb300 import geometry as G
-from rbc3d_gb300.abi import FP32C, FP32D, FP64, TERM_CORR, TERM_LINEAR, TERM_REAL, TLIST_RAW, TLIST_RBC, Context
+from rbc3d_gb300.abi import (FP32C, FP32D, FP64, TERM_CORR, TERM_LINEAR, TERM_PME, TERM_REAL, TLIST_RAW, TLIST_RBC,
+                              Context)
 
 pytestmark = pytest.mark.gpu
 C = 1 / (4 * math.pi)
@@ -93,3 +94,24 @@ def test_few_points(gpu, oracle, n, prec):
     # FP64: rounding of the sums; FP32: of single pairs and of the mesh
     tol = 1e-10 if prec == FP64 else 2e-6
     assert x.shape[1] == n and np.linalg.norm(out[1] - out[0]) <= tol * np.linalg.norm(out[0])
+
+
+@pytest.mark.parametrize("P", [2, 4, 6, 8])
+def test_spread_orders(gpu, oracle, P):
+    """PME at every even spline order (an odd one's factor vanishes at an even
+    mesh's highest wave): the tiled spread's rounds of nodes, full and partly
+    filled, all at once or (many rounds) one at a time."""
+    L = 14.0
+    rng = np.random.default_rng(P)
+    cells = G.make_cells(rng, 3, [L] * 3, 3.2, nlat=12, nlon=24, with_g=True)
+    prm = dict(Lb=[L] * 3, alpha=G.alpha_for_cutoff(3.0, 1e-6), rc=3.0, eps=1e-6, Nb=[24, 20, 18], P=P, nlat=12, nlon=24,
+               ncelltypes=1, viscRat=[5.0])
+    out = []
+    for lib in (oracle, gpu):
+        c = Context(lib, prm)
+        c.set_cells(cells)
+        c.set_cell_density(f=cells.f, g=cells.g, spl_F=cells.spl_F, spl_G=cells.spl_G)
+        out.append(c.matvec(TLIST_RBC, C, C, TERM_PME, FP32C if lib is gpu else FP64))
+        c.close()
+    # FP32 rounding of the mesh part, as test_few_points
+    assert np.linalg.norm(out[1] - out[0]) <= 2e-6 * np.linalg.norm(out[0])
