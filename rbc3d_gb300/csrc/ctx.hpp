@@ -219,6 +219,7 @@ struct rbc3d_ctx {
   DBuf<double> s_rec64;         // FP64 pair-sum records (12 doubles a source)
   DBuf<float4> s_op0, s_op1;    // own-cell pair records in point order (k_pair_own32)
   DBuf<int> s_inv;              // point -> sorted source position
+  DBuf<int> s_wide;             // per cell: its pairs may meet at another image (k_own_records)
   int s_ntiles = 0;
   DBuf<unsigned long long> near_queue;  // work counter of the near-singular kernel
   DBuf<double> dBcoef;                  // Bcoef per cell type on the device

@@ -15,7 +15,8 @@
 // candidates in bit lists and evaluates them, so lanes work on sources of
 // their own.  Cell targets: the own cell's pairs (79% of the pairs of dense
 // suspensions) go to a dense pass per cell (k_pair_own32, k_pair_own64), which
-// evaluates a pair once for both points.
+// evaluates a pair once for both points (cells that nearly meet their own
+// image keep to the walk: k_own_records).
 // FP32: sources carry hi/lo FP32
 // coordinates relative to their own cell centre (from FP64, once per
 // position update) and the targets are shifted into each neighbour cell's
@@ -151,11 +152,12 @@ __global__ void k_gather_units(int cap, const int* __restrict__ idx, const int4*
   if (i < cap) out[i] = in[idx[i]];
 }
 
-// Gather cell-point geometry into cell-list order.
+// Gather cell-point geometry into cell-list order; clears the cells' flags of k_own_records.
 __global__ void k_gather_src(int n, int nlat, int nv, const int* __restrict__ order, const double* __restrict__ x,
-                             double* __restrict__ sx, int4* __restrict__ meta) {
+                             double* __restrict__ sx, int4* __restrict__ meta, int* __restrict__ wide) {
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
+  if (q < n / nv) wide[q] = 0;
   int p = order[q];
   for (int k = 0; k < 3; ++k) sx[q + (size_t)k * n] = x[p + (size_t)k * n];
   int cell = p / nv, r = p - cell * nv;
@@ -243,11 +245,14 @@ __global__ void k_tile_boxes(const int2* __restrict__ tiles, const float4* __res
 }
 
 // Point-order records of the own-cell pair sums: hi/lo FP32 of the position
-// relative to the cell's first point (minimum image: a cell spans less than
-// half the box), the grid indices, and the point's sorted source position.
+// relative to the cell's first point (at the minimum image), the grid indices, and
+// the point's sorted source position.  The difference of two such positions is
+// the pair's minimum image, or the pair is out of reach, while every component
+// is under L - rc; a cell with a component of (L - rc) / 2 or more is flagged
+// in wide[cell], and its own pairs stay in the cell-list walk.
 __global__ void k_own_records(int n, int nlat, int nv, const double* __restrict__ x, const int* __restrict__ order,
-                              double L0, double L1, double L2, float4* __restrict__ op0, float4* __restrict__ op1,
-                              int* __restrict__ sinv) {
+                              double L0, double L1, double L2, double rc, float4* __restrict__ op0,
+                              float4* __restrict__ op1, int* __restrict__ sinv, int* __restrict__ wide) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q < n) sinv[order[q]] = q;
   const int p = q;
@@ -257,6 +262,7 @@ __global__ void k_own_records(int n, int nlat, int nv, const double* __restrict_
   float hi[3], lo[3];
   for (int k = 0; k < 3; ++k) {
     const double d = min_image(x[p + (size_t)k * n] - x[(size_t)cell * nv + (size_t)k * n], L[k], 1.0 / L[k]);
+    if (2.0 * fabs(d) >= L[k] - 1.000001 * rc) wide[cell] = 1;  // (margin: the FP32 cutoff)
     hi[k] = (float)d;
     lo[k] = (float)(d - (double)hi[k]);
   }
@@ -371,8 +377,9 @@ struct PairArgs {
   int cap;
   unsigned long long* cnt;  // [0] items, [1] pairs, [2] overflow
   // own-cell pairs (cell targets, same-cell weight table): the dense pass takes
-  // them and k_pair skips same-surface sources
+  // them and k_pair skips same-surface sources, but for the cells in wide
   int own_split;
+  const int* wide;
   const float4* op0;  // per point (point order): (x, y, z) hi relative to its cell's first point, id bits
   const float4* op1;  // lo
   const int* sinv;    // point -> sorted source position
@@ -550,7 +557,7 @@ __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs 
   const int ti = active ? a.torder[unit.y + lane / SUB] : 0;
   double t64[3] = {0, 0, 0};
   float th_[3] = {0, 0, 0}, tl_[3] = {0, 0, 0};
-  int surf_i = -2, tlat = 0, tlon = 0;
+  int surf_i = -2, own = -7, tlat = 0, tlon = 0;  // own: the surface whose pairs the dense pass takes
   bool grid = false;
   if (active) {
     for (int k = 0; k < 3; ++k) {
@@ -560,6 +567,7 @@ __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs 
     }
     const int4 m = a.tmeta[ti];
     surf_i = m.x;
+    if (a.own_split && !a.wide[m.x - 1]) own = m.x;
     if (m.y >= 0) { tlat = m.y; tlon = m.z; grid = true; }
   }
   float3 wlo0, whi0;
@@ -581,8 +589,8 @@ __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs 
   // targets share one (whole tiles and chunks of it are skipped), else -7
   int wsurf = -7;
   if (a.own_split) {
-    const int s0 = __shfl_sync(0xffffffffu, surf_i, 0);
-    wsurf = __all_sync(0xffffffffu, !active || surf_i == s0) ? s0 : -7;
+    const int s0 = __shfl_sync(0xffffffffu, own, 0);
+    wsurf = __all_sync(0xffffffffu, !active || own == s0) ? s0 : -7;
   }
 
   // 1 - MaskFunc of a pair on one cell
@@ -719,7 +727,7 @@ __global__ void __launch_bounds__(TILE, sizeof(R) == 8 ? 3 : 5) k_pair(PairArgs 
           const float4 p = F64 ? D.p0[32 * word + j] : C.r[32 * word + j][0];
           const float hx = p.x - tsh[0], hy = p.y - tsh[1], hz = p.z - tsh[2];
           const float h2 = fmaf(hx, hx, fmaf(hy, hy, hz * hz));
-          if (h2 <= a.rc2_loose && !(a.own_split && __float_as_int(p.w) == surf_i)) m |= 1u << j;
+          if (h2 <= a.rc2_loose && __float_as_int(p.w) != own) m |= 1u << j;
         }
         bits[w] = m;
       }
@@ -898,6 +906,7 @@ __global__ void __launch_bounds__(OWN_TILE) k_pair_own32(PairArgs a) {
   const int nlat = a.nlat, nlon = a.nlon, nv = nlat * nlon, rowlen = nlat * a.nhalf;
   const int ntile = (nv + OWN_TILE - 1) / OWN_TILE, npt = ntile * (ntile + 1) / 2;
   const int cell = blockIdx.x / npt;
+  if (a.wide[cell]) return;  // k_pair takes this cell's pairs
   int r = blockIdx.x - cell * npt, T = 0;
   while (r >= ntile - T) { r -= ntile - T; ++T; }
   const int S = T + r;
@@ -1040,6 +1049,7 @@ __global__ void __launch_bounds__(OT) k_pair_own64(PairArgs a) {
   const int nlat = a.nlat, nlon = a.nlon, nv = nlat * nlon, rowlen = nlat * a.nhalf;
   const int ntile = (nv + OT - 1) / OT, npt = ntile * (ntile + 1) / 2;
   const int cell = blockIdx.x / npt;
+  if (a.wide[cell]) return;  // k_pair takes this cell's pairs
   int r = blockIdx.x - cell * npt, T = 0;
   while (r >= ntile - T) { r -= ntile - T; ++T; }
   const int S = T + r;
@@ -1328,8 +1338,9 @@ rbc3d_status build_source_list(rbc3d_ctx* ctx, bool with_normals) {
   if (s) return s;
   CUDA_TRY(ctx->s_x.alloc(3 * (size_t)n)); CUDA_TRY(ctx->s_a3.alloc(3 * (size_t)n)); CUDA_TRY(ctx->s_meta.alloc(n));
   CUDA_TRY(ctx->s_f.alloc(3 * (size_t)n)); CUDA_TRY(ctx->s_g.alloc(3 * (size_t)n));
+  CUDA_TRY(ctx->s_wide.alloc(ctx->ncell));
   { k_gather_src<<<nblk(n, 256), 256, 0, ctx->st>>>(n, ctx->nlat, ctx->nlat * ctx->nlon, ctx->s_order.p, ctx->x.p,
-                                                   ctx->s_x.p, ctx->s_meta.p); ++ctx->launches; }
+                                                   ctx->s_x.p, ctx->s_meta.p, ctx->s_wide.p); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());
   // FP32 pair-sum records and tile boxes
   CUDA_TRY(ctx->s_p0.alloc(n)); CUDA_TRY(ctx->s_p1.alloc(n)); CUDA_TRY(ctx->s_u4.alloc(n)); CUDA_TRY(ctx->s_a4.alloc(n));
@@ -1342,8 +1353,8 @@ rbc3d_status build_source_list(rbc3d_ctx* ctx, bool with_normals) {
     ++ctx->launches;
     CUDA_TRY(ctx->s_op0.alloc(n)); CUDA_TRY(ctx->s_op1.alloc(n)); CUDA_TRY(ctx->s_inv.alloc(n));
     { k_own_records<<<nblk(n, 256), 256, 0, ctx->st>>>(n, ctx->nlat, ctx->nlat * ctx->nlon, ctx->x.p, ctx->s_order.p,
-                                                       hg.L[0], hg.L[1], hg.L[2], ctx->s_op0.p, ctx->s_op1.p,
-                                                       ctx->s_inv.p); ++ctx->launches; }
+                                                       hg.L[0], hg.L[1], hg.L[2], ctx->prm.rc, ctx->s_op0.p,
+                                                       ctx->s_op1.p, ctx->s_inv.p, ctx->s_wide.p); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
     const int nc = hg.ncells;
     // tiles of TILE and chunks of 32 consecutive sources of one cell, with
@@ -1467,7 +1478,7 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
   const size_t own_sm = (f64 ? sizeof(double) : sizeof(float)) * (size_t)nrow * ctx->nlat * a.nhalf;
   const bool own = tlist == RBC3D_TLIST_RBC && a.mtab32 && t.n == n && ctx->s_op0.p && own_sm <= 160 * 1024;
   a.own_split = own ? 1 : 0;
-  a.op0 = ctx->s_op0.p; a.op1 = ctx->s_op1.p; a.sinv = ctx->s_inv.p;
+  a.op0 = ctx->s_op0.p; a.op1 = ctx->s_op1.p; a.sinv = ctx->s_inv.p; a.wide = ctx->s_wide.p;
   if (f64) {
     CUDA_TRY(ctx->s_rec64.alloc(12 * (size_t)n));
     a.rec64 = ctx->s_rec64.p;
