@@ -565,7 +565,8 @@ rbc3d_status rbc3d_set_cell_grid(rbc3d_ctx* ctx, const double* th, const double*
   if (!ctx || !th || !phi || !w) return RBC3D_ERR_ARG;
   const int nlat = ctx->nlat, nlon = ctx->nlon;
   ctx->h_th.assign(th, th + nlat); ctx->h_phi.assign(phi, phi + nlon); ctx->h_w.assign(w, w + nlat);
-  ctx->shtab.L = 0;  // transform tables of the previous grid
+  ctx->shtab.L = ctx->mb.L = 0;  // transform and membrane tables of the previous grid
+  spl_wait(ctx);                 // (a set_cells_x whose side stream still reads them)
   CUDA_TRY(ctx->th.upload(th, nlat, ctx->st)); CUDA_TRY(ctx->phi.upload(phi, nlon, ctx->st));
   CUDA_TRY(ctx->w.upload(w, nlat, ctx->st));
   std::vector<float4> us(nlat * nlon);
