@@ -332,8 +332,8 @@ rbc3d_status sh_anal(rbc3d_ctx* ctx, const CellSolveTabs& T, const double* v, co
                      int nvar = 3) {
   ShArgs a = sh_args(ctx, T, false, nvar);
   const size_t sm = sizeof(double) * ((size_t)a.nlat * a.nlon + 2 * (size_t)T.L * a.nlat);
-  if (sm > 227 * 1024) return ctx_fail(ctx, RBC3D_ERR_ARG, "sh_anal: cell grid too large for one block");
-  if (sm > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(k_sh_anal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (sm > SMEM_BLOCK) return ctx_fail(ctx, RBC3D_ERR_ARG, "sh_anal: cell grid too large for one block");
+  if (sm > 48 * 1024) CUDA_TRY(smem_opt_in(k_sh_anal, sm));
   { k_sh_anal<<<nvar * ctx->ncell, 128, sm, ctx->st>>>(a, v, fac, c); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());
   return RBC3D_OK;
@@ -341,8 +341,8 @@ rbc3d_status sh_anal(rbc3d_ctx* ctx, const CellSolveTabs& T, const double* v, co
 rbc3d_status sh_synth(rbc3d_ctx* ctx, const CellSolveTabs& T, const double* c, double* out, bool equi, int nvar = 3) {
   ShArgs a = sh_args(ctx, T, equi, nvar);
   const size_t sm = sizeof(double) * (2 * (size_t)T.L * T.L + 2 * (size_t)T.L * a.nrow);
-  if (sm > 227 * 1024) return ctx_fail(ctx, RBC3D_ERR_ARG, "sh_synth: degree too large for one block");
-  if (sm > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(k_sh_synth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (sm > SMEM_BLOCK) return ctx_fail(ctx, RBC3D_ERR_ARG, "sh_synth: degree too large for one block");
+  if (sm > 48 * 1024) CUDA_TRY(smem_opt_in(k_sh_synth, sm));
   { k_sh_synth<<<nvar * ctx->ncell, 128, sm, ctx->st>>>(a, c, out, equi ? 1 : 0); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());
   return RBC3D_OK;
@@ -359,8 +359,8 @@ rbc3d_status build_spline_set(rbc3d_ctx* ctx, const CellSolveTabs& T, const doub
   a.PG = T.PG.p; a.PE = T.PE.p; a.dPE = T.dPE.p; a.wf = T.wf.p; a.tab = T.fold.p;
   const size_t L = T.L, R = ctx->nlat + 1;
   const size_t sm = sizeof(double) * (2 * L * L + std::max(4 * L * R, (size_t)ctx->nlat * ctx->nlon + 2 * L * ctx->nlat));
-  if (sm > 227 * 1024) return ctx_fail(ctx, RBC3D_ERR_ARG, "spline build: cell grid too large for one block");
-  if (sm > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(k_sh_spline, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (sm > SMEM_BLOCK) return ctx_fail(ctx, RBC3D_ERR_ARG, "spline build: cell grid too large for one block");
+  if (sm > 48 * 1024) CUDA_TRY(smem_opt_in(k_sh_spline, sm));
   { k_sh_spline<<<nvar * ctx->ncell, SPL_THREADS, sm, ctx->st>>>(a, v, fac, ctx->spl.p); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());
   return RBC3D_OK;

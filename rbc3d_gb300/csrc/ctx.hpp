@@ -33,6 +33,17 @@ struct DBuf {
   ~DBuf() { release(); }
 };
 
+// Dynamic shared memory a block may take.  A kernel's opt-in above 48 KB is the
+// process's, so every launch names one bound for all its sizes: a launch that
+// named its own would lower it under a context of another grid in another
+// thread, between that thread's opt-in and its launch.
+constexpr size_t SMEM_BLOCK = 227 * 1024;
+template <class Kernel>
+inline cudaError_t smem_opt_in(Kernel kern, size_t bytes, size_t most = SMEM_BLOCK) {
+  if (bytes > most) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // Uniform cell list over the periodic box (HashTable_ComputeNumBlocks,
 // ModHashTable.F90:99-126, single rank): Nc = max(floor(L/rc), 3) per axis.
 struct HashGrid {

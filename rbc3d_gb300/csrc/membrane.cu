@@ -464,8 +464,8 @@ rbc3d_status mb_tables(rbc3d_ctx* ctx) {
   CUDA_TRY(M.sn.upload(sn.data(), sn.size(), ctx->st)); CUDA_TRY(M.sinth.upload(st.data(), st.size(), ctx->st));
   const size_t sm = grad_smem(L, nlat, nlat * nlon);
   if (sm > 48 * 1024) {
-    CUDA_TRY(cudaFuncSetAttribute(k_mb_grad<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    CUDA_TRY(cudaFuncSetAttribute(k_mb_grad<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    CUDA_TRY(smem_opt_in(k_mb_grad<true>, sm));
+    CUDA_TRY(smem_opt_in(k_mb_grad<false>, sm));
   }
   bool equi = nlon % 2 == 0;
   for (int j = 0; j < nlon && equi; ++j)

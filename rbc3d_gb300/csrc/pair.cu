@@ -897,6 +897,7 @@ constexpr int OWN_TILE = 128;
 // 1761 -> 1533, 3 cells of 12 x 24 839 -> 675, 8 cells 3085 -> 2797, 12 cells
 // 3850 -> 3800, 20 cells (1100) 6596 -> 6589, 64 cells (3520) 19927 -> 20133.
 constexpr int OWN64_BLOCKS = 1216;
+constexpr size_t OWN_MASK_MAX = 160 * 1024;  // weight-table rows of a block; wider grids keep their pairs in the walk
 template <bool SL, bool DL>
 __global__ void __launch_bounds__(OWN_TILE) k_pair_own32(PairArgs a) {
   __shared__ __align__(16) float s_src[15][OWN_TILE];  // hi xyz, lo xyz, f xyz, g xyz, normal xyz
@@ -1476,7 +1477,7 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
   const int own_tile = f64 && own_blocks(OWN_TILE) < OWN64_BLOCKS ? 32 : OWN_TILE;
   const int nrow = std::min(ctx->nlat, (own_tile - 1) / std::max(ctx->nlon, 1) + 2);
   const size_t own_sm = (f64 ? sizeof(double) : sizeof(float)) * (size_t)nrow * ctx->nlat * a.nhalf;
-  const bool own = tlist == RBC3D_TLIST_RBC && a.mtab32 && t.n == n && ctx->s_op0.p && own_sm <= 160 * 1024;
+  const bool own = tlist == RBC3D_TLIST_RBC && a.mtab32 && t.n == n && ctx->s_op0.p && own_sm <= OWN_MASK_MAX;
   a.own_split = own ? 1 : 0;
   a.op0 = ctx->s_op0.p; a.op1 = ctx->s_op1.p; a.sinv = ctx->s_inv.p; a.wide = ctx->s_wide.p;
   if (f64) {
@@ -1492,9 +1493,9 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
     { k_src_dens4<<<nblk(n, 256), 256, 0, ctx->st>>>(n, c1, c2, ctx->s_f.p, ctx->s_g.p, sl, dl,
                                                      ctx->s_F4.p, ctx->s_G4.p); ++ctx->launches; }
   }
-  auto launch = [&](auto kern, int blocks, size_t bytes, int threads = TILE) -> rbc3d_status {
+  auto launch = [&](auto kern, int blocks, size_t bytes, size_t most, int threads = TILE) -> rbc3d_status {
     // (static and dynamic shared memory together may pass the 48 KB that need no opt-in)
-    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    CUDA_TRY(smem_opt_in(kern, bytes, most));
     kern<<<blocks, threads, bytes, ctx->st>>>(a);
     ++ctx->launches;
     CUDA_TRY(cudaGetLastError());
@@ -1503,16 +1504,16 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
   auto pairs = [&](auto R, auto SL, auto DL) -> rbc3d_status {
     using T = decltype(R);
     const size_t bytes = TILE / 32 * warp_tile_bytes<T, SL.value, DL.value>();
-    if (t.sub == 4 && t.n <= (sizeof(T) == 8 ? PAIR_SPLIT_MAX64 : PAIR_SPLIT_MAX32)) return launch(k_pair<T, SL.value, DL.value, 4, 4>, t.nunits, bytes);
-    if (t.sub == 4) return launch(k_pair<T, SL.value, DL.value, 4, 1>, nb, bytes);
-    if (t.sub == 2) return launch(k_pair<T, SL.value, DL.value, 2, 1>, nb, bytes);
-    return launch(k_pair<T, SL.value, DL.value, 1, 1>, nb, bytes);
+    if (t.sub == 4 && t.n <= (sizeof(T) == 8 ? PAIR_SPLIT_MAX64 : PAIR_SPLIT_MAX32)) return launch(k_pair<T, SL.value, DL.value, 4, 4>, t.nunits, bytes, bytes);
+    if (t.sub == 4) return launch(k_pair<T, SL.value, DL.value, 4, 1>, nb, bytes, bytes);
+    if (t.sub == 2) return launch(k_pair<T, SL.value, DL.value, 2, 1>, nb, bytes, bytes);
+    return launch(k_pair<T, SL.value, DL.value, 1, 1>, nb, bytes, bytes);
   };
   auto own_pairs = [&](auto R, auto SL, auto DL) -> rbc3d_status {
     const int blocks = (int)own_blocks(own_tile);
-    if (sizeof(R) == 4) return launch(k_pair_own32<SL.value, DL.value>, blocks, own_sm);
-    if (own_tile == 32) return launch(k_pair_own64<SL.value, DL.value, 32>, blocks, own_sm, 32);
-    return launch(k_pair_own64<SL.value, DL.value, OWN_TILE>, blocks, own_sm);
+    if (sizeof(R) == 4) return launch(k_pair_own32<SL.value, DL.value>, blocks, own_sm, OWN_MASK_MAX);
+    if (own_tile == 32) return launch(k_pair_own64<SL.value, DL.value, 32>, blocks, own_sm, OWN_MASK_MAX, 32);
+    return launch(k_pair_own64<SL.value, DL.value, OWN_TILE>, blocks, own_sm, OWN_MASK_MAX);
   };
   const std::true_type yes{};
   const std::false_type no{};

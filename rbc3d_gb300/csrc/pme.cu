@@ -732,12 +732,12 @@ rbc3d_status launch_spread_p(rbc3d_ctx* ctx, const SpreadArgs& a, const SpreadPl
   // warps (3-plane groups) per launch: as many as the 227 KB of shared memory hold
   const int gfirst = a.sl ? 0 : 1, glast = a.dl ? 4 : 1;
   int per = glast - gfirst;
-  while (per > 1 && spread_smem_bytes(t.B, per, sizeof(R)) > 227 * 1024) --per;
+  while (per > 1 && spread_smem_bytes(t.B, per, sizeof(R)) > SMEM_BLOCK) --per;
   for (int g = gfirst; g < glast; g += per) {
     const int nw = std::min(per, glast - g);
     t.c0 = 3 * g;
     const size_t bytes = spread_smem_bytes(t.B, nw, sizeof(R));
-    CUDA_TRY(cudaFuncSetAttribute(k_spread_tile<R, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    CUDA_TRY(smem_opt_in(k_spread_tile<R, PT>, bytes));
     { k_spread_tile<R, PT><<<pl.nchunk, 32 * nw, bytes, ctx->st>>>(a, t, pl.perm.p, pl.chunk.p, grid); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
   }

@@ -632,7 +632,7 @@ rbc3d_status run_self_ff(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
     return sizeof(float4) * 4 * np * cols + sizeof(FFCell) * G + sizeof(float2) * 9 * cols;
   };
   // a ring wider than shared memory holds (about 500 columns) goes to the FP64 patch
-  if (smem(1) > 227 * 1024) return run_self_corr(ctx, tlist, sl ? c1 : 0., dl ? c2 : 0.);
+  if (smem(1) > SMEM_BLOCK) return run_self_corr(ctx, tlist, sl ? c1 : 0., dl ? c2 : 0.);
   // records this call reads: x always, f for SL, g and a3 for DL
   rbc3d_status s = self_ff_records(ctx, 1 | (sl ? 2 : 0) | (dl ? 4 | 8 : 0));
   if (s) return s;
@@ -657,7 +657,7 @@ rbc3d_status run_self_ff(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   a.parts = ring_parts(a.NC, blocks, nsm);
   const size_t bytes = smem(a.G);
   auto launch = [&](auto kern) -> rbc3d_status {
-    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    CUDA_TRY(smem_opt_in(kern, bytes));
     kern<<<blocks * a.parts, thr, bytes, ctx->st>>>(a);
     ++ctx->launches;
     CUDA_TRY(cudaGetLastError());

@@ -372,7 +372,7 @@ rbc3d_status run_self_mixed(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
     return sizeof(float4) * 2 * 3 * cols + sizeof(float2) * 9 * cols;
   };
   // a ring wider than shared memory holds (about 1,300 columns) goes to the FP64 patch
-  if (smem(1) > 227 * 1024) return run_self_corr(ctx, tlist, sl ? c1 : 0., dl ? c2 : 0.);
+  if (smem(1) > SMEM_BLOCK) return run_self_corr(ctx, tlist, sl ? c1 : 0., dl ? c2 : 0.);
   // FP32 node records of the current geometry and densities (bit 0 geometry, 1 f, 2 g)
   const size_t per = 4 * (size_t)ctx->m * ctx->nlon * MIX_ROW;
   if (!ctx->mix_rec.p || ctx->mix_rec.n < ctx->ncell * per) {
@@ -409,7 +409,7 @@ rbc3d_status run_self_mixed(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   a.parts = ring_parts(a.NC, blocks, nsm);
   const size_t bytes = smem(a.G);
   auto launch = [&](auto kern) -> rbc3d_status {
-    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    CUDA_TRY(smem_opt_in(kern, bytes));
     kern<<<blocks * a.parts, thr, bytes, ctx->st>>>(a);
     ++ctx->launches;
     CUDA_TRY(cudaGetLastError());

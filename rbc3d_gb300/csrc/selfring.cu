@@ -85,7 +85,9 @@ __global__ void __launch_bounds__(128) k_ring_rec(int m, int n, const double* __
   }
 }
 
-template <bool SL, bool DL>
+// FEW: the form for few points, the same code with another shared-memory split
+// (a kernel's split is the process's, as its opt-in: run_self_ring).
+template <bool SL, bool DL, bool FEW>
 __global__ void __launch_bounds__(256, 1) k_self_ring(RingArgs a) {
   constexpr int NV = 3 + (SL ? 3 : 0) + (DL ? 6 : 0);  // x, f, g, a3
   constexpr int OF = 3, OG = 3 + (SL ? 3 : 0), OA = OG + 3;
@@ -294,20 +296,21 @@ rbc3d_status run_self_ring(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   a.th = ctx->th.p; a.phi = ctx->phi.p; a.tA = t.Acoef.p; a.v = t.v.p; a.celltype = ctx->celltype.p; a.Bc = ctx->dBcoef.p;
   a.T = ctx->T;
   a.c1 = c1; a.c2 = c2;
+  // few points: the pair kernels' shared-memory split of the SM, as no block
+  // of another split starts beside this one (3 cells of 12 x 24: matvec 661 ->
+  // 459 us, of 14 x 28 841 -> 617; of 25 x 50 1224 -> 1281, where the L1 counts)
+  const bool few = t.n <= 2000;
   auto launch = [&](auto kern, int nv) -> rbc3d_status {
     const size_t bytes = sizeof(double) * (size_t)thr * (2 * nv + 9);
-    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    // few points: the pair kernels' shared-memory split of the SM, as no block
-    // of another split starts beside this one (3 cells of 12 x 24: matvec 661 ->
-    // 459 us, of 14 x 28 841 -> 617; of 25 x 50 1224 -> 1281, where the L1 counts)
-    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                  t.n <= 2000 ? cudaSharedmemCarveoutMaxShared : cudaSharedmemCarveoutDefault));
+    CUDA_TRY(smem_opt_in(kern, bytes));
+    if (few)
+      CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     kern<<<blocks * a.parts, thr, bytes, ctx->st>>>(a);
     ++ctx->launches;
     CUDA_TRY(cudaGetLastError());
     return RBC3D_OK;
   };
-  if (sl && dl) return launch(k_self_ring<true, true>, 12);
-  if (sl) return launch(k_self_ring<true, false>, 6);
-  return launch(k_self_ring<false, true>, 9);
+  if (sl && dl) return few ? launch(k_self_ring<true, true, true>, 12) : launch(k_self_ring<true, true, false>, 12);
+  if (sl) return few ? launch(k_self_ring<true, false, true>, 6) : launch(k_self_ring<true, false, false>, 6);
+  return few ? launch(k_self_ring<false, true, true>, 9) : launch(k_self_ring<false, true, false>, 9);
 }

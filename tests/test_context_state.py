@@ -1,11 +1,12 @@
 """What one context or call leaves behind for the next."""
 import math
+import threading
 
 import numpy as np
 import pytest
 
 from rbc3d_gb300 import geometry as G
-from rbc3d_gb300.abi import Context
+from rbc3d_gb300.abi import FP32D, FP32M, FP64, TERM_ALL, TLIST_RBC, Context
 
 pytestmark = pytest.mark.gpu
 C = 1 / (4 * math.pi)
@@ -35,3 +36,50 @@ def test_second_grid_on_one_context(gpu, warp):
     for a, b in zip(*geom):
         assert np.array_equal(a, b)  # the same tables, the same kernel
 
+
+
+def test_larger_grid_after_a_smaller_one(gpu):
+    """The shared-memory limit of a kernel is the process's: a context of a
+    smaller grid leaves it where a larger one needs it."""
+    L = 14.0
+    ctx, geom = [], []
+    for nlat, nlon in ((36, 72), (33, 66)):
+        cells = G.make_cells(np.random.default_rng(2), 1, [L] * 3, 3.2, nlat=nlat, nlon=nlon)
+        c = Context(gpu, params(L, nlat, nlon))
+        c.set_cell_grid(cells.th, cells.phi, cells.w)
+        geom.append(c.cell_geometry(cells.x, 1))
+        ctx.append((c, cells))
+    c, cells = ctx[0]
+    for a, b in zip(c.cell_geometry(cells.x, 1), geom[0]):
+        assert np.array_equal(a, b)
+    for c, _ in ctx:
+        c.close()
+
+
+def test_grids_in_two_threads(gpu):
+    """A context per host thread, each of another grid, whose kernels take
+    other amounts of shared memory: every call of both succeeds."""
+    L, failed = 14.0, []
+
+    def work(nlat, nlon):
+        try:
+            cells = G.make_cells(np.random.default_rng(nlat), 2, [L] * 3, 3.2, nlat=nlat, nlon=nlon, with_g=True)
+            c = Context(gpu, params(L, nlat, nlon))
+            c.set_cells(cells)
+            c.set_cell_density(f=cells.f, g=cells.g, spl_F=cells.spl_F, spl_G=cells.spl_G)
+            ref = {p: c.matvec(TLIST_RBC, C, C, TERM_ALL, p) for p in (FP64, FP32D, FP32M)}
+            for _ in range(40):
+                for p, r in ref.items():
+                    v = c.matvec(TLIST_RBC, C, C, TERM_ALL, p)
+                    # the atomics' order: of FP64 sums, and of FP32 mesh sums (test_few_points)
+                    assert np.linalg.norm(v - r) <= (1e-13 if p == FP64 else 2e-6) * np.linalg.norm(r)
+            c.close()
+        except Exception as e:
+            failed.append((nlat, e))
+
+    threads = [threading.Thread(target=work, args=g) for g in ((12, 24), (25, 50))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
