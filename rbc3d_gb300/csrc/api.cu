@@ -347,6 +347,19 @@ rbc3d_status rbcs_dev(rbc3d_ctx* ctx, int which, double c1, double c2, int prec,
 
 }  // namespace
 
+// A matvec that fails leaves nothing in flight beside the main stream: what runs
+// there reads sources and densities that the next call may replace.
+struct SideDrain {
+  rbc3d_ctx* ctx;
+  bool armed;
+  ~SideDrain() {
+    if (!armed) return;
+    cudaStreamSynchronize(ctx->st2);
+    cudaStreamSynchronize(ctx->st3);
+    cudaStreamSynchronize(ctx->st4);
+  }
+};
+
 // Composite device-resident matvec used by the ABI calls (defined here so the
 // wall solver can call it too).
 rbc3d_status matvec_dev(rbc3d_ctx* ctx, int which, double c1, double c2, unsigned terms, int prec) {
@@ -377,15 +390,10 @@ rbc3d_status matvec_dev(rbc3d_ctx* ctx, int which, double c1, double c2, unsigne
   const bool late = side && rbc && late_patch(prec);
   const bool self_side = side && rbc && !late;
   const bool pme_side = !rbc || prec != RBC3D_FP32C;
+  SideDrain drain{ctx, side};
   if (side && (s = fork_side(ctx, which, c1, c2, terms, prec, self_side, pme_side))) return s;
   if (terms & (RBC3D_TERM_REAL | RBC3D_TERM_CORR | RBC3D_TERM_LINEAR))
-    if ((s = rbcs_dev(ctx, which, c1, c2, prec, terms, self_side, late))) {
-      if (side) {  // leave nothing in flight beside the main stream
-        cudaStreamSynchronize(ctx->st2);
-        cudaStreamSynchronize(ctx->st4);
-      }
-      return s;
-    }
+    if ((s = rbcs_dev(ctx, which, c1, c2, prec, terms, self_side, late))) return s;
   if (terms & RBC3D_TERM_WALLS) {
     StageScope sc(ctx, 4);
     if (which == RBC3D_TLIST_WALL) { if ((s = run_wall_self(ctx, c1))) return s; }
@@ -402,6 +410,7 @@ rbc3d_status matvec_dev(rbc3d_ctx* ctx, int which, double c1, double c2, unsigne
   } else if (terms & RBC3D_TERM_PME) {
     if ((s = pme_stages(ctx, which, c1, c2, terms, prec))) return s;
   }
+  drain.armed = false;
   return RBC3D_OK;
 }
 

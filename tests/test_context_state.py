@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from rbc3d_gb300 import geometry as G
-from rbc3d_gb300.abi import FP32D, FP32M, FP64, TERM_ALL, TLIST_RBC, Context
+from rbc3d_gb300.abi import FP32C, FP32D, FP32M, FP64, TERM_ALL, TLIST_RBC, TLIST_WALL, Context, RBC3DError
 
 pytestmark = pytest.mark.gpu
 C = 1 / (4 * math.pi)
@@ -83,3 +83,36 @@ def test_grids_in_two_threads(gpu):
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+@pytest.mark.parametrize("prec", [FP64, FP32C])
+def test_cells_replaced_after_a_failed_matvec(gpu, prec):
+    """A wall-list matvec before prepare_sing_int_on_wall is refused with the
+    mesh part already under way; cells and densities replaced right after it
+    give a fresh context's velocities."""
+    L = 14.0
+    wall = G.make_tube(5.0, L, 16, 8, (7.0, 7.0))
+    rng = np.random.default_rng(4)
+    first, second = (G.make_cells(rng, n, [L] * 3, 2.8, with_g=True) for n in (12, 3))
+    fw = rng.normal(size=(3, wall.nvert))
+    out = []
+    for fails in (20, 0):
+        c = Context(gpu, params(L, 25, 50))
+        for k in range(max(fails, 1)):
+            if fails:
+                c.set_cells(first)
+                c.set_cell_density(f=first.f, g=first.g, spl_F=first.spl_F, spl_G=first.spl_G)
+            c.set_walls(wall)
+            c.set_wall_density(fw)
+            if fails:
+                with pytest.raises(RBC3DError) as e:
+                    c.matvec(TLIST_WALL, C, C, TERM_ALL, prec)
+                assert e.value.code == 6  # ERR_STATE
+            c.set_cells(second)
+            c.set_cell_density(f=second.f, g=second.g, spl_F=second.spl_F, spl_G=second.spl_G)
+            v = c.matvec(TLIST_RBC, C, C, TERM_ALL, prec)
+            out.append(v)
+        c.close()
+    for v in out[:-1]:
+        # the atomics' order, as test_grids_in_two_threads
+        assert np.linalg.norm(v - out[-1]) <= (1e-13 if prec == FP64 else 2e-6) * np.linalg.norm(out[-1])
