@@ -106,6 +106,7 @@ struct PmeState {
   DBuf<double2> infl64;
   DBuf<float> wave32;
   DBuf<double> wave64;
+  bool infl32_built = false, infl64_built = false;
   cufftHandle r2c32_3 = 0, r2c32_12 = 0, c2r32_3 = 0;
   cufftHandle r2c64_3 = 0, r2c64_12 = 0, c2r64_3 = 0;
   bool planned32 = false, planned64 = false;

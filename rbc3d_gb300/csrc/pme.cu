@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "ctx.hpp"
+#include "once.hpp"
 
 namespace {
 
@@ -853,10 +854,13 @@ rbc3d_status pme_transform(rbc3d_ctx* ctx) {
     CUDA_TRY(P.spec32.alloc(12 * P.GC)); CUDA_TRY(P.vspec32.alloc(3 * P.GC)); CUDA_TRY(P.vel32.alloc(3 * P.G));
     if (P.dl) { if (cufftExecR2C(P.r2c32_12, P.grid32.p, (cufftComplex*)P.spec32.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecR2C"); }
     else if (cufftExecR2C(P.r2c32_3, P.grid32.p, (cufftComplex*)P.spec32.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecR2C");
-    if (!P.infl32.p) {
+    const rbc3d_status s = build_once(P.infl32_built, [&]() -> rbc3d_status {
       CUDA_TRY(P.infl32.alloc(P.GC)); CUDA_TRY(P.wave32.alloc(nwave));
       { k_influence_table<float><<<nblk(std::max(P.GC, nwave), 256), 256, 0, ctx->st>>>(a, P.infl32.p, P.wave32.p); ++ctx->launches; }
-    }
+      CUDA_TRY(cudaGetLastError());
+      return RBC3D_OK;
+    });
+    if (s) return s;
     { k_influence<float, float2><<<nblk(P.GC, 256), 256, 0, ctx->st>>>(a, P.infl32.p, P.wave32.p, P.spec32.p, P.vspec32.p); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
     if (cufftExecC2R(P.c2r32_3, (cufftComplex*)P.vspec32.p, P.vel32.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecC2R");
@@ -864,10 +868,13 @@ rbc3d_status pme_transform(rbc3d_ctx* ctx) {
     CUDA_TRY(P.spec64.alloc(12 * P.GC)); CUDA_TRY(P.vspec64.alloc(3 * P.GC)); CUDA_TRY(P.vel64.alloc(3 * P.G));
     if (P.dl) { if (cufftExecD2Z(P.r2c64_12, P.grid64.p, (cufftDoubleComplex*)P.spec64.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecD2Z"); }
     else if (cufftExecD2Z(P.r2c64_3, P.grid64.p, (cufftDoubleComplex*)P.spec64.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecD2Z");
-    if (!P.infl64.p) {
+    const rbc3d_status s = build_once(P.infl64_built, [&]() -> rbc3d_status {
       CUDA_TRY(P.infl64.alloc(P.GC)); CUDA_TRY(P.wave64.alloc(nwave));
       { k_influence_table<double><<<nblk(std::max(P.GC, nwave), 256), 256, 0, ctx->st>>>(a, P.infl64.p, P.wave64.p); ++ctx->launches; }
-    }
+      CUDA_TRY(cudaGetLastError());
+      return RBC3D_OK;
+    });
+    if (s) return s;
     { k_influence<double, double2><<<nblk(P.GC, 256), 256, 0, ctx->st>>>(a, P.infl64.p, P.wave64.p, P.spec64.p, P.vspec64.p); ++ctx->launches; }
     CUDA_TRY(cudaGetLastError());
     if (cufftExecZ2D(P.c2r64_3, (cufftDoubleComplex*)P.vspec64.p, P.vel64.p)) return ctx_fail(ctx, RBC3D_ERR_CUDA, "cufftExecZ2D");
