@@ -35,15 +35,6 @@ struct Tables {
   long long eps2b, rc2b;
 };
 
-// 1/sqrt(x) for a positive, normal x: the hardware's approximation and one
-// step of third order (y <- y + y e (1/2 + 3/8 e), e = 1 - x y^2).
-__device__ __forceinline__ double rsqrt_step(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // EwaldCoeff_SL / EwaldCoeff_DL (ModEwaldFunc.F90:86-180) from a squared
 // distance: EA, EB, ED with v = EA (x.f) x + EB f + ED (x.g)(x.n) x.  False where
 // they are zero or not evaluated: below r_eps, from rc on, NaN (positive
@@ -53,7 +44,7 @@ template <bool SL, bool DL>
 __device__ __forceinline__ bool ewald_coef64(const Tables& T, double r2, double& EA, double& EB, double& ED) {
   const long long bits = __double_as_longlong(r2);
   if (bits < T.eps2b || bits >= T.rc2b) return false;
-  const double ir = rsqrt_step(r2), rr = r2 * ir;
+  const double ir = rsqrt(r2), rr = r2 * ir;
   const double magic = 6755399441055744.0;
   const double ft = __fma_rd(rr, T.ntab_over_rc, magic);
   const int it = __double2loint(ft);

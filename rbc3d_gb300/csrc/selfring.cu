@@ -21,8 +21,8 @@
 // threads meet).
 //
 // Bound by the FP64 pipe (2 lanes a clock and SM): about 140 FP64
-// instructions a patch point, against about 350 (counting conversions and the
-// library's rsqrt) with one warp per target and 16-term interpolations.  256
+// instructions a patch point, against about 350 (counting conversions) with one
+// warp per target and 16-term interpolations.  256
 // cells, SL+DL, inside the FP32C matvec: 46.1 -> 19.6 ms, the matvec 46.5 ->
 // 20.1.  The node values are kept per row in column
 // order (rec, built when positions or densities change), so that a warp reads
