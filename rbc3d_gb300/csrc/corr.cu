@@ -71,8 +71,8 @@ __device__ __forceinline__ const double* set_ptr(const CorrArgs& a, int cell, in
   return a.spl + ((size_t)cell * SPL_NSET + set) * (size_t)a.m * a.nlon * SPL_NODE;
 }
 
-// RBC_SingInt on any longitude grid: one warp per cell target (uniform grids
-// of up to RING_MAX_NLON columns: selfring.cu)
+// RBC_SingInt on any longitude grid: one warp per cell target (uniform grids:
+// selfring.cu)
 __global__ void __launch_bounds__(256) k_self(CorrArgs a) {
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
@@ -1005,7 +1005,7 @@ rbc3d_status run_self_corr(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   CorrArgs a;
   fill_args(ctx, tlist, c1, (c2 != 0 && ctx->has_g) ? c2 : 0.0, a, Bc);
   if (c1 != 0 && !ctx->has_f) a.c1 = 0;
-  if (ctx->phi_uniform && ctx->nlon <= RING_MAX_NLON) return run_self_ring(ctx, tlist, a.c1, a.c2);
+  if (ctx->phi_uniform) return run_self_ring(ctx, tlist, a.c1, a.c2);
   long long threads = (long long)t.n * 32;
   { k_self<<<(int)((threads + 255) / 256), 256, 0, ctx->st>>>(a); ++ctx->launches; }
   CUDA_TRY(cudaGetLastError());

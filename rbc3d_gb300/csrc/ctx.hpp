@@ -372,11 +372,13 @@ rbc3d_status wall_spec_add_dev(rbc3d_ctx* ctx, const double* b_dev, const double
 rbc3d_status wall_spec_apply_dev(rbc3d_ctx* ctx, const double* v_dev, double* out_dev);
 void wall_spec_release(rbc3d_ctx* ctx);
 
-// selfring.cu: the FP64 patch by latitude rings (uniform longitudes, nlon <= RING_MAX_NLON)
+// selfring.cu: the FP64 patch by latitude rings (uniform longitudes; more than
+// RING_MAX_NLON columns, a block's threads, go by segments of a ring)
 constexpr int RING_MAX_NLON = 256;
 std::vector<RingClass> ring_classes(const rbc3d_ctx* ctx, const std::vector<double>& thG,
                                     const std::vector<double>& phiA, const std::vector<double>& pw);
 int ring_cells(int ncell, int nlon);                  // cells of one block
+int ring_segment(int nlon, int most);                 // targets of one block of a wide ring
 int ring_parts(int classes, int blocks, int nsm);     // blocks that share a ring's classes
 rbc3d_status self_ring_grid(rbc3d_ctx* ctx, const std::vector<RingClass>& C);
 rbc3d_status self_ring_tables(rbc3d_ctx* ctx, const std::vector<double>& c1, const std::vector<double>& c2,

@@ -56,6 +56,9 @@
 namespace {
 
 constexpr int FF_ROW = 12;   // 32-byte entries of a node: 4 slots x 3 quads
+// Targets of a ring segment's block: 44 KB of shared memory, five blocks of three
+// warps an SM (63 and 127 targets within 3 % of it at 260 to 1,000 columns)
+constexpr int FF_SEG = 95;
 
 // A class of patch points (RingClass) in hi/lo parts, each weight as the
 // operands (h, h, l, l): the theta weights of (u, u', u_th, u'_th), per side
@@ -135,6 +138,7 @@ struct FFArgs {
   ff c1;                // c1
   ff c2B[RBC3D_MAX_CELLTYPES];  // c2 Bcoef per cell type
   ff rc2, r_eps, ntab_over_rc;
+  int seg, segs;        // targets of a ring segment's block, blocks a ring
 };
 
 // float-float arithmetic on two points at once (packed FP32x2)
@@ -334,36 +338,50 @@ __device__ __forceinline__ void patch_points(const FFArgs& a, const Dot2* A, con
 // then every column evaluates the points in the interval [j, j + 1]: of the
 // targets j - j[0] and j - j[1] (mod nlon), whose sums lie in shared memory, a
 // side each, so no two threads meet between two barriers.
-template <bool SL, bool DL>
-__global__ void __launch_bounds__(256, 2) k_self_ff(FFArgs a) {
+// WIDE: a segment of the targets of one cell's ring, thread = target; the theta
+// parts of a class are of the columns that these targets' points fall into, for
+// each side apart (so each twice in a ring).
+template <bool SL, bool DL, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? FF_SEG + 1 : 256, WIDE ? 5 : 2) k_self_ff(FFArgs a) {
   constexpr int NP = DL ? (SL ? 6 : 5) : 3;  // pairs kept; without SL the pair (f.y f.z) is left out
   extern __shared__ __align__(16) unsigned char smem_ff[];
-  const int nlon = a.nlon, cols = a.G * nlon;
-  float4* ex = reinterpret_cast<float4*>(smem_ff);            // [2][NP][U, D][cols]: (s, s, c, c)
-  FFCell* sC = reinterpret_cast<FFCell*>(ex + (size_t)4 * NP * cols);  // [G]
-  float2* acc = reinterpret_cast<float2*>(sC + a.G);          // [2 sides][3][cols]
-  float2* sT = acc + 6 * cols;                                // [3][cols] target positions
+  const int nlon = a.nlon, cols = WIDE ? 2 * (a.seg + 1) : a.G * nlon, ntg = WIDE ? a.seg : cols;
+  float4* ex = reinterpret_cast<float4*>(smem_ff);            // [2, WIDE 1][NP][U, D][cols]: (s, s, c, c)
+  FFCell* sC = reinterpret_cast<FFCell*>(ex + (size_t)(WIDE ? 2 : 4) * NP * cols);  // [G]
+  float2* acc = reinterpret_cast<float2*>(sC + a.G);          // [2 sides][3][ntg]
+  float2* sT = acc + 6 * ntg;                                 // [3][ntg] target positions
   int b = blockIdx.x;
   const int part = b % a.parts; b /= a.parts;
+  const int q0 = WIDE ? b % a.segs * a.seg : 0;               // the first target
+  if (WIDE) b /= a.segs;
   const int ring = b % a.nlat, cell0 = (b / a.nlat) * a.G;
-  const int ncl = min(a.G, a.ncell - cell0), ncol = ncl * nlon;
+  const int ncl = min(a.G, a.ncell - cell0), ncol = WIDE ? min(a.seg, nlon - q0) : ncl * nlon;
   const int nv = a.nlat * nlon;
   for (int t = threadIdx.x; t < ncl; t += blockDim.x) cell_offsets(a, cell0 + t, sC[t]);
   for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
-    const int lc = t / nlon, j = t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
+    const int lc = WIDE ? 0 : t / nlon, j = q0 + t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
     const float4 h = a.thi[p], l = a.tlo[p];
-    sT[t] = make_float2(h.x, l.x); sT[cols + t] = make_float2(h.y, l.y); sT[2 * cols + t] = make_float2(h.z, l.z);
-    for (int k = 0; k < 6; ++k) acc[k * cols + t] = make_float2(0.f, 0.f);
+    sT[t] = make_float2(h.x, l.x); sT[ntg + t] = make_float2(h.y, l.y); sT[2 * ntg + t] = make_float2(h.z, l.z);
+    for (int k = 0; k < 6; ++k) acc[k * ntg + t] = make_float2(0.f, 0.f);
   }
   __syncthreads();
   const int k0 = (int)((long long)a.NC * part / a.parts), k1 = (int)((long long)a.NC * (part + 1) / a.parts);
   const FFClass* cls = a.cls + (size_t)ring * a.NC;
   for (int k = k0; k < k1; ++k) {
     const FFClass& c = cls[k];
-    float4* buf = ex + (size_t)((k & 1) * NP * 2) * cols;
+    float4* buf = WIDE ? ex : ex + (size_t)((k & 1) * NP * 2) * cols;
     const int i1 = c.i1, i2 = i1 + 1 == a.m ? 0 : i1 + 1;
-    for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
-      const int lc = t / nlon, j = t - lc * nlon;
+    if (WIDE) __syncthreads();  // the previous class's values are done with
+    for (int t = threadIdx.x; t < (WIDE ? 2 * (ncol + 1) : ncol); t += blockDim.x) {
+      int lc = 0, j;
+      if (WIDE) {
+        const int side = t > ncol;
+        j = q0 + t - side * (ncol + 1) + c.j[side];
+        if (j >= nlon) j -= nlon;
+      } else {
+        lc = t / nlon;
+        j = t - lc * nlon;
+      }
       const FFCell& C = sC[lc];
       const float4* rc = a.rec + 2 * ((size_t)(cell0 + lc) * a.m * FF_ROW * nlon + j);
       const float4 w0 = __ldg(c.x), w1 = __ldg(c.x + 1), w2 = __ldg(c.x + 2), w3 = __ldg(c.x + 3);
@@ -405,21 +423,25 @@ __global__ void __launch_bounds__(256, 2) k_self_ff(FFArgs a) {
     // nobody is past this barrier before the previous class's sums are in
     __syncthreads();
     for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
-      const int lc = t / nlon, j = t - lc * nlon, base = t - j;
-      const int tn = j + 1 == nlon ? base : t + 1;
+      const int lc = WIDE ? 0 : t / nlon, j = t - lc * nlon, base = t - j;
+      const int tn = !WIDE && j + 1 == nlon ? base : t + 1;
       const FFCell& C = sC[lc];
-      const int qa = base + (j >= c.j[0] ? j - c.j[0] : j - c.j[0] + nlon);  // the targets' columns
-      const int qb = base + (j >= c.j[1] ? j - c.j[1] : j - c.j[1] + nlon);
+      const int qa = WIDE ? t : base + (j >= c.j[0] ? j - c.j[0] : j - c.j[0] + nlon);  // the targets' columns
+      const int qb = WIDE ? t : base + (j >= c.j[1] ? j - c.j[1] : j - c.j[1] + nlon);
       Dot2 da[FF_PAIRS], db[FF_PAIRS];
 #pragma unroll
       for (int P = 0; P < FF_PAIRS; ++P) {
         if ((!DL && P >= 3) || (!SL && P == 2)) continue;
         const int S = (!SL && P > 2) ? P - 1 : P;
         const float4* o = buf + (size_t)(2 * S) * cols;
-        const float4 D0 = o[cols + t], D1 = o[cols + tn], U0 = o[t], U1 = o[tn];
+        float4 D0 = o[cols + t], D1 = o[cols + tn], U0 = o[t], U1 = o[tn];
         const float2 off = C.p[P];
 #pragma unroll
         for (int side = 0; side < 2; ++side) {
+          if (WIDE && side) {
+            const int u = ncol + 1 + t;
+            D0 = o[cols + u]; D1 = o[cols + u + 1]; U0 = o[u]; U1 = o[u + 1];
+          }
           const float4* y = c.y[side];
           const float4 w0 = __ldg(y), w1 = __ldg(y + 1), w2 = __ldg(y + 2), w3 = __ldg(y + 3);
           Dot2& d = side ? db[P] : da[P];
@@ -437,15 +459,15 @@ __global__ void __launch_bounds__(256, 2) k_self_ff(FFArgs a) {
           }
         }
       }
-      patch_points<SL, DL>(a, da, db, sT + qa, sT + qb, {C.c2m.x, C.c2m.y}, __ldg(&c.w), acc + qa, acc + 3 * cols + qb, cols);
+      patch_points<SL, DL>(a, da, db, sT + qa, sT + qb, {C.c2m.x, C.c2m.y}, __ldg(&c.w), acc + qa, acc + 3 * ntg + qb, ntg);
     }
   }
   __syncthreads();
   for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
-    const int lc = t / nlon, j = t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
+    const int lc = WIDE ? 0 : t / nlon, j = q0 + t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
     const double iA = 1.0 / a.tA[p];
     for (int k = 0; k < 3; ++k) {
-      const float2 z0 = acc[k * cols + t], z1 = acc[(3 + k) * cols + t];
+      const float2 z0 = acc[k * ntg + t], z1 = acc[(3 + k) * ntg + t];
       const double dv = (((double)z0.x + (double)z1.x) + ((double)z0.y + (double)z1.y)) * iA;
       if (a.parts == 1) a.v[p + (size_t)k * a.nt] += dv;
       else atomicAdd(a.v + p + (size_t)k * a.nt, dv);
@@ -627,12 +649,6 @@ rbc3d_status run_self_ff(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   const bool sl = c1 != 0 && ctx->has_f, dl = c2 != 0 && ctx->has_g;
   if (!sl && !dl) return RBC3D_OK;
   const int np = dl ? (sl ? 6 : 5) : 3;
-  auto smem = [&](int G) {
-    const size_t cols = (size_t)G * ctx->nlon;
-    return sizeof(float4) * 4 * np * cols + sizeof(FFCell) * G + sizeof(float2) * 9 * cols;
-  };
-  // a ring wider than shared memory holds (about 500 columns) goes to the FP64 patch
-  if (smem(1) > SMEM_BLOCK) return run_self_corr(ctx, tlist, sl ? c1 : 0., dl ? c2 : 0.);
   // records this call reads: x always, f for SL, g and a3 for DL
   rbc3d_status s = self_ff_records(ctx, 1 | (sl ? 2 : 0) | (dl ? 4 | 8 : 0));
   if (s) return s;
@@ -652,10 +668,22 @@ rbc3d_status run_self_ff(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
   a.NC = ctx->nrad * (ctx->nazm / 2 + 1);
-  a.G = ring_cells(ctx->ncell, ctx->nlon);
-  const int blocks = (ctx->ncell + a.G - 1) / a.G * ctx->nlat, thr = std::min(256, (a.G * ctx->nlon + 31) / 32 * 32);
+  // A ring of more columns than threads goes by segments, unless it fits in
+  // shared memory (498 columns) and leaves few threads without a second column
+  // (us, whole ring / segments: 4 cells of 16 x 260 706 / 670, 16 x 300 774 /
+  // 749, 2 cells of 40 x 264 1470 / 1310, of 16 x 480 665 / 692).  Over that it
+  // went to the FP64 patch: 2 cells of 16 x 520 2165 -> 775, of 16 x 1000 5115 -> 2410.
+  const size_t column = sizeof(float4) * 4 * np + sizeof(float2) * 9;
+  const bool wide = ctx->nlon > RING_MAX_NLON &&
+                    (ctx->nlon < 432 || column * ctx->nlon + sizeof(FFCell) > SMEM_BLOCK);
+  a.G = wide ? 1 : ring_cells(ctx->ncell, ctx->nlon);
+  a.seg = wide ? ring_segment(ctx->nlon, FF_SEG) : 0;
+  a.segs = wide ? (ctx->nlon + a.seg - 1) / a.seg : 1;
+  const int blocks = (ctx->ncell + a.G - 1) / a.G * ctx->nlat * a.segs;
+  const int thr = std::min(256, ((wide ? a.seg + 1 : a.G * ctx->nlon) + 31) / 32 * 32);
   a.parts = ring_parts(a.NC, blocks, nsm);
-  const size_t bytes = smem(a.G);
+  const size_t cols = wide ? a.seg : a.G * ctx->nlon, ent = wide ? 2 * (a.seg + 1) : 2 * cols;  // (both buffers)
+  const size_t bytes = sizeof(float4) * 2 * np * ent + sizeof(FFCell) * a.G + sizeof(float2) * 9 * cols;
   auto launch = [&](auto kern) -> rbc3d_status {
     CUDA_TRY(smem_opt_in(kern, bytes));
     kern<<<blocks * a.parts, thr, bytes, ctx->st>>>(a);
@@ -663,7 +691,7 @@ rbc3d_status run_self_ff(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
     CUDA_TRY(cudaGetLastError());
     return RBC3D_OK;
   };
-  if (sl && dl) return launch(k_self_ff<true, true>);
-  if (sl) return launch(k_self_ff<true, false>);
-  return launch(k_self_ff<false, true>);
+  if (sl && dl) return wide ? launch(k_self_ff<true, true, true>) : launch(k_self_ff<true, true, false>);
+  if (sl) return wide ? launch(k_self_ff<true, false, true>) : launch(k_self_ff<true, false, false>);
+  return wide ? launch(k_self_ff<false, true, true>) : launch(k_self_ff<false, true, false>);
 }

@@ -22,6 +22,7 @@
 // 1.72 ms alone (two blocks an SM 1.82).  With the theta part for the positions
 // and normals too, relative to the ring's target, 1.41 ms, but outputs 1.3e-7
 // from these by rounding alone.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -35,6 +36,7 @@ inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 // x hi(3) lo(3), a3(3), then u_th, u_ph, u_thph of x (9) and of a3 (9), pad;
 // from quad 7 on f and g (6 floats) of the slots u, u_th, u_ph, u_thph.
 constexpr int MIX_ROW = 13, MIX_XA = 7;
+constexpr int MIX_SEG = 127;  // targets of a ring segment's block
 
 // A class of patch points (RingClass): theta weights of (u, u', u_th, u'_th);
 // per side the phi weights of (U_j, U_j+1, D_j, D_j+1) and, per stencil node
@@ -147,28 +149,31 @@ struct MixArgs {
   float c1, c2;
   float rc2, sqpa, two_isqa, m8_ispi, q75_spi;
   float erfcx_q[ERFCX_DEG + 1];
+  int seg, segs;  // as FFArgs (selfff.cu)
 };
 
 // One block: a ring of G cells, thread = column (cols = G nlon; more than 256
 // columns: several a thread).  One barrier a class: the densities' theta parts
 // alternate between two buffers; the targets' sums lie in shared memory, a side
-// each, so no two threads meet between two barriers.
-template <bool SL, bool DL>
-__global__ void __launch_bounds__(256, 3) k_self_mix(MixArgs a) {
+// each, so no two threads meet between two barriers.  WIDE: a segment of the targets of one cell's ring, as k_self_ff.
+template <bool SL, bool DL, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? MIX_SEG + 1 : 256, WIDE ? 5 : 3) k_self_mix(MixArgs a) {
   extern __shared__ __align__(16) unsigned char smem_mix[];
-  const int nlon = a.nlon, cols = a.G * nlon;
+  const int nlon = a.nlon, cols = WIDE ? 2 * (a.seg + 1) : a.G * nlon, ntg = WIDE ? a.seg : cols;
   float4* ex = reinterpret_cast<float4*>(smem_mix);            // [2][3][cols]: (f0 f1) (f2 g0) (g1 g2) of U, D
-  float2* acc = reinterpret_cast<float2*>(ex + 2 * 3 * cols);  // [2 sides][3][cols]: Kahan sum and error
-  float2* sT = acc + 6 * cols;                                 // [3][cols]: target position hi, lo
+  float2* acc = reinterpret_cast<float2*>(ex + 2 * 3 * cols);  // [2 sides][3][ntg]: Kahan sum and error
+  float2* sT = acc + 6 * ntg;                                   // [3][ntg]: target position hi, lo
   int b = blockIdx.x;
   const int part = b % a.parts; b /= a.parts;
+  const int q0 = WIDE ? b % a.segs * a.seg : 0;                // the first target
+  if (WIDE) b /= a.segs;
   const int ring = b % a.nlat, cell0 = (b / a.nlat) * a.G;
-  const int ncol = min(a.G, a.ncell - cell0) * nlon, nv = a.nlat * nlon;
+  const int ncol = WIDE ? min(a.seg, nlon - q0) : min(a.G, a.ncell - cell0) * nlon, nv = a.nlat * nlon;
   for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
-    const int lc = t / nlon, j = t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
+    const int lc = WIDE ? 0 : t / nlon, j = q0 + t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
     const float4 h = a.thi[p], l = a.tlo[p];
-    sT[t] = make_float2(h.x, l.x); sT[cols + t] = make_float2(h.y, l.y); sT[2 * cols + t] = make_float2(h.z, l.z);
-    for (int k = 0; k < 6; ++k) acc[k * cols + t] = make_float2(0.f, 0.f);
+    sT[t] = make_float2(h.x, l.x); sT[ntg + t] = make_float2(h.y, l.y); sT[2 * ntg + t] = make_float2(h.z, l.z);
+    for (int k = 0; k < 6; ++k) acc[k * ntg + t] = make_float2(0.f, 0.f);
   }
   __syncthreads();
   const int k0 = (int)((long long)a.NC * part / a.parts), k1 = (int)((long long)a.NC * (part + 1) / a.parts);
@@ -178,8 +183,16 @@ __global__ void __launch_bounds__(256, 3) k_self_mix(MixArgs a) {
     const MixClass& c = cls[kc];
     float4* buf = ex + (size_t)((kc & 1) * 3) * cols;
     const int i1 = c.i1, i2 = i1 + 1 == a.m ? 0 : i1 + 1;
-    for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
-      const int lc = t / nlon, j = t - lc * nlon;
+    for (int t = threadIdx.x; t < (WIDE ? 2 * (ncol + 1) : ncol); t += blockDim.x) {
+      int lc = 0, j;
+      if (WIDE) {
+        const int side = t > ncol;
+        j = q0 + t - side * (ncol + 1) + c.j[side];
+        if (j >= nlon) j -= nlon;
+      } else {
+        lc = t / nlon;
+        j = t - lc * nlon;
+      }
       const float4* r1 = a.rec + (((size_t)(cell0 + lc) * a.m + i1) * MIX_ROW + MIX_XA) * nlon + j;
       const float4* r2 = a.rec + (((size_t)(cell0 + lc) * a.m + i2) * MIX_ROW + MIX_XA) * nlon + j;
       const float4 w = *reinterpret_cast<const float4*>(c.x);
@@ -202,31 +215,49 @@ __global__ void __launch_bounds__(256, 3) k_self_mix(MixArgs a) {
     }
     __syncthreads();
     for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
-      const int lc = t / nlon, j = t - lc * nlon, base = t - j, jn = j + 1 == nlon ? 0 : j + 1, tn = base + jn;
-      const int qs[2] = {base + (j >= c.j[0] ? j - c.j[0] : j - c.j[0] + nlon),
-                         base + (j >= c.j[1] ? j - c.j[1] : j - c.j[1] + nlon)};
+      // the sides' targets, columns and places of their theta parts
+      int lc = 0, qs[2] = {t, t}, js[2], jn[2], ts[2] = {t, ncol + 1 + t}, tn[2] = {t + 1, ncol + 2 + t};
+      if (WIDE) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          js[s] = q0 + t + c.j[s];
+          if (js[s] >= nlon) js[s] -= nlon;
+          jn[s] = js[s] + 1 == nlon ? 0 : js[s] + 1;
+        }
+      } else {
+        lc = t / nlon;
+        const int j = t - lc * nlon, base = t - j;
+        js[0] = js[1] = j;
+        jn[0] = jn[1] = j + 1 == nlon ? 0 : j + 1;
+        ts[1] = t;
+        tn[0] = tn[1] = base + jn[0];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) qs[s] = base + (j >= c.j[s] ? j - c.j[s] : j - c.j[s] + nlon);
+      }
       float xx[2][3], A3[2][3], FG[2][6], th_[2][3], tl_[2][3];
 #pragma unroll
       for (int s = 0; s < 2; ++s)
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          const float2 T = sT[k * cols + qs[s]];
+          const float2 T = sT[k * ntg + qs[s]];
           th_[s][k] = T.x; tl_[s][k] = T.y;
           xx[s][k] = 0.f; A3[s][k] = 0.f;
         }
       const float4* rows = a.rec + (size_t)(cell0 + lc) * a.m * MIX_ROW * nlon;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {  // the stencil nodes
-        const float4* r = rows + (size_t)(k < 2 ? i1 : i2) * MIX_ROW * nlon + (k & 1 ? jn : j);
         float v[4 * MIX_XA];
 #pragma unroll
-        for (int q = 0; q < MIX_XA; ++q) {
-          if (!DL && q >= 5) continue;  // a3's derivatives
-          const float4 u = __ldg(r + q * nlon);
-          v[4 * q] = u.x; v[4 * q + 1] = u.y; v[4 * q + 2] = u.z; v[4 * q + 3] = u.w;
-        }
-#pragma unroll
         for (int s = 0; s < 2; ++s) {
+          if (WIDE || s == 0) {  // the sides share a column unless WIDE
+            const float4* r = rows + (size_t)(k < 2 ? i1 : i2) * MIX_ROW * nlon + (k & 1 ? jn[s] : js[s]);
+#pragma unroll
+            for (int q = 0; q < MIX_XA; ++q) {
+              if (!DL && q >= 5) continue;  // a3's derivatives
+              const float4 u = __ldg(r + q * nlon);
+              v[4 * q] = u.x; v[4 * q + 1] = u.y; v[4 * q + 2] = u.z; v[4 * q + 3] = u.w;
+            }
+          }
           const float4 w = *reinterpret_cast<const float4*>(c.n[s][k]);
 #pragma unroll
           for (int e = 0; e < 3; ++e) {
@@ -241,9 +272,10 @@ __global__ void __launch_bounds__(256, 3) k_self_mix(MixArgs a) {
       }
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
-        const float4 A = buf[q * cols + t], B = buf[q * cols + tn];
+        float4 A = buf[q * cols + ts[0]], B = buf[q * cols + tn[0]];
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
+          if (WIDE && s) { A = buf[q * cols + ts[1]]; B = buf[q * cols + tn[1]]; }
           const float4 y = *reinterpret_cast<const float4*>(c.y[s]);
           FG[s][2 * q] = fmaf(y.w, B.z, fmaf(y.z, A.z, fmaf(y.y, B.x, y.x * A.x)));
           FG[s][2 * q + 1] = fmaf(y.w, B.w, fmaf(y.z, A.w, fmaf(y.y, B.y, y.x * A.y)));
@@ -281,23 +313,23 @@ __global__ void __launch_bounds__(256, 3) k_self_mix(MixArgs a) {
           const float tt = c2m * Ad * dg * da;
           v0 += tt * x[0]; v1 += tt * x[1]; v2 += tt * x[2];
         }
-        float2* z = acc + 3 * s * cols + qs[s];
+        float2* z = acc + 3 * s * ntg + qs[s];
         const float v[3] = {v0, v1, v2};
 #pragma unroll
         for (int k = 0; k < 3; ++k) {  // Kahan: (sum, error)
-          const float2 o = z[k * cols];
+          const float2 o = z[k * ntg];
           const float y = __fsub_rn(v[k], o.y), n = __fadd_rn(o.x, y);
-          z[k * cols] = make_float2(n, __fsub_rn(__fsub_rn(n, o.x), y));
+          z[k * ntg] = make_float2(n, __fsub_rn(__fsub_rn(n, o.x), y));
         }
       }
     }
   }
   __syncthreads();
   for (int t = threadIdx.x; t < ncol; t += blockDim.x) {
-    const int lc = t / nlon, j = t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
+    const int lc = WIDE ? 0 : t / nlon, j = q0 + t - lc * nlon, p = (cell0 + lc) * nv + j * a.nlat + ring;
     const double iA = 1.0 / a.tA[p];
     for (int k = 0; k < 3; ++k) {
-      const float2 z0 = acc[k * cols + t], z1 = acc[(3 + k) * cols + t];
+      const float2 z0 = acc[k * ntg + t], z1 = acc[(3 + k) * ntg + t];
       const double dv = (((double)z0.x - (double)z0.y) + ((double)z1.x - (double)z1.y)) * iA;
       if (a.parts == 1) a.v[p + (size_t)k * a.nt] += dv;
       else atomicAdd(a.v + p + (size_t)k * a.nt, dv);
@@ -367,12 +399,6 @@ rbc3d_status run_self_mixed(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   if (tlist != RBC3D_TLIST_RBC || t.n == 0 || ctx->ncell == 0) return RBC3D_OK;
   const bool sl = c1 != 0 && ctx->has_f, dl = c2 != 0 && ctx->has_g;
   if (!sl && !dl) return RBC3D_OK;
-  auto smem = [&](int G) {
-    const size_t cols = (size_t)G * ctx->nlon;
-    return sizeof(float4) * 2 * 3 * cols + sizeof(float2) * 9 * cols;
-  };
-  // a ring wider than shared memory holds (about 1,300 columns) goes to the FP64 patch
-  if (smem(1) > SMEM_BLOCK) return run_self_corr(ctx, tlist, sl ? c1 : 0., dl ? c2 : 0.);
   // FP32 node records of the current geometry and densities (bit 0 geometry, 1 f, 2 g)
   const size_t per = 4 * (size_t)ctx->m * ctx->nlon * MIX_ROW;
   if (!ctx->mix_rec.p || ctx->mix_rec.n < ctx->ncell * per) {
@@ -404,10 +430,21 @@ rbc3d_status run_self_mixed(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
   a.NC = ctx->nrad * (ctx->nazm / 2 + 1);
-  a.G = ring_cells(ctx->ncell, ctx->nlon);
-  const int blocks = (ctx->ncell + a.G - 1) / a.G * ctx->nlat, thr = std::min(256, (a.G * ctx->nlon + 31) / 32 * 32);
+  // a ring that does not fit in shared memory (about 1,300 columns) goes by
+  // segments; under that a ring of more than 256 columns, several a thread, is
+  // the faster (us, whole ring / segments: 4 cells of 16 x 260 585 / 610, 2 of
+  // 16 x 520 606 / 639, of 16 x 1000 2270 / 2270).  Over it a ring went to the
+  // FP64 patch: 1 cell of 10 x 1400 1820 -> 790.
+  constexpr size_t COLUMN = sizeof(float4) * 2 * 3 + sizeof(float2) * 9;
+  const bool wide = COLUMN * ctx->nlon > SMEM_BLOCK;
+  a.G = wide ? 1 : ring_cells(ctx->ncell, ctx->nlon);
+  a.seg = wide ? ring_segment(ctx->nlon, MIX_SEG) : 0;
+  a.segs = wide ? (ctx->nlon + a.seg - 1) / a.seg : 1;
+  const int blocks = (ctx->ncell + a.G - 1) / a.G * ctx->nlat * a.segs;
+  const int thr = std::min(256, ((wide ? a.seg + 1 : a.G * ctx->nlon) + 31) / 32 * 32);
   a.parts = ring_parts(a.NC, blocks, nsm);
-  const size_t bytes = smem(a.G);
+  const size_t cols = wide ? a.seg : a.G * ctx->nlon, ent = wide ? 2 * (a.seg + 1) : cols;
+  const size_t bytes = sizeof(float4) * 2 * 3 * ent + sizeof(float2) * 9 * cols;
   auto launch = [&](auto kern) -> rbc3d_status {
     CUDA_TRY(smem_opt_in(kern, bytes));
     kern<<<blocks * a.parts, thr, bytes, ctx->st>>>(a);
@@ -415,7 +452,7 @@ rbc3d_status run_self_mixed(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
     CUDA_TRY(cudaGetLastError());
     return RBC3D_OK;
   };
-  if (sl && dl) return launch(k_self_mix<true, true>);
-  if (sl) return launch(k_self_mix<true, false>);
-  return launch(k_self_mix<false, true>);
+  if (sl && dl) return wide ? launch(k_self_mix<true, true, true>) : launch(k_self_mix<true, true, false>);
+  if (sl) return wide ? launch(k_self_mix<true, false, true>) : launch(k_self_mix<true, false, false>);
+  return wide ? launch(k_self_mix<false, true, true>) : launch(k_self_mix<false, true, false>);
 }

@@ -51,6 +51,8 @@ struct RingArgs {
   const double* Bc;
   Tables T;
   double c1, c2;
+  int seg, segs;  // targets of a ring segment's block, blocks a ring (last: k_self_ring is
+                  // 0.3 % slower with these before the pointers)
 };
 
 // Node values of the sets in `sets` (bit 0 x, 1 f, 2 g, 3 a3) in column order;
@@ -85,12 +87,54 @@ __global__ void __launch_bounds__(128) k_ring_rec(int m, int n, const double* __
   }
 }
 
+// The values of a node or point: x, f, g, a3.
+template <bool SL, bool DL>
+struct RingVal {
+  static constexpr int NV = 3 + (SL ? 3 : 0) + (DL ? 6 : 0), OF = 3, OG = 3 + (SL ? 3 : 0), OA = OG + 3;
+  // U_j and D_j of a class from the column's node values (rc: row 0)
+  static __device__ __forceinline__ void theta(const RingArgs& a, const RingClass& c, const double* rc, double* U,
+                                               double* D) {
+    const int nlon = a.nlon;
+    const size_t rowlen = (size_t)RSLOT * RVAL * nlon;
+    const double* r1 = rc + (size_t)c.i1 * rowlen;
+    const double* r2 = rc + (size_t)(c.i1 + 1 == a.m ? 0 : c.i1 + 1) * rowlen;
+    const double x1 = c.x[0], x2 = c.x[1], x3 = c.x[2];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const int rv = (v < 3 || SL) ? v : v + 3;  // without f: g and a3 follow x
+      U[v] = fma(x3, __ldg(r2 + (2 * RVAL + rv) * nlon),
+                 fma(x2, __ldg(r1 + (2 * RVAL + rv) * nlon), fma(x1, __ldg(r1 + (RVAL + rv) * nlon), __ldg(r1 + rv * nlon))));
+      D[v] = fma(x3, __ldg(r2 + (5 * RVAL + rv) * nlon),
+                 fma(x2, __ldg(r1 + (5 * RVAL + rv) * nlon),
+                     fma(x1, __ldg(r1 + (4 * RVAL + rv) * nlon), __ldg(r1 + (3 * RVAL + rv) * nlon))));
+    }
+  }
+  // the point's term is cx p + cf f, p relative to the target; false: none
+  static __device__ __forceinline__ bool term(const RingArgs& a, const double* p, double w1, double w2, bool dl,
+                                              double& cx, double& cf) {
+    const double r2 = fma(p[0], p[0], fma(p[1], p[1], p[2] * p[2]));
+    double EA, EB, ED;
+    if (!ewald_coef64<SL, DL>(a.T, r2, EA, EB, ED)) return false;  // rr >= rc: ModRbcSingInt.F90:65
+    cx = cf = 0.;
+    if (SL) {
+      cx = w1 * EA * fma(p[0], p[OF], fma(p[1], p[OF + 1], p[2] * p[OF + 2]));
+      cf = w1 * EB;
+    }
+    if (DL && dl) {
+      const double dg = fma(p[0], p[OG], fma(p[1], p[OG + 1], p[2] * p[OG + 2]));
+      const double da = fma(p[0], p[OA], fma(p[1], p[OA + 1], p[2] * p[OA + 2]));
+      cx = fma(w2 * ED * dg, da, cx);
+    }
+    return true;
+  }
+};
+
 // FEW: the form for few points, the same code with another shared-memory split
 // (a kernel's split is the process's, as its opt-in: run_self_ring).
 template <bool SL, bool DL, bool FEW>
 __global__ void __launch_bounds__(256, 1) k_self_ring(RingArgs a) {
-  constexpr int NV = 3 + (SL ? 3 : 0) + (DL ? 6 : 0);  // x, f, g, a3
-  constexpr int OF = 3, OG = 3 + (SL ? 3 : 0), OA = OG + 3;
+  using V = RingVal<SL, DL>;
+  constexpr int NV = V::NV;
   extern __shared__ double sm[];
   const int t = threadIdx.x, W = blockDim.x, nlon = a.nlon;
   double* exU = sm;             // [NV][W]
@@ -114,25 +158,11 @@ __global__ void __launch_bounds__(256, 1) k_self_ring(RingArgs a) {
   }
   for (int k = 0; k < 6; ++k) acc[k * W + t] = 0.;
   const double* rc = a.rec + (size_t)(valid ? cell : 0) * a.m * RSLOT * RVAL * nlon + j;
-  const size_t rowlen = (size_t)RSLOT * RVAL * nlon;
   const int k0 = (int)((long long)a.NC * part / a.parts), k1 = (int)((long long)a.NC * (part + 1) / a.parts);
   for (int kc = k0; kc < k1; ++kc) {
     const RingClass& c = a.cls[(size_t)ring * a.NC + kc];
     double U[NV], D[NV];
-    if (valid) {
-      const double* r1 = rc + (size_t)c.i1 * rowlen;
-      const double* r2 = rc + (size_t)(c.i1 + 1 == a.m ? 0 : c.i1 + 1) * rowlen;
-      const double x1 = c.x[0], x2 = c.x[1], x3 = c.x[2];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const int rv = (v < 3 || SL) ? v : v + 3;  // without f: g and a3 follow x
-        U[v] = fma(x3, __ldg(r2 + (2 * RVAL + rv) * nlon),
-                   fma(x2, __ldg(r1 + (2 * RVAL + rv) * nlon), fma(x1, __ldg(r1 + (RVAL + rv) * nlon), __ldg(r1 + rv * nlon))));
-        D[v] = fma(x3, __ldg(r2 + (5 * RVAL + rv) * nlon),
-                   fma(x2, __ldg(r1 + (5 * RVAL + rv) * nlon),
-                       fma(x1, __ldg(r1 + (4 * RVAL + rv) * nlon), __ldg(r1 + (3 * RVAL + rv) * nlon))));
-      }
-    }
+    if (valid) V::theta(a, c, rc, U, D);
     __syncthreads();  // the previous class's values and sums are done with
     if (valid) {
 #pragma unroll
@@ -154,24 +184,13 @@ __global__ void __launch_bounds__(256, 1) k_self_ring(RingArgs a) {
 #pragma unroll
       for (int v = 0; v < NV; ++v) p[v] = fma(y3, E[v], fma(y2, D[v], fma(y1, dU[v], U[v])));
       for (int k = 0; k < 3; ++k) p[k] -= sT[k * W + q];
-      const double r2 = fma(p[0], p[0], fma(p[1], p[1], p[2] * p[2]));
-      double EA, EB, ED;
-      if (!ewald_coef64<SL, DL>(a.T, r2, EA, EB, ED)) continue;  // rr >= rc: ModRbcSingInt.F90:65
-      double cx = 0., cf = 0.;  // dv = cx xx + cf f
-      if (SL) {
-        cx = w1 * EA * fma(p[0], p[OF], fma(p[1], p[OF + 1], p[2] * p[OF + 2]));
-        cf = w1 * EB;
-      }
-      if (DL && c2m != 0.) {
-        const double dg = fma(p[0], p[OG], fma(p[1], p[OG + 1], p[2] * p[OG + 2]));
-        const double da = fma(p[0], p[OA], fma(p[1], p[OA + 1], p[2] * p[OA + 2]));
-        cx = fma(w2 * ED * dg, da, cx);
-      }
+      double cx, cf;
+      if (!V::term(a, p, w1, w2, c2m != 0., cx, cf)) continue;
       double* s = acc + 3 * side * W + q;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         double z = s[k * W];
-        if (SL) z = fma(cf, p[OF + k], z);
+        if (SL) z = fma(cf, p[V::OF + k], z);
         s[k * W] = fma(cx, p[k], z);
       }
     }
@@ -187,7 +206,90 @@ __global__ void __launch_bounds__(256, 1) k_self_ring(RingArgs a) {
   }
 }
 
+// Rings of more than RING_MAX_NLON columns: a block takes a segment of the
+// targets of one cell's ring, a thread a target.  Per class and side the theta
+// parts of the segment's columns (and the next) go through shared memory to
+// the neighbour as above, each column's twice in a ring (a side each), 6.6 +
+// 3.5 FMA a value; the sums stay in registers.  FP32C matvecs against one warp per
+// target and 16-term interpolations (us): 4 cells of 16 x 260 2210 -> 1300, 2 cells
+// of 40 x 264 5290 -> 2830, of 16 x 520 2400 -> 1450, of 16 x 1000 5843 -> 3610.
+template <bool SL, bool DL>
+__global__ void __launch_bounds__(256, 1) k_self_ring_wide(RingArgs a) {
+  using V = RingVal<SL, DL>;
+  constexpr int NV = V::NV;
+  extern __shared__ double sm[];
+  const int t = threadIdx.x, W = blockDim.x, nlon = a.nlon;
+  double* exU = sm;            // [NV][W]
+  double* exD = exU + NV * W;  // [NV][W]
+  int b = blockIdx.x;
+  const int part = b % a.parts; b /= a.parts;
+  const int q0 = b % a.segs * a.seg; b /= a.segs;
+  const int ring = b % a.nlat, cell = b / a.nlat, n = min(a.seg, nlon - q0);
+  double xi[3] = {0, 0, 0}, dv[3] = {0, 0, 0}, c2m = 0.;
+  if (t < n) {
+    SplW sw;
+    spline_weights(a.th[ring], a.phi[q0 + t], a.m, nlon, sw);
+    spline_eval(a.spl + ((size_t)cell * SPL_NSET + SPL_X) * (size_t)a.m * nlon * SPL_NODE, sw, 3, xi);
+    if (DL) c2m = a.c2 * a.Bc[a.celltype[cell]];
+  }
+  const double* rc = a.rec + (size_t)cell * a.m * RSLOT * RVAL * nlon;
+  const int k0 = (int)((long long)a.NC * part / a.parts), k1 = (int)((long long)a.NC * (part + 1) / a.parts);
+  for (int kc = k0; kc < k1; ++kc) {
+    const RingClass& c = a.cls[(size_t)ring * a.NC + kc];
+    const double w1 = SL ? a.c1 * c.w : 0., w2 = DL ? c2m * c.w : 0.;
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {
+      if (c.j[side] < 0) break;  // the points on the meridian have no mirror image
+      double U[NV], D[NV];
+      if (t <= n) {
+        const int j = q0 + t + c.j[side];
+        V::theta(a, c, rc + (j >= nlon ? j - nlon : j), U, D);
+      }
+      __syncthreads();  // the previous values are done with
+      if (t <= n) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) { exU[v * W + t] = U[v]; exD[v * W + t] = D[v]; }
+      }
+      __syncthreads();
+      if (t >= n) continue;
+      const double y1 = c.y[side][0], y2 = c.y[side][1], y3 = c.y[side][2];
+      double p[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        p[v] = fma(y3, exD[v * W + t + 1], fma(y2, D[v], fma(y1, exU[v * W + t + 1] - U[v], U[v])));
+      for (int k = 0; k < 3; ++k) p[k] -= xi[k];
+      double cx, cf;
+      if (!V::term(a, p, w1, w2, c2m != 0., cx, cf)) continue;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (SL) dv[k] = fma(cf, p[V::OF + k], dv[k]);
+        dv[k] = fma(cx, p[k], dv[k]);
+      }
+    }
+  }
+  if (t >= n) return;
+  const int p = cell * a.nlat * nlon + (q0 + t) * a.nlat + ring;
+  const double iA = 1.0 / a.tA[p];
+  for (int k = 0; k < 3; ++k) {
+    if (a.parts == 1) a.v[p + (size_t)k * a.nt] += dv[k] * iA;
+    else atomicAdd(a.v + p + (size_t)k * a.nt, dv[k] * iA);
+  }
+}
+
 }  // namespace
+
+// Targets of one block of a wide ring, `most` at most (a block's threads are
+// these and one column more): the most lanes in use.
+int ring_segment(int nlon, int most) {
+  int best = most;
+  double top = -1.;
+  for (int segs = (nlon + most - 1) / most; segs <= 2 * ((nlon + most - 1) / most) + 1; ++segs) {
+    const int seg = (nlon + segs - 1) / segs, thr = (seg + 32) / 32 * 32;
+    const double used = (double)nlon / ((double)segs * thr);
+    if (used > top + 1e-9) { top = used; best = seg; }
+  }
+  return best;
+}
 
 // Cells per block: the most lanes in use (full warps of columns, no empty
 // places in the last block).
@@ -289,8 +391,12 @@ rbc3d_status run_self_ring(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   RingArgs a;
   a.ncell = ctx->ncell; a.nlat = ctx->nlat; a.nlon = ctx->nlon; a.m = ctx->m; a.nt = t.n;
   a.NC = ctx->nrad * (ctx->nazm / 2 + 1);
-  a.G = ring_cells(ctx->ncell, ctx->nlon);
-  const int blocks = (ctx->ncell + a.G - 1) / a.G * ctx->nlat, thr = (a.G * ctx->nlon + 31) / 32 * 32;
+  const bool wide = ctx->nlon > RING_MAX_NLON;
+  a.G = wide ? 1 : ring_cells(ctx->ncell, ctx->nlon);
+  a.seg = wide ? ring_segment(ctx->nlon, RING_MAX_NLON - 1) : 0;
+  a.segs = wide ? (ctx->nlon + a.seg - 1) / a.seg : 1;
+  const int blocks = (ctx->ncell + a.G - 1) / a.G * ctx->nlat * a.segs;
+  const int thr = ((wide ? a.seg + 1 : a.G * ctx->nlon) + 31) / 32 * 32;
   a.parts = ring_parts(a.NC, blocks, nsm);
   a.rec = ctx->ring_rec.p; a.cls = reinterpret_cast<const RingClass*>(ctx->ring_cls.p); a.spl = ctx->spl.p;
   a.th = ctx->th.p; a.phi = ctx->phi.p; a.tA = t.Acoef.p; a.v = t.v.p; a.celltype = ctx->celltype.p; a.Bc = ctx->dBcoef.p;
@@ -301,15 +407,20 @@ rbc3d_status run_self_ring(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   // 459 us, of 14 x 28 841 -> 617; of 25 x 50 1224 -> 1281, where the L1 counts)
   const bool few = t.n <= 2000;
   auto launch = [&](auto kern, int nv) -> rbc3d_status {
-    const size_t bytes = sizeof(double) * (size_t)thr * (2 * nv + 9);
+    const size_t bytes = sizeof(double) * (size_t)thr * (2 * nv + (wide ? 0 : 9));
     CUDA_TRY(smem_opt_in(kern, bytes));
-    if (few)
+    if (few && !wide)
       CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     kern<<<blocks * a.parts, thr, bytes, ctx->st>>>(a);
     ++ctx->launches;
     CUDA_TRY(cudaGetLastError());
     return RBC3D_OK;
   };
+  if (wide) {
+    if (sl && dl) return launch(k_self_ring_wide<true, true>, 12);
+    if (sl) return launch(k_self_ring_wide<true, false>, 6);
+    return launch(k_self_ring_wide<false, true>, 9);
+  }
   if (sl && dl) return few ? launch(k_self_ring<true, true, true>, 12) : launch(k_self_ring<true, true, false>, 12);
   if (sl) return few ? launch(k_self_ring<true, false, true>, 6) : launch(k_self_ring<true, false, false>, 6);
   return few ? launch(k_self_ring<false, true, true>, 9) : launch(k_self_ring<false, true, false>, 9);
