@@ -645,7 +645,7 @@ rbc3d_status rbc3d_set_cell_grid(rbc3d_ctx* ctx, const double* th, const double*
     // phi0 moves the stencil by whole columns
     const std::vector<RingClass> R = ring_classes(ctx, thG, phiA, pw);
     rbc3d_status s;
-    if ((s = self_ff_grid(ctx, R)) || (s = self_mixed_grid(ctx, R)) || (s = self_ring_grid(ctx, R))) return s;
+    if ((s = proj_table(ctx)) || (s = self_ff_grid(ctx, R)) || (s = self_mixed_grid(ctx, R)) || (s = self_ring_grid(ctx, R))) return s;
   }
   CUDA_TRY(ctx->thG.upload(thG.data(), thG.size(), ctx->st));
   CUDA_TRY(ctx->phiA.upload(phiA.data(), phiA.size(), ctx->st));

@@ -10,8 +10,10 @@
 // lanes 0..16 and the 27 normal-equation sums are butterfly warp reductions,
 // which leave bit-identical values on every lane so the subsequent 6x6 solve
 // and every branch stay warp-uniform.  In ReAdd lane = azimuth (nazm = 32).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <vector>
 
 #include "ctx.hpp"
 
@@ -65,6 +67,7 @@ struct CorrArgs {
   int screen;  // screen items before the FP64 projection (FP32C path)
   double rthr;  // FP32C path: cross-surface pairs closer than rthr are added here in FP64
   int verify;  // evaluate screened items in FP64 anyway and count disagreements
+  const double* proj;  // proj_table
 };
 
 __device__ __forceinline__ const double* set_ptr(const CorrArgs& a, int cell, int set) {
@@ -178,25 +181,19 @@ __device__ __forceinline__ double atan2_r(double y, double x) { return atan2(y, 
 __device__ __forceinline__ float atan2_r(float y, float x) { return atan2f(y, x); }
 
 // A lane's fit point: azimuth and radii of the three levels, and its weights
-// in the fit of u = px/h, v = py/h, uv, u^2 - v^2 and u^2 + v^2.
+// in the fit of u = px/h, v = py/h, uv, u^2 - v^2 and u^2 + v^2.  From a table
+// (proj_table), as they depend on the grid only: formed by every warp of a
+// resident wave, the FP64 sines and cosines held up the near pass without a
+// candidate by 55 us (FP32D, 8 cells: 94 us, 37 from the table).
+constexpr int PROJ_LANE = 13;
 template <typename R>
 struct ProjLane {
   R cph, sph, sL[3], cL[3], wu, wv, wuv, wd, wr;
-  __device__ __forceinline__ void init(double h0) {
-    const int k = threadIdx.x & 15;
-    const double r = 0.5 * (k % 2 + 1), a = (k / 2) * RBC3D_TWO_PI / 8;
-    double s, c;
-    sincos(a, &s, &c);
-    const double u = r * c, v = r * s;
-    cph = (R)c; sph = (R)s;
-    // sums over the points: u^2 5, (uv)^2 17/16, (u^2 - v^2)^2 17/4, and of
-    // r^2 10, r^4 8.5 over 17 points
-    wu = (R)(u / 5); wv = (R)(v / 5); wuv = (R)(u * v / 1.0625); wd = (R)((u * u - v * v) / 4.25);
-    wr = (R)((r * r - 10. / 17) / (8.5 - 100. / 17));
-    for (int l = 0; l < 3; ++l, h0 *= 0.5) {
-      sincos(r * h0, &s, &c);
-      sL[l] = (R)s; cL[l] = (R)c;
-    }
+  __device__ __forceinline__ void init(const double* __restrict__ tab) {
+    const double* t = tab + PROJ_LANE * (threadIdx.x & 15);
+    cph = (R)__ldg(t); sph = (R)__ldg(t + 1);
+    for (int l = 0; l < 3; ++l) { sL[l] = (R)__ldg(t + 2 + l); cL[l] = (R)__ldg(t + 5 + l); }
+    wu = (R)__ldg(t + 8); wv = (R)__ldg(t + 9); wuv = (R)__ldg(t + 10); wd = (R)__ldg(t + 11); wr = (R)__ldg(t + 12);
   }
 };
 template <typename R>
@@ -528,7 +525,7 @@ __global__ void __launch_bounds__(128) k_near_replay(CorrArgs a, const int* __re
   const long long n = (long long)*nin;
   const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
   ProjLane<float> P;
-  P.init(fmax(a.G.hx, a.G.hy));
+  P.init(a.proj);
   for (long long w = 2 * ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); w < n; w += 2 * nw) {
     const bool on = w + half < n;
     const int idx = in[on ? w + half : w];
@@ -552,9 +549,9 @@ __global__ void __launch_bounds__(128) k_near(CorrArgs a) {
   if (nitem > (unsigned long long)a.cap) nitem = a.cap;
   if (nitem == 0) return;
   ProjLane<double> PL;
-  PL.init(fmax(a.G.hx, a.G.hy));
+  PL.init(a.proj);
   ProjLane<float> PF;
-  if (a.screen) PF.init(fmax(a.G.hx, a.G.hy));
+  if (a.screen) PF.init(a.proj);
   // warps take items from a shared counter (the grid is one resident wave)
   for (;;) {
     unsigned long long g0 = 0;
@@ -664,7 +661,7 @@ __global__ void __launch_bounds__(128) k_near_proj(CorrArgs a, NearPlan* __restr
   unsigned long long nn = a.list ? *a.nlist : *a.nitems;
   const long long n = (long long)(nn > (unsigned long long)a.cap ? (unsigned long long)a.cap : nn);
   ProjLane<double> PL;
-  PL.init(fmax(a.G.hx, a.G.hy));
+  PL.init(a.proj);
   unsigned done = 0, hits = 0;
   for (;;) {
     unsigned long long g0 = 0;
@@ -830,6 +827,7 @@ struct RepArgs {
   double* dx;           // 3 x n, moves (zero where none)
   unsigned long long* dmin;   // minimum surface separation (double bits)
   unsigned long long* nmoved;
+  const double* proj;   // proj_table
 };
 
 __device__ __forceinline__ double rep_minimg(double d, double L, double iL) { return d - round(d * iL) * L; }
@@ -884,7 +882,7 @@ __global__ void __launch_bounds__(128) k_inter_rep(RepArgs a) {
     const double* sx = a.spl + ((size_t)cell0 * SPL_NSET + SPL_X) * (size_t)a.m * a.nlon * SPL_NODE;
     const SplGrid G = a.G;
     ProjLane<double> PL;
-    PL.init(fmax(G.hx, G.hy));
+    PL.init(a.proj);
     project64(PL, sx, G, xtar, th0, phi0, x1);
     double d2 = 0;
     for (int d = 0; d < 3; ++d) d2 += (xtar[d] - x1[d]) * (xtar[d] - x1[d]);
@@ -994,9 +992,32 @@ void fill_args(rbc3d_ctx* ctx, int tlist, double c1, double c2, CorrArgs& a, con
   for (int d = 0; d < 3; ++d) { a.L[d] = ctx->prm.Lb[d]; a.iL[d] = ctx->iLb[d]; }
   a.T = ctx->T;
   a.items = ctx->items.p; a.nitems = ctx->dcnt.p; a.cap = ctx->items_cap; a.cnt = ctx->dcnt.p;
+  a.proj = ctx->proj.p;
 }
 
 }  // namespace
+
+// ProjLane of the 16 fit points: cos, sin of the azimuth, sin (3) and cos (3) of
+// the radius at the three levels, and the five weights.
+rbc3d_status proj_table(rbc3d_ctx* ctx) {
+  const SplGrid G = spl_grid(ctx->m, ctx->nlon);
+  std::vector<double> tab(16 * PROJ_LANE);
+  for (int k = 0; k < 16; ++k) {
+    double* t = &tab[PROJ_LANE * k];
+    const double r = 0.5 * (k % 2 + 1), a = (k / 2) * RBC3D_TWO_PI / 8;
+    const double c = std::cos(a), s = std::sin(a), u = r * c, v = r * s;
+    t[0] = c; t[1] = s;
+    double h = std::max(G.hx, G.hy);
+    for (int l = 0; l < 3; ++l, h *= 0.5) { t[2 + l] = std::sin(r * h); t[5 + l] = std::cos(r * h); }
+    // sums over the points: u^2 5, (uv)^2 17/16, (u^2 - v^2)^2 17/4, and of
+    // r^2 10, r^4 8.5 over 17 points
+    t[8] = u / 5; t[9] = v / 5; t[10] = u * v / 1.0625; t[11] = (u * u - v * v) / 4.25;
+    t[12] = (r * r - 10. / 17) / (8.5 - 100. / 17);
+  }
+  CUDA_TRY(ctx->proj.upload(tab.data(), tab.size(), ctx->st));
+  CUDA_TRY(cudaStreamSynchronize(ctx->st));
+  return RBC3D_OK;
+}
 
 rbc3d_status run_self_corr(rbc3d_ctx* ctx, int tlist, double c1, double c2) {
   TargetSet& t = ctx->tl[tlist];
@@ -1094,7 +1115,7 @@ extern "C" rbc3d_status rbc3d_inter_cell_repulsion(rbc3d_ctx* ctx, double epsDis
   a.n = n; a.nv = ctx->nlat * ctx->nlon; a.nlat = ctx->nlat; a.nlon = ctx->nlon; a.m = ctx->m;
   a.G = spl_grid(ctx->m, ctx->nlon);
   a.x = ctx->x.p; a.sx = ctx->s_x.p; a.smeta = ctx->s_meta.p; a.cs = ctx->s_cstart.p; a.ce = ctx->s_cend.p;
-  a.spl = ctx->spl.p; a.th = ctx->th.p; a.phi = ctx->phi.p;
+  a.spl = ctx->spl.p; a.th = ctx->th.p; a.phi = ctx->phi.p; a.proj = ctx->proj.p;
   for (int d = 0; d < 3; ++d) { a.Nc[d] = ctx->hg.Nc[d]; a.L[d] = ctx->prm.Lb[d]; a.iL[d] = ctx->iLb[d]; }
   a.eps = epsDist;
   a.nvert = W.nvert; a.nele = W.nele; a.wx = W.x.p; a.e2v = W.e2v.p;

@@ -238,6 +238,7 @@ struct rbc3d_ctx {
   DBuf<char> ring_cls;                  // patch-point classes per latitude (RingClass)
   DBuf<double> ring_tab, ring_rec;      // FP64 patch: Ewald tables with steps, node values in column order
   int ring_sets = 0;                    // ring_rec's current sets (bit 0 x, 1 f, 2 g, 3 a3)
+  DBuf<double> proj;                    // the projection's fit points (proj_table)
   DBuf<double> mtab64;                  // same-cell mask per (latitude, latitude, longitude gap)
   DBuf<float> mtab32;                   // 1 - mask, FP32
   DBuf<int> near_l1, near_l2;           // near-singular candidates after the screen / the FP32 replay
@@ -375,6 +376,7 @@ void wall_spec_release(rbc3d_ctx* ctx);
 // selfring.cu: the FP64 patch by latitude rings (uniform longitudes; more than
 // RING_MAX_NLON columns, a block's threads, go by segments of a ring)
 constexpr int RING_MAX_NLON = 256;
+rbc3d_status proj_table(rbc3d_ctx* ctx);  // corr.cu
 std::vector<RingClass> ring_classes(const rbc3d_ctx* ctx, const std::vector<double>& thG,
                                     const std::vector<double>& phiA, const std::vector<double>& pw);
 int ring_cells(int ncell, int nlon);                  // cells of one block
