@@ -4,12 +4,15 @@
 // Spline_FindProjection (ModSpline.F90:203-269) and QuadFit_2D (normal
 // equations + Cholesky, ModBasicMath.F90:234-284).
 //
-// Mapping: one warp per target for the self patch (nrad*nazm quadrature points
-// spread over the lanes), one warp per (target, neighbour cell) work item for
-// the near-singular correction.  In the projection the 17 fit points sit on
-// lanes 0..16 and the 27 normal-equation sums are butterfly warp reductions,
-// which leave bit-identical values on every lane so the subsequent 6x6 solve
-// and every branch stay warp-uniform.  In ReAdd lane = azimuth (nazm = 32).
+// Mapping.  Self patch on uneven longitudes: one warp per target, its nrad*nazm
+// quadrature points over the lanes (equispaced longitudes: selfring.cu).
+// Near-singular pass, staged so that its work spreads evenly (see NearPlan): a
+// thread per candidate for the geometric screen and a half-warp for the FP32
+// replay of the projection (FP32 modes), a half-warp per item for the FP64
+// projection, a warp per quarter of a re-add or per subtract, a thread per
+// item for the sum.  In the projection the 16 fit points sit on the 16 lanes and
+// an iteration needs five butterfly sums (find_projection), which leave the same
+// bits on every lane.  In ReAdd lane = azimuth (nazm = 32).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -172,7 +175,7 @@ __device__ __forceinline__ void patch_point(double st0, double ct0, double phi0,
 // (ModBasicMath.F90:234-284) are solved once and for all: five weighted sums
 // of the distances less the centre's.  An iteration takes about 600 FP64
 // instructions for two targets, against 1600 for one with 27 sums, a Cholesky
-// factorisation and the angles' sines anew (see run_near_corr).
+// factorisation and the angles' sines anew.
 __device__ __forceinline__ void sincos_r(double x, double* s, double* c) { sincos(x, s, c); }
 __device__ __forceinline__ void sincos_r(float x, float* s, float* c) { sincosf(x, s, c); }
 __device__ __forceinline__ double acos_r(double x) { return acos(x); }
@@ -480,7 +483,6 @@ __device__ __forceinline__ float projection_dist32(const ProjLane<float>& P, con
   return a30[0] * (xt[0] - x0[0]) + a30[1] * (xt[1] - x0[1]) + a30[2] * (xt[2] - x0[2]);
 }
 
-// RBC_NearSingInt over the work list (persistent warps)
 // Target position in the item's cell frame (minimum image about the closest
 // mesh point x0), as RBC_NearSingInt receives it.
 __device__ __forceinline__ void item_geometry(const CorrArgs& a, int4 item, double* x0, double* xt, size_t& q0) {

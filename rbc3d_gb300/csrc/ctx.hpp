@@ -173,7 +173,7 @@ struct rbc3d_ctx {
   cudaStream_t st2 = nullptr;  // matvec side stream: self patch and PME next to the pair sums
   cudaStream_t st3 = nullptr;  // the pair sums' own-cell pass, from ev_pair to ev_own
   cudaEvent_t ev_pair = nullptr, ev_own = nullptr;
-  cudaStream_t st4 = nullptr;  // PME of large FP32D matvecs, done at ev_pme
+  cudaStream_t st4 = nullptr;  // PME of large FP32D and FP32M matvecs, done at ev_pme
   cudaEvent_t ev_pme = nullptr;
   cudaEvent_t ev_vup = nullptr;  // the caller's values are in vadd (vadd_up: on their way, on st3)
   bool vadd_up = false;

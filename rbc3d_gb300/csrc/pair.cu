@@ -108,13 +108,8 @@ __global__ void k_fill_pieces(int nc, const int* __restrict__ cs, const int* __r
 
 // Work units of the pair sums (the cells' targets in equal-sized units of at
 // most `tile`), keyed by their work: targets x the sources of the 27
-// neighbour cells.  Unit counts first, then the units at the scanned offsets.
-__global__ void k_unit_counts(int nc, int tile, const int* __restrict__ cs, const int* __restrict__ ce,
-                              int* __restrict__ cnt) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c > nc) return;
-  cnt[c] = c < nc ? (ce[c] - cs[c] + tile - 1) / tile : 0;
-}
+// neighbour cells.  Unit counts first (k_piece_counts), then the units at the
+// scanned offsets.
 __global__ void k_fill_units(int nc, int tile, int Nc0, int Nc1, int Nc2, const int* __restrict__ cs, const int* __restrict__ ce,
                              const int* __restrict__ ss, const int* __restrict__ se, const int* __restrict__ off,
                              int cap, int4* __restrict__ units, long long* __restrict__ key, int* __restrict__ idx) {
@@ -1236,7 +1231,7 @@ rbc3d_status fill_units(rbc3d_ctx* ctx, const DBuf<int>& cs, const DBuf<int>& ce
   CUDA_TRY(ctx->unit_tmp.alloc(cap)); CUDA_TRY(units.alloc(cap));
   CUDA_TRY(ctx->unit_key.alloc(2 * (size_t)cap)); CUDA_TRY(ctx->unit_idx.alloc(2 * (size_t)cap));
   const int g1 = nblk(nc + 1, 256);
-  { k_unit_counts<<<g1, 256, 0, ctx->st>>>(nc, tile, cs.p, ce.p, cnt.p); ++ctx->launches; }
+  { k_piece_counts<<<g1, 256, 0, ctx->st>>>(nc, cs.p, ce.p, tile, cnt.p); ++ctx->launches; }
   if ((s = scan_counts(ctx, nc, cnt.p, ctx->unit_off.p))) return s;
   long long* key = ctx->unit_key.p;
   int* idx = ctx->unit_idx.p;
@@ -1259,15 +1254,16 @@ rbc3d_status fill_units(rbc3d_ctx* ctx, const DBuf<int>& cs, const DBuf<int>& ce
 }
 
 // Lanes per target of the pair sums.  With one lane each and few units the
-// longest warps set the time (256 cells: SMs active 74 % of the kernel's);
-// more lanes a target cost tile walks.  FP32D, pair stage alone and whole
-// matvec (us) with 1 / 2 / 4 lanes: 8 cells (10,000 targets) 653 / - / 325 and
-// 918 / - / 609; 24 cells - / 664 / 529 and - / 1308 / 1164; 40 cells - / 828 /
-// 740 and - / 1588 / 1597; 64 cells 1197 / 874 / 884 and 2242 / 1970 / 2032;
-// 97 cells 1686 / 1175 / - and 3320 / 2970 / -; 128 cells 1744 / 1492 / 1693 and
-// 3983 / 3908 / 4313 (the wider walk holds up the mesh beside it); 160 cells
-// 2073 / 1767 / - but 4887 / 4944 / -; 256 cells 2718 / 2596 / 3029 but 7155 /
-// 7225 / -.  FP64 matvec (ms): 64 cells - / 19.2 / 19.5, 160 cells 50.9 / 50.9.
+// longest warps set the time (256 cells: the walk's SMs active 74 % of its
+// time); more lanes a target cost tile walks.  FP32D, the pair stage alone and
+// the whole matvec (us) with 1 / 2 / 4 lanes, the own-cell pass beside the walk:
+// 8 cells of 1,250 points 728 / 434 / 233 and 812 / 613 / 433; 24 cells 1112 / 689 /
+// 570 and 1589 / 1223 / 1070; 40 cells 1287 / 818 / 654 and 1905 / 1394 / 1418; 64
+// cells 1163 / 736 / 752 and 2012 / 1803 / 1915; 97 cells 1499 / 993 / 1103 and 3036 /
+// 2634 / 2845; 128 cells 1519 / 1195 / 1506 and 3573 / 3532 / 3839; 160 cells 1746 /
+// 1501 / 1886 and 4507 / 4475 / 4845 (FP32M 3369 / 3505 / 3884); 256 cells 2106 /
+// 2250 / 2840 and 6468 / 6624 / 7204; 512 cells 13446 / 13781 / 14941.  FP64 matvecs
+// (ms): 64 cells 19.3 / 19.2 / 19.5, 160 cells 50.9 / 50.9 / 51.9.
 int pair_sub(int n) { return n <= 50000 ? 4 : n <= 180000 ? 2 : 1; }
 
 rbc3d_status make_units(rbc3d_ctx* ctx, TargetSet& t, const DBuf<int>& cs, const DBuf<int>& ce) {
@@ -1526,7 +1522,7 @@ rbc3d_status run_pair_sum(rbc3d_ctx* ctx, int tlist, double c1, double c2, int p
     // 54844.  At the walk's priority 7018 and 5417.  FP64 with PME on the side
     // stream: 3 cells 1490 / 1218, 3 cells of 12 x 24 525 / 459, 8 cells 2812 /
     // 2770, 64 cells 19385 / 19287, 9 cells of 36 x 72 9203 / 9317.
-      const bool beside = own && ctx->st3;
+    const bool beside = own && ctx->st3;
     if (beside) {
       CUDA_TRY(cudaEventRecord(ctx->ev_pair, ctx->st));
       CUDA_TRY(cudaStreamWaitEvent(ctx->st3, ctx->ev_pair, 0));

@@ -3,9 +3,11 @@
 //   PME_Distrib_Source (ModPME.F90:58-133, 405-443): B-spline spreading of
 //     c1*f (3 grids) and c2*g (x) Bcoef*a3 (9 grids); walls spread one
 //     centroid source per triangle.  Sources are binned by 8^3 grid tiles
-//     (once per position update); a CTA accumulates one tile's sources into
-//     a (8+P-1)^3 box in shared memory and adds the box to the grids with
-//     one global atomic per touched node.
+//     (once per position update).  FP32 cell sources: a CTA accumulates one
+//     tile's sources into a (8+P-1)^3 box in shared memory and adds the box
+//     to the grids with one global atomic per touched node (k_spread_tile);
+//     FP64 and wall sources go straight to the grids, a warp each in tile
+//     order (k_spread_direct, see launch_spread).
 //   PME_Transform (ModPME.F90:137-222): batched 3-D R2C FFTs (cuFFT), one
 //     fused kernel for the Stokeslet / stresslet influence and the B-spline
 //     factor bb, 3 C2R FFTs.  Unnormalised, as Get_That / Get_R.
@@ -87,7 +89,6 @@ constexpr int GATHER_WARP64 = 8192;
 struct TileArgs {
   int ntile[3];        // tiles per axis
   int B;               // box edge, SPREAD_TILE + P - 1
-  int cg;              // grid planes per warp (3)
   const int2* sched;   // [rounds][32] stencil-node schedule
   int c0;              // first grid plane of the launch (3 per warp from there)
 };
@@ -633,11 +634,10 @@ rbc3d_status pme_release(rbc3d_ctx* ctx) {
   return RBC3D_OK;
 }
 
-TileArgs tile_args(const rbc3d_ctx* ctx, size_t elem) {
+TileArgs tile_args(const rbc3d_ctx* ctx) {
   TileArgs t;
   for (int d = 0; d < 3; ++d) t.ntile[d] = (ctx->prm.Nb[d] + SPREAD_TILE - 1) / SPREAD_TILE;
   t.B = SPREAD_TILE + ctx->prm.P - 1;
-  t.cg = 3;
   return t;
 }
 
@@ -669,7 +669,7 @@ rbc3d_status build_spread_plan(rbc3d_ctx* ctx, int n, const double* x, SpreadArg
   pl.nchunk = 0;
   pl.valid = true;
   if (n == 0) return RBC3D_OK;
-  TileArgs t = tile_args(ctx, 4);
+  TileArgs t = tile_args(ctx);
   DBuf<int>&key = ctx->plan_key, &key2 = ctx->plan_key2, &idx = ctx->plan_idx;
   CUDA_TRY(key.alloc(n)); CUDA_TRY(key2.alloc(n)); CUDA_TRY(idx.alloc(n)); CUDA_TRY(pl.perm.alloc(n));
   { k_tile_keys<<<nblk(n, 256), 256, 0, ctx->st>>>(n, x, a, t, key.p, idx.p); ++ctx->launches; }
@@ -727,21 +727,17 @@ rbc3d_status spread_schedule(rbc3d_ctx* ctx, int P, TileArgs& t) {
 
 template <typename R, int PT>
 rbc3d_status launch_spread_p(rbc3d_ctx* ctx, const SpreadArgs& a, const SpreadPlan& pl, R* grid) {
-  TileArgs t = tile_args(ctx, sizeof(R));
+  TileArgs t = tile_args(ctx);
   rbc3d_status st = spread_schedule(ctx, PT, t);
   if (st) return st;
-  // warps (3-plane groups) per launch: as many as the 227 KB of shared memory hold
-  const int gfirst = a.sl ? 0 : 1, glast = a.dl ? 4 : 1;
-  int per = glast - gfirst;
-  while (per > 1 && spread_smem_bytes(t.B, per, sizeof(R)) > SMEM_BLOCK) --per;
-  for (int g = gfirst; g < glast; g += per) {
-    const int nw = std::min(per, glast - g);
-    t.c0 = 3 * g;
-    const size_t bytes = spread_smem_bytes(t.B, nw, sizeof(R));
-    CUDA_TRY(smem_opt_in(k_spread_tile<R, PT>, bytes));
-    { k_spread_tile<R, PT><<<pl.nchunk, 32 * nw, bytes, ctx->st>>>(a, t, pl.perm.p, pl.chunk.p, grid); ++ctx->launches; }
-    CUDA_TRY(cudaGetLastError());
-  }
+  // a warp per vector quantity; four boxes in FP32 at the highest order take 167 KB
+  static_assert(sizeof(R) == 4, "FP64 spreads directly");
+  const int gfirst = a.sl ? 0 : 1, nw = (a.dl ? 4 : 1) - gfirst;
+  t.c0 = 3 * gfirst;
+  const size_t bytes = spread_smem_bytes(t.B, nw, sizeof(R));
+  CUDA_TRY(smem_opt_in(k_spread_tile<R, PT>, bytes));
+  { k_spread_tile<R, PT><<<pl.nchunk, 32 * nw, bytes, ctx->st>>>(a, t, pl.perm.p, pl.chunk.p, grid); ++ctx->launches; }
+  CUDA_TRY(cudaGetLastError());
   return RBC3D_OK;
 }
 // The spread without boxes (k_spread_direct) for wall sources, a dozen a tile: a
