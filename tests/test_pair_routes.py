@@ -91,3 +91,26 @@ def test_weight_table_too_large_for_the_dense_pass(gpu, oracle):
     # as test_wide_rings
     assert np.linalg.norm(out[1] - out[0]) <= 1e-11 * norm
     assert np.linalg.norm(out[2] - out[0]) <= 1e-6 * norm
+
+
+@pytest.mark.parametrize("cap", ["0", "7"])
+def test_near_stage_capacity_fp64(gpu, monkeypatch, cap):
+    """The FP64 near pass past its staged capacity: every item is taken once,
+    as test_gpu_parity has it for the FP32 modes."""
+    rng = np.random.default_rng(5)
+    cells = G.make_cells(rng, 3, [10.0] * 3, 3.2, nlat=12, nlon=24, with_g=True)
+    p = rng.integers(0, cells.x.shape[1], size=300)
+    x = np.ascontiguousarray(cells.x[:, p] + rng.uniform(0.03, 0.4, size=300) * cells.a3[:, p])
+    out = []
+    for env in (None, cap):
+        if env is not None:
+            monkeypatch.setenv("RBC3D_NEAR_STAGE_CAP", env)
+        c = context(gpu, cells, 10.0, 16)
+        c.set_raw_targets(x)
+        v = c.matvec(TLIST_RAW, C, C, TERM_CORR, FP64)
+        out.append((v, c.counts()))
+        c.close()
+    (ref, cref), (v, cnt) = out
+    assert cref["nearsing_items"] >= 300
+    assert cnt["near_projections"] == cref["near_projections"] and cnt["nearsing_items"] == cref["nearsing_items"]
+    assert np.abs(v - ref).max() <= 1e-12 * np.abs(ref).max()
